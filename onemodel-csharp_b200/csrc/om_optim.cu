@@ -14,7 +14,14 @@
 namespace om {
 
 constexpr int kMaxTensors = 40;
-constexpr int kChunk = 16384;  // elements per CTA visit
+constexpr int kChunk = 16384;  // elements per CTA visit where partial sums are formed: the order of the norm's doubles hangs on it
+
+// Elements per CTA visit of the element-wise updates, by the launch's total. A visit is one or four 16-byte rounds of a CTA:
+// with the 16384 elements of the norm's chunks a small model kept a handful of CTAs busy for sixteen rounds each (0.03 M
+// parameters: 25 us, 0.1 M: 37 us, 0.67 M: 16 us; now 4 to 5 us), and a large one ended in a part round of long visits.
+// The line is where visits of 4096 fill the eight CTAs that an SM holds.
+constexpr int kUpdateChunkSmall = 1024, kUpdateChunk = 4096;
+static int update_chunk(int64_t total) { return total < (int64_t)8 * 148 * kUpdateChunk ? kUpdateChunkSmall : kUpdateChunk; }
 
 struct TensorTable {
   float* p[kMaxTensors];
@@ -27,6 +34,7 @@ struct TensorTable {
   int32_t chunk_prefix[kMaxTensors + 1];
   int32_t first[kMaxTensors];
   int32_t n;
+  int32_t chunk;  // elements per CTA visit
 };
 
 __device__ __forceinline__ int find_tensor(const TensorTable& t, int chunk) {
@@ -70,8 +78,8 @@ adam_kernel(TensorTable t, om_adam_hyper hv, const om_adam_hyper* __restrict__ h
   const int total = t.chunk_prefix[t.n];
   for (int chunk = blockIdx.x; chunk < total; chunk += gridDim.x) {
     int ti = find_tensor(t, chunk);
-    int64_t start = (int64_t)(chunk - t.chunk_prefix[ti]) * kChunk;
-    int64_t end = min(t.len[ti], start + kChunk);
+    int64_t start = (int64_t)(chunk - t.chunk_prefix[ti]) * t.chunk;
+    int64_t end = min(t.len[ti], start + t.chunk);
     float* p = t.p[ti];
     const float* g = t.g[ti];
     float* m = t.a[ti];
@@ -115,6 +123,20 @@ adam_kernel(TensorTable t, om_adam_hyper hv, const om_adam_hyper* __restrict__ h
   }
 }
 
+__device__ __forceinline__ void sgd_element(float& p, float g, float& buf, bool first, const om_sgd_hyper& h, float keep) {
+  if (h.grad_scale != 1.0f) g = __fmul_rn(g, h.grad_scale);
+  const float pi = p;
+  if (h.weight_decay != 0.0f) g = __fadd_rn(g, __fmul_rn(h.weight_decay, pi));
+  if (h.has_momentum) {
+    const float bv = first ? g : __fadd_rn(__fmul_rn(h.momentum, buf), __fmul_rn(keep, g));
+    buf = bv;
+    g = h.nesterov ? __fadd_rn(g, __fmul_rn(h.momentum, bv)) : bv;
+  }
+  p = __fsub_rn(pi, __fmul_rn(h.lr, g));
+}
+
+// 16-byte accesses where the three arrays allow them: 4.7 M parameters with momentum (94 MB) took 44 us with 4-byte ones
+// in visits of 16384 elements. On the first step the momentum buffer is written without being read, as before.
 __global__ void __launch_bounds__(256)
 sgd_kernel(TensorTable t, om_sgd_hyper hv, const om_sgd_hyper* __restrict__ hd) {
   const om_sgd_hyper h = hd ? *hd : hv;
@@ -122,23 +144,29 @@ sgd_kernel(TensorTable t, om_sgd_hyper hv, const om_sgd_hyper* __restrict__ hd) 
   const int total = t.chunk_prefix[t.n];
   for (int chunk = blockIdx.x; chunk < total; chunk += gridDim.x) {
     int ti = find_tensor(t, chunk);
-    int64_t start = (int64_t)(chunk - t.chunk_prefix[ti]) * kChunk;
-    int64_t end = min(t.len[ti], start + kChunk);
+    int64_t start = (int64_t)(chunk - t.chunk_prefix[ti]) * t.chunk;
+    int64_t end = min(t.len[ti], start + t.chunk);
     float* p = t.p[ti];
     const float* gr = t.g[ti];
-    float* buf = t.a[ti];
-    const bool first = t.first[ti] != 0;
-    for (int64_t i = start + threadIdx.x; i < end; i += 256) {
-      float g = gr[i];
-      if (h.grad_scale != 1.0f) g = __fmul_rn(g, h.grad_scale);
-      float pi = p[i];
-      if (h.weight_decay != 0.0f) g = __fadd_rn(g, __fmul_rn(h.weight_decay, pi));
-      if (h.has_momentum) {
-        float bv = first ? g : __fadd_rn(__fmul_rn(h.momentum, buf[i]), __fmul_rn(keep, g));
-        buf[i] = bv;
-        g = h.nesterov ? __fadd_rn(g, __fmul_rn(h.momentum, bv)) : bv;
-      }
-      p[i] = __fsub_rn(pi, __fmul_rn(h.lr, g));
+    float* buf = h.has_momentum ? t.a[ti] : nullptr;
+    const bool first = t.first[ti] != 0, read_buf = buf != nullptr && !first;
+    const bool vec = (((uintptr_t)p | (uintptr_t)gr | (uintptr_t)buf) & 15) == 0;
+    const int64_t e4 = vec ? start + ((end - start) & ~(int64_t)3) : start;
+    for (int64_t i = start + threadIdx.x * 4; i < e4; i += 256 * 4) {
+      float4 pp = *reinterpret_cast<float4*>(p + i);
+      const float4 gg = *reinterpret_cast<const float4*>(gr + i);
+      float4 bb = read_buf ? *reinterpret_cast<float4*>(buf + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      sgd_element(pp.x, gg.x, bb.x, first, h, keep);
+      sgd_element(pp.y, gg.y, bb.y, first, h, keep);
+      sgd_element(pp.z, gg.z, bb.z, first, h, keep);
+      sgd_element(pp.w, gg.w, bb.w, first, h, keep);
+      *reinterpret_cast<float4*>(p + i) = pp;
+      if (buf) *reinterpret_cast<float4*>(buf + i) = bb;
+    }
+    for (int64_t i = e4 + threadIdx.x; i < end; i += 256) {
+      float bv = read_buf ? buf[i] : 0.f;
+      sgd_element(p[i], gr[i], bv, first, h, keep);
+      if (buf) buf[i] = bv;
     }
   }
 }
@@ -152,8 +180,8 @@ sumsq_kernel(TensorTable t, int infinity, double* __restrict__ partial, int chun
   const int total = t.chunk_prefix[t.n];
   for (int chunk = blockIdx.x; chunk < total; chunk += gridDim.x) {
     int ti = find_tensor(t, chunk);
-    int64_t start = (int64_t)(chunk - t.chunk_prefix[ti]) * kChunk;
-    int64_t end = min(t.len[ti], start + kChunk);
+    int64_t start = (int64_t)(chunk - t.chunk_prefix[ti]) * t.chunk;
+    int64_t end = min(t.len[ti], start + t.chunk);
     const float* g = t.g[ti];
     double acc = 0.0;
     for (int64_t i = start + threadIdx.x; i < end; i += 256) {
@@ -216,8 +244,8 @@ scale_by_coef_kernel(TensorTable t, const float* __restrict__ coef_ptr) {
   const int total = t.chunk_prefix[t.n];
   for (int chunk = blockIdx.x; chunk < total; chunk += gridDim.x) {
     int ti = find_tensor(t, chunk);
-    int64_t start = (int64_t)(chunk - t.chunk_prefix[ti]) * kChunk;
-    int64_t end = min(t.len[ti], start + kChunk);
+    int64_t start = (int64_t)(chunk - t.chunk_prefix[ti]) * t.chunk;
+    int64_t end = min(t.len[ti], start + t.chunk);
     float* g = t.p[ti];
     for (int64_t i = start + threadIdx.x; i < end; i += 256) g[i] = __fmul_rn(g[i], coef);
   }
@@ -228,8 +256,8 @@ clip_value_kernel(TensorTable t, float clip) {
   const int total = t.chunk_prefix[t.n];
   for (int chunk = blockIdx.x; chunk < total; chunk += gridDim.x) {
     int ti = find_tensor(t, chunk);
-    int64_t start = (int64_t)(chunk - t.chunk_prefix[ti]) * kChunk;
-    int64_t end = min(t.len[ti], start + kChunk);
+    int64_t start = (int64_t)(chunk - t.chunk_prefix[ti]) * t.chunk;
+    int64_t end = min(t.len[ti], start + t.chunk);
     float* g = t.p[ti];
     for (int64_t i = start + threadIdx.x; i < end; i += 256) {
       float v = g[i];
@@ -240,8 +268,9 @@ clip_value_kernel(TensorTable t, float clip) {
 
 // Fills one table with tensors [base, base + count) and returns the number of chunks.
 static int fill_table(TensorTable& t, int base, int count, float* const* p, const float* const* g, float* const* a,
-                      float* const* b, float* const* c, const int32_t* first, const int64_t* len) {
+                      float* const* b, float* const* c, const int32_t* first, const int64_t* len, int chunk) {
   t.n = count;
+  t.chunk = chunk;
   int chunks = 0;
   for (int i = 0; i < count; i++) {
     int s = base + i;
@@ -254,10 +283,16 @@ static int fill_table(TensorTable& t, int base, int count, float* const* p, cons
     t.first[i] = first ? first[s] : 0;
     t.len[i] = len[s];
     t.chunk_prefix[i] = chunks;
-    chunks += (int)ceil_div(len[s] > 0 ? len[s] : 0, kChunk);
+    chunks += (int)ceil_div(len[s] > 0 ? len[s] : 0, chunk);
   }
   t.chunk_prefix[count] = chunks;
   return chunks;
+}
+
+static int64_t table_total(int base, int count, const int64_t* len) {
+  int64_t total = 0;
+  for (int i = 0; i < count; i++) total += len[base + i] > 0 ? len[base + i] : 0;
+  return total;
 }
 
 static int grid_chunks(om_ctx* ctx, int chunks) {
@@ -386,7 +421,7 @@ int32_t om_optim_adam_step_b16(om_ctx* ctx, int32_t n_tensors, float* const* p, 
   for (int base = 0; base < n_tensors; base += kMaxTensors) {
     TensorTable t;
     int count = std::min(kMaxTensors, n_tensors - base);
-    int chunks = fill_table(t, base, count, p, g, m, v, vmax, nullptr, len);
+    int chunks = fill_table(t, base, count, p, g, m, v, vmax, nullptr, len, update_chunk(table_total(base, count, len)));
     if (chunks == 0) continue;
     if (p16)
       for (int i = 0; i < count; i++) t.p16[i] = p16[base + i];
@@ -408,7 +443,7 @@ int32_t om_optim_sgd_step(om_ctx* ctx, int32_t n_tensors, float* const* p, const
   for (int base = 0; base < n_tensors; base += kMaxTensors) {
     TensorTable t;
     int count = std::min(kMaxTensors, n_tensors - base);
-    int chunks = fill_table(t, base, count, p, g, buf, nullptr, nullptr, first, len);
+    int chunks = fill_table(t, base, count, p, g, buf, nullptr, nullptr, first, len, update_chunk(table_total(base, count, len)));
     if (chunks == 0) continue;
     sgd_kernel<<<grid_chunks(ctx, chunks), 256, 0, ctx->stream>>>(t, *hyper_host, hyper_dev);
     OM_LAUNCH_CHECK(ctx, "om_optim_sgd_step");
@@ -436,7 +471,7 @@ int32_t om_grad_norm_clip(om_ctx* ctx, int32_t n_tensors, float* const* g, const
   for (int base = 0; base < n_tensors; base += kMaxTensors) {
     TensorTable t;
     int count = std::min(kMaxTensors, n_tensors - base);
-    int chunks = fill_table(t, base, count, nullptr, (const float* const*)g, nullptr, nullptr, nullptr, nullptr, len);
+    int chunks = fill_table(t, base, count, nullptr, (const float* const*)g, nullptr, nullptr, nullptr, nullptr, len, kChunk);
     if (chunks == 0) continue;
     launch_chained(ctx, sumsq_kernel, grid_chunks(ctx, chunks), 256, 0, t, infinity_norm, partial, chunk_base);
     chunk_base += chunks;
@@ -445,7 +480,7 @@ int32_t om_grad_norm_clip(om_ctx* ctx, int32_t n_tensors, float* const* g, const
   for (int base = 0; base < n_tensors; base += kMaxTensors) {
     TensorTable t;
     int count = std::min(kMaxTensors, n_tensors - base);
-    int chunks = fill_table(t, base, count, g, nullptr, nullptr, nullptr, nullptr, nullptr, len);
+    int chunks = fill_table(t, base, count, g, nullptr, nullptr, nullptr, nullptr, nullptr, len, kChunk);
     if (chunks == 0) continue;
     launch_chained(ctx, scale_by_coef_kernel, grid_chunks(ctx, chunks), 256, 0, t, coef);
   }
@@ -462,7 +497,7 @@ int32_t om_grad_clip_value(om_ctx* ctx, int32_t n_tensors, float* const* g, cons
   for (int base = 0; base < n_tensors; base += kMaxTensors) {
     TensorTable t;
     int count = std::min(kMaxTensors, n_tensors - base);
-    int chunks = fill_table(t, base, count, g, nullptr, nullptr, nullptr, nullptr, nullptr, len);
+    int chunks = fill_table(t, base, count, g, nullptr, nullptr, nullptr, nullptr, nullptr, len, kChunk);
     if (chunks == 0) continue;
     clip_value_kernel<<<grid_chunks(ctx, chunks), 256, 0, ctx->stream>>>(t, clip);
     OM_LAUNCH_CHECK(ctx, "om_grad_clip_value");
