@@ -11,6 +11,8 @@
 //
 // Every mbarrier wait is bounded (om_tc.cuh): on expiry the kernel raises OM_ERR_TIMEOUT in the status word, all roles
 // leave, TMEM is released.
+#include <type_traits>
+
 #include "om_tc.cuh"
 
 namespace om {
@@ -24,6 +26,7 @@ struct AttFwdParams {
   float scale;
   const float* mask;
   long long mask_batch_stride;
+  int mask_vec;          // mask rows can be read 16 bytes at a time
   float* out;
   long long o_batch, o_head, o_row;
   float* lse;            // [B*H, lq] or null
@@ -51,6 +54,44 @@ __device__ __forceinline__ float fast_ex2(float x) {
 __device__ __forceinline__ uint32_t att_idesc(int n, bool a_mn, bool b_mn) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) |
          ((uint32_t)(ATT_TILE >> 4) << 24);
+}
+
+// The additive mask of a warp's 32 x 32 block of scores. A thread owns a score row, so reading the mask where it is used
+// would touch 32 different rows with every 4-byte load (B 16, H 8, L 320, D 32: 161 us forward and 106 us backward front per
+// layer, most of it those loads; 61 and 59 us this way). Instead the warp reads the block by rows (eight lanes cover the 128
+// bytes of one, before the wait for the scores) and turns it through 4 KB of shared memory whose 16-byte chunk c of row r
+// sits at c ^ (r & 7). Rows and columns outside the mask read as zero.
+__device__ __forceinline__ void mask_fetch(float4 (&m)[8], const float* __restrict__ mask, int row0, int lq, int col0, int lk, int lane) {
+  const int col = col0 + (lane & 7) * 4;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int row = row0 + i * 4 + (lane >> 3);
+    m[i] = row < lq && col < lk ? __ldg(reinterpret_cast<const float4*>(mask + (long long)row * lk + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+// Without 16-byte rows (vec == false) the warp fetches here, a row per step.
+__device__ __forceinline__ void mask_deposit(uint8_t* blk, const float4 (&m)[8], bool vec, const float* __restrict__ mask, int row0, int lq, int col0,
+                                             int lk, int lane) {
+  if (vec) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const int r = i * 4 + (lane >> 3);
+      *reinterpret_cast<float4*>(blk + r * 128 + (((lane & 7) ^ (r & 7)) << 4)) = m[i];
+    }
+  } else {
+#pragma unroll 8
+    for (int r = 0; r < 32; r++)
+      *reinterpret_cast<float*>(blk + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4) =
+          row0 + r < lq && col0 + lane < lk ? __ldg(mask + (long long)(row0 + r) * lk + col0 + lane) : 0.f;
+  }
+  __syncwarp();
+}
+// Columns 4 c .. 4 c + 3 of the lane's own row.
+__device__ __forceinline__ float4 mask_row4(const uint8_t* blk, int lane, int c) {
+  return *reinterpret_cast<const float4*>(blk + lane * 128 + ((c ^ (lane & 7)) << 4));
+}
+static int mask_rows_vec(const float* mask, long long batch_stride, int lk) {
+  return mask && (lk & 3) == 0 && (batch_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(mask) & 15) == 0;
 }
 
 // Writes one accumulator row (values v[0..127], already TF32) into a K-major operand tile of 4 blocks [128 rows x 128 B]
@@ -150,7 +191,7 @@ attention_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     // ---- one row per thread ----
     const int row = warp * 32 + lane;
     const uint32_t lane_base = tmem_base + ((uint32_t)(warp * 32) << 16);
-    bool ok = mbar_wait(bar_s, 0, abort_flag, p.status, 13);
+    bool ok = __all_sync(0xffffffffu, mbar_wait(bar_s, 0, abort_flag, p.status, 13));   // the warp works together from here on
     tc_fence_after();
     float v[ATT_TILE];
     if (ok) {
@@ -164,10 +205,31 @@ attention_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       }
       // scale * s + mask, row maximum, exponentials and their sum; four independent chains keep the pipes busy. The
       // exponential is 2^(x * log2 e) on the special-function unit; the sum runs in fp32 (128 terms).
-      const float* mrow = nullptr;
-      if (p.mask && row < p.lq) mrow = p.mask + (long long)bi * p.mask_batch_stride + (long long)row * p.lk;
+      const float* mask = p.mask ? p.mask + (long long)bi * p.mask_batch_stride : nullptr;
       float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-      if (mrow == nullptr && p.lk == ATT_TILE) {
+      if (mask) {
+        // Turned through this warp's rows of the P region: S is complete, so the Q and K tiles under it are dead.
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          uint8_t* blk = p_s + c * ATT_BLOCK_BYTES + warp * 4096;
+          float4 mk[8];
+          if (p.mask_vec) mask_fetch(mk, mask, warp * 32, p.lq, c * 32, p.lk, lane);
+          mask_deposit(blk, mk, p.mask_vec, mask, warp * 32, p.lq, c * 32, p.lk, lane);
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            const float4 m = mask_row4(blk, lane, j);
+            const float mj[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              const int col = c * 32 + j * 4 + e;
+              const float s = col < p.lk ? (v[col] * p.scale) + mj[e] : -INFINITY;
+              v[col] = s;
+              m4[e] = fmaxf(m4[e], s);
+            }
+          }
+        }
+        __syncwarp();
+      } else if (p.lk == ATT_TILE) {
 #pragma unroll
         for (int j = 0; j < ATT_TILE; j++) {
           v[j] = v[j] * p.scale;
@@ -177,7 +239,7 @@ attention_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 #pragma unroll
         for (int j = 0; j < ATT_TILE; j++) {
           float s = -INFINITY;
-          if (j < p.lk) s = (v[j] * p.scale) + (mrow ? mrow[j] : 0.f);
+          if (j < p.lk) s = (v[j] * p.scale) + 0.f;
           v[j] = s;
           m4[j & 3] = fmaxf(m4[j & 3], s);
         }
@@ -253,6 +315,7 @@ struct AttBwdParams {
   float scale;
   const float* mask;
   long long mask_batch_stride;
+  int mask_vec;          // mask rows can be read 16 bytes at a time
   const float* lse;
   float *dq, *dk, *dv;
   long long dq_batch, dq_head, dq_row, dk_batch, dk_head, dk_row, dv_batch, dv_head, dv_row;
@@ -407,26 +470,35 @@ attention_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid
     const int row = quad * 32 + lane;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
     const float LOG2E = 1.4426950408889634f;
-    bool ok = mbar_wait(bar_sdp, 0, abort_flag, p.status, 26);
+    bool ok = __all_sync(0xffffffffu, mbar_wait(bar_sdp, 0, abort_flag, p.status, 26));   // the warp works together from here on
     tc_fence_after();
     float pv[64], dp[64];
     float dot = 0.f;
     if (ok) {
       const float lse_l = (row < p.lq ? p.lse[(long long)bh * p.lq + row] : 0.f) * LOG2E;
-      const float* mrow = nullptr;
-      if (p.mask && row < p.lq) mrow = p.mask + (long long)bi * p.mask_batch_stride + (long long)row * p.lk;
+      const float* mask = p.mask ? p.mask + (long long)bi * p.mask_batch_stride : nullptr;
       float d4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int c = 0; c < 2; c++) {
         const int col0 = half * 64 + c * 32;
+        uint8_t* blk = stage_b + (half * 2 + c) * ATT_BLOCK_BYTES + quad * 4096;   // this warp's rows of dS, not yet written
+        if (mask) {
+          float4 mk[8];
+          if (p.mask_vec) mask_fetch(mk, mask, quad * 32, p.lq, col0, p.lk, lane);
+          mask_deposit(blk, mk, p.mask_vec, mask, quad * 32, p.lq, col0, p.lk, lane);
+        }
         uint32_t rs[32], rd[32];
         tmem_ld_32x32b_x32(lane_base + COL_S + col0, rs);
         tmem_ld_32x32b_x32(lane_base + COL_DP + col0, rd);
         tmem_ld_wait();
+        float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int j = 0; j < 32; j++) {
           float s = __uint_as_float(rs[j]) * p.scale;
-          if (mrow && col0 + j < p.lk) s = s + mrow[col0 + j];
+          if (mask) {
+            if ((j & 3) == 0) m = mask_row4(blk, lane, j >> 2);
+            s = s + ((j & 3) == 0 ? m.x : (j & 3) == 1 ? m.y : (j & 3) == 2 ? m.z : m.w);
+          }
           float e = exp2f(fmaf(s, LOG2E, -lse_l));
           if (col0 + j >= p.lk) e = 0.f;
           const float d = __uint_as_float(rd[j]);
@@ -510,7 +582,8 @@ constexpr int ATT_MT_PARTS = 4;              // threads per score row: each owns
 constexpr int ATT_MT_ISSUE_WARP = 4 * ATT_MT_PARTS;
 constexpr int ATT_MT_THREADS = 32 * (ATT_MT_ISSUE_WARP + 1);   // 16 row warps (enough of them to hide each other's latencies) + TMA / MMA issue
 
-template <int D>
+// MASKED: with an additive mask (its block in registers would make the plain form spill).
+template <int D, bool MASKED>
 __global__ void __launch_bounds__(ATT_MT_THREADS, 1)
 attention_fwd_mt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                         const __grid_constant__ CUtensorMap map_v, AttFwdParams p) {
@@ -534,7 +607,8 @@ attention_fwd_mt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   uint64_t* bar_pv = bars + 10;     // P V product complete (P buffer and that tile's V buffer free)
   uint64_t* bar_x = bars + 11;      // all parts of every row have published their pass-1 statistics
   uint64_t* bar_x2 = bars + 12;     // ... and have read them: the statistics share their memory with the first P
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+  uint64_t* bar_m = bars + 13;      // all row warps have read the last mask block of pass 1
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -555,6 +629,7 @@ attention_fwd_mt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     mbar_init(bar_pv, 1);
     mbar_init(bar_x, ATT_MT_PARTS * ATT_TILE);
     mbar_init(bar_x2, ATT_MT_PARTS * ATT_TILE);
+    mbar_init(bar_m, ATT_MT_ISSUE_WARP);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -652,14 +727,19 @@ attention_fwd_mt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
     const float LOG2E = 1.4426950408889634f;
     const float sl2 = p.scale * LOG2E;
-    const float* mrow = nullptr;
-    if (p.mask && qrow < p.lq) mrow = p.mask + (long long)bi * p.mask_batch_stride + (long long)qrow * p.lk;
+    const float* mask = MASKED ? p.mask + (long long)bi * p.mask_batch_stride : nullptr;
+    uint8_t* blk = p_s + part * ATT_BLOCK_BYTES + quad * 4096;   // this warp's 32 x 32 block of P: the mask is turned through it
     float run_max = -INFINITY, run_sum = 0.f, inv_sum = 0.f, max_l2 = 0.f;
     bool ok = true;
     float v[32];
     for (int g = 0; g < steps && ok; g++) {
       const int i = g & 1, j = g % nk, col0 = j * ATT_TILE + part * 32;
+      float4 mk[8];
+      if (MASKED && p.mask_vec) mask_fetch(mk, mask, q0 + quad * 32, p.lq, col0, p.lk, lane);
       ok = __all_sync(0xffffffffu, mbar_wait(&bar_s[i], (uint32_t)(g >> 1) & 1, abort_flag, p.status, 49));
+      // P is free for the mask of pass 2 once the previous P has been consumed and, at first, everyone has read the statistics.
+      if (MASKED && ok && g >= nk) ok = __all_sync(0xffffffffu, g > nk ? mbar_wait(bar_pv, (uint32_t)(g - nk - 1) & 1, abort_flag, p.status, 50)
+                                                                     : mbar_wait(bar_x2, 0, abort_flag, p.status, 53));
       if (!ok) break;
       tc_fence_after();
       {
@@ -674,17 +754,23 @@ attention_fwd_mt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       if (lane == 0) mbar_arrive(&bar_sr[i]);       // the next product may overwrite this S buffer (one arrival per warp:
                                                     // hundreds of arrivals on one barrier word would serialise)
       // Scores in the base-2 domain from here on: t = (scale s + mask) log2 e, so that an exponential is one ex2.
-      const bool full = mrow == nullptr && col0 + 32 <= p.lk;
-      if (full) {
+      if (MASKED) {
+        mask_deposit(blk, mk, p.mask_vec, mask, q0 + quad * 32, p.lq, col0, p.lk, lane);
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+          const float4 m = mask_row4(blk, lane, c);
+          v[4 * c] = col0 + 4 * c < p.lk ? fmaf(v[4 * c], sl2, m.x * LOG2E) : -INFINITY;
+          v[4 * c + 1] = col0 + 4 * c + 1 < p.lk ? fmaf(v[4 * c + 1], sl2, m.y * LOG2E) : -INFINITY;
+          v[4 * c + 2] = col0 + 4 * c + 2 < p.lk ? fmaf(v[4 * c + 2], sl2, m.z * LOG2E) : -INFINITY;
+          v[4 * c + 3] = col0 + 4 * c + 3 < p.lk ? fmaf(v[4 * c + 3], sl2, m.w * LOG2E) : -INFINITY;
+        }
+        __syncwarp();
+      } else if (col0 + 32 <= p.lk) {
 #pragma unroll
         for (int jj = 0; jj < 32; jj++) v[jj] = v[jj] * sl2;
       } else {
 #pragma unroll
-        for (int jj = 0; jj < 32; jj++) {
-          float sv = -INFINITY;
-          if (col0 + jj < p.lk) sv = fmaf(v[jj], sl2, mrow ? mrow[col0 + jj] * LOG2E : 0.f);
-          v[jj] = sv;
-        }
+        for (int jj = 0; jj < 32; jj++) v[jj] = col0 + jj < p.lk ? fmaf(v[jj], sl2, 0.f) : -INFINITY;
       }
       if (g < nk) {
         // pass 1: running maximum and sum of exponentials of this thread's columns
@@ -702,6 +788,12 @@ attention_fwd_mt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           run_max = new_max;
         }
         if (g == nk - 1) {
+          // (the statistics lie where warp 0 turned its mask: not before it has read it)
+          if (MASKED) {
+            if (lane == 0) mbar_arrive(bar_m);
+            ok = __all_sync(0xffffffffu, mbar_wait(bar_m, 0, abort_flag, p.status, 54));
+            if (!ok) break;
+          }
           // the threads of a row exchange their statistics once and combine them in the order of the column ranges, so that
           // all of them hold the same bits
           stats[(part * ATT_TILE + row) * 2] = run_max;
@@ -728,7 +820,8 @@ attention_fwd_mt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         const int t = g - nk;
 #pragma unroll
         for (int jj = 0; jj < 32; jj++) v[jj] = to_tf32(fast_ex2(v[jj] - max_l2) * inv_sum);
-        if (t >= 1) ok = __all_sync(0xffffffffu, mbar_wait(bar_pv, (uint32_t)(t - 1) & 1, abort_flag, p.status, 50));   // the previous P has been consumed
+        if (MASKED) ok = true;                                                                                             // waited for above
+        else if (t >= 1) ok = __all_sync(0xffffffffu, mbar_wait(bar_pv, (uint32_t)(t - 1) & 1, abort_flag, p.status, 50));   // the previous P has been consumed
         else ok = __all_sync(0xffffffffu, mbar_wait(bar_x2, 0, abort_flag, p.status, 53));                               // everyone has read the statistics
         if (ok) {
           store_seg_kmajor(p_s + part * ATT_BLOCK_BYTES, row, v);
@@ -773,6 +866,7 @@ struct AttFrontParams {
   float scale;
   const float* mask;
   long long mask_batch_stride;
+  int mask_vec;          // mask rows can be read 16 bytes at a time
   const float* lse;      // [B*H, lq]
   const float* g;        // dO and O as strided [B, H, L, D] views (ONE_PASS)
   const float* o;
@@ -807,7 +901,7 @@ __device__ __forceinline__ void store_block_32(float* stg, int lane, const float
   __syncwarp();
 }
 
-template <int D, bool ONE_PASS>
+template <int D, bool ONE_PASS, bool MASKED>
 __global__ void __launch_bounds__(ATT_MT_THREADS, 1)
 attention_bwd_front_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_g,
                            const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, AttFrontParams p) {
@@ -916,8 +1010,7 @@ attention_bwd_front_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
     const float LOG2E = 1.4426950408889634f;
     const float sl2 = p.scale * LOG2E;
-    const float* mrow = nullptr;
-    if (p.mask && qrow < p.lq) mrow = p.mask + (long long)bi * p.mask_batch_stride + (long long)qrow * p.lk;
+    const float* mask = MASKED ? p.mask + (long long)bi * p.mask_batch_stride : nullptr;
     const float lse_l = (qrow < p.lq ? p.lse[(long long)bh * p.lq + qrow] : 0.f) * LOG2E;
     const bool vec_ok = (p.lk & 3) == 0 && ((reinterpret_cast<uintptr_t>(p.p_out) | reinterpret_cast<uintptr_t>(p.ds_out)) & 15) == 0;
     float* stg = stage + warp * 32 * ATT_STG_LD;
@@ -955,6 +1048,12 @@ attention_bwd_front_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     float pv[32], dp[32];
     for (int g = 0; g < steps && ok; g++) {
       const int i = g & 1, j = g % nk, col0 = j * ATT_TILE + part * 32;
+      uint8_t* blk = reinterpret_cast<uint8_t*>(stg);   // the mask is turned where the results will be
+      if (MASKED) {
+        float4 mk[8];
+        if (p.mask_vec) mask_fetch(mk, mask, q0 + quad * 32, p.lq, col0, p.lk, lane);
+        mask_deposit(blk, mk, p.mask_vec, mask, q0 + quad * 32, p.lq, col0, p.lk, lane);
+      }
       ok = __all_sync(0xffffffffu, mbar_wait(&bar_s[i], (uint32_t)(g >> 1) & 1, abort_flag, p.status, 66));
       if (!ok) break;
       tc_fence_after();
@@ -963,7 +1062,20 @@ attention_bwd_front_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         tmem_ld_32x32b_x32(lane_base + (uint32_t)(i * ATT_TILE + part * 32), rs);
         tmem_ld_32x32b_x32(lane_base + COL_DP + (uint32_t)(i * ATT_TILE + part * 32), rd);
         tmem_ld_wait();
-        if (mrow == nullptr && col0 + 32 <= p.lk) {
+        if (MASKED) {
+#pragma unroll
+          for (int c = 0; c < 8; c++) {
+            const float4 m = mask_row4(blk, lane, c);
+            const float mj[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              const int jj = 4 * c + e;
+              pv[jj] = col0 + jj < p.lk ? fast_ex2(fmaf(__uint_as_float(rs[jj]), sl2, mj[e] * LOG2E - lse_l)) : 0.f;
+              dp[jj] = __uint_as_float(rd[jj]);
+            }
+          }
+          __syncwarp();
+        } else if (col0 + 32 <= p.lk) {
 #pragma unroll
           for (int jj = 0; jj < 32; jj++) {
             pv[jj] = fast_ex2(fmaf(__uint_as_float(rs[jj]), sl2, -lse_l));
@@ -972,10 +1084,7 @@ attention_bwd_front_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         } else {
 #pragma unroll
           for (int jj = 0; jj < 32; jj++) {
-            const int col = col0 + jj;
-            float e = 0.f;
-            if (col < p.lk) e = fast_ex2(fmaf(__uint_as_float(rs[jj]), sl2, (mrow ? mrow[col] * LOG2E : 0.f) - lse_l));
-            pv[jj] = e;
+            pv[jj] = col0 + jj < p.lk ? fast_ex2(fmaf(__uint_as_float(rs[jj]), sl2, 0.f - lse_l)) : 0.f;
             dp[jj] = __uint_as_float(rd[jj]);
           }
         }
@@ -1037,6 +1146,18 @@ bool attention_tc_fwd_supported(om_ctx* ctx, const float* q, const om_head_strid
   return true;
 }
 
+template <int D, bool MASKED>
+static int32_t launch_mt(om_ctx* ctx, dim3 grid, size_t smem, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                         const AttFwdParams& p) {
+  static bool set = false;
+  if (!set) {
+    OM_CUDA(ctx, cudaFuncSetAttribute(attention_fwd_mt_kernel<D, MASKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    set = true;
+  }
+  launch_chained(ctx, attention_fwd_mt_kernel<D, MASKED>, grid, ATT_MT_THREADS, smem, mq, mk, mv, p);
+  return OM_OK;
+}
+
 int32_t attention_tc_fwd(om_ctx* ctx, const float* q, const om_head_strides* qs, const float* k, const om_head_strides* ks, const float* v,
                          const om_head_strides* vs, const float* mask, long long mask_batch_stride, int b, int h, int lq, int lk, int d,
                          float scale, float* out, const om_head_strides* os, float* lse) {
@@ -1045,27 +1166,16 @@ int32_t attention_tc_fwd(om_ctx* ctx, const float* q, const om_head_strides* qs,
       !att_map(&mv, v, d, lk, h, b, vs->row, vs->head, vs->batch, true))
     return fail(ctx, OM_ERR_CUDA, "cuTensorMapEncodeTiled failed for the attention operands");
   AttFwdParams p;
-  p.lq = lq; p.lk = lk; p.d = d; p.heads = h; p.scale = scale; p.mask = mask; p.mask_batch_stride = mask_batch_stride;
+  p.lq = lq; p.lk = lk; p.d = d; p.heads = h; p.scale = scale; p.mask = mask; p.mask_batch_stride = mask_batch_stride; p.mask_vec = mask_rows_vec(mask, mask_batch_stride, lk);
   p.out = out; p.o_batch = os->batch; p.o_head = os->head; p.o_row = os->row; p.lse = lse; p.status = ctx->status_dev;
   if (lq > ATT_TILE || lk > ATT_TILE) {
     // Several tiles: one CTA per 128 queries walks the key tiles (two passes, see attention_fwd_mt_kernel).
     const size_t smem_mt = (size_t)(5 * (d / 32) + 4) * ATT_BLOCK_BYTES + 1024 + 256;
     const dim3 grid_mt((unsigned)((lq + ATT_TILE - 1) / ATT_TILE), (unsigned)(b * h));
-    if (d == 32) {
-      static bool set = false;
-      if (!set) {
-        OM_CUDA(ctx, cudaFuncSetAttribute(attention_fwd_mt_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_mt));
-        set = true;
-      }
-      launch_chained(ctx, attention_fwd_mt_kernel<32>, grid_mt, ATT_MT_THREADS, smem_mt, mq, mk, mv, p);
-    } else {
-      static bool set = false;
-      if (!set) {
-        OM_CUDA(ctx, cudaFuncSetAttribute(attention_fwd_mt_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_mt));
-        set = true;
-      }
-      launch_chained(ctx, attention_fwd_mt_kernel<64>, grid_mt, ATT_MT_THREADS, smem_mt, mq, mk, mv, p);
-    }
+    int32_t st;
+    if (d == 32) st = mask ? launch_mt<32, true>(ctx, grid_mt, smem_mt, mq, mk, mv, p) : launch_mt<32, false>(ctx, grid_mt, smem_mt, mq, mk, mv, p);
+    else st = mask ? launch_mt<64, true>(ctx, grid_mt, smem_mt, mq, mk, mv, p) : launch_mt<64, false>(ctx, grid_mt, smem_mt, mq, mk, mv, p);
+    OM_TRY(st);
     OM_LAUNCH_CHECK(ctx, "attention_fwd_mt");
     return OM_OK;
   }
@@ -1115,7 +1225,7 @@ int32_t attention_tc_bwd(om_ctx* ctx, const float* g, const om_head_strides* gs,
              att_map(&gm, g, 32, lq, h, b, gs->row, gs->head, gs->batch, true);
   if (!okm) return fail(ctx, OM_ERR_CUDA, "cuTensorMapEncodeTiled failed for the attention backward operands");
   AttBwdParams p;
-  p.lq = lq; p.lk = lk; p.heads = h; p.scale = scale; p.mask = mask; p.mask_batch_stride = mask_batch_stride; p.lse = lse;
+  p.lq = lq; p.lk = lk; p.heads = h; p.scale = scale; p.mask = mask; p.mask_batch_stride = mask_batch_stride; p.mask_vec = mask_rows_vec(mask, mask_batch_stride, lk); p.lse = lse;
   p.dq = dq; p.dk = dk; p.dv = dv;
   p.dq_batch = dq ? dqs->batch : 0; p.dq_head = dq ? dqs->head : 0; p.dq_row = dq ? dqs->row : 0;
   p.dk_batch = dk ? dks->batch : 0; p.dk_head = dk ? dks->head : 0; p.dk_row = dk ? dks->row : 0;
@@ -1141,15 +1251,15 @@ bool attention_bwd_front_supported(om_ctx* ctx, const float* g, const om_head_st
   return att_operand_ok(g, gs, h, b) && att_operand_ok(q, qs, h, b) && att_operand_ok(k, ks, h, b) && att_operand_ok(v, vs, h, b);
 }
 
-template <int D, bool ONE_PASS>
+template <int D, bool ONE_PASS, bool MASKED>
 static int32_t launch_front(om_ctx* ctx, dim3 grid, size_t smem, const CUtensorMap& mq, const CUtensorMap& mg, const CUtensorMap& mk,
                             const CUtensorMap& mv, const AttFrontParams& p) {
   static bool set = false;
   if (!set) {
-    OM_CUDA(ctx, cudaFuncSetAttribute(attention_bwd_front_kernel<D, ONE_PASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    OM_CUDA(ctx, cudaFuncSetAttribute(attention_bwd_front_kernel<D, ONE_PASS, MASKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     set = true;
   }
-  launch_chained(ctx, attention_bwd_front_kernel<D, ONE_PASS>, grid, ATT_MT_THREADS, smem, mq, mg, mk, mv, p);
+  launch_chained(ctx, attention_bwd_front_kernel<D, ONE_PASS, MASKED>, grid, ATT_MT_THREADS, smem, mq, mg, mk, mv, p);
   return OM_OK;
 }
 
@@ -1165,16 +1275,21 @@ int32_t attention_bwd_front(om_ctx* ctx, const float* g, const om_head_strides* 
   const bool one_pass = o != nullptr && os != nullptr && (reinterpret_cast<uintptr_t>(o) & 15) == 0 && (os->row & 3) == 0 &&
                         (os->head & 3) == 0 && (os->batch & 3) == 0;
   AttFrontParams p;
-  p.lq = lq; p.lk = lk; p.heads = h; p.d = d; p.scale = scale; p.mask = mask; p.mask_batch_stride = mask_batch_stride; p.lse = lse;
+  p.lq = lq; p.lk = lk; p.heads = h; p.d = d; p.scale = scale; p.mask = mask; p.mask_batch_stride = mask_batch_stride; p.mask_vec = mask_rows_vec(mask, mask_batch_stride, lk); p.lse = lse;
   p.g = g; p.g_batch = gs->batch; p.g_head = gs->head; p.g_row = gs->row;
   p.o = one_pass ? o : nullptr; p.o_batch = one_pass ? os->batch : 0; p.o_head = one_pass ? os->head : 0; p.o_row = one_pass ? os->row : 0;
   p.p_out = p_out; p.ds_out = ds_out; p.status = ctx->status_dev;
   const size_t smem = (size_t)(4 * (d / 32)) * ATT_BLOCK_BYTES + 1024 + (ATT_MT_ISSUE_WARP * 32 * ATT_STG_LD + ATT_MT_PARTS * ATT_TILE) * sizeof(float) + 256;
   const dim3 grid((unsigned)((lq + ATT_TILE - 1) / ATT_TILE), (unsigned)(b * h));
-  int32_t st;
-  if (d == 32) st = one_pass ? launch_front<32, true>(ctx, grid, smem, mq, mg, mk, mv, p) : launch_front<32, false>(ctx, grid, smem, mq, mg, mk, mv, p);
-  else st = one_pass ? launch_front<64, true>(ctx, grid, smem, mq, mg, mk, mv, p) : launch_front<64, false>(ctx, grid, smem, mq, mg, mk, mv, p);
-  OM_TRY(st);
+  auto launch = [&](auto dim, auto pass) -> int32_t {
+    constexpr int D = decltype(dim)::value;
+    constexpr bool ONE = decltype(pass)::value;
+    return mask ? launch_front<D, ONE, true>(ctx, grid, smem, mq, mg, mk, mv, p) : launch_front<D, ONE, false>(ctx, grid, smem, mq, mg, mk, mv, p);
+  };
+  using D32 = std::integral_constant<int, 32>;
+  using D64 = std::integral_constant<int, 64>;
+  if (d == 32) OM_TRY(one_pass ? launch(D32{}, std::true_type{}) : launch(D32{}, std::false_type{}));
+  else OM_TRY(one_pass ? launch(D64{}, std::true_type{}) : launch(D64{}, std::false_type{}));
   OM_LAUNCH_CHECK(ctx, "attention_bwd_front");
   return OM_OK;
 }

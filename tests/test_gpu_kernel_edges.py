@@ -49,3 +49,34 @@ def test_sgd_visits_are_bit_exact(ctx, K, sizes, momentum, nesterov, wd):
         assert np.array_equal(P[i].numpy()[s:], ps[i]), sizes[i]
         if momentum:
             assert np.array_equal(B[i].numpy()[s:], bufs[i]), sizes[i]
+
+
+@pytest.mark.parametrize("tf32", [0, 1])
+@pytest.mark.parametrize("b,h,lq,lk,d,batched", [(2, 3, 128, 128, 32, 1), (3, 2, 97, 61, 32, 1), (2, 2, 100, 128, 64, 0), (2, 2, 129, 130, 32, 1),
+                                                 (2, 2, 320, 320, 32, 1), (1, 3, 200, 259, 64, 0), (2, 1, 256, 384, 64, 1)])
+def test_attention_masks_of_every_alignment(ctx, K, tf32, b, h, lq, lk, d, batched):
+    """The mask is brought in by rows and turned: one tile and several, ragged rows and columns, rows off the 16-byte grid, a
+    mask base off it, a mask for all batches and one for each, padded keys with a large negative score and with -inf. Three
+    chained TF32 products: 2e-3 scaled, the gate of the attention tests without a mask."""
+    ctx.set_flags(omb.OM_TF32 if tf32 else 0)
+    try:
+        q, k, v, g = (normal(i, b, h, l, d) for i, l in ((1, lq), (2, lk), (3, lk), (4, lq)))
+        r = np.random.default_rng(5)
+        mask = normal(6, *((b, lq, lk) if batched else (lq, lk)))
+        mask[..., lk - lk // 4:] = np.where(r.random(mask[..., lk - lk // 4:].shape) < 0.5, np.float32(-1e9), np.float32(-np.inf))
+        scale = 1.0 / np.sqrt(d)
+        for shift in (0, 1):
+            Q, Kk, V, G = (ctx.to_device(a) for a in (q, k, v, g))
+            M = ctx.to_device(np.concatenate([np.zeros(shift, np.float32), mask.reshape(-1)]))
+            O, LSE = ctx.empty(q.shape), ctx.empty((b, h, lq))
+            DQ, DK, DV = ctx.empty(q.shape), ctx.empty(k.shape), ctx.empty(v.shape)
+            at = C.c_void_p(M.ptr.value + 4 * shift)
+            mbs = lq * lk if batched else 0
+            ctx.call("om_attention_fwd", ctx.handle, Q.ptr, Kk.ptr, V.ptr, at, i64(mbs), i32(b), i32(h), i32(lq), i32(lk), i32(d), f32(scale), O.ptr, LSE.ptr)
+            ctx.call("om_attention_bwd", ctx.handle, G.ptr, Q.ptr, Kk.ptr, V.ptr, at, i64(mbs), LSE.ptr, i32(b), i32(h), i32(lq), i32(lk), i32(d), f32(scale),
+                     DQ.ptr, DK.ptr, DV.ptr)
+            dq, dk, dv = K.attention_bwd(g, q, k, v, mask)
+            for got, want in ((O, K.attention_fwd(q, k, v, mask)), (DQ, dq), (DK, dk), (DV, dv)):
+                assert scaled_diff(got.numpy(), want) <= (2e-3 if tf32 else 1e-4)
+    finally:
+        ctx.set_flags(0)
