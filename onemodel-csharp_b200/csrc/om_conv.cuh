@@ -1,0 +1,20 @@
+// Geometry of a 2-D convolution, shared by the unfolding path (om_spatial.cu), the tensor-pipe kernels (om_conv_tc.cu).
+#pragma once
+#include "om_common.cuh"
+
+namespace om {
+
+struct ConvGeom {
+  int n, cin, h, w, cout, kh, kw, sh, sw, pt, pl, dh, dw, groups, oh, ow;
+};
+
+// The TF32 products without an unfolded matrix (om_conv_tc.cu). *_fits says whether the kernel takes the geometry; the caller
+// has already decided that the product runs on the tensor pipe.
+bool conv_tc_fwd_fits(const ConvGeom& g);
+int32_t conv_tc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y);
+bool conv_tc_dgrad_fits(const ConvGeom& g);
+int32_t conv_tc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx);
+bool conv_tc_wgrad_fits(const ConvGeom& g);
+int32_t conv_tc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, float* dw, int accumulate);
+
+}  // namespace om

@@ -1,0 +1,714 @@
+// Convolution on the tensor pipe without an unfolded matrix: implicit products over NCHW tensors (ConvBackward and its forward,
+// BackwardNn.cs:317-462 of the reference), TF32 operands, fp32 accumulators in tensor memory.
+//
+//   forward  y[co, pixel]  = sum over k = (c, tap)    W[co, k]          x[c, pixel's input position of the tap]
+//   dgrad    dx[c, pixel]  = sum over k = (co, tap)   W[co, c, tap]     g[co, pixel's output position of the tap]
+//   wgrad    dW[co, n]     = sum over k = pixels      g[co, pixel]      x[n's channel, pixel's input position of n's tap]
+//
+// The operand that an unfolded matrix would hold is gathered by eight warps straight into the K-major, 128-byte-swizzled
+// operand tile, rounded to TF32 (nearest even, as TMA rounds) on the way. Lanes own consecutive pixels, so a load is one or
+// two row segments. k runs in units of eight channels of one tap: inside a unit the source position moves by whole planes
+// and lies inside the image or outside for all eight, so an element costs an addition, a load, a rounding and a quarter of a
+// 16-byte store. (With k in the weights' own order, channel by channel, each element looked its offset and its tap up in a table:
+// 17 instructions and 12 load/store wavefronts, 202 us for 256 images of 64 x 32 x 32 through a 3 x 3 window to 64
+// channels; the unfolded form took 455.) Units of four neighbouring channel groups share a tap before the next tap comes, so the
+// taps of a window find each other's lines in L1. The weights are turned into the order of the units by a small kernel.
+// What bounds the kernels is the load/store unit: 128 x 32 gathered elements a 128 x 128 x 32 product.
+//
+// dgrad with stride s works on the s * s classes of input positions modulo the stride (grid z): each is a stride-1
+// problem over the taps that reach it, so no product is formed with the zeros between the strides.
+#include "om_conv.cuh"
+#include "om_tc.cuh"
+
+namespace om {
+
+constexpr int CV_TILE = 128;                      // channels (accumulator rows) and pixels / unit columns (columns) of a tile
+constexpr int CV_BK = 32;                         // one 128-byte swizzle row of k
+constexpr int CV_UNIT = 8;                        // channels of one tap
+constexpr int CV_GROUP = 4;                       // units of one tap that follow one another
+constexpr int CV_BLOCK = CV_TILE * 128;           // one operand block: 16 KiB
+constexpr int CV_PRODUCERS = 8;                   // gathering warps, also the epilogue
+constexpr int CV_THREADS = 32 * (CV_PRODUCERS + 2);   // + one warp issuing products, one issuing TMA loads
+constexpr int CV_MAX_TAPS = 32;                   // a thread keeps the taps that lie inside the image as a bit mask
+constexpr int CV_MAX_PHASES = 4;
+constexpr int CV_STG_LD = CV_TILE + 4;            // floats per staged result row
+
+// n / d for 0 <= n < 2^31 by a multiplication (Granlund and Montgomery, "Division by invariant integers using
+// multiplication", 1994): s = ceil(log2 d), mul = floor(2^32 (2^s - d) / d) + 1, n / d = (mulhi(n, mul) + n) >> s.
+struct CvDiv {
+  uint32_t mul, shift;
+};
+static CvDiv cv_div(uint32_t d) {
+  CvDiv r;
+  r.shift = 0;
+  while ((1ull << r.shift) < d) r.shift++;
+  r.mul = (uint32_t)(((1ull << 32) * ((1ull << r.shift) - d)) / d + 1);
+  return r;
+}
+__device__ __forceinline__ int cv_quot(int n, CvDiv d) { return (int)((__umulhi((uint32_t)n, d.mul) + (uint32_t)n) >> d.shift); }
+
+// Unit u of channels x taps: its tap, and its first channel.
+__host__ __device__ __forceinline__ void cv_unit(int u, int channels, int taps, int* tap, int* c0) {
+  const int c8 = (channels + CV_UNIT - 1) / CV_UNIT;
+  const int sg = u / (CV_GROUP * taps), r = u - sg * CV_GROUP * taps;
+  const int width = c8 - sg * CV_GROUP < CV_GROUP ? c8 - sg * CV_GROUP : CV_GROUP;
+  *tap = r / width;
+  *c0 = (sg * CV_GROUP + r % width) * CV_UNIT;
+}
+static int cv_units(int channels, int taps) { return (channels + CV_UNIT - 1) / CV_UNIT * taps; }
+
+struct ConvPhase {
+  int ph, pw;                  // grid of pixels
+  CvDiv div_plane, div_w;
+  int oy0, ox0;                // output position of pixel (0, 0)
+  int taps, units;
+  int dy[CV_MAX_TAPS], dx[CV_MAX_TAPS];
+};
+
+struct ConvTcParams {
+  const float* src;
+  float* out;
+  const float* bias;
+  int32_t* status;
+  int images, m;               // output channels
+  int sc, sh, sw;              // source channels and plane
+  int out_w, out_plane;
+  int step_y, step_x, base_y, base_x;   // source position of pixel (y, x) and tap t: y * step_y + base_y + dy[t], likewise x
+  int ostep_y, ostep_x;        // output position of pixel (y, x): y * ostep_y + oy0, likewise x
+  int vec;                     // four consecutive pixels are 16 aligned bytes of the output
+  ConvPhase phase[CV_MAX_PHASES];
+};
+struct ConvMaps {
+  CUtensorMap a[CV_MAX_PHASES];
+};
+
+__device__ __forceinline__ uint32_t rn_tf32(float x) {
+  uint32_t r;
+  asm("cvt.rn.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ void cv_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__host__ __device__ constexpr uint32_t cv_idesc() {   // kind::tf32, fp32 accumulator, both operands K-major, N = M = 128
+  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(CV_TILE >> 3) << 17) | ((uint32_t)(CV_TILE >> 4) << 24);
+}
+
+// The products of one stage: MT accumulators of 128 rows share the gathered tile.
+template <int MT>
+__device__ __forceinline__ void cv_issue(uint32_t tmem, uint32_t a_addr, uint32_t b_addr, int mts, bool first) {
+#pragma unroll
+  for (int mt = 0; mt < MT; mt++) {
+    if (mt >= mts) break;
+#pragma unroll
+    for (int ks = 0; ks < CV_BK / 8; ks++)
+      umma_tf32(tmem + mt * CV_TILE, make_desc(a_addr + mt * CV_BLOCK + ks * 32, 16, 1024, 2), make_desc(b_addr + ks * 32, 16, 1024, 2), cv_idesc(),
+                (!first || ks > 0) ? 1u : 0u);
+  }
+}
+
+// Turns this CTA's 128 x 128 accumulator into rows of CV_STG_LD floats in shared memory (the dead operand stages).
+__device__ __forceinline__ void cv_stage_rows(float* stg, uint32_t tmem, int warp, int lane, bool any) {
+  const int quad = warp & 3, half = warp >> 2;
+#pragma unroll
+  for (int c = 0; c < 2; c++) {
+    uint32_t r[32];
+    const int col = half * 64 + c * 32;
+    if (any) {
+      tmem_ld_32x32b_x32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)col, r);
+      tmem_ld_wait();
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; j++) r[j] = 0u;
+    }
+    float* dst = stg + (quad * 32 + lane) * CV_STG_LD + col;
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(dst + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+  }
+}
+
+// Eight channels of one tap for this lane's pixel. o: byte offset of the first (modulo 2^32), step: bytes of a plane.
+__device__ __forceinline__ void cv_load_unit(float* v, const float* __restrict__ src, uint32_t o, uint32_t step, int count) {
+#pragma unroll
+  for (int j = 0; j < CV_UNIT; j++) v[j] = 0.f;
+  const char* base = reinterpret_cast<const char*>(src);
+  if (count == CV_UNIT) {
+#pragma unroll
+    for (int j = 0; j < CV_UNIT; j++) {
+      v[j] = __ldg(reinterpret_cast<const float*>(base + o));
+      o += step;
+    }
+  } else if (count > 0) {        // the last channels
+#pragma unroll
+    for (int j = 0; j < CV_UNIT; j++) {
+      if (j < count) v[j] = __ldg(reinterpret_cast<const float*>(base + o));
+      o += step;
+    }
+  }
+}
+
+// ---- forward and input gradient ------------------------------------------------------------------------------------------
+// MT: 128-row accumulators per CTA; two (three stages become two, so that two CTAs still share an SM) halve the gathering
+// per product where there are more than 128 output channels and pixels enough to fill the device.
+template <int MT>
+__global__ void __launch_bounds__(CV_THREADS, 2)
+conv_tc_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvTcParams p) {
+  constexpr int STAGES = MT == 1 ? 3 : 2;
+  constexpr int STAGE_BYTES = (MT + 1) * CV_BLOCK;
+  constexpr uint32_t TMEM_COLS = MT * CV_TILE;
+  const ConvPhase& ph = p.phase[blockIdx.z];
+  const int plane = ph.ph * ph.pw;
+  const int pixels = p.images * plane;
+  const int q0 = blockIdx.x * CV_TILE;
+  if (q0 >= pixels) return;       // the classes of a strided gradient differ in size
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* empty = full + STAGES;
+  uint64_t* acc_full = empty + STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int2* units = reinterpret_cast<int2*>(smem + STAGES * STAGE_BYTES + 128);   // byte offset; tap | channels << 8
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m0 = blockIdx.y * (MT * CV_TILE);
+  const int mts = min(MT, (p.m - m0 + CV_TILE - 1) / CV_TILE);
+  const int k_blocks = (ph.units * CV_UNIT + CV_BK - 1) / CV_BK;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; s++) {
+      mbar_init(&full[s], 1 + CV_PRODUCERS);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(acc_full, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (int u = threadIdx.x; u < k_blocks * (CV_BK / CV_UNIT); u += CV_THREADS) {
+    int2 e = make_int2(0, 0);
+    if (u < ph.units) {
+      int t, c0;
+      cv_unit(u, p.sc, ph.taps, &t, &c0);
+      e.x = (int)(4u * (uint32_t)(c0 * p.sh * p.sw + ph.dy[t] * p.sw + ph.dx[t]));
+      e.y = t | (min(CV_UNIT, p.sc - c0) << 8);
+    }
+    units[u] = e;
+  }
+  if (warp == CV_PRODUCERS) {
+    tmem_alloc(tmem_slot, TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp < CV_PRODUCERS) {
+    // ---- gather: a thread owns a pixel and two of a stage's four units ----
+    const int half = warp >> 2;
+    const int px = (warp & 3) * 32 + lane;
+    const int q = q0 + px;
+    uint32_t mask = 0, base = 0;
+    if (q < pixels) {
+      const int n = cv_quot(q, ph.div_plane), r = q - n * plane;
+      const int y = cv_quot(r, ph.div_w), x = r - y * ph.pw;
+      const int y0 = y * p.step_y + p.base_y, x0 = x * p.step_x + p.base_x;
+      for (int t = 0; t < ph.taps; t++)
+        if ((unsigned)(y0 + ph.dy[t]) < (unsigned)p.sh && (unsigned)(x0 + ph.dx[t]) < (unsigned)p.sw) mask |= 1u << t;
+      base = 4u * ((uint32_t)n * (uint32_t)(p.sc * p.sh * p.sw) + (uint32_t)(y0 * p.sw + x0));
+    }
+    const uint32_t step = 4u * (uint32_t)(p.sh * p.sw);
+    auto fetch = [&](float (&v)[16], int kb) {
+      if (kb >= k_blocks) return;
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const int2 e = units[kb * 4 + half * 2 + i];
+        cv_load_unit(v + 8 * i, p.src, base + (uint32_t)e.x, step, (mask >> (e.y & 31)) & 1 ? e.y >> 8 : 0);
+      }
+    };
+    bool ok = true;
+    auto deposit = [&](const float (&v)[16], int kb) {
+      if (!ok || kb >= k_blocks) return;
+      const int s = kb % STAGES;
+      const uint32_t round = kb / STAGES;
+      if (round > 0) ok = __all_sync(0xffffffffu, mbar_wait(&empty[s], (round - 1) & 1, abort_flag, p.status, 71));
+      if (!ok) return;
+      uint8_t* row = smem + (size_t)s * STAGE_BYTES + MT * CV_BLOCK + px * 128;
+#pragma unroll
+      for (int c = 0; c < 4; c++)
+        *reinterpret_cast<uint4*>(row + (((half * 4 + c) ^ (px & 7)) << 4)) =
+            make_uint4(rn_tf32(v[4 * c]), rn_tf32(v[4 * c + 1]), rn_tf32(v[4 * c + 2]), rn_tf32(v[4 * c + 3]));
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) cv_arrive(&full[s]);
+    };
+    float v0[16], v1[16], v2[16];     // the loads of two blocks are in flight while one is stored
+    fetch(v0, 0);
+    fetch(v1, 1);
+    for (int kb = 0; kb < k_blocks && ok; kb += 3) {
+      fetch(v2, kb + 2);
+      deposit(v0, kb);
+      fetch(v0, kb + 3);
+      deposit(v1, kb + 1);
+      fetch(v1, kb + 4);
+      deposit(v2, kb + 2);
+    }
+    // ---- results: accumulator rows through shared memory to rows of consecutive pixels ----
+    if (k_blocks > 0) {
+      const bool done = mbar_wait(acc_full, 0, abort_flag, p.status, 72);
+      ok = __all_sync(0xffffffffu, done) && ok;
+    }
+    tc_fence_after();
+    float* stg = reinterpret_cast<float*>(smem);
+    long long at[4];               // output positions of this lane's pixels relative to their image's first channel; -1 past the end
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int qi = q0 + (p.vec ? 4 * lane : lane + 32 * i);
+      at[i] = -1;
+      if (qi < pixels) {
+        const int n = cv_quot(qi, ph.div_plane), r = qi - n * plane;
+        const int y = cv_quot(r, ph.div_w), x = r - y * ph.pw;
+        at[i] = (long long)n * p.m * p.out_plane + (y * p.ostep_y + ph.oy0) * p.out_w + x * p.ostep_x + ph.ox0;
+      }
+    }
+    for (int mt = 0; mt < mts; mt++) {
+      if (ok) cv_stage_rows(stg, tmem_base + mt * CV_TILE, warp, lane, k_blocks > 0);
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (ok) {
+#pragma unroll 4
+        for (int i = 0; i < 16; i++) {
+          const int row = warp * 16 + i, co = m0 + mt * CV_TILE + row;
+          if (co >= p.m) break;
+          const float bv = p.bias ? __ldg(p.bias + co) : 0.f;
+          float* out = p.out + (long long)co * p.out_plane;
+          const float* sr = stg + row * CV_STG_LD;
+          if (p.vec) {
+            if (at[0] >= 0) {
+              float4 v = *reinterpret_cast<const float4*>(sr + 4 * lane);
+              if (p.bias) { v.x += bv; v.y += bv; v.z += bv; v.w += bv; }
+              *reinterpret_cast<float4*>(out + at[0]) = v;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+              if (at[j] >= 0) out[at[j]] = p.bias ? sr[lane + 32 * j] + bv : sr[lane + 32 * j];
+          }
+        }
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+    }
+  } else if (warp == CV_PRODUCERS) {
+    if (lane == 0 && k_blocks > 0) {
+      for (int kb = 0; kb < k_blocks; kb++) {
+        const int s = kb % STAGES;
+        if (!mbar_wait(&full[s], (kb / STAGES) & 1, abort_flag, p.status, 73)) break;
+        tc_fence_after();
+        const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES);
+        cv_issue<MT>(tmem_base, a, a + MT * CV_BLOCK, mts, kb == 0);
+        umma_commit(&empty[s]);
+      }
+      umma_commit(acc_full);
+    }
+  } else if (lane == 0) {
+    for (int kb = 0; kb < k_blocks; kb++) {
+      const int s = kb % STAGES;
+      const uint32_t round = kb / STAGES;
+      if (round > 0 && !mbar_wait(&empty[s], (round - 1) & 1, abort_flag, p.status, 74)) break;
+      mbar_expect_tx(&full[s], (uint32_t)(mts * CV_BLOCK));
+      for (int mt = 0; mt < mts; mt++)
+        tma_load_4d(smem + (size_t)s * STAGE_BYTES + mt * CV_BLOCK, &maps.a[blockIdx.z], kb * CV_BK, m0 + mt * CV_TILE, 0, 0, &full[s]);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == CV_PRODUCERS) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, TMEM_COLS);
+  }
+}
+
+// The weights in the order of the units, one K-major row per output channel of the product: wt[phase][m][8 u + i] is the weight of
+// tap(u) and source channel c0(u) + i, zero past the last channel. Weights are addressed by their strides over (m, source channel).
+struct ConvTurn {
+  int m, sc;
+  long long stride_m, stride_sc;
+  int taps[CV_MAX_PHASES], ld[CV_MAX_PHASES];
+  long long start[CV_MAX_PHASES];
+  int tap[CV_MAX_PHASES][CV_MAX_TAPS];
+};
+__global__ void __launch_bounds__(256) conv_turn_weights_kernel(const float* __restrict__ w, float* __restrict__ wt, const __grid_constant__ ConvTurn t) {
+  const int z = blockIdx.z, m = blockIdx.y;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < t.ld[z]; i += gridDim.x * blockDim.x) {
+    int tap, c0;
+    cv_unit(i / CV_UNIT, t.sc, t.taps[z], &tap, &c0);
+    const int c = c0 + i % CV_UNIT;
+    wt[t.start[z] + (long long)m * t.ld[z] + i] = c < t.sc ? __ldg(w + m * t.stride_m + c * t.stride_sc + t.tap[z][tap]) : 0.f;
+  }
+}
+
+// ---- weight gradient -------------------------------------------------------------------------------------------------------
+struct ConvWgradParams {
+  const float* gr;
+  const float* x;
+  float* part;                 // [splits][cout][8 * units]
+  int32_t* status;
+  int cout, units, cin, h, w, kw, taps, sh, sw, pt, pl, dh, dw, ow, plane;
+  CvDiv div_plane, div_w;
+  int pixels;
+  int blocks_per_split;
+};
+
+// One CTA: 128 output channels x 128 columns (16 units of eight channels of a tap) over a slice of the pixels, 32 of them a stage. A lane
+// owns a pixel and a warp two units, so both operands are loaded along rows and written as whole 128-byte operand rows.
+// A_TMA: whole stages of the gradient come by TMA (planes of a multiple of 32 pixels); otherwise the warps load its rows too.
+template <bool A_TMA>
+__global__ void __launch_bounds__(CV_THREADS, 2)
+conv_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ ConvWgradParams p) {
+  constexpr int STAGES = 3;
+  constexpr int STAGE_BYTES = 2 * CV_BLOCK;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* empty = full + STAGES;
+  uint64_t* acc_full = empty + STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = blockIdx.x * CV_TILE, m0 = blockIdx.y * CV_TILE;
+  const int all_blocks = (p.pixels + CV_BK - 1) / CV_BK;
+  const int b0 = blockIdx.z * p.blocks_per_split;
+  const int k_blocks = min(p.blocks_per_split, all_blocks - b0);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; s++) {
+      mbar_init(&full[s], CV_PRODUCERS + (A_TMA ? 1 : 0));
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(acc_full, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == CV_PRODUCERS) {
+    tmem_alloc(tmem_slot, CV_TILE);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp < CV_PRODUCERS) {
+    bool ok = true;
+    const int row0 = warp * 16;
+    // This warp's two units (columns) and 16 output channels (rows): the same for every stage.
+    int dy[2] = {0, 0}, dx[2] = {0, 0}, count[2] = {0, 0};
+    uint32_t off[2] = {0, 0};
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const int u = (n0 + row0) / CV_UNIT + i;
+      if (u < p.units) {
+        int t, c0;
+        cv_unit(u, p.cin, p.taps, &t, &c0);
+        dy[i] = (t / p.kw) * p.dh - p.pt;
+        dx[i] = (t % p.kw) * p.dw - p.pl;
+        count[i] = min(CV_UNIT, p.cin - c0);
+        off[i] = 4u * (uint32_t)(c0 * p.h * p.w);
+      }
+    }
+    const uint32_t step = 4u * (uint32_t)(p.h * p.w), gstep = 4u * (uint32_t)p.plane;
+    const int rows = min(16, p.cout - m0 - row0);
+    auto fetch = [&](float (&vb)[16], float (&va)[A_TMA ? 1 : 16], int kb) {
+      if (kb >= k_blocks) return;
+      const int q = (b0 + kb) * CV_BK + lane;
+      const bool inside = q < p.pixels;
+      const int n = cv_quot(inside ? q : 0, p.div_plane), r = (inside ? q : 0) - n * p.plane;
+      const int oy = cv_quot(r, p.div_w), ox = r - oy * p.ow;
+      const uint32_t image = (uint32_t)n * (uint32_t)(p.cin * p.h * p.w);
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const int y = oy * p.sh + dy[i], x = ox * p.sw + dx[i];
+        const bool in = inside && (unsigned)y < (unsigned)p.h && (unsigned)x < (unsigned)p.w;
+        cv_load_unit(vb + 8 * i, p.x, off[i] + 4u * (image + (uint32_t)(y * p.w + x)), step, in ? count[i] : 0);
+      }
+      if (!A_TMA) {
+        const uint32_t o = 4u * (((uint32_t)n * (uint32_t)p.cout + (uint32_t)(m0 + row0)) * (uint32_t)p.plane + (uint32_t)r);
+        cv_load_unit(va, p.gr, o, gstep, inside ? max(0, min(CV_UNIT, rows)) : 0);
+        cv_load_unit(va + (A_TMA ? 0 : 8), p.gr, o + 8u * gstep, gstep, inside ? max(0, min(CV_UNIT, rows - CV_UNIT)) : 0);
+      }
+    };
+    auto deposit = [&](const float (&vb)[16], const float (&va)[A_TMA ? 1 : 16], int kb) {
+      if (!ok || kb >= k_blocks) return;
+      const int s = kb % STAGES;
+      const uint32_t round = kb / STAGES;
+      if (round > 0) ok = __all_sync(0xffffffffu, mbar_wait(&empty[s], (round - 1) & 1, abort_flag, p.status, 75));
+      if (!ok) return;
+      uint8_t* a = smem + (size_t)s * STAGE_BYTES;
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        const int at = (row0 + i) * 128 + (((lane >> 2) ^ (i & 7)) << 4) + (lane & 3) * 4;      // (row0 is a multiple of 8)
+        *reinterpret_cast<uint32_t*>(a + CV_BLOCK + at) = rn_tf32(vb[i]);
+        if (!A_TMA) *reinterpret_cast<uint32_t*>(a + at) = rn_tf32(va[A_TMA ? 0 : i]);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) cv_arrive(&full[s]);
+    };
+    float vb0[16], vb1[16], va0[A_TMA ? 1 : 16], va1[A_TMA ? 1 : 16];
+    fetch(vb0, va0, 0);
+    for (int kb = 0; kb < k_blocks && ok; kb += 2) {
+      fetch(vb1, va1, kb + 1);
+      deposit(vb0, va0, kb);
+      fetch(vb0, va0, kb + 2);
+      deposit(vb1, va1, kb + 1);
+    }
+    ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, p.status, 76)) && ok;
+    tc_fence_after();
+    float* stg = reinterpret_cast<float*>(smem);
+    if (ok) cv_stage_rows(stg, tmem_base, warp, lane, true);
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    if (ok) {
+      const int ld = p.units * CV_UNIT, col = n0 + 4 * lane;
+      float* out = p.part + (long long)blockIdx.z * p.cout * ld + col;
+      if (col < ld) {
+#pragma unroll 4
+        for (int i = 0; i < rows; i++)
+          *reinterpret_cast<float4*>(out + (long long)(m0 + row0 + i) * ld) = *reinterpret_cast<const float4*>(stg + (row0 + i) * CV_STG_LD + 4 * lane);
+      }
+    }
+  } else if (warp == CV_PRODUCERS) {
+    if (lane == 0) {
+      for (int kb = 0; kb < k_blocks; kb++) {
+        const int s = kb % STAGES;
+        if (!mbar_wait(&full[s], (kb / STAGES) & 1, abort_flag, p.status, 77)) break;
+        tc_fence_after();
+        const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES);
+        cv_issue<1>(tmem_base, a, a + CV_BLOCK, 1, kb == 0);
+        umma_commit(&empty[s]);
+      }
+      umma_commit(acc_full);
+    }
+  } else if (lane == 0 && A_TMA) {
+    for (int kb = 0; kb < k_blocks; kb++) {
+      const int s = kb % STAGES;
+      const uint32_t round = kb / STAGES;
+      if (round > 0 && !mbar_wait(&empty[s], (round - 1) & 1, abort_flag, p.status, 78)) break;
+      const int q = (b0 + kb) * CV_BK, n = cv_quot(q, p.div_plane);
+      mbar_expect_tx(&full[s], CV_BLOCK);
+      tma_load_4d(smem + (size_t)s * STAGE_BYTES, &map_g, q - n * p.plane, m0, n, 0, &full[s]);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == CV_PRODUCERS) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, CV_TILE);
+  }
+}
+
+// dW[co][c][tap] (+)= the slices' sums. A CTA: 32 unit columns of an output channel x 8 shares of the slices (share y takes slices
+// y, y + 8, ... in order), the shares added in order: with up to 296 slices one thread a value was a chain of as many loads.
+__global__ void __launch_bounds__(256)
+conv_wgrad_finish_kernel(const float* __restrict__ part, int splits, int cout, int units, int cin, int taps, float* __restrict__ dw, int accumulate) {
+  __shared__ float sums[8][32];
+  const int ld = units * CV_UNIT, lane = threadIdx.x & 31, share = threadIdx.x >> 5;
+  const int col = blockIdx.x * 32 + lane, co = blockIdx.y;
+  float acc = 0.f;
+  if (col < ld) {
+    const float* src = part + (long long)co * ld + col;
+    const long long stride = (long long)cout * ld;
+#pragma unroll 4
+    for (int s = share; s < splits; s += 8) acc += src[s * stride];
+  }
+  sums[share][lane] = acc;
+  __syncthreads();
+  if (share == 0 && col < ld) {
+    int t, c0;
+    cv_unit(col / CV_UNIT, cin, taps, &t, &c0);
+    const int c = c0 + col % CV_UNIT;
+    if (c >= cin) return;
+    for (int y = 1; y < 8 && y < splits; y++) acc += sums[y][lane];
+    float* dst = dw + ((long long)co * cin + c) * taps + t;
+    *dst = accumulate ? *dst + acc : acc;
+  }
+}
+
+// ---- host side -------------------------------------------------------------------------------------------------------------
+// K-major TF32 operand [rows, inner] (planes of them) with boxes of 32 x 128.
+static bool cv_map(CUtensorMap* map, const float* base, long long inner, long long rows, long long ld, long long count, long long stride) {
+  cuuint64_t dims[4] = {(cuuint64_t)inner, (cuuint64_t)rows, (cuuint64_t)count, 1};
+  const cuuint64_t filler = (((cuuint64_t)ld * rows * 4) + 15) & ~(cuuint64_t)15;
+  cuuint64_t strides[3] = {(cuuint64_t)ld * 4, count > 1 ? (cuuint64_t)stride * 4 : filler, filler};
+  cuuint32_t box[4] = {CV_BK, CV_TILE, 1, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  return encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_TFLOAT32, 4, const_cast<float*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Byte offsets into a tensor are 32-bit and pixels (with a tile's or a slice's overhang) 31-bit numbers, taps a 32-bit mask.
+static bool cv_sizes_fit(const ConvGeom& g) {
+  const long long in = (long long)g.n * g.cin * g.h * g.w, out = (long long)g.n * g.cout * g.oh * g.ow;
+  return g.groups == 1 && (long long)g.kh * g.kw <= CV_MAX_TAPS && in < (1ll << 30) && out < (1ll << 30) &&
+         (long long)g.n * g.oh * g.ow < (1ll << 30) && (long long)g.n * g.h * g.w < (1ll << 30) &&
+         (long long)g.cin * g.kh * g.kw <= 65535 && (long long)g.cout * g.kh * g.kw <= 65535 && g.n <= 65535 &&
+         (long long)(g.kh - 1) * g.dh * g.w + (long long)g.kw * g.dw + (long long)g.pt * g.w + g.pl < (1ll << 28);
+}
+
+template <int MT>
+static int32_t launch_conv_as(om_ctx* ctx, const ConvMaps& maps, const ConvTcParams& p, dim3 grid, int units) {
+  constexpr int STAGES = MT == 1 ? 3 : 2;
+  constexpr size_t stages = (size_t)STAGES * (MT + 1) * CV_BLOCK;
+  constexpr int most = 227 * 1024;
+  static_assert(stages >= (size_t)CV_TILE * CV_STG_LD * 4, "the result rows are staged in the operand stages");
+  static_assert(stages + 1024 + 128 + (65535 + CV_MAX_TAPS * CV_UNIT) / CV_UNIT * sizeof(int2) + 64 <= most, "every table of units fits");
+  const size_t smem = stages + 1024 + 128 + (size_t)((units + 3) & ~3) * sizeof(int2);
+  static bool set = false;
+  if (!set) {
+    OM_CUDA(ctx, cudaFuncSetAttribute(conv_tc_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    set = true;
+  }
+  conv_tc_kernel<MT><<<grid, CV_THREADS, smem, ctx->stream>>>(maps, p);
+  OM_LAUNCH_CHECK(ctx, "conv_tc");
+  return OM_OK;
+}
+
+// Turns the weights and runs the product of every phase. p holds all but the phases' divisors and units, turn the taps.
+static int32_t run_conv(om_ctx* ctx, ConvTcParams& p, ConvTurn& turn, int phases, const float* w) {
+  ConvMaps maps = {};
+  long long floats = 0, most = 0, all = 0;
+  int most_units = 0;
+  for (int z = 0; z < phases; z++) {
+    ConvPhase& f = p.phase[z];
+    f.div_plane = cv_div((uint32_t)std::max(1, f.ph * f.pw));
+    f.div_w = cv_div((uint32_t)std::max(1, f.pw));
+    f.units = cv_units(p.sc, f.taps);
+    turn.taps[z] = f.taps;
+    turn.ld[z] = f.units * CV_UNIT;
+    turn.start[z] = floats;
+    floats += (long long)turn.ld[z] * p.m;
+    most_units = std::max(most_units, f.units);
+    const long long tiles = ceil_div((long long)p.images * f.ph * f.pw, CV_TILE);
+    most = std::max(most, tiles);
+    all += tiles;
+  }
+  if (most == 0) return OM_OK;
+  float* wt = nullptr;
+  OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)std::max<long long>(floats, 4), false, (void**)&wt));
+  int32_t st = OM_OK;
+  for (int z = 0; z < phases && st == OM_OK; z++)
+    if (turn.ld[z] > 0 && !cv_map(&maps.a[z], wt + turn.start[z], turn.ld[z], p.m, turn.ld[z], 1, 0))
+      st = fail(ctx, OM_ERR_CUDA, "cuTensorMapEncodeTiled failed for a convolution's turned weights");
+  if (st == OM_OK) {
+    if (most_units > 0)
+      conv_turn_weights_kernel<<<dim3((unsigned)std::min<int64_t>(ceil_div(most_units * CV_UNIT, 256), 64), (unsigned)p.m, (unsigned)phases), 256, 0, ctx->stream>>>(
+          w, wt, turn);
+    // Two accumulators once that still leaves a CTA for every SM.
+    const bool two = p.m > CV_TILE && all * ceil_div(p.m, 2 * CV_TILE) >= 148;
+    const dim3 grid((unsigned)most, (unsigned)ceil_div(p.m, two ? 2 * CV_TILE : CV_TILE), (unsigned)phases);
+    st = two ? launch_conv_as<2>(ctx, maps, p, grid, most_units) : launch_conv_as<1>(ctx, maps, p, grid, most_units);
+  }
+  pool_free(ctx, wt);
+  return st;
+}
+
+bool conv_tc_fwd_fits(const ConvGeom& g) { return encode_fn() && cv_sizes_fit(g); }
+
+int32_t conv_tc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y) {
+  ConvTcParams p = {};
+  ConvTurn turn = {};
+  const int plane = g.oh * g.ow;
+  p.src = x; p.out = y; p.bias = bias; p.status = ctx->status_dev;
+  p.images = g.n; p.m = g.cout; p.sc = g.cin; p.sh = g.h; p.sw = g.w;
+  p.out_w = g.ow; p.out_plane = plane;
+  p.step_y = g.sh; p.step_x = g.sw; p.base_y = -g.pt; p.base_x = -g.pl;
+  p.ostep_y = p.ostep_x = 1;
+  p.vec = (plane & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+  ConvPhase& f = p.phase[0];
+  f.ph = g.oh; f.pw = g.ow; f.taps = g.kh * g.kw;
+  for (int t = 0; t < f.taps; t++) {
+    f.dy[t] = (t / g.kw) * g.dh;
+    f.dx[t] = (t % g.kw) * g.dw;
+    turn.tap[0][t] = t;
+  }
+  turn.m = g.cout; turn.sc = g.cin;
+  turn.stride_m = (long long)g.cin * f.taps; turn.stride_sc = f.taps;
+  return run_conv(ctx, p, turn, 1, w);
+}
+
+bool conv_tc_dgrad_fits(const ConvGeom& g) { return encode_fn() && cv_sizes_fit(g) && g.sh * g.sw <= CV_MAX_PHASES; }
+
+int32_t conv_tc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx) {
+  ConvTcParams p = {};
+  ConvTurn turn = {};
+  p.src = gr; p.out = dx; p.status = ctx->status_dev;
+  p.images = g.n; p.m = g.cin; p.sc = g.cout; p.sh = g.oh; p.sw = g.ow;
+  p.out_w = g.w; p.out_plane = g.h * g.w;
+  p.step_y = p.step_x = 1;
+  p.ostep_y = g.sh; p.ostep_x = g.sw;
+  p.vec = g.sh == 1 && g.sw == 1 && (p.out_plane & 3) == 0 && (reinterpret_cast<uintptr_t>(dx) & 15) == 0;
+  for (int z = 0; z < g.sh * g.sw; z++) {
+    ConvPhase& f = p.phase[z];
+    f.oy0 = z / g.sw;
+    f.ox0 = z % g.sw;
+    f.ph = f.oy0 < g.h ? (g.h - f.oy0 + g.sh - 1) / g.sh : 0;
+    f.pw = f.ox0 < g.w ? (g.w - f.ox0 + g.sw - 1) / g.sw : 0;
+    for (int t = 0; t < g.kh * g.kw; t++) {
+      const int ty = f.oy0 + g.pt - (t / g.kw) * g.dh, tx = f.ox0 + g.pl - (t % g.kw) * g.dw;
+      if (ty % g.sh || tx % g.sw) continue;      // (exact for negative values too)
+      f.dy[f.taps] = ty / g.sh;
+      f.dx[f.taps] = tx / g.sw;
+      turn.tap[z][f.taps++] = t;
+    }
+  }
+  turn.m = g.cin; turn.sc = g.cout;
+  turn.stride_m = g.kh * g.kw; turn.stride_sc = (long long)g.cin * g.kh * g.kw;
+  return run_conv(ctx, p, turn, g.sh * g.sw, w);
+}
+
+bool conv_tc_wgrad_fits(const ConvGeom& g) { return encode_fn() && cv_sizes_fit(g); }
+
+template <bool A_TMA>
+static int32_t launch_wgrad(om_ctx* ctx, const CUtensorMap& map, const ConvWgradParams& p, dim3 grid) {
+  constexpr size_t smem = (size_t)3 * 2 * CV_BLOCK + 1024 + 128;
+  static bool set = false;
+  if (!set) {
+    OM_CUDA(ctx, cudaFuncSetAttribute(conv_wgrad_tc_kernel<A_TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    set = true;
+  }
+  conv_wgrad_tc_kernel<A_TMA><<<grid, CV_THREADS, smem, ctx->stream>>>(map, p);
+  return OM_OK;
+}
+
+int32_t conv_tc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, float* dw, int accumulate) {
+  ConvWgradParams p = {};
+  p.gr = gr; p.x = x; p.status = ctx->status_dev;
+  p.cout = g.cout; p.cin = g.cin; p.h = g.h; p.w = g.w; p.kw = g.kw; p.taps = g.kh * g.kw; p.sh = g.sh; p.sw = g.sw;
+  p.pt = g.pt; p.pl = g.pl; p.dh = g.dh; p.dw = g.dw; p.ow = g.ow; p.plane = g.oh * g.ow;
+  p.units = cv_units(g.cin, p.taps);
+  p.div_plane = cv_div((uint32_t)p.plane);
+  p.div_w = cv_div((uint32_t)g.ow);
+  p.pixels = g.n * p.plane;
+  const bool a_tma = (p.plane & 31) == 0 && (reinterpret_cast<uintptr_t>(gr) & 15) == 0;
+  CUtensorMap map = {};
+  if (a_tma && !cv_map(&map, gr, p.plane, g.cout, p.plane, g.n, (long long)g.cout * p.plane))
+    return fail(ctx, OM_ERR_CUDA, "cuTensorMapEncodeTiled failed for a convolution's gradient");
+  // Slices of the pixels for one round of two CTAs an SM, each at least eight stages long: a function of the shape alone.
+  const int ld = p.units * CV_UNIT;
+  const int tn = (int)ceil_div(ld, CV_TILE), tm = (int)ceil_div(g.cout, CV_TILE);
+  const long long blocks = ceil_div(p.pixels, CV_BK);
+  int splits = (int)std::max<long long>(1, std::min<long long>(kSplitSlots / ((long long)tn * tm), blocks / 8));
+  p.blocks_per_split = (int)ceil_div(blocks, splits);
+  splits = (int)ceil_div(blocks, p.blocks_per_split);
+  OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)splits * g.cout * ld, false, (void**)&p.part));
+  const dim3 grid((unsigned)tn, (unsigned)tm, (unsigned)splits);
+  int32_t st = a_tma ? launch_wgrad<true>(ctx, map, p, grid) : launch_wgrad<false>(ctx, map, p, grid);
+  if (st == OM_OK)
+    conv_wgrad_finish_kernel<<<dim3((unsigned)ceil_div(ld, 32), (unsigned)g.cout), 256, 0, ctx->stream>>>(p.part, splits, g.cout, p.units, g.cin, p.taps, dw,
+                                                                                                        accumulate);
+  pool_free(ctx, p.part);
+  OM_TRY(st);
+  OM_LAUNCH_CHECK(ctx, "conv_wgrad_tc");
+  return OM_OK;
+}
+
+}  // namespace om

@@ -13,7 +13,7 @@
 //   forward  y_t [Cout, N*P] = W [Cout, K] * cols [K, N*P]          (then back to NCHW with the bias in the same pass)
 //   dgrad    dcols [K, N*P]  = W^T * g_t [Cout, N*P]                 (then the same col2im gather)
 //   wgrad    dW [Cout, K]    = g_t [Cout, N*P] * cols^T              (one product with k = N*P, fixed split of k)
-#include "om_common.cuh"
+#include "om_conv.cuh"
 
 namespace om {
 
@@ -27,10 +27,6 @@ bool gemm_tc_supported(om_ctx* ctx, int ta, int tb, int m, int n, int k, const f
                        int ldb, const float* C, int ldc);
 int32_t gemm_tc(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, const float* B, int ldb,
                 float* C, int ldc, int acc, const float* bias);
-
-struct ConvGeom {
-  int n, cin, h, w, cout, kh, kw, sh, sw, pt, pl, dh, dw, groups, oh, ow;
-};
 
 static bool conv_geom(const om_conv_shape* s, ConvGeom* g) {
   g->n = s->n; g->cin = s->cin; g->h = s->h; g->w = s->w; g->cout = s->cout; g->kh = s->kh; g->kw = s->kw;
@@ -535,7 +531,9 @@ int32_t om_conv2d_fwd(om_ctx* ctx, const om_conv_shape* s, const float* x, const
   const int cg = g.cin / g.groups, og = g.cout / g.groups, kk = cg * g.kh * g.kw, plane = g.oh * g.ow;
   if (g.n > 65535) return fail(ctx, OM_ERR_UNSUPPORTED, "om_conv2d_fwd: more than 65535 images in one call");
   ProfileScope prof(ctx, "om_conv2d_fwd", 2.0 * g.n * g.cout * (double)kk * plane, 4.0 * ((double)g.n * g.cin * g.h * g.w + (double)g.n * g.cout * plane));
-  if (conv_on_tensor_pipe(ctx, g, true)) {
+  const bool tensor_pipe = conv_on_tensor_pipe(ctx, g, true);
+  if (tensor_pipe && conv_tc_fwd_fits(g)) return conv_tc_fwd(ctx, g, x, w, bias, y);
+  if (tensor_pipe) {
     const int np = g.n * plane;
     float *cols = nullptr, *yt = nullptr;
     OM_TRY(unfold(ctx, g, x, &cols, true));
@@ -578,10 +576,12 @@ int32_t om_conv2d_dgrad(om_ctx* ctx, const om_conv_shape* s, const float* gr, co
   if (g.n > 65535) return fail(ctx, OM_ERR_UNSUPPORTED, "om_conv2d_dgrad: more than 65535 images in one call");
   const int cg = g.cin / g.groups, og = g.cout / g.groups, kk = cg * g.kh * g.kw, plane = g.oh * g.ow;
   ProfileScope prof(ctx, "om_conv2d_dgrad", 2.0 * g.n * g.cout * (double)kk * plane, 4.0 * ((double)g.n * g.cin * g.h * g.w + (double)g.n * g.cout * plane));
+  const bool tensor_pipe = conv_on_tensor_pipe(ctx, g, true);
+  if (tensor_pipe && conv_tc_dgrad_fits(g)) return conv_tc_dgrad(ctx, g, gr, w, dx);
   float* dcols = nullptr;
   int64_t total_cols = (int64_t)g.n * g.groups * kk * plane;
   OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)total_cols, false, (void**)&dcols));
-  if (conv_on_tensor_pipe(ctx, g, true)) {
+  if (tensor_pipe) {
     const int np = g.n * plane;
     float* gt = nullptr;
     int32_t st = to_cnhw(ctx, g, gr, &gt);
@@ -622,7 +622,9 @@ int32_t om_conv2d_wgrad(om_ctx* ctx, const om_conv_shape* s, const float* gr, co
     return OM_OK;
   }
   ProfileScope prof(ctx, "om_conv2d_wgrad", 2.0 * g.n * g.cout * (double)kk * plane, 4.0 * ((double)g.n * g.cin * g.h * g.w + (double)g.n * g.cout * plane));
-  if (conv_on_tensor_pipe(ctx, g, false)) {
+  const bool tensor_pipe = conv_on_tensor_pipe(ctx, g, false);
+  if (tensor_pipe && conv_tc_wgrad_fits(g)) return conv_tc_wgrad(ctx, g, gr, x, dw, accumulate);
+  if (tensor_pipe) {
     const int np = g.n * plane;
     float *cols = nullptr, *gt = nullptr;
     OM_TRY(unfold(ctx, g, x, &cols, true));

@@ -80,3 +80,72 @@ def test_attention_masks_of_every_alignment(ctx, K, tf32, b, h, lq, lk, d, batch
                 assert scaled_diff(got.numpy(), want) <= (2e-3 if tf32 else 1e-4)
     finally:
         ctx.set_flags(0)
+
+
+class ConvShape(C.Structure):
+    _fields_ = [(n, C.c_int32) for n in ("n", "cin", "h", "w", "cout", "kh", "kw", "stride_h", "stride_w", "pad_top", "pad_left",
+                                         "pad_bottom", "pad_right", "dil_h", "dil_w", "groups")]
+
+
+def to_tf32(a):
+    """Round to nearest even at 10 mantissa bits."""
+    u = a.view(np.uint32).astype(np.uint64)
+    return ((u + 0xFFF + ((u >> 13) & 1)) & ~np.uint64(0x1FFF)).astype(np.uint32).view(np.float32)
+
+
+def conv_case(n, cin, h, w, cout, kh, kw, sh, sw, pads, dh, dw, seed=0):
+    """Geometry, TF32-valued operands and the exact results (float64 PyTorch on the CPU)."""
+    import torch
+    pt, pl, pb, pr = pads
+    s = ConvShape(n, cin, h, w, cout, kh, kw, sh, sw, pt, pl, pb, pr, dh, dw, 1)
+    x, wt, b = to_tf32(normal(seed, n, cin, h, w)), to_tf32(normal(seed + 1, cout, cin, kh, kw, scale=0.2)), normal(seed + 2, cout)
+    xt, wtt = (torch.from_numpy(a).double().requires_grad_(True) for a in (x, wt))
+    y = torch.nn.functional.conv2d(torch.nn.functional.pad(xt, (pl, pr, pt, pb)), wtt, torch.from_numpy(b).double(), (sh, sw), 0, (dh, dw))
+    g = to_tf32(normal(seed + 3, *y.shape))
+    y.backward(torch.from_numpy(g).double())
+    return s, x, wt, b, g, y.detach().numpy(), xt.grad.numpy(), wtt.grad.numpy()
+
+
+def run_conv(ctx, s, x, wt, b, g):
+    X, W, B, G = (ctx.to_device(a) for a in (x, wt, b, g))
+    Y, DX, DW = ctx.empty(g.shape), ctx.empty(x.shape), ctx.empty(wt.shape)
+    ctx.call("om_conv2d_fwd", ctx.handle, C.byref(s), X.ptr, W.ptr, B.ptr, Y.ptr)
+    ctx.call("om_conv2d_dgrad", ctx.handle, C.byref(s), G.ptr, W.ptr, DX.ptr)
+    ctx.call("om_conv2d_wgrad", ctx.handle, C.byref(s), G.ptr, X.ptr, DW.ptr, i32(0))
+    first = DW.numpy().copy()
+    ctx.call("om_conv2d_wgrad", ctx.handle, C.byref(s), G.ptr, X.ptr, DW.ptr, i32(1))
+    ctx.sync()
+    return Y.numpy(), DX.numpy(), first, DW.numpy()
+
+
+CONV_EDGES = [
+    # n, cin, h, w, cout, kh, kw, sh, sw, (top, left, bottom, right), dh, dw
+    (2, 4, 8, 8, 5, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1),            # one ragged tile of everything
+    (4, 8, 5, 7, 130, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1),          # planes off the 16-byte grid, a second block of channels
+    (20, 8, 32, 32, 200, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1),       # two accumulators, the second ragged
+    (20, 8, 32, 32, 384, 1, 1, 1, 1, (0, 0, 0, 0), 1, 1),       # two accumulators, then one
+    (4, 12, 9, 11, 20, 3, 3, 2, 2, (1, 1, 1, 1), 1, 1),         # classes of a strided gradient of different sizes
+    (4, 16, 8, 6, 12, 1, 1, 2, 2, (0, 0, 0, 0), 1, 1),          # classes that no tap reaches
+    (4, 8, 13, 10, 12, 3, 2, 1, 2, (2, 0, 1, 1), 1, 1),         # strides and pads of their own
+    (4, 4, 20, 18, 9, 5, 5, 1, 1, (4, 4, 4, 4), 2, 2),          # dilation, 25 taps
+    (4, 4, 12, 12, 9, 4, 8, 2, 1, (1, 3, 2, 4), 1, 1),          # 32 taps
+    (4, 4, 12, 12, 9, 6, 6, 1, 1, (2, 2, 2, 2), 1, 1),          # 36 taps: the unfolded matrix
+    (4, 4, 14, 14, 9, 3, 3, 3, 3, (1, 1, 1, 1), 1, 1),          # nine classes: the unfolded matrix for the input gradient
+    (3, 4, 64, 4, 136, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1),         # planes of whole stages: the gradient by TMA
+    (64, 160, 4, 4, 144, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1),       # several column tiles, planes of half a stage
+]
+
+
+@pytest.mark.parametrize("case", CONV_EDGES)
+def test_conv2d_without_an_unfolded_matrix(ctx, case):
+    """TF32-valued operands, so that only the order of the fp32 sums is left: 2e-5 scaled, the gate of the plain products."""
+    s, x, wt, b, g, y, dx, dw = conv_case(*case)
+    ctx.set_flags(omb.OM_TF32)
+    try:
+        Y, DX, DW, DW2 = run_conv(ctx, s, x, wt, b, g)
+    finally:
+        ctx.set_flags(0)
+    assert scaled_diff(Y, y) <= 2e-5
+    assert scaled_diff(DX, dx) <= 2e-5
+    assert scaled_diff(DW, dw) <= 2e-5
+    assert scaled_diff(DW2, 2 * dw) <= 2e-5
