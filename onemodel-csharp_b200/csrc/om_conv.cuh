@@ -1,4 +1,4 @@
-// Geometry of a 2-D convolution, shared by the unfolding path (om_spatial.cu), the tensor-pipe kernels (om_conv_tc.cu).
+// Geometry of a 2-D convolution, shared by the unfolding path (om_spatial.cu), the kernels of om_conv_tc.cu and om_conv_fma.cu.
 #pragma once
 #include "om_common.cuh"
 
@@ -16,5 +16,13 @@ bool conv_tc_dgrad_fits(const ConvGeom& g);
 int32_t conv_tc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx);
 bool conv_tc_wgrad_fits(const ConvGeom& g);
 int32_t conv_tc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, float* dw, int accumulate);
+
+// The fp32 products of small shapes without an unfolded matrix (om_conv_fma.cu).
+bool conv_fma_fwd_fits(const ConvGeom& g);
+int32_t conv_fma_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y);
+bool conv_fma_dgrad_fits(const ConvGeom& g);
+int32_t conv_fma_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx);
+bool conv_fma_wgrad_fits(const ConvGeom& g);
+int32_t conv_fma_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, float* dw, int accumulate);
 
 }  // namespace om

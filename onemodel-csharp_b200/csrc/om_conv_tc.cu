@@ -506,28 +506,34 @@ conv_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
   }
 }
 
-// dW[co][c][tap] (+)= the slices' sums. A CTA: 32 unit columns of an output channel x 8 shares of the slices (share y takes slices
-// y, y + 8, ... in order), the shares added in order: with up to 296 slices one thread a value was a chain of as many loads.
+// dW[co][c][tap] (+)= the slices' sums. A CTA: 256 / SHARES unit columns of an output channel x SHARES shares of the slices (share y
+// takes slices y, y + SHARES, ... in order), the shares added in order. Eight shares for many slices: with up to 296 of them one
+// thread a value is a chain of as many loads (21 us against 5). One share for a few: 512 x 4608 weights in two slices took 67 us
+// with eight, most of whose threads had nothing to add.
+template <int SHARES>
 __global__ void __launch_bounds__(256)
 conv_wgrad_finish_kernel(const float* __restrict__ part, int splits, int cout, int units, int cin, int taps, float* __restrict__ dw, int accumulate) {
-  __shared__ float sums[8][32];
-  const int ld = units * CV_UNIT, lane = threadIdx.x & 31, share = threadIdx.x >> 5;
-  const int col = blockIdx.x * 32 + lane, co = blockIdx.y;
+  constexpr int COLS = 256 / SHARES;
+  __shared__ float sums[SHARES][COLS];
+  const int ld = units * CV_UNIT, lane = threadIdx.x % COLS, share = threadIdx.x / COLS;
+  const int col = blockIdx.x * COLS + lane, co = blockIdx.y;
   float acc = 0.f;
   if (col < ld) {
     const float* src = part + (long long)co * ld + col;
     const long long stride = (long long)cout * ld;
 #pragma unroll 4
-    for (int s = share; s < splits; s += 8) acc += src[s * stride];
+    for (int s = share; s < splits; s += SHARES) acc += src[s * stride];
   }
-  sums[share][lane] = acc;
-  __syncthreads();
+  if (SHARES > 1) {
+    sums[share][lane] = acc;
+    __syncthreads();
+  }
   if (share == 0 && col < ld) {
     int t, c0;
     cv_unit(col / CV_UNIT, cin, taps, &t, &c0);
     const int c = c0 + col % CV_UNIT;
     if (c >= cin) return;
-    for (int y = 1; y < 8 && y < splits; y++) acc += sums[y][lane];
+    for (int y = 1; y < SHARES && y < splits; y++) acc += sums[y][lane];
     float* dst = dw + ((long long)co * cin + c) * taps + t;
     *dst = accumulate ? *dst + acc : acc;
   }
@@ -702,9 +708,14 @@ int32_t conv_tc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const flo
   OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)splits * g.cout * ld, false, (void**)&p.part));
   const dim3 grid((unsigned)tn, (unsigned)tm, (unsigned)splits);
   int32_t st = a_tma ? launch_wgrad<true>(ctx, map, p, grid) : launch_wgrad<false>(ctx, map, p, grid);
-  if (st == OM_OK)
-    conv_wgrad_finish_kernel<<<dim3((unsigned)ceil_div(ld, 32), (unsigned)g.cout), 256, 0, ctx->stream>>>(p.part, splits, g.cout, p.units, g.cin, p.taps, dw,
-                                                                                                        accumulate);
+  if (st == OM_OK) {
+    if (splits <= 8)
+      conv_wgrad_finish_kernel<1><<<dim3((unsigned)ceil_div(ld, 256), (unsigned)g.cout), 256, 0, ctx->stream>>>(p.part, splits, g.cout, p.units, g.cin, p.taps, dw,
+                                                                                                             accumulate);
+    else
+      conv_wgrad_finish_kernel<8><<<dim3((unsigned)ceil_div(ld, 32), (unsigned)g.cout), 256, 0, ctx->stream>>>(p.part, splits, g.cout, p.units, g.cin, p.taps, dw,
+                                                                                                            accumulate);
+  }
   pool_free(ctx, p.part);
   OM_TRY(st);
   OM_LAUNCH_CHECK(ctx, "conv_wgrad_tc");

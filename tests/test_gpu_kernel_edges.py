@@ -149,3 +149,26 @@ def test_conv2d_without_an_unfolded_matrix(ctx, case):
     assert scaled_diff(DX, dx) <= 2e-5
     assert scaled_diff(DW, dw) <= 2e-5
     assert scaled_diff(DW2, 2 * dw) <= 2e-5
+
+
+@pytest.mark.parametrize("tf32", [0, 1])
+@pytest.mark.parametrize("case", [
+    (3, 3, 45, 51, 24, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1), (3, 24, 11, 13, 48, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1),
+    (1, 1, 9, 7, 33, 3, 3, 2, 2, (1, 1, 1, 1), 1, 1), (2, 33, 7, 9, 64, 1, 1, 1, 1, (0, 0, 0, 0), 1, 1),
+    (3, 32, 5, 5, 65, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1),      # the weight and input gradients on the unfolded matrix
+    (3, 33, 5, 5, 7, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1),       # 297 terms: forward and weight gradient on the unfolded matrix
+    (1, 2, 11, 10, 5, 4, 8, 2, 1, (1, 3, 2, 4), 2, 1)] + [c for c in CONV_EDGES if c[0] == 4])
+def test_conv2d_on_the_fma_pipe(ctx, case, tf32):
+    """fp32 products without an unfolded matrix where they are small, in both tiers (with TF32 asked for: planes off the 16-byte
+    grid). The operands are TF32 values, so every path is held to the fp32 gates: 1e-6 a short sum, 1e-5 a sum over pixels."""
+    s, x, wt, b, g, y, dx, dw = conv_case(*case)
+    ctx.set_flags(omb.OM_TF32 if tf32 else 0)
+    try:
+        Y, DX, DW, DW2 = run_conv(ctx, s, x, wt, b, g)
+    finally:
+        ctx.set_flags(0)
+    tc = tf32 and (s.n * y.shape[2] * y.shape[3]) % 4 == 0
+    assert scaled_diff(Y, y) <= (2e-5 if tc else 1e-6)
+    assert scaled_diff(DX, dx) <= (2e-5 if tc else 1e-6)
+    assert scaled_diff(DW, dw) <= (2e-5 if tc else 1e-5)
+    assert scaled_diff(DW2, 2 * dw) <= (2e-5 if tc else 1e-5)
