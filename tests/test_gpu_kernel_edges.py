@@ -172,3 +172,24 @@ def test_conv2d_on_the_fma_pipe(ctx, case, tf32):
     assert scaled_diff(DX, dx) <= (2e-5 if tc else 1e-6)
     assert scaled_diff(DW, dw) <= (2e-5 if tc else 1e-5)
     assert scaled_diff(DW2, 2 * dw) <= (2e-5 if tc else 1e-5)
+
+
+def test_ctc_chains_and_classes_are_bit_exact(ctx, K):
+    """Extended targets of more positions than a CTA has threads, repeated labels, an empty target, more labels than steps, no steps, and a
+    number of steps whose rows no longer fit on the chip: the reference's doubles bit for bit."""
+    r = np.random.default_rng(4)
+    for t, c, tl, il in ((150, 7, [70, 0, 3, 149, 2], [150, 150, 2, 150, 0]), (1300, 5, [90, 1], [1300, 640])):
+        tl, il = np.array(tl, np.int32), np.array(il, np.int32)
+        b = len(tl)
+        z = r.standard_normal((t, b, c))
+        lp = (z - np.log(np.exp(z).sum(-1, keepdims=True))).astype(np.float32)
+        tg = r.integers(1, c, int(tl.sum())).astype(np.int32)
+        for red in (0, 1, 2):
+            g = normal(red, b if red == 0 else 1)
+            LP, TG, TL, IL, G = (ctx.to_device(a) for a in (lp, tg, tl, il, g))
+            NLL, L, GR = ctx.empty((b,)), ctx.empty(()), ctx.empty(lp.shape)
+            ctx.call("om_ctc_loss", ctx.handle, LP.ptr, i32(t), i32(b), i32(c), TG.ptr, TL.ptr, IL.ptr, i32(0), i32(red), i32(1), NLL.ptr, L.ptr)
+            ctx.call("om_ctc_grad", ctx.handle, G.ptr, LP.ptr, i32(t), i32(b), i32(c), TG.ptr, TL.ptr, IL.ptr, None, i32(0), i32(red), i32(1), GR.ptr)
+            ctx.sync()
+            assert np.array_equal(NLL.numpy(), K.ctc_loss(lp, tg, tl, il, 0, red, True)[1])
+            assert np.array_equal(GR.numpy(), K.ctc_grad(g, lp, tg, tl, il, 0, red))
