@@ -8,6 +8,9 @@ namespace om {
 void splitk_reduce_launch(om_ctx* ctx, const float* part, int splits, int64_t mn, int n, int64_t ldc, const float* bias, float* out, int accumulate);
 int32_t gemm_simt(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, int64_t sA,
                   const float* B, int ldb, int64_t sB, float* C, int ldc, int64_t sC, int batch, int acc);
+bool gemm_simt_takes_bias(int m, int n);
+int32_t gemm_simt_bias(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, const float* B, int ldb, float* C, int ldc,
+                       int acc, const float* bias);
 bool gemm_tc_supported(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, const float* B,
                        int ldb, const float* C, int ldc);
 int32_t gemm_tc(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, const float* B, int ldb,
@@ -73,6 +76,7 @@ int32_t gemm_dispatch(om_ctx* ctx, int ta, int tb, int m, int n, int k, const fl
       return st;
     }
   }
+  if (bias && gemm_simt_takes_bias(m, n)) return gemm_simt_bias(ctx, ta, tb, m, n, k, A, lda, B, ldb, C, ldc, acc, bias);
   OM_TRY(gemm_simt(ctx, ta, tb, m, n, k, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, acc));
   if (bias) {
     add_bias_rows_kernel<<<grid_for(ctx, ((int64_t)m * n + 3) / 4, 256), 256, 0, ctx->stream>>>(C, bias, m, n, ldc);

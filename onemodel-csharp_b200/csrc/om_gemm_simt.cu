@@ -116,6 +116,78 @@ gemm_simt_kernel(int m, int n, int k, const float* __restrict__ A, int lda, int6
   }
 }
 
+// Small results: one output element per thread, 16 x 16 a CTA, so that even a 16 x 128 layer spreads over eight CTAs, and the next 64 k's
+// are on their way from memory while these are multiplied (the tiles of 64 x 64 wait for every 16 of them: 8 to 17 us for 16 rows
+// and 64 to 128 k's, 17.6 us for 10 x 512 over 128 k's). Latency bounds it: the chain of one accumulator, and one round trip to
+// memory. The same chain of fmaf per element, so the bits do not depend on which kernel ran. A bias is added to the finished sum.
+constexpr int kSmallTile = 16, kSmallK = 64;
+// The line: four CTAs an SM on 148 SMs. Up to there a k costs the load/store unit no more than one 64 x 64 tile an SM does.
+constexpr int64_t kSmallOutputs = (int64_t)4 * 148 * kSmallTile * kSmallTile;
+
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(kSmallTile * kSmallTile)
+gemm_small_kernel(int m, int n, int k, const float* __restrict__ A, int lda, int64_t strideA, const float* __restrict__ B, int ldb,
+                  int64_t strideB, float* __restrict__ C, int ldc, int64_t strideC, int accumulate, int inner, int64_t innerA,
+                  int64_t innerB, int64_t innerC, const float* __restrict__ bias) {
+  __shared__ __align__(16) float As[kSmallTile][kSmallK + 4];
+  __shared__ __align__(16) float Bs[kSmallTile][kSmallK + 4];
+  constexpr int THREADS = kSmallTile * kSmallTile, LOADS = kSmallTile * kSmallK / THREADS;
+  const int zo = blockIdx.z / inner, zi = blockIdx.z % inner;
+  A += zo * strideA + zi * innerA;
+  B += zo * strideB + zi * innerB;
+  C += zo * strideC + zi * innerC;
+  const int tid = threadIdx.x, tx = tid % kSmallTile, ty = tid / kSmallTile;
+  const int m0 = blockIdx.y * kSmallTile, n0 = blockIdx.x * kSmallTile;
+  float ra[LOADS], rb[LOADS];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < LOADS; i++) {
+      const int e = tid + i * THREADS;
+      // consecutive threads walk the index that is contiguous in memory
+      const int am = m0 + (TA ? e % kSmallTile : e / kSmallK), ak = k0 + (TA ? e / kSmallTile : e % kSmallK);
+      const int bn = n0 + (TB ? e / kSmallK : e % kSmallTile), bk = k0 + (TB ? e % kSmallK : e / kSmallTile);
+      ra[i] = am < m && ak < k ? __ldg(A + (TA ? (int64_t)ak * lda + am : (int64_t)am * lda + ak)) : 0.f;
+      rb[i] = bn < n && bk < k ? __ldg(B + (TB ? (int64_t)bn * ldb + bk : (int64_t)bk * ldb + bn)) : 0.f;
+    }
+  };
+  float acc = 0.f;
+  fetch(0);
+  for (int k0 = 0; k0 < k; k0 += kSmallK) {
+#pragma unroll
+    for (int i = 0; i < LOADS; i++) {
+      const int e = tid + i * THREADS;
+      As[TA ? e % kSmallTile : e / kSmallK][TA ? e / kSmallTile : e % kSmallK] = ra[i];
+      Bs[TB ? e / kSmallK : e % kSmallTile][TB ? e % kSmallK : e / kSmallTile] = rb[i];
+    }
+    __syncthreads();
+    if (k0 + kSmallK < k) fetch(k0 + kSmallK);
+    const int kmax = min(kSmallK, k - k0);
+    const float *a = As[ty], *b = Bs[tx];
+    if (kmax == kSmallK) {
+#pragma unroll
+      for (int kk = 0; kk < kSmallK; kk += 4) {
+        const float4 av = *reinterpret_cast<const float4*>(a + kk), bv = *reinterpret_cast<const float4*>(b + kk);
+        acc = fmaf(av.x, bv.x, acc);
+        acc = fmaf(av.y, bv.y, acc);
+        acc = fmaf(av.z, bv.z, acc);
+        acc = fmaf(av.w, bv.w, acc);
+      }
+    } else {
+      for (int kk = 0; kk < kmax; kk++) acc = fmaf(a[kk], b[kk], acc);   // (the padding must not enter the sum)
+    }
+    __syncthreads();
+  }
+  const int gm = m0 + ty, gn = n0 + tx;
+  if (gm < m && gn < n) {
+    float* c = C + (int64_t)gm * ldc + gn;
+    float v = accumulate ? *c + acc : acc;
+    if (bias) v += __ldg(bias + gn);
+    *c = v;
+  }
+}
+
+bool gemm_simt_takes_bias(int m, int n) { return (int64_t)m * n <= kSmallOutputs; }
+
 template <int BM, int BN, int BK, int TM, int TN>
 static void launch_simt(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, int64_t sA,
                         const float* B, int ldb, int64_t sB, float* C, int ldc, int64_t sC, int batch, int acc, int bpz = 0,
@@ -128,11 +200,23 @@ static void launch_simt(om_ctx* ctx, int ta, int tb, int m, int n, int k, const 
   else gemm_simt_kernel<BM, BN, BK, TM, TN, true, true><<<grid, T, 0, ctx->stream>>>(m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, acc, batch, bpz, inner, iA, iB, iC);
 }
 
-int32_t gemm_simt_heads(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, int64_t sA, int64_t iA,
-                        const float* B, int ldb, int64_t sB, int64_t iB, float* C, int ldc, int64_t sC, int64_t iC, int batch,
-                        int inner, int acc) {
+static int32_t gemm_simt_any(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, int64_t sA, int64_t iA,
+                             const float* B, int ldb, int64_t sB, int64_t iB, float* C, int ldc, int64_t sC, int64_t iC, int batch,
+                             int inner, int acc, const float* bias) {
   if (m == 0 || n == 0 || batch == 0) return OM_OK;
   if (inner < 1) inner = 1;
+  if ((int64_t)m * n * batch <= kSmallOutputs && batch <= 65535) {
+    const dim3 grid((unsigned)ceil_div(n, kSmallTile), (unsigned)ceil_div(m, kSmallTile), (unsigned)batch);
+#define OM_SMALL(TA, TB) \
+  gemm_small_kernel<TA, TB><<<grid, kSmallTile * kSmallTile, 0, ctx->stream>>>(m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, acc, inner, iA, iB, iC, bias)
+    if (!ta && !tb) OM_SMALL(false, false);
+    else if (!ta) OM_SMALL(false, true);
+    else if (!tb) OM_SMALL(true, false);
+    else OM_SMALL(true, true);
+#undef OM_SMALL
+    OM_LAUNCH_CHECK(ctx, "gemm_small");
+    return OM_OK;
+  }
   int64_t tiles128 = ceil_div(m, 128) * ceil_div(n, 128) * batch;
   if (tiles128 >= ctx->sm_count) {
     launch_simt<128, 128, 16, 8, 8>(ctx, ta, tb, m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, acc, 0, inner, iA, iB, iC);
@@ -145,7 +229,19 @@ int32_t gemm_simt_heads(om_ctx* ctx, int ta, int tb, int m, int n, int k, const 
 
 int32_t gemm_simt(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, int64_t sA,
                   const float* B, int ldb, int64_t sB, float* C, int ldc, int64_t sC, int batch, int acc) {
-  return gemm_simt_heads(ctx, ta, tb, m, n, k, A, lda, sA, 0, B, ldb, sB, 0, C, ldc, sC, 0, batch, 1, acc);
+  return gemm_simt_any(ctx, ta, tb, m, n, k, A, lda, sA, 0, B, ldb, sB, 0, C, ldc, sC, 0, batch, 1, acc, nullptr);
+}
+
+int32_t gemm_simt_heads(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, int64_t sA, int64_t iA,
+                        const float* B, int ldb, int64_t sB, int64_t iB, float* C, int ldc, int64_t sC, int64_t iC, int batch,
+                        int inner, int acc) {
+  return gemm_simt_any(ctx, ta, tb, m, n, k, A, lda, sA, iA, B, ldb, sB, iB, C, ldc, sC, iC, batch, inner, acc, nullptr);
+}
+
+// One product with a bias over its columns (only where gemm_simt_takes_bias says so).
+int32_t gemm_simt_bias(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, const float* B, int ldb, float* C, int ldc,
+                       int acc, const float* bias) {
+  return gemm_simt_any(ctx, ta, tb, m, n, k, A, lda, 0, 0, B, ldb, 0, 0, C, ldc, 0, 0, 1, 1, acc, bias);
 }
 
 // Sums the products of `batch` matrix pairs in chunks of batch_per_chunk: partial[c] = sum over the chunk's matrices

@@ -193,3 +193,22 @@ def test_ctc_chains_and_classes_are_bit_exact(ctx, K):
             ctx.sync()
             assert np.array_equal(NLL.numpy(), K.ctc_loss(lp, tg, tl, il, 0, red, True)[1])
             assert np.array_equal(GR.numpy(), K.ctc_grad(g, lp, tg, tl, il, 0, red))
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("m,n,k", [(16, 16, 64), (17, 15, 65), (1, 1, 1), (16, 128, 63), (10, 512, 128), (389, 389, 129), (4 * 148 * 16, 16, 3), (4 * 148 * 16 + 1, 16, 3)])
+def test_small_fp32_products_are_bit_exact(ctx, K, ta, tb, m, n, k):
+    """Either side of the line between one output a thread and tiles of 64 x 64, ragged tiles and k's: the scalar chain's bits,
+    with and without a bias, accumulating or not."""
+    ctx.set_flags(0)
+    a, b = normal(m + k, *((k, m) if ta else (m, k))), normal(n + 3 * k, *((n, k) if tb else (k, n)))
+    A, B, Cm = ctx.to_device(a), ctx.to_device(b), ctx.empty((m, n))
+    ref = K.gemm(a, b, bool(ta), bool(tb))
+    for acc in (0, 1):
+        ctx.call("om_matmul", ctx.handle, i32(ta), i32(tb), i32(m), i32(n), i32(k), A.ptr, i32(a.shape[1]), B.ptr, i32(b.shape[1]), Cm.ptr, i32(n), i32(acc))
+        assert np.array_equal(Cm.numpy(), ref + ref if acc else ref)
+    if not ta and tb:
+        bias = normal(9, n)
+        Bv = ctx.to_device(bias)
+        ctx.call("om_linear_fwd", ctx.handle, A.ptr, B.ptr, Bv.ptr, i32(m), i32(k), i32(n), Cm.ptr)
+        assert np.array_equal(Cm.numpy(), ref + bias)
