@@ -5,12 +5,12 @@
 // few microseconds of work and the sequence is bound by launch and dependency latency. Here the work of a step is
 // tiled over CTAs as (16 hidden units) x (a group of batch rows): a CTA keeps the rows (forward) or columns (backward)
 // of W_hh that belong to its units in shared memory for the whole sequence, and per step brings in only the previous
-// state (forward: h, 16 rows x H) or the gate gradients (backward: 16 rows x 4H) of its own batch rows, computes with
-// fp32 FMAs from shared memory, applies the cell, and meets the CTAs that share its batch rows (the other unit slices)
-// at a barrier, once per time step. CTAs of different row groups and directions never wait for one another.
+// state (forward: h, 16 rows x H) or the shares of its units' state gradient (backward: 16 rows x 16 units from H / 16
+// slices) of its own batch rows, computes with fp32 FMAs from shared memory, applies the cell, and meets the CTAs that
+// share its batch rows (the other unit slices) at a barrier, once per time step. CTAs of different row groups and directions never wait for one another.
 //
 // Arithmetic: fp32 throughout (more accurate than the TF32 product of the step-by-step fast path). A dot product is
-// split in two (forward) or eight (backward) k ranges summed in a fixed order, so results do not depend on scheduling;
+// split in eight (forward) or 2 H / 16 (backward) k ranges summed in a fixed order, so results do not depend on scheduling;
 // they are not the one-accumulator order of the reference's exact tier, which stays on the step-by-step path.
 //
 // CTAs wait on one another, so the launch is cooperative (all CTAs resident at once; the host checks the occupancy
@@ -52,11 +52,31 @@ __device__ __forceinline__ bool seq_barrier(unsigned* counter, unsigned target, 
   return *failed == 0;
 }
 
+// Copies rows r0 .. r0 + 15 of src [B, 4 * q4] (written by other CTAs of this launch: past L1) into rows of ld floats, zero beyond B; the loads
+// of four rounds are in flight together.
+__device__ __forceinline__ void seq_stage_rows(float* dst, int ld, const float* src, int r0, int B, int q4, int tid) {
+  for (int base = tid; base < kSeqRows * q4; base += 4 * kSeqThreads) {
+    float4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int idx = base + i * kSeqThreads, r = idx / q4, b = r0 + r;
+      v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (idx < kSeqRows * q4 && b < B) v[i] = __ldcg(reinterpret_cast<const float4*>(src + (size_t)b * 4 * q4) + (idx - r * q4));
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int idx = base + i * kSeqThreads, r = idx / q4;
+      if (idx < kSeqRows * q4) *reinterpret_cast<float4*>(dst + (size_t)r * ld + 4 * (idx - r * q4)) = v[i];
+    }
+  }
+}
+
 // Forward. Grid (H / 16, row groups, directions). Shared memory: ws [64][H + 4] (row q * 16 + j = W_hh[q * H + j0 + j, :]),
-// hs [16][H + 4] (previous h of the pass's rows), red [128][8] (the upper k half's partial sums).
-// Threads: k half = tid / 128; within a half, row pair = (tid % 128) / 16, unit = tid % 16: a thread forms the four gate
-// dot products of one unit for two batch rows over its half of k; the lower half then adds the upper half's sums and
-// applies the cell to its two (row, unit) elements.
+// hs [16][H + 4] (previous h of the pass's rows).
+// Threads: k lane = tid % 8, unit = tid / 8 % 16, row half = tid / 128: a thread forms the four gate dot products of one unit for eight
+// batch rows over every eighth float4 of k (12 shared-memory reads for 128 multiply-adds: the reads bound the product, and
+// with two rows a thread they were 6 for 32); the eight k lanes then fold their sums by halves, each keeping half of the rows
+// it holds, so that every thread ends with the four gates of one (row, unit) and applies the cell to it.
 __global__ void __launch_bounds__(kSeqThreads) lstm_seq_fwd_kernel(const LstmSeqFwdParams p) {
   extern __shared__ __align__(16) float seq_smem[];
   __shared__ int failed;
@@ -66,7 +86,6 @@ __global__ void __launch_bounds__(kSeqThreads) lstm_seq_fwd_kernel(const LstmSeq
   const int group_rows = p.passes * kSeqRows, row_base = blockIdx.y * group_rows;
   float* ws = seq_smem;
   float* hs = ws + (size_t)64 * ldw;
-  float* red = hs + (size_t)kSeqRows * ldw;
   const int hq = H / 4;
   for (int idx = tid; idx < 64 * hq; idx += kSeqThreads) {
     const int row = idx / hq, k4 = idx % hq, q = row / kSeqUnits, j = row % kSeqUnits;
@@ -74,14 +93,16 @@ __global__ void __launch_bounds__(kSeqThreads) lstm_seq_fwd_kernel(const LstmSeq
   }
   if (tid == 0) failed = 0;
   __syncthreads();
-  const int half = tid >> 7, rp = (tid & 127) >> 4, cg = tid & 15;
-  const int kspan4 = hq / 2;
+  const int kl = tid & 7, un = (tid >> 3) & 15, rh = tid >> 7;
   const size_t bh = (size_t)B * H;
   unsigned* counter = D.counter + blockIdx.y;
-  const int jg = j0 + cg;
+  const int jg = j0 + un;
   float bias[4] = {0.f, 0.f, 0.f, 0.f};
   if (D.bias != nullptr)
     for (int q = 0; q < 4; q++) bias[q] = D.bias[q * H + jg];
+  // With one pass a CTA the thread's (row, unit) is the same at every step: its cell state stays in a register and the next step's
+  // pre-activations are fetched ahead of the barrier (they do not depend on the other CTAs).
+  float pre[4] = {0.f, 0.f, 0.f, 0.f}, c_own = 0.f;
   for (int f = 0; f < T; f++) {
     const int tt = D.reverse ? T - 1 - f : f;
     const int pt = D.reverse ? tt + 1 : tt - 1;
@@ -91,123 +112,116 @@ __global__ void __launch_bounds__(kSeqThreads) lstm_seq_fwd_kernel(const LstmSeq
     for (int pass = 0; pass < p.passes; pass++) {
       const int r0 = row_base + pass * kSeqRows;
       if (r0 >= B) break;
-      // The cell's own inputs do not depend on the other CTAs: issue their loads before the dot products.
-      float pre[2][4], cprev[2];
+      const int b = r0 + rh * 8 + kl;
+      float cprev = c_own;
+      if (b < B && (p.passes > 1 || f == 0)) {
 #pragma unroll
-      for (int u = 0; u < 2; u++) {
-        cprev[u] = 0.f;
-#pragma unroll
-        for (int q = 0; q < 4; q++) pre[u][q] = 0.f;
+        for (int q = 0; q < 4; q++) pre[q] = gates_t[(size_t)b * H4 + q * H + jg];
+        cprev = cp != nullptr ? __ldcg(cp + (size_t)b * H + jg) : 0.f;
       }
-      if (half == 0) {
+      float acc[8][4];
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-          const int b = r0 + 2 * rp + u;
-          if (b < B) {
+      for (int r = 0; r < 8; r++)
 #pragma unroll
-            for (int q = 0; q < 4; q++) pre[u][q] = gates_t[(size_t)b * H4 + q * H + jg];
-            if (cp != nullptr) cprev[u] = __ldcg(cp + (size_t)b * H + jg);
+        for (int q = 0; q < 4; q++) acc[r][q] = 0.f;
+      if (hp != nullptr) {
+        seq_stage_rows(hs, ldw, hp, r0, B, hq, tid);
+        __syncthreads();
+        const float* hrow = hs + (size_t)rh * 8 * ldw;
+        const float* wrow = ws + (size_t)un * ldw;
+#pragma unroll 2
+        for (int k4 = kl; k4 < hq; k4 += 8) {
+          float4 w[4];
+#pragma unroll
+          for (int q = 0; q < 4; q++) w[q] = *reinterpret_cast<const float4*>(wrow + (size_t)q * kSeqUnits * ldw + 4 * k4);
+#pragma unroll
+          for (int r = 0; r < 8; r++) {
+            const float4 a = *reinterpret_cast<const float4*>(hrow + (size_t)r * ldw + 4 * k4);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+              acc[r][q] = fmaf(a.x, w[q].x, acc[r][q]);
+              acc[r][q] = fmaf(a.y, w[q].y, acc[r][q]);
+              acc[r][q] = fmaf(a.z, w[q].z, acc[r][q]);
+              acc[r][q] = fmaf(a.w, w[q].w, acc[r][q]);
+            }
           }
         }
       }
-      float acc[2][4];
+      // fold the eight k lanes: after the step of width w a lane holds w rows, the last one is row rh * 8 + kl
 #pragma unroll
-      for (int u = 0; u < 2; u++)
+      for (int w = 4; w > 0; w >>= 1) {
+        const bool high = (kl & w) != 0;
 #pragma unroll
-        for (int q = 0; q < 4; q++) acc[u][q] = 0.f;
-      if (hp != nullptr) {
-        // h of the previous step was written by other CTAs of this launch: read it past L1, into shared memory.
-        for (int idx = tid; idx < kSeqRows * hq; idx += kSeqThreads) {
-          const int r = idx / hq, k4 = idx % hq, b = r0 + r;
-          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (b < B) v = __ldcg(reinterpret_cast<const float4*>(hp + (size_t)b * H) + k4);
-          *reinterpret_cast<float4*>(hs + (size_t)r * ldw + 4 * k4) = v;
-        }
-        __syncthreads();
-        const float4* h0p = reinterpret_cast<const float4*>(hs + (size_t)(2 * rp) * ldw) + half * kspan4;
-        const float4* h1p = reinterpret_cast<const float4*>(hs + (size_t)(2 * rp + 1) * ldw) + half * kspan4;
-        const float4* w0p = reinterpret_cast<const float4*>(ws + (size_t)(0 * kSeqUnits + cg) * ldw) + half * kspan4;
-        const float4* w1p = reinterpret_cast<const float4*>(ws + (size_t)(1 * kSeqUnits + cg) * ldw) + half * kspan4;
-        const float4* w2p = reinterpret_cast<const float4*>(ws + (size_t)(2 * kSeqUnits + cg) * ldw) + half * kspan4;
-        const float4* w3p = reinterpret_cast<const float4*>(ws + (size_t)(3 * kSeqUnits + cg) * ldw) + half * kspan4;
-#pragma unroll 4
-        for (int k4 = 0; k4 < kspan4; k4++) {
-          const float4 a0 = h0p[k4], a1 = h1p[k4];
-          float4 w = w0p[k4];
-          acc[0][0] = fmaf(a0.x, w.x, acc[0][0]); acc[0][0] = fmaf(a0.y, w.y, acc[0][0]); acc[0][0] = fmaf(a0.z, w.z, acc[0][0]); acc[0][0] = fmaf(a0.w, w.w, acc[0][0]);
-          acc[1][0] = fmaf(a1.x, w.x, acc[1][0]); acc[1][0] = fmaf(a1.y, w.y, acc[1][0]); acc[1][0] = fmaf(a1.z, w.z, acc[1][0]); acc[1][0] = fmaf(a1.w, w.w, acc[1][0]);
-          w = w1p[k4];
-          acc[0][1] = fmaf(a0.x, w.x, acc[0][1]); acc[0][1] = fmaf(a0.y, w.y, acc[0][1]); acc[0][1] = fmaf(a0.z, w.z, acc[0][1]); acc[0][1] = fmaf(a0.w, w.w, acc[0][1]);
-          acc[1][1] = fmaf(a1.x, w.x, acc[1][1]); acc[1][1] = fmaf(a1.y, w.y, acc[1][1]); acc[1][1] = fmaf(a1.z, w.z, acc[1][1]); acc[1][1] = fmaf(a1.w, w.w, acc[1][1]);
-          w = w2p[k4];
-          acc[0][2] = fmaf(a0.x, w.x, acc[0][2]); acc[0][2] = fmaf(a0.y, w.y, acc[0][2]); acc[0][2] = fmaf(a0.z, w.z, acc[0][2]); acc[0][2] = fmaf(a0.w, w.w, acc[0][2]);
-          acc[1][2] = fmaf(a1.x, w.x, acc[1][2]); acc[1][2] = fmaf(a1.y, w.y, acc[1][2]); acc[1][2] = fmaf(a1.z, w.z, acc[1][2]); acc[1][2] = fmaf(a1.w, w.w, acc[1][2]);
-          w = w3p[k4];
-          acc[0][3] = fmaf(a0.x, w.x, acc[0][3]); acc[0][3] = fmaf(a0.y, w.y, acc[0][3]); acc[0][3] = fmaf(a0.z, w.z, acc[0][3]); acc[0][3] = fmaf(a0.w, w.w, acc[0][3]);
-          acc[1][3] = fmaf(a1.x, w.x, acc[1][3]); acc[1][3] = fmaf(a1.y, w.y, acc[1][3]); acc[1][3] = fmaf(a1.z, w.z, acc[1][3]); acc[1][3] = fmaf(a1.w, w.w, acc[1][3]);
-        }
-      }
-      if (half == 1) {
-        float* dst = red + (size_t)(tid & 127) * 8;
-        *reinterpret_cast<float4*>(dst) = make_float4(acc[0][0], acc[0][1], acc[0][2], acc[0][3]);
-        *reinterpret_cast<float4*>(dst + 4) = make_float4(acc[1][0], acc[1][1], acc[1][2], acc[1][3]);
-      }
-      __syncthreads();
-      if (half == 0) {
-        const float* src = red + (size_t)tid * 8;
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-          const int b = r0 + 2 * rp + u;
-          if (b >= B) continue;
-          float v[4];
+        for (int r = 0; r < 4; r++) {
+          if (r >= w) break;
 #pragma unroll
           for (int q = 0; q < 4; q++) {
-            const float rec = acc[u][q] + src[u * 4 + q];
-            float tv = pre[u][q] + rec;
-            if (D.bias != nullptr) tv = tv + bias[q];
-            v[q] = tv;
+            const float keep = high ? acc[r + w][q] : acc[r][q], send = high ? acc[r][q] : acc[r + w][q];
+            acc[r][q] = keep + __shfl_xor_sync(0xffffffffu, send, w);
           }
-          const float gi = seq_sigm(v[0]), gf = seq_sigm(v[1]), gg = tanhf(v[2]), go = seq_sigm(v[3]);
-          float* g = gates_t + (size_t)b * H4;
-          g[jg] = gi;
-          g[H + jg] = gf;
-          g[2 * H + jg] = gg;
-          g[3 * H + jg] = go;
-          const size_t idx = (size_t)b * H + jg;
-          const float fc = gf * cprev[u];
-          const float ig = gi * gg;
-          const float cn = fc + ig;
-          D.c[(size_t)tt * bh + idx] = cn;
-          const float tc = tanhf(cn);
-          D.tanh_c[(size_t)tt * bh + idx] = tc;
-          D.y[(size_t)tt * bh + idx] = go * tc;
         }
       }
-      __syncthreads();   // hs and red are reused by the next pass
+      if (b < B) {
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          float tv = pre[q] + acc[0][q];
+          if (D.bias != nullptr) tv = tv + bias[q];
+          v[q] = tv;
+        }
+        const float gi = seq_sigm(v[0]), gf = seq_sigm(v[1]), gg = tanhf(v[2]), go = seq_sigm(v[3]);
+        const size_t idx = (size_t)b * H + jg;
+        const float fc = gf * cprev;
+        const float ig = gi * gg;
+        const float cn = fc + ig;
+        const float tc = tanhf(cn);
+        D.y[(size_t)tt * bh + idx] = go * tc;
+        float* g = gates_t + (size_t)b * H4;
+        g[jg] = gi;
+        g[H + jg] = gf;
+        g[2 * H + jg] = gg;
+        g[3 * H + jg] = go;
+        D.c[(size_t)tt * bh + idx] = cn;
+        D.tanh_c[(size_t)tt * bh + idx] = tc;
+        c_own = cn;
+        if (p.passes == 1 && f + 1 < T) {
+          const float* next = D.gates + (size_t)(D.reverse ? tt - 1 : tt + 1) * B * H4 + (size_t)b * H4 + jg;
+#pragma unroll
+          for (int q = 0; q < 4; q++) pre[q] = next[q * H];
+        }
+      }
+      __syncthreads();   // hs is reused by the next pass
     }
     if (f + 1 < T && !seq_barrier(counter, (unsigned)(f + 1) * gridDim.x, p.status, &failed, 9100 + (int)blockIdx.z)) return;
   }
 }
 
-// Backward. Grid as forward. Shared memory: wcol [4H][16] (W_hh[c, j0 .. j0 + 15]), ds [16][4H + 4] (the gate gradients
-// of the pass's rows), red [8][16][16], dh_s and dc_s [group rows][16] (the state gradients of this CTA's units).
-// Threads for the product: k eighth = tid / 32; within it row pair = (tid % 32) / 4, unit quad = tid % 4: two rows x four
-// units over an eighth of the 4H gate columns. Threads for the cell: row = tid / 16, unit = tid % 16.
+// Backward. Grid as forward. dh of the previous step is dG_t W_hh, a sum over all 4 H gate columns. A CTA owns 64 of them (its 16 units'
+// gates): it forms their share of the sum for ALL units and leaves it in `part`, and after the barrier every CTA adds the
+// shares of its own units in the order of the slices. (Exchanging dG_t itself instead, every CTA read 16 rows x 4 H a step,
+// four times what the shares of its units are.) Shares of even and odd steps lie apart: a CTA may write step s + 1's while another still
+// reads step s's, and all have read step s's before anyone passes the barrier of s + 1.
+// Shared memory: ws [64][H] (row q * 16 + j = W_hh[q * H + j0 + j, :]), ds [64][16] (the gate gradients of the pass's rows, turned), red
+// [128][36] (the second k half's sums), dh_s and dc_s [group rows][16] (the state gradients of this CTA's units).
+// Threads of the product: k half = tid / 128, row half = tid / 64 % 2, column quad = tid % 64 (+ 64 a round): eight rows x four columns
+// over 32 gate columns, three shared-memory reads for 32 multiply-adds. Threads of the cell: row = tid / 16, unit = tid % 16.
+constexpr int kSeqRedLd = 36;
 __global__ void __launch_bounds__(kSeqThreads) lstm_seq_bwd_kernel(const LstmSeqBwdParams p) {
   extern __shared__ __align__(16) float seq_smem[];
   __shared__ int failed;
   const LstmSeqBwdDir& D = p.d[blockIdx.z];
-  const int H = p.h, B = p.b, T = p.t, H4 = 4 * p.h, ldd = 4 * p.h + kSeqPad;
+  const int H = p.h, B = p.b, T = p.t, H4 = 4 * p.h, hq = p.h / 4;
   const int j0 = blockIdx.x * kSeqUnits, tid = threadIdx.x;
   const int group_rows = p.passes * kSeqRows, row_base = blockIdx.y * group_rows;
-  float* wcol = seq_smem;
-  float* ds = wcol + (size_t)H4 * kSeqUnits;
-  float* red = ds + (size_t)kSeqRows * ldd;
-  float* dh_s = red + 8 * kSeqRows * kSeqUnits;
+  const int slices = gridDim.x, all_rows = gridDim.y * group_rows;
+  float* ws = seq_smem;
+  float* ds = ws + (size_t)64 * H;
+  float* red = ds + 64 * kSeqRows;
+  float* dh_s = red + 128 * kSeqRedLd;
   float* dc_s = dh_s + (size_t)group_rows * kSeqUnits;
-  for (int idx = tid; idx < H4 * 4; idx += kSeqThreads) {
-    const int c = idx >> 2, part = idx & 3;
-    *reinterpret_cast<float4*>(wcol + (size_t)c * kSeqUnits + 4 * part) = __ldg(reinterpret_cast<const float4*>(D.w_hh + (size_t)c * H + j0) + part);
+  for (int idx = tid; idx < 64 * hq; idx += kSeqThreads) {
+    const int row = idx / hq, k4 = idx % hq, q = row / kSeqUnits, j = row % kSeqUnits;
+    *reinterpret_cast<float4*>(ws + (size_t)row * H + 4 * k4) = __ldg(reinterpret_cast<const float4*>(D.w_hh + (size_t)(q * H + j0 + j) * H) + k4);
   }
   for (int e = tid; e < group_rows * kSeqUnits; e += kSeqThreads) {
     const int b = row_base + e / kSeqUnits;
@@ -217,10 +231,10 @@ __global__ void __launch_bounds__(kSeqThreads) lstm_seq_bwd_kernel(const LstmSeq
   }
   if (tid == 0) failed = 0;
   __syncthreads();
-  const int eighth = tid >> 5, rp = (tid & 31) >> 2, uq = tid & 3;
+  const int khalf = tid >> 7, rhalf = (tid >> 6) & 1, cq0 = tid & 63;
   const int cr = tid >> 4, cj = tid & 15;            // the cell's (row, unit) of this thread
-  const int kspan4 = H4 / 4 / 8;
-  const size_t bh = (size_t)B * H;
+  const size_t bh = (size_t)B * H, slice_floats = (size_t)all_rows * H;
+  float* part_dir = p.part + (size_t)blockIdx.z * 2 * slices * slice_floats;
   unsigned* counter = D.counter + blockIdx.y;
   float pre[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   for (int s = 0; s < T; s++) {
@@ -230,38 +244,88 @@ __global__ void __launch_bounds__(kSeqThreads) lstm_seq_bwd_kernel(const LstmSeq
     const float* cp = first ? D.c0 : D.c + (size_t)pt * bh;
     const float* gates_t = D.gates + (size_t)tt * B * H4;
     float* dg_t = D.dG + (size_t)tt * B * H4;
-    // Gate gradients of this CTA's units (BackwardRecurrent.cs:37-57 of the reference, the same operation order). With one
-    // pass per CTA the step's saved values were fetched ahead (they do not depend on dh), under the previous step's product.
+    float* part_s = part_dir + (size_t)(s & 1) * slices * slice_floats;
+    const bool last = s == T - 1 && D.dh0 == nullptr;
     for (int pass = 0; pass < p.passes; pass++) {
+      if (row_base + pass * kSeqRows >= B) break;
+      // Gate gradients of this CTA's units (BackwardRecurrent.cs:37-57 of the reference, the same operation order). With one
+      // pass per CTA the step's saved values were fetched ahead (they do not depend on dh).
       const int b = row_base + pass * kSeqRows + cr;
-      if (b >= B) continue;
-      const int e = (pass * kSeqRows + cr) * kSeqUnits + cj, jg = j0 + cj;
-      const size_t idx = (size_t)b * H + jg;
-      float* d = dg_t + (size_t)b * H4;
-      float gi, gf, gg, go, tc, gyv, cpv;
-      if (p.passes == 1 && s > 0) {
-        gi = pre[0]; gf = pre[1]; gg = pre[2]; go = pre[3]; tc = pre[4]; gyv = pre[5]; cpv = pre[6];
-      } else {
-        const float* g = gates_t + (size_t)b * H4;
-        gi = g[jg]; gf = g[H + jg]; gg = g[2 * H + jg]; go = g[3 * H + jg];
-        tc = D.tanh_c[(size_t)tt * bh + idx];
-        gyv = D.gy[(size_t)tt * bh + idx];
-        cpv = cp ? cp[idx] : 0.f;
+      float dg[4] = {0.f, 0.f, 0.f, 0.f};
+      if (b < B) {
+        const int e = (pass * kSeqRows + cr) * kSeqUnits + cj, jg = j0 + cj;
+        const size_t idx = (size_t)b * H + jg;
+        float* d = dg_t + (size_t)b * H4;
+        float gi, gf, gg, go, tc, gyv, cpv;
+        if (p.passes == 1 && s > 0) {
+          gi = pre[0]; gf = pre[1]; gg = pre[2]; go = pre[3]; tc = pre[4]; gyv = pre[5]; cpv = pre[6];
+        } else {
+          const float* g = gates_t + (size_t)b * H4;
+          gi = g[jg]; gf = g[H + jg]; gg = g[2 * H + jg]; go = g[3 * H + jg];
+          tc = D.tanh_c[(size_t)tt * bh + idx];
+          gyv = D.gy[(size_t)tt * bh + idx];
+          cpv = cp ? cp[idx] : 0.f;
+        }
+        const float dH = gyv + dh_s[e];
+        const float dO = dH * tc;
+        const float dC = dc_s[e] + ((dH * go) * (1.f - (tc * tc)));
+        const float dI = dC * gg, dF = dC * cpv, dGg = dC * gi;
+        dc_s[e] = dC * gf;
+        dg[0] = (dI * gi) * (1.f - gi);
+        dg[1] = (dF * gf) * (1.f - gf);
+        dg[2] = dGg * (1.f - (gg * gg));
+        dg[3] = (dO * go) * (1.f - go);
+#pragma unroll
+        for (int q = 0; q < 4; q++) d[q * H + jg] = dg[q];
       }
-      const float dH = gyv + dh_s[e];
-      const float dO = dH * tc;
-      const float dC = dc_s[e] + ((dH * go) * (1.f - (tc * tc)));
-      const float dI = dC * gg, dF = dC * cpv, dGg = dC * gi;
-      dc_s[e] = dC * gf;
-      d[jg] = (dI * gi) * (1.f - gi);
-      d[H + jg] = (dF * gf) * (1.f - gf);
-      d[2 * H + jg] = dGg * (1.f - (gg * gg));
-      d[3 * H + jg] = (dO * go) * (1.f - go);
+      if (last) continue;
+#pragma unroll
+      for (int q = 0; q < 4; q++) ds[(q * kSeqUnits + cj) * kSeqRows + cr] = dg[q];
+      __syncthreads();
+      // this slice's share of dh, all units: rows of the pass x H
+      for (int q0 = 0; q0 < hq; q0 += 64) {
+        const int cq = q0 + cq0;
+        float acc[8][4];
+#pragma unroll
+        for (int r = 0; r < 8; r++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) acc[r][j] = 0.f;
+        if (cq < hq) {
+#pragma unroll 4
+          for (int k = khalf * 32; k < khalf * 32 + 32; k++) {
+            const float4 w = *reinterpret_cast<const float4*>(ws + (size_t)k * H + 4 * cq);
+            const float4 d0 = *reinterpret_cast<const float4*>(ds + k * kSeqRows + rhalf * 8);
+            const float4 d1 = *reinterpret_cast<const float4*>(ds + k * kSeqRows + rhalf * 8 + 4);
+            const float dv[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+              acc[r][0] = fmaf(dv[r], w.x, acc[r][0]);
+              acc[r][1] = fmaf(dv[r], w.y, acc[r][1]);
+              acc[r][2] = fmaf(dv[r], w.z, acc[r][2]);
+              acc[r][3] = fmaf(dv[r], w.w, acc[r][3]);
+            }
+          }
+        }
+        float* mine = red + (size_t)(tid & 127) * kSeqRedLd;
+        if (khalf == 1) {
+#pragma unroll
+          for (int r = 0; r < 8; r++) *reinterpret_cast<float4*>(mine + 4 * r) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+        }
+        __syncthreads();
+        if (khalf == 0 && cq < hq) {
+          float* out = part_s + (size_t)blockIdx.x * slice_floats + (size_t)(row_base + pass * kSeqRows + rhalf * 8) * H + 4 * cq;
+#pragma unroll
+          for (int r = 0; r < 8; r++) {
+            const float4 o = *reinterpret_cast<const float4*>(mine + 4 * r);
+            *reinterpret_cast<float4*>(out + (size_t)r * H) = make_float4(acc[r][0] + o.x, acc[r][1] + o.y, acc[r][2] + o.z, acc[r][3] + o.w);
+          }
+        }
+        __syncthreads();   // red and ds are used again
+      }
     }
-    if (s == T - 1 && D.dh0 == nullptr) break;
-    if (!seq_barrier(counter, (unsigned)(s + 1) * gridDim.x, p.status, &failed, 9200 + (int)blockIdx.z)) return;
+    if (last) break;
     if (p.passes == 1 && s + 1 < T) {
-      // the next step's saved values: issued now, used after the product below
+      // the next step's saved values: on their way during the barrier
       const int b = row_base + cr;
       if (b < B) {
         const int tn = D.reverse ? s + 1 : T - 2 - s;
@@ -276,55 +340,15 @@ __global__ void __launch_bounds__(kSeqThreads) lstm_seq_bwd_kernel(const LstmSeq
         pre[6] = cpn ? cpn[idx] : 0.f;
       }
     }
-    // dh of the next processed step, this CTA's units: dG_t[b, :] . W_hh[:, j]
+    if (!seq_barrier(counter, (unsigned)(s + 1) * gridDim.x, p.status, &failed, 9200 + (int)blockIdx.z)) return;
     for (int pass = 0; pass < p.passes; pass++) {
-      const int r0 = row_base + pass * kSeqRows;
-      if (r0 >= B) break;
-      for (int idx = tid; idx < kSeqRows * (H4 / 4); idx += kSeqThreads) {
-        const int r = idx / (H4 / 4), k4 = idx % (H4 / 4), b = r0 + r;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (b < B) v = __ldcg(reinterpret_cast<const float4*>(dg_t + (size_t)b * H4) + k4);
-        *reinterpret_cast<float4*>(ds + (size_t)r * ldd + 4 * k4) = v;
-      }
-      __syncthreads();
-      float acc[2][4];
-#pragma unroll
-      for (int u = 0; u < 2; u++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[u][j] = 0.f;
-      const float4* d0p = reinterpret_cast<const float4*>(ds + (size_t)(2 * rp) * ldd) + eighth * kspan4;
-      const float4* d1p = reinterpret_cast<const float4*>(ds + (size_t)(2 * rp + 1) * ldd) + eighth * kspan4;
-      const float* wbase = wcol + (size_t)(eighth * kspan4 * 4) * kSeqUnits + 4 * uq;
-#pragma unroll 2
-      for (int k4 = 0; k4 < kspan4; k4++) {
-        const float4 a0 = d0p[k4], a1 = d1p[k4];
-        const float4 w0 = *reinterpret_cast<const float4*>(wbase + (size_t)(4 * k4) * kSeqUnits);
-        const float4 w1 = *reinterpret_cast<const float4*>(wbase + (size_t)(4 * k4 + 1) * kSeqUnits);
-        const float4 w2 = *reinterpret_cast<const float4*>(wbase + (size_t)(4 * k4 + 2) * kSeqUnits);
-        const float4 w3 = *reinterpret_cast<const float4*>(wbase + (size_t)(4 * k4 + 3) * kSeqUnits);
-        acc[0][0] = fmaf(a0.x, w0.x, acc[0][0]); acc[0][1] = fmaf(a0.x, w0.y, acc[0][1]); acc[0][2] = fmaf(a0.x, w0.z, acc[0][2]); acc[0][3] = fmaf(a0.x, w0.w, acc[0][3]);
-        acc[1][0] = fmaf(a1.x, w0.x, acc[1][0]); acc[1][1] = fmaf(a1.x, w0.y, acc[1][1]); acc[1][2] = fmaf(a1.x, w0.z, acc[1][2]); acc[1][3] = fmaf(a1.x, w0.w, acc[1][3]);
-        acc[0][0] = fmaf(a0.y, w1.x, acc[0][0]); acc[0][1] = fmaf(a0.y, w1.y, acc[0][1]); acc[0][2] = fmaf(a0.y, w1.z, acc[0][2]); acc[0][3] = fmaf(a0.y, w1.w, acc[0][3]);
-        acc[1][0] = fmaf(a1.y, w1.x, acc[1][0]); acc[1][1] = fmaf(a1.y, w1.y, acc[1][1]); acc[1][2] = fmaf(a1.y, w1.z, acc[1][2]); acc[1][3] = fmaf(a1.y, w1.w, acc[1][3]);
-        acc[0][0] = fmaf(a0.z, w2.x, acc[0][0]); acc[0][1] = fmaf(a0.z, w2.y, acc[0][1]); acc[0][2] = fmaf(a0.z, w2.z, acc[0][2]); acc[0][3] = fmaf(a0.z, w2.w, acc[0][3]);
-        acc[1][0] = fmaf(a1.z, w2.x, acc[1][0]); acc[1][1] = fmaf(a1.z, w2.y, acc[1][1]); acc[1][2] = fmaf(a1.z, w2.z, acc[1][2]); acc[1][3] = fmaf(a1.z, w2.w, acc[1][3]);
-        acc[0][0] = fmaf(a0.w, w3.x, acc[0][0]); acc[0][1] = fmaf(a0.w, w3.y, acc[0][1]); acc[0][2] = fmaf(a0.w, w3.z, acc[0][2]); acc[0][3] = fmaf(a0.w, w3.w, acc[0][3]);
-        acc[1][0] = fmaf(a1.w, w3.x, acc[1][0]); acc[1][1] = fmaf(a1.w, w3.y, acc[1][1]); acc[1][2] = fmaf(a1.w, w3.z, acc[1][2]); acc[1][3] = fmaf(a1.w, w3.w, acc[1][3]);
-      }
-      // red[eighth][row][unit]
-#pragma unroll
-      for (int u = 0; u < 2; u++)
-        *reinterpret_cast<float4*>(red + ((size_t)eighth * kSeqRows + 2 * rp + u) * kSeqUnits + 4 * uq) =
-            make_float4(acc[u][0], acc[u][1], acc[u][2], acc[u][3]);
-      __syncthreads();
-      {
-        const float* rpn = red + (size_t)cr * kSeqUnits + cj;
-        float t = rpn[0];
-#pragma unroll
-        for (int k = 1; k < 8; k++) t += rpn[(size_t)k * kSeqRows * kSeqUnits];
-        dh_s[(pass * kSeqRows + cr) * kSeqUnits + cj] = t;
-      }
-      __syncthreads();
+      if (row_base + pass * kSeqRows >= B) break;
+      // written by other CTAs of this launch: past L1
+      const float* src = part_s + (size_t)(row_base + pass * kSeqRows + cr) * H + j0 + cj;
+      float t = 0.f;
+#pragma unroll 8
+      for (int k = 0; k < slices; k++) t += __ldcg(src + (size_t)k * slice_floats);
+      dh_s[(pass * kSeqRows + cr) * kSeqUnits + cj] = t;     // read by this thread alone
     }
   }
   __syncthreads();
@@ -339,10 +363,9 @@ __global__ void __launch_bounds__(kSeqThreads) lstm_seq_bwd_kernel(const LstmSeq
 
 static_assert(kSeqThreads == kSeqRows * kSeqUnits, "the cell phases map one thread to one (row, unit)");
 
-static size_t seq_fwd_smem(int h) { return sizeof(float) * ((size_t)(64 + kSeqRows) * (h + kSeqPad) + 128 * 8); }
+static size_t seq_fwd_smem(int h) { return sizeof(float) * ((size_t)(64 + kSeqRows) * (h + kSeqPad)); }
 static size_t seq_bwd_smem(int h, int passes) {
-  return sizeof(float) * ((size_t)4 * h * kSeqUnits + (size_t)kSeqRows * (4 * h + kSeqPad) + 8 * kSeqRows * kSeqUnits +
-                          2 * (size_t)passes * kSeqRows * kSeqUnits);
+  return sizeof(float) * ((size_t)64 * h + 64 * kSeqRows + 128 * kSeqRedLd + 2 * (size_t)passes * kSeqRows * kSeqUnits);
 }
 
 // The launch shape: row groups of `passes` x 16 rows, as few passes as lets all CTAs of `dirs` directions be resident at
@@ -407,6 +430,12 @@ int32_t lstm_seq_bwd(om_ctx* ctx, int dirs, int t, int b, int h, const LstmSeqBw
   if (!seq_plan(ctx, dirs, b, h, true, &p.passes, &p.groups)) return fail(ctx, OM_ERR_UNSUPPORTED, "lstm_seq_bwd: B %d H %d", b, h);
   unsigned* counters = nullptr;
   OM_TRY(pool_alloc(ctx, 2 * kSeqMaxGroups * sizeof(unsigned), true, (void**)&counters));
+  // the slices' shares of dh: two steps x (H / 16) slices x rows x H a direction (4 MB at 64 rows, H 256)
+  const int32_t st = pool_alloc(ctx, sizeof(float) * (size_t)dirs * 2 * (h / kSeqUnits) * ((size_t)p.groups * p.passes * kSeqRows) * h, false, (void**)&p.part);
+  if (st != OM_OK) {
+    pool_free(ctx, counters);
+    return st;
+  }
   for (int k = 0; k < 2; k++) {
     p.d[k] = d[k < dirs ? k : 0];
     p.d[k].counter = counters + k * kSeqMaxGroups;
@@ -419,6 +448,7 @@ int32_t lstm_seq_bwd(om_ctx* ctx, int dirs, int t, int b, int h, const LstmSeqBw
   cudaError_t e = cudaLaunchCooperativeKernel((const void*)lstm_seq_bwd_kernel, dim3((unsigned)(h / kSeqUnits), (unsigned)p.groups, (unsigned)dirs),
                                               dim3(kSeqThreads), args, seq_bwd_smem(h, p.passes), ctx->stream);
   pool_free(ctx, counters);
+  pool_free(ctx, p.part);
   if (e != cudaSuccess) return check_cuda(ctx, e, "lstm_seq_bwd");
   return OM_OK;
 }

@@ -42,6 +42,7 @@ struct LstmSeqBwdParams {
   LstmSeqBwdDir d[2];
   int t, b, h;
   int passes, groups;
+  float* part;           // [dirs][2][H / 16][rows][H]: shares of dh between the CTAs of a row group
   int32_t* status;
 };
 

@@ -212,3 +212,29 @@ def test_small_fp32_products_are_bit_exact(ctx, K, ta, tb, m, n, k):
         Bv = ctx.to_device(bias)
         ctx.call("om_linear_fwd", ctx.handle, A.ptr, B.ptr, Bv.ptr, i32(m), i32(k), i32(n), Cm.ptr)
         assert np.array_equal(Cm.numpy(), ref + bias)
+
+
+@pytest.mark.parametrize("t,b,h", [(3, 5, 64), (4, 33, 144), (3, 17, 272), (3, 40, 400), (5, 16, 16)])
+def test_whole_sequence_lstm_shapes(ctx, K, t, b, h):
+    """Widths off the eight k lanes and off the 256 columns of a round, row groups with idle rows, both directions: fp32 products, 1e-4, the gate of the exact tier (only the order of the recurrent sums differs)."""
+    r = np.random.default_rng(h)
+    bound = 1.0 / np.sqrt(h)
+    gx = r.standard_normal((t, b, 12)).astype(np.float32)
+    w_ih, w_hh = (r.uniform(-bound, bound, (4 * h, n)).astype(np.float32) for n in (12, h))
+    b_ih, b_hh = (r.uniform(-bound, bound, 4 * h).astype(np.float32) for _ in range(2))
+    proj = r.standard_normal((t, b, h)).astype(np.float32)
+    results = []
+    for flags in (0, omb.OM_SEQ_KERNELS):
+        ctx.set_flags(flags)
+        try:
+            out = []
+            for reverse in (False, True):
+                x, ws = omb.Tensor.from_numpy(gx, requires_grad=True), [omb.Tensor.from_numpy(a, requires_grad=True) for a in (w_ih, w_hh, b_ih, b_hh)]
+                y = omb.call("lstm_layer", [x] + ws, ints=[int(reverse)])
+                omb.call("sum", [omb.call("mul", [y, omb.Tensor.from_numpy(proj)])]).backward()
+                out += [y.numpy(), x.grad.numpy()] + [w.grad.numpy() for w in ws]
+            results.append(out)
+        finally:
+            ctx.set_flags(0)
+    for k, (p, q) in enumerate(zip(*results)):
+        assert scaled_diff(q, p) <= 1e-4, k
