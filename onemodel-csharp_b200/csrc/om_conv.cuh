@@ -17,6 +17,14 @@ int32_t conv_tc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const flo
 bool conv_tc_wgrad_fits(const ConvGeom& g);
 int32_t conv_tc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, float* dw, int accumulate);
 
+// The same from channels-last copies of the activations, for the geometries whose pixels and channels tile well.
+bool conv_nhwc_fwd_fits(const ConvGeom& g);
+int32_t conv_nhwc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y);
+bool conv_nhwc_dgrad_fits(const ConvGeom& g);
+int32_t conv_nhwc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx);
+bool conv_nhwc_wgrad_fits(const ConvGeom& g);
+int32_t conv_nhwc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, float* dw, int accumulate);
+
 // The fp32 products of small shapes without an unfolded matrix (om_conv_fma.cu).
 bool conv_fma_fwd_fits(const ConvGeom& g);
 int32_t conv_fma_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y);

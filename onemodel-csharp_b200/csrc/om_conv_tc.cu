@@ -32,6 +32,7 @@ constexpr int CV_THREADS = 32 * (CV_PRODUCERS + 2);   // + one warp issuing prod
 constexpr int CV_MAX_TAPS = 32;                   // a thread keeps the taps that lie inside the image as a bit mask
 constexpr int CV_MAX_PHASES = 4;
 constexpr int CV_STG_LD = CV_TILE + 4;            // floats per staged result row
+constexpr double CN_MIN_FLOPS = 1e9;              // below, turning the source costs more than it gives
 
 // n / d for 0 <= n < 2^31 by a multiplication (Granlund and Montgomery, "Division by invariant integers using
 // multiplication", 1994): s = ceil(log2 d), mul = floor(2^32 (2^s - d) / d) + 1, n / d = (mulhi(n, mul) + n) >> s.
@@ -47,15 +48,17 @@ static CvDiv cv_div(uint32_t d) {
 }
 __device__ __forceinline__ int cv_quot(int n, CvDiv d) { return (int)((__umulhi((uint32_t)n, d.mul) + (uint32_t)n) >> d.shift); }
 
-// Unit u of channels x taps: its tap, and its first channel.
+// Unit u of channels x taps (UNIT channels of a tap, GROUP neighbouring channel blocks of a tap before the next tap): its tap, and its
+// first channel.
+template <int UNIT, int GROUP>
 __host__ __device__ __forceinline__ void cv_unit(int u, int channels, int taps, int* tap, int* c0) {
-  const int c8 = (channels + CV_UNIT - 1) / CV_UNIT;
-  const int sg = u / (CV_GROUP * taps), r = u - sg * CV_GROUP * taps;
-  const int width = c8 - sg * CV_GROUP < CV_GROUP ? c8 - sg * CV_GROUP : CV_GROUP;
+  const int blocks = (channels + UNIT - 1) / UNIT;
+  const int sg = u / (GROUP * taps), r = u - sg * GROUP * taps;
+  const int width = blocks - sg * GROUP < GROUP ? blocks - sg * GROUP : GROUP;
   *tap = r / width;
-  *c0 = (sg * CV_GROUP + r % width) * CV_UNIT;
+  *c0 = (sg * GROUP + r % width) * UNIT;
 }
-static int cv_units(int channels, int taps) { return (channels + CV_UNIT - 1) / CV_UNIT * taps; }
+static int cv_units(int channels, int taps, int unit) { return (channels + unit - 1) / unit * taps; }
 
 struct ConvPhase {
   int ph, pw;                  // grid of pixels
@@ -188,7 +191,7 @@ conv_tc_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
     int2 e = make_int2(0, 0);
     if (u < ph.units) {
       int t, c0;
-      cv_unit(u, p.sc, ph.taps, &t, &c0);
+      cv_unit<CV_UNIT, CV_GROUP>(u, p.sc, ph.taps, &t, &c0);
       e.x = (int)(4u * (uint32_t)(c0 * p.sh * p.sw + ph.dy[t] * p.sw + ph.dx[t]));
       e.y = t | (min(CV_UNIT, p.sc - c0) << 8);
     }
@@ -327,7 +330,7 @@ conv_tc_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
   }
 }
 
-// The weights in the order of the units, one K-major row per output channel of the product: wt[phase][m][8 u + i] is the weight of
+// The weights in the order of the units, one K-major row per output channel of the product: wt[phase][m][UNIT u + i] is the weight of
 // tap(u) and source channel c0(u) + i, zero past the last channel. Weights are addressed by their strides over (m, source channel).
 struct ConvTurn {
   int m, sc;
@@ -336,12 +339,13 @@ struct ConvTurn {
   long long start[CV_MAX_PHASES];
   int tap[CV_MAX_PHASES][CV_MAX_TAPS];
 };
+template <int UNIT, int GROUP>
 __global__ void __launch_bounds__(256) conv_turn_weights_kernel(const float* __restrict__ w, float* __restrict__ wt, const __grid_constant__ ConvTurn t) {
   const int z = blockIdx.z, m = blockIdx.y;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < t.ld[z]; i += gridDim.x * blockDim.x) {
     int tap, c0;
-    cv_unit(i / CV_UNIT, t.sc, t.taps[z], &tap, &c0);
-    const int c = c0 + i % CV_UNIT;
+    cv_unit<UNIT, GROUP>(i / UNIT, t.sc, t.taps[z], &tap, &c0);
+    const int c = c0 + i % UNIT;
     wt[t.start[z] + (long long)m * t.ld[z] + i] = c < t.sc ? __ldg(w + m * t.stride_m + c * t.stride_sc + t.tap[z][tap]) : 0.f;
   }
 }
@@ -409,7 +413,7 @@ conv_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
       const int u = (n0 + row0) / CV_UNIT + i;
       if (u < p.units) {
         int t, c0;
-        cv_unit(u, p.cin, p.taps, &t, &c0);
+        cv_unit<CV_UNIT, CV_GROUP>(u, p.cin, p.taps, &t, &c0);
         dy[i] = (t / p.kw) * p.dh - p.pt;
         dx[i] = (t % p.kw) * p.dw - p.pl;
         count[i] = min(CV_UNIT, p.cin - c0);
@@ -510,12 +514,12 @@ conv_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
 // takes slices y, y + SHARES, ... in order), the shares added in order. Eight shares for many slices: with up to 296 of them one
 // thread a value is a chain of as many loads (21 us against 5). One share for a few: 512 x 4608 weights in two slices took 67 us
 // with eight, most of whose threads had nothing to add.
-template <int SHARES>
+template <int SHARES, int UNIT, int GROUP>
 __global__ void __launch_bounds__(256)
 conv_wgrad_finish_kernel(const float* __restrict__ part, int splits, int cout, int units, int cin, int taps, float* __restrict__ dw, int accumulate) {
   constexpr int COLS = 256 / SHARES;
   __shared__ float sums[SHARES][COLS];
-  const int ld = units * CV_UNIT, lane = threadIdx.x % COLS, share = threadIdx.x / COLS;
+  const int ld = units * UNIT, lane = threadIdx.x % COLS, share = threadIdx.x / COLS;
   const int col = blockIdx.x * COLS + lane, co = blockIdx.y;
   float acc = 0.f;
   if (col < ld) {
@@ -530,12 +534,300 @@ conv_wgrad_finish_kernel(const float* __restrict__ part, int splits, int cout, i
   }
   if (share == 0 && col < ld) {
     int t, c0;
-    cv_unit(col / CV_UNIT, cin, taps, &t, &c0);
-    const int c = c0 + col % CV_UNIT;
+    cv_unit<UNIT, GROUP>(col / UNIT, cin, taps, &t, &c0);
+    const int c = c0 + col % UNIT;
     if (c >= cin) return;
     for (int y = 1; y < SHARES && y < splits; y++) acc += sums[y][lane];
     float* dst = dw + ((long long)co * cin + c) * taps + t;
     *dst = accumulate ? *dst + acc : acc;
+  }
+}
+
+// ---- channels last ---------------------------------------------------------------------------------------------------------
+// Where pixels tile well, the source is first turned to [n][h][w][c] (one pass over the activation), and everything the products read
+// comes by TMA: 128 pixels are a box of the turned tensor, a tap moves the box by whole pixels, and what lies outside the image
+// reads as zero. No warp touches an operand, so the pace is that of operand delivery to shared memory, as for the plain products
+// (the gathering kernels above are held up by the load/store unit).
+//   forward, dgrad   D [128 pixels, NT channels] += x [pixels + tap, 32 c] W [NT, (32 c, tap)]      both K-major
+//   wgrad            D [128 co, 4 x (32 c, tap)] += g [32 pixels, co] x [32 pixels + tap, 32 c]      both MN-major
+// Accumulator rows are pixels, so a warp's store of one channel is 32 neighbouring pixels of the NCHW result.
+struct ConvBox {
+  int w, h, n;                 // a tile of w x h x n pixels (powers of two)
+  int tw, th, tn;              // tiles along each
+};
+struct ConvNhwcPhase {
+  int ph, pw, oy0, ox0, taps, k_blocks;
+  ConvBox box;
+  int dy[CV_MAX_TAPS], dx[CV_MAX_TAPS];
+};
+struct ConvNhwcParams {
+  float* out;
+  const float* bias;
+  int32_t* status;
+  int images, m, out_w, out_plane;
+  int step_y, step_x, base_y, base_x, ostep_y, ostep_x;
+  ConvNhwcPhase phase[CV_MAX_PHASES];
+};
+struct ConvNhwcMaps {
+  CUtensorMap src[CV_MAX_PHASES], w[CV_MAX_PHASES];
+};
+
+// t[q][c] = s[n][c][p] for pixel q = n * plane + p; rows of cp floats (c rounded up to a multiple of four, zero there).
+constexpr int CN_PX = 64;
+__global__ void __launch_bounds__(256) conv_channels_last_kernel(const float* __restrict__ src, float* __restrict__ t, int pixels, int plane, CvDiv div_plane, int c, int cp) {
+  __shared__ float tile[32][CN_PX + 1];
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  const int q0 = blockIdx.x * CN_PX, c0 = blockIdx.y * 32;
+#pragma unroll
+  for (int i = 0; i < CN_PX / 32; i++) {
+    const int q = q0 + 32 * i + lane;
+    const int n = cv_quot(q < pixels ? q : 0, div_plane), p = (q < pixels ? q : 0) - n * plane;
+    const float* base = src + (long long)n * c * plane + p;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int ch = c0 + row + 8 * j;
+      tile[row + 8 * j][32 * i + lane] = q < pixels && ch < c ? __ldg(base + (long long)ch * plane) : 0.f;
+    }
+  }
+  __syncthreads();
+  if (c0 + lane >= cp) return;
+#pragma unroll
+  for (int i = 0; i < CN_PX / 8; i++) {
+    const int q = q0 + row + 8 * i;
+    if (q < pixels) t[(long long)q * cp + c0 + lane] = tile[lane][row + 8 * i];
+  }
+}
+
+constexpr int CN_THREADS = 192;      // warp 0: TMA, warp 1: products, warps 2-5: results
+template <int NT>
+__global__ void __launch_bounds__(CN_THREADS, 2)
+conv_nhwc_kernel(const __grid_constant__ ConvNhwcMaps maps, const __grid_constant__ ConvNhwcParams p) {
+  constexpr int STAGES = NT == 64 ? 4 : 3;
+  constexpr int STAGE_BYTES = CV_BLOCK + NT * 128;
+  const ConvNhwcPhase& ph = p.phase[blockIdx.z];
+  const ConvBox& box = ph.box;
+  const int tile = blockIdx.x;
+  if (tile >= box.tw * box.th * box.tn) return;       // the classes of a strided gradient differ in size
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* empty = full + STAGES;
+  uint64_t* acc_full = empty + STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m0 = blockIdx.y * NT, k_blocks = ph.k_blocks;
+  const int tx = tile % box.tw, ty = tile / box.tw % box.th, tn = tile / (box.tw * box.th);
+  const int x0 = tx * box.w, y0 = ty * box.h, n0 = tn * box.n;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; s++) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(acc_full, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, NT);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int t = 0, c0 = 0;
+      for (int kb = 0; kb < k_blocks; kb++) {
+        const int s = kb % STAGES;
+        const uint32_t round = kb / STAGES;
+        if (round > 0 && !mbar_wait(&empty[s], (round - 1) & 1, abort_flag, p.status, 81)) break;
+        uint8_t* a = smem + (size_t)s * STAGE_BYTES;
+        mbar_expect_tx(&full[s], STAGE_BYTES);
+        tma_load_4d(a, &maps.src[blockIdx.z], c0, x0 * p.step_x + p.base_x + ph.dx[t], y0 * p.step_y + p.base_y + ph.dy[t], n0, &full[s]);
+        tma_load_4d(a + CV_BLOCK, &maps.w[blockIdx.z], kb * CV_BK, m0, 0, 0, &full[s]);
+        if (++t == ph.taps) {
+          t = 0;
+          c0 += CV_BK;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && k_blocks > 0) {
+      constexpr uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(CV_TILE >> 4) << 24);
+      for (int kb = 0; kb < k_blocks; kb++) {
+        const int s = kb % STAGES;
+        if (!mbar_wait(&full[s], (kb / STAGES) & 1, abort_flag, p.status, 82)) break;
+        tc_fence_after();
+        const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES), b = a + CV_BLOCK;
+#pragma unroll
+        for (int ks = 0; ks < CV_BK / 8; ks++)
+          umma_tf32(tmem_base, make_desc(a + ks * 32, 16, 1024, 2), make_desc(b + ks * 32, 16, 1024, 2), idesc, (kb > 0 || ks > 0) ? 1u : 0u);
+        umma_commit(&empty[s]);
+      }
+      umma_commit(acc_full);
+    }
+  } else {
+    const int quad = warp & 3, slot = quad * 32 + lane;
+    const int ix = slot % box.w, iy = slot / box.w % box.h, in = slot / (box.w * box.h);
+    const int x = x0 + ix, y = y0 + iy, n = n0 + in;
+    const bool valid = x < ph.pw && y < ph.ph && n < p.images;
+    float* out = p.out + ((long long)n * p.m + m0) * p.out_plane + (long long)(y * p.ostep_y + ph.oy0) * p.out_w + x * p.ostep_x + ph.ox0;
+    bool ok = true;
+    if (k_blocks > 0) ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, p.status, 83));
+    tc_fence_after();
+    if (ok) {
+#pragma unroll 1
+      for (int c = 0; c < NT && m0 + c < p.m; c += 32) {
+        uint32_t r[32];
+        if (k_blocks > 0) {
+          tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c, r);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; j++) r[j] = 0u;
+        }
+        if (p.bias) add_bias32(r, p.bias, m0 + c, p.m);
+        if (valid) {
+#pragma unroll
+          for (int j = 0; j < 32; j++)
+            if (m0 + c + j < p.m) out[(long long)(c + j) * p.out_plane] = __uint_as_float(r[j]);
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, NT);
+  }
+}
+
+struct ConvNhwcWgradParams {
+  float* part;                 // [splits][cout][32 * units]
+  int32_t* status;
+  int cout, units, cin, kw, taps, sh, sw, pt, pl, dh, dw;
+  ConvBox box;                 // 32 pixels, tiling the output exactly
+  int blocks, blocks_per_split;
+};
+// One CTA: 128 output channels x four units of 32 channels of a tap, over a slice of the pixel boxes.
+__global__ void __launch_bounds__(CN_THREADS, 2)
+conv_nhwc_wgrad_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ ConvNhwcWgradParams p) {
+  constexpr int STAGES = 3;
+  constexpr int STAGE_BYTES = 2 * CV_BLOCK, CHUNK = CV_BK * 128;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* empty = full + STAGES;
+  uint64_t* acc_full = empty + STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int u0 = blockIdx.x * 4, m0 = blockIdx.y * CV_TILE;
+  const int b0 = blockIdx.z * p.blocks_per_split;
+  const int k_blocks = min(p.blocks_per_split, p.blocks - b0);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; s++) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(acc_full, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, CV_TILE);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int dy[4], dx[4], c0[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        int t;
+        cv_unit<CV_BK, 1>(min(u0 + j, p.units - 1), p.cin, p.taps, &t, &c0[j]);    // (past the last unit: its columns are not stored)
+        dy[j] = (t / p.kw) * p.dh - p.pt;
+        dx[j] = (t % p.kw) * p.dw - p.pl;
+      }
+      for (int kb = 0; kb < k_blocks; kb++) {
+        const int s = kb % STAGES;
+        const uint32_t round = kb / STAGES;
+        if (round > 0 && !mbar_wait(&empty[s], (round - 1) & 1, abort_flag, p.status, 84)) break;
+        const int b = b0 + kb;
+        const int x0 = b % p.box.tw * p.box.w, y0 = b / p.box.tw % p.box.th * p.box.h, n0 = b / (p.box.tw * p.box.th) * p.box.n;
+        uint8_t* a = smem + (size_t)s * STAGE_BYTES;
+        // Channels past the last 32-channel block of the gradient are outside the tensor (zero), as are taps outside the image.
+        int rows = 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) rows += m0 + 32 * j < p.cout;
+        mbar_expect_tx(&full[s], (uint32_t)((rows + 4) * CHUNK));
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          if (j < rows) tma_load_4d(a + j * CHUNK, &map_g, m0 + 32 * j, x0, y0, n0, &full[s]);
+          tma_load_4d(a + CV_BLOCK + j * CHUNK, &map_x, c0[j], x0 * p.sw + dx[j], y0 * p.sh + dy[j], n0, &full[s]);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(CV_TILE >> 3) << 17) | ((uint32_t)(CV_TILE >> 4) << 24);
+      for (int kb = 0; kb < k_blocks; kb++) {
+        const int s = kb % STAGES;
+        if (!mbar_wait(&full[s], (kb / STAGES) & 1, abort_flag, p.status, 85)) break;
+        tc_fence_after();
+        const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES), b = a + CV_BLOCK;
+#pragma unroll
+        for (int ks = 0; ks < CV_BK / 8; ks++)
+          umma_tf32(tmem_base, make_desc(a + ks * 1024, CHUNK, 512, 1), make_desc(b + ks * 1024, CHUNK, 512, 1), idesc, (kb > 0 || ks > 0) ? 1u : 0u);
+        umma_commit(&empty[s]);
+      }
+      umma_commit(acc_full);
+    }
+  } else {
+    const int quad = warp & 3;
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, p.status, 86));
+    tc_fence_after();
+    // Accumulator rows through the dead operand stages, then whole rows of 128 columns.
+    float* stg = reinterpret_cast<float*>(smem) + quad * 32 * CV_STG_LD;
+    if (ok) {
+#pragma unroll 1
+      for (int c = 0; c < 4; c++) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 32), r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(stg + lane * CV_STG_LD + c * 32 + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+      }
+      __syncwarp();
+      const int ld = p.units * CV_BK, col = u0 * CV_BK + 4 * lane;
+      float* out = p.part + (long long)blockIdx.z * p.cout * ld + col;
+      if (col < ld) {
+#pragma unroll 4
+        for (int i = 0; i < 32; i++) {
+          const int co = m0 + quad * 32 + i;
+          if (co >= p.cout) break;
+          *reinterpret_cast<float4*>(out + (long long)co * ld) = *reinterpret_cast<const float4*>(stg + i * CV_STG_LD + 4 * lane);
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, CV_TILE);
   }
 }
 
@@ -587,7 +879,7 @@ static int32_t run_conv(om_ctx* ctx, ConvTcParams& p, ConvTurn& turn, int phases
     ConvPhase& f = p.phase[z];
     f.div_plane = cv_div((uint32_t)std::max(1, f.ph * f.pw));
     f.div_w = cv_div((uint32_t)std::max(1, f.pw));
-    f.units = cv_units(p.sc, f.taps);
+    f.units = cv_units(p.sc, f.taps, CV_UNIT);
     turn.taps[z] = f.taps;
     turn.ld[z] = f.units * CV_UNIT;
     turn.start[z] = floats;
@@ -606,7 +898,7 @@ static int32_t run_conv(om_ctx* ctx, ConvTcParams& p, ConvTurn& turn, int phases
       st = fail(ctx, OM_ERR_CUDA, "cuTensorMapEncodeTiled failed for a convolution's turned weights");
   if (st == OM_OK) {
     if (most_units > 0)
-      conv_turn_weights_kernel<<<dim3((unsigned)std::min<int64_t>(ceil_div(most_units * CV_UNIT, 256), 64), (unsigned)p.m, (unsigned)phases), 256, 0, ctx->stream>>>(
+      conv_turn_weights_kernel<CV_UNIT, CV_GROUP><<<dim3((unsigned)std::min<int64_t>(ceil_div(most_units * CV_UNIT, 256), 64), (unsigned)p.m, (unsigned)phases), 256, 0, ctx->stream>>>(
           w, wt, turn);
     // Two accumulators once that still leaves a CTA for every SM.
     const bool two = p.m > CV_TILE && all * ceil_div(p.m, 2 * CV_TILE) >= 148;
@@ -643,6 +935,19 @@ int32_t conv_tc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const float*
 
 bool conv_tc_dgrad_fits(const ConvGeom& g) { return encode_fn() && cv_sizes_fit(g) && g.sh * g.sw <= CV_MAX_PHASES; }
 
+// The taps that reach the input positions (oy0, ox0) modulo the stride, and where in the gradient from a pixel of that class.
+static int class_taps(const ConvGeom& g, int oy0, int ox0, int* dy, int* dx, int* tap) {
+  int n = 0;
+  for (int t = 0; t < g.kh * g.kw; t++) {
+    const int ty = oy0 + g.pt - (t / g.kw) * g.dh, tx = ox0 + g.pl - (t % g.kw) * g.dw;
+    if (ty % g.sh || tx % g.sw) continue;      // (exact for negative values too)
+    dy[n] = ty / g.sh;
+    dx[n] = tx / g.sw;
+    tap[n++] = t;
+  }
+  return n;
+}
+
 int32_t conv_tc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx) {
   ConvTcParams p = {};
   ConvTurn turn = {};
@@ -658,17 +963,22 @@ int32_t conv_tc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const flo
     f.ox0 = z % g.sw;
     f.ph = f.oy0 < g.h ? (g.h - f.oy0 + g.sh - 1) / g.sh : 0;
     f.pw = f.ox0 < g.w ? (g.w - f.ox0 + g.sw - 1) / g.sw : 0;
-    for (int t = 0; t < g.kh * g.kw; t++) {
-      const int ty = f.oy0 + g.pt - (t / g.kw) * g.dh, tx = f.ox0 + g.pl - (t % g.kw) * g.dw;
-      if (ty % g.sh || tx % g.sw) continue;      // (exact for negative values too)
-      f.dy[f.taps] = ty / g.sh;
-      f.dx[f.taps] = tx / g.sw;
-      turn.tap[z][f.taps++] = t;
-    }
+    f.taps = class_taps(g, f.oy0, f.ox0, f.dy, f.dx, turn.tap[z]);
   }
   turn.m = g.cin; turn.sc = g.cout;
   turn.stride_m = g.kh * g.kw; turn.stride_sc = (long long)g.cin * g.kh * g.kw;
   return run_conv(ctx, p, turn, g.sh * g.sw, w);
+}
+
+template <int UNIT, int GROUP>
+static void launch_finish(om_ctx* ctx, const float* part, int splits, const ConvGeom& g, int units, float* dw, int accumulate) {
+  const int ld = units * UNIT;
+  if (splits <= 8)
+    conv_wgrad_finish_kernel<1, UNIT, GROUP><<<dim3((unsigned)ceil_div(ld, 256), (unsigned)g.cout), 256, 0, ctx->stream>>>(part, splits, g.cout, units, g.cin,
+                                                                                                                        g.kh * g.kw, dw, accumulate);
+  else
+    conv_wgrad_finish_kernel<8, UNIT, GROUP><<<dim3((unsigned)ceil_div(ld, 32), (unsigned)g.cout), 256, 0, ctx->stream>>>(part, splits, g.cout, units, g.cin,
+                                                                                                                       g.kh * g.kw, dw, accumulate);
 }
 
 bool conv_tc_wgrad_fits(const ConvGeom& g) { return encode_fn() && cv_sizes_fit(g); }
@@ -690,7 +1000,7 @@ int32_t conv_tc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const flo
   p.gr = gr; p.x = x; p.status = ctx->status_dev;
   p.cout = g.cout; p.cin = g.cin; p.h = g.h; p.w = g.w; p.kw = g.kw; p.taps = g.kh * g.kw; p.sh = g.sh; p.sw = g.sw;
   p.pt = g.pt; p.pl = g.pl; p.dh = g.dh; p.dw = g.dw; p.ow = g.ow; p.plane = g.oh * g.ow;
-  p.units = cv_units(g.cin, p.taps);
+  p.units = cv_units(g.cin, p.taps, CV_UNIT);
   p.div_plane = cv_div((uint32_t)p.plane);
   p.div_w = cv_div((uint32_t)g.ow);
   p.pixels = g.n * p.plane;
@@ -708,18 +1018,207 @@ int32_t conv_tc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const flo
   OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)splits * g.cout * ld, false, (void**)&p.part));
   const dim3 grid((unsigned)tn, (unsigned)tm, (unsigned)splits);
   int32_t st = a_tma ? launch_wgrad<true>(ctx, map, p, grid) : launch_wgrad<false>(ctx, map, p, grid);
-  if (st == OM_OK) {
-    if (splits <= 8)
-      conv_wgrad_finish_kernel<1><<<dim3((unsigned)ceil_div(ld, 256), (unsigned)g.cout), 256, 0, ctx->stream>>>(p.part, splits, g.cout, p.units, g.cin, p.taps, dw,
-                                                                                                             accumulate);
-    else
-      conv_wgrad_finish_kernel<8><<<dim3((unsigned)ceil_div(ld, 32), (unsigned)g.cout), 256, 0, ctx->stream>>>(p.part, splits, g.cout, p.units, g.cin, p.taps, dw,
-                                                                                                            accumulate);
-  }
+  if (st == OM_OK) launch_finish<CV_UNIT, CV_GROUP>(ctx, p.part, splits, g, p.units, dw, accumulate);
   pool_free(ctx, p.part);
   OM_TRY(st);
   OM_LAUNCH_CHECK(ctx, "conv_wgrad_tc");
   return OM_OK;
+}
+
+// ---- channels last, host side ----------------------------------------------------------------------------------------------
+// The box of `size` pixels (a power of two) that covers a grid of w x h x n pixels in the fewest tiles, the widest of those.
+static ConvBox cn_box(int size, int w, int h, int n) {
+  ConvBox best = {};
+  long long fewest = -1;
+  for (int bw = size; bw >= 1; bw /= 2)
+    for (int bh = size / bw; bh >= 1; bh /= 2) {
+      const ConvBox b = {bw, bh, size / bw / bh, (int)ceil_div(w, bw), (int)ceil_div(h, bh), (int)ceil_div(n, size / bw / bh)};
+      const long long tiles = (long long)b.tw * b.th * b.tn;
+      if (fewest < 0 || tiles < fewest) {
+        fewest = tiles;
+        best = b;
+      }
+    }
+  return best;
+}
+static int cn_pitch(int c) { return (c + 3) & ~3; }
+
+// The turned tensor [n][h][w][c] with boxes of 32 channels x `box`, taken every (sy, sx) pixels.
+static bool cn_map(CUtensorMap* map, const float* base, int c, int w, int h, int n, const ConvBox& box, int sx, int sy, bool mn_major) {
+  const cuuint64_t row = (cuuint64_t)cn_pitch(c) * 4;
+  cuuint64_t dims[4] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
+  cuuint64_t strides[3] = {row, row * w, row * w * h};
+  cuuint32_t bx[4] = {CV_BK, (cuuint32_t)(box.w * sx), (cuuint32_t)(box.h * sy), (cuuint32_t)box.n};
+  cuuint32_t estr[4] = {1, (cuuint32_t)sx, (cuuint32_t)sy, 1};
+  return encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_TFLOAT32, 4, const_cast<float*>(base), dims, strides, bx, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     mn_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+static int32_t cn_turn(om_ctx* ctx, const float* src, int n, int c, int plane, float** out) {
+  const int pixels = n * plane, cp = cn_pitch(c);
+  OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)pixels * cp, false, (void**)out));
+  conv_channels_last_kernel<<<dim3((unsigned)ceil_div(pixels, CN_PX), (unsigned)ceil_div(cp, 32)), 256, 0, ctx->stream>>>(src, *out, pixels, plane,
+                                                                                                                      cv_div((uint32_t)plane), c, cp);
+  return OM_OK;
+}
+
+// A block of 32 channels may be partly empty, and a box partly outside the grid: at least two thirds of the work has to be real.
+static bool cn_channels_fit(int c) { return 3 * c >= 2 * (int)ceil_div(c, 32) * 32; }
+static bool cn_worth(const ConvGeom& g) {
+  return 2.0 * g.n * g.oh * g.ow * (double)g.cout * g.cin * g.kh * g.kw >= CN_MIN_FLOPS && g.sh <= 2 && g.sw <= 2 && (long long)g.n * g.h * g.w * cn_pitch(g.cin) < (1ll << 30) &&
+         (long long)g.n * g.oh * g.ow * cn_pitch(g.cout) < (1ll << 30);
+}
+
+// Runs the product of every phase from the turned source; the phases' grids, taps and output positions are set.
+static int32_t run_conv_nhwc(om_ctx* ctx, ConvNhwcParams& p, ConvTurn& turn, int phases, const float* src, int sc, int sh, int sw, const float* w) {
+  ConvNhwcMaps maps = {};
+  float *t = nullptr, *wt = nullptr;
+  OM_TRY(cn_turn(ctx, src, p.images, sc, sh * sw, &t));
+  const int nt = p.m <= 64 ? 64 : 128;
+  long long floats = 0, most = 0;
+  int most_ld = 0;
+  for (int z = 0; z < phases; z++) {
+    ConvNhwcPhase& f = p.phase[z];
+    f.box = cn_box(CV_TILE, f.pw, f.ph, p.images);
+    const int units = cv_units(sc, f.taps, CV_BK);
+    f.k_blocks = units;
+    turn.taps[z] = f.taps;
+    turn.ld[z] = units * CV_BK;
+    turn.start[z] = floats;
+    floats += (long long)turn.ld[z] * p.m;
+    most_ld = std::max(most_ld, turn.ld[z]);
+    most = std::max(most, (long long)f.box.tw * f.box.th * f.box.tn);
+  }
+  int32_t st = pool_alloc(ctx, sizeof(float) * (size_t)std::max<long long>(floats, 4), false, (void**)&wt);
+  for (int z = 0; z < phases && st == OM_OK; z++) {
+    const ConvNhwcPhase& f = p.phase[z];
+    if (f.k_blocks == 0) continue;
+    bool ok = cn_map(&maps.src[z], t, sc, sw, sh, p.images, f.box, p.step_x, p.step_y, false);
+    cuuint64_t dims[4] = {(cuuint64_t)turn.ld[z], (cuuint64_t)p.m, 1, 1};
+    const cuuint64_t row = (cuuint64_t)turn.ld[z] * 4;
+    cuuint64_t strides[3] = {row, row * p.m, row * p.m};
+    cuuint32_t bx[4] = {CV_BK, (cuuint32_t)nt, 1, 1}, estr[4] = {1, 1, 1, 1};
+    ok = ok && encode_fn()(&maps.w[z], CU_TENSOR_MAP_DATA_TYPE_TFLOAT32, 4, wt + turn.start[z], dims, strides, bx, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    if (!ok) st = fail(ctx, OM_ERR_CUDA, "cuTensorMapEncodeTiled failed for a convolution's operands");
+  }
+  if (st == OM_OK && most > 0) {
+    if (most_ld > 0)
+      conv_turn_weights_kernel<CV_BK, 1><<<dim3((unsigned)std::min<int64_t>(ceil_div(most_ld, 256), 64), (unsigned)p.m, (unsigned)phases), 256, 0, ctx->stream>>>(w, wt, turn);
+    const dim3 grid((unsigned)most, (unsigned)ceil_div(p.m, nt), (unsigned)phases);
+    static bool set = false;
+    constexpr size_t smem64 = (size_t)4 * (CV_BLOCK + 64 * 128) + 1024 + 128, smem128 = (size_t)3 * (CV_BLOCK + 128 * 128) + 1024 + 128;
+    if (!set) {
+      st = check_cuda(ctx, cudaFuncSetAttribute(conv_nhwc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem64), "conv_nhwc");
+      if (st == OM_OK) st = check_cuda(ctx, cudaFuncSetAttribute(conv_nhwc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem128), "conv_nhwc");
+      set = st == OM_OK;
+    }
+    if (st == OM_OK) {
+      if (nt == 64) conv_nhwc_kernel<64><<<grid, CN_THREADS, smem64, ctx->stream>>>(maps, p);
+      else conv_nhwc_kernel<128><<<grid, CN_THREADS, smem128, ctx->stream>>>(maps, p);
+      st = check_cuda(ctx, cudaGetLastError(), "conv_nhwc");
+    }
+  }
+  pool_free(ctx, t);
+  if (wt) pool_free(ctx, wt);
+  return st;
+}
+
+static bool cn_grid_fits(int w, int h, int n) {
+  const ConvBox b = cn_box(CV_TILE, w, h, n);
+  return 3 * (long long)w * h * n >= 2 * (long long)b.tw * b.th * b.tn * CV_TILE;
+}
+bool conv_nhwc_fwd_fits(const ConvGeom& g) {
+  return encode_fn() && cv_sizes_fit(g) && cn_worth(g) && cn_channels_fit(g.cin) && cn_grid_fits(g.ow, g.oh, g.n);
+}
+
+int32_t conv_nhwc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y) {
+  ConvNhwcParams p = {};
+  ConvTurn turn = {};
+  p.out = y; p.bias = bias; p.status = ctx->status_dev;
+  p.images = g.n; p.m = g.cout; p.out_w = g.ow; p.out_plane = g.oh * g.ow;
+  p.step_y = g.sh; p.step_x = g.sw; p.base_y = -g.pt; p.base_x = -g.pl; p.ostep_y = p.ostep_x = 1;
+  ConvNhwcPhase& f = p.phase[0];
+  f.ph = g.oh; f.pw = g.ow; f.taps = g.kh * g.kw;
+  for (int t = 0; t < f.taps; t++) {
+    f.dy[t] = (t / g.kw) * g.dh;
+    f.dx[t] = (t % g.kw) * g.dw;
+    turn.tap[0][t] = t;
+  }
+  turn.m = g.cout; turn.sc = g.cin;
+  turn.stride_m = (long long)g.cin * f.taps; turn.stride_sc = f.taps;
+  return run_conv_nhwc(ctx, p, turn, 1, x, g.cin, g.h, g.w, w);
+}
+
+bool conv_nhwc_dgrad_fits(const ConvGeom& g) {
+  return encode_fn() && cv_sizes_fit(g) && cn_worth(g) && cn_channels_fit(g.cout) && cn_grid_fits((int)ceil_div(g.w, g.sw), (int)ceil_div(g.h, g.sh), g.n);
+}
+
+int32_t conv_nhwc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx) {
+  ConvNhwcParams p = {};
+  ConvTurn turn = {};
+  p.out = dx; p.status = ctx->status_dev;
+  p.images = g.n; p.m = g.cin; p.out_w = g.w; p.out_plane = g.h * g.w;
+  p.step_y = p.step_x = 1; p.ostep_y = g.sh; p.ostep_x = g.sw;
+  for (int z = 0; z < g.sh * g.sw; z++) {
+    ConvNhwcPhase& f = p.phase[z];
+    f.oy0 = z / g.sw;
+    f.ox0 = z % g.sw;
+    f.ph = f.oy0 < g.h ? (g.h - f.oy0 + g.sh - 1) / g.sh : 0;
+    f.pw = f.ox0 < g.w ? (g.w - f.ox0 + g.sw - 1) / g.sw : 0;
+    f.taps = class_taps(g, f.oy0, f.ox0, f.dy, f.dx, turn.tap[z]);
+  }
+  turn.m = g.cin; turn.sc = g.cout;
+  turn.stride_m = g.kh * g.kw; turn.stride_sc = (long long)g.cin * g.kh * g.kw;
+  return run_conv_nhwc(ctx, p, turn, g.sh * g.sw, gr, g.cout, g.oh, g.ow, w);
+}
+
+// The pixel boxes have to tile the output exactly: a slot outside it would multiply its zero gradient with values of the input, which may
+// be infinite.
+bool conv_nhwc_wgrad_fits(const ConvGeom& g) {
+  if (!encode_fn() || !cv_sizes_fit(g) || !cn_worth(g) || !cn_channels_fit(g.cin)) return false;
+  const ConvBox b = cn_box(CV_BK, g.ow, g.oh, g.n);
+  return g.ow % b.w == 0 && g.oh % b.h == 0 && g.n % b.n == 0;
+}
+
+int32_t conv_nhwc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, float* dw, int accumulate) {
+  ConvNhwcWgradParams p = {};
+  p.status = ctx->status_dev;
+  p.cout = g.cout; p.cin = g.cin; p.kw = g.kw; p.taps = g.kh * g.kw; p.sh = g.sh; p.sw = g.sw; p.pt = g.pt; p.pl = g.pl; p.dh = g.dh; p.dw = g.dw;
+  p.units = cv_units(g.cin, p.taps, CV_BK);
+  p.box = cn_box(CV_BK, g.ow, g.oh, g.n);
+  p.blocks = p.box.tw * p.box.th * p.box.tn;
+  const int ld = p.units * CV_BK;
+  const int tn = (int)ceil_div(p.units, 4), tm = (int)ceil_div(g.cout, CV_TILE);
+  // Slices of the pixels for one round of two CTAs an SM, each at least eight stages long: a function of the shape alone.
+  int splits = (int)std::max<long long>(1, std::min<long long>(kSplitSlots / ((long long)tn * tm), p.blocks / 8));
+  p.blocks_per_split = (int)ceil_div(p.blocks, splits);
+  splits = (int)ceil_div(p.blocks, p.blocks_per_split);
+  float *gt = nullptr, *xt = nullptr;
+  CUtensorMap map_g = {}, map_x = {};
+  int32_t st = cn_turn(ctx, gr, g.n, g.cout, g.oh * g.ow, &gt);
+  if (st == OM_OK) st = cn_turn(ctx, x, g.n, g.cin, g.h * g.w, &xt);
+  if (st == OM_OK) st = pool_alloc(ctx, sizeof(float) * (size_t)splits * g.cout * ld, false, (void**)&p.part);
+  if (st == OM_OK && (!cn_map(&map_g, gt, g.cout, g.ow, g.oh, g.n, p.box, 1, 1, true) || !cn_map(&map_x, xt, g.cin, g.w, g.h, g.n, p.box, g.sw, g.sh, true)))
+    st = fail(ctx, OM_ERR_CUDA, "cuTensorMapEncodeTiled failed for a convolution's operands");
+  if (st == OM_OK) {
+    constexpr size_t smem = (size_t)3 * 2 * CV_BLOCK + 1024 + 128;
+    static bool set = false;
+    if (!set) {
+      st = check_cuda(ctx, cudaFuncSetAttribute(conv_nhwc_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "conv_nhwc_wgrad");
+      set = st == OM_OK;
+    }
+    if (st == OM_OK) {
+      conv_nhwc_wgrad_kernel<<<dim3((unsigned)tn, (unsigned)tm, (unsigned)splits), CN_THREADS, smem, ctx->stream>>>(map_g, map_x, p);
+      launch_finish<CV_BK, 1>(ctx, p.part, splits, g, p.units, dw, accumulate);
+      st = check_cuda(ctx, cudaGetLastError(), "conv_nhwc_wgrad");
+    }
+  }
+  if (gt) pool_free(ctx, gt);
+  if (xt) pool_free(ctx, xt);
+  if (p.part) pool_free(ctx, p.part);
+  return st;
 }
 
 }  // namespace om

@@ -532,6 +532,7 @@ int32_t om_conv2d_fwd(om_ctx* ctx, const om_conv_shape* s, const float* x, const
   if (g.n > 65535) return fail(ctx, OM_ERR_UNSUPPORTED, "om_conv2d_fwd: more than 65535 images in one call");
   ProfileScope prof(ctx, "om_conv2d_fwd", 2.0 * g.n * g.cout * (double)kk * plane, 4.0 * ((double)g.n * g.cin * g.h * g.w + (double)g.n * g.cout * plane));
   const bool tensor_pipe = conv_on_tensor_pipe(ctx, g, true);
+  if (tensor_pipe && conv_nhwc_fwd_fits(g)) return conv_nhwc_fwd(ctx, g, x, w, bias, y);
   if (tensor_pipe && conv_tc_fwd_fits(g)) return conv_tc_fwd(ctx, g, x, w, bias, y);
   if (!tensor_pipe && conv_fma_fwd_fits(g)) return conv_fma_fwd(ctx, g, x, w, bias, y);
   if (tensor_pipe) {
@@ -578,6 +579,7 @@ int32_t om_conv2d_dgrad(om_ctx* ctx, const om_conv_shape* s, const float* gr, co
   const int cg = g.cin / g.groups, og = g.cout / g.groups, kk = cg * g.kh * g.kw, plane = g.oh * g.ow;
   ProfileScope prof(ctx, "om_conv2d_dgrad", 2.0 * g.n * g.cout * (double)kk * plane, 4.0 * ((double)g.n * g.cin * g.h * g.w + (double)g.n * g.cout * plane));
   const bool tensor_pipe = conv_on_tensor_pipe(ctx, g, true);
+  if (tensor_pipe && conv_nhwc_dgrad_fits(g)) return conv_nhwc_dgrad(ctx, g, gr, w, dx);
   if (tensor_pipe && conv_tc_dgrad_fits(g)) return conv_tc_dgrad(ctx, g, gr, w, dx);
   if (!tensor_pipe && conv_fma_dgrad_fits(g)) return conv_fma_dgrad(ctx, g, gr, w, dx);
   float* dcols = nullptr;
@@ -625,6 +627,7 @@ int32_t om_conv2d_wgrad(om_ctx* ctx, const om_conv_shape* s, const float* gr, co
   }
   ProfileScope prof(ctx, "om_conv2d_wgrad", 2.0 * g.n * g.cout * (double)kk * plane, 4.0 * ((double)g.n * g.cin * g.h * g.w + (double)g.n * g.cout * plane));
   const bool tensor_pipe = conv_on_tensor_pipe(ctx, g, false);
+  if (tensor_pipe && conv_nhwc_wgrad_fits(g)) return conv_nhwc_wgrad(ctx, g, gr, x, dw, accumulate);
   if (tensor_pipe && conv_tc_wgrad_fits(g)) return conv_tc_wgrad(ctx, g, gr, x, dw, accumulate);
   if (!tensor_pipe && conv_fma_wgrad_fits(g)) return conv_fma_wgrad(ctx, g, gr, x, dw, accumulate);
   if (tensor_pipe) {

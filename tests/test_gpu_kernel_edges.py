@@ -238,3 +238,23 @@ def test_whole_sequence_lstm_shapes(ctx, K, t, b, h):
             ctx.set_flags(0)
     for k, (p, q) in enumerate(zip(*results)):
         assert scaled_diff(q, p) <= 1e-4, k
+
+
+@pytest.mark.parametrize("case", [
+    (80, 32, 16, 16, 96, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1), (20, 48, 32, 32, 64, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1),     # half a block of channels empty
+    (33, 64, 16, 16, 129, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1),     # a second block of one channel, images that no box divides
+    (64, 64, 16, 16, 256, 3, 3, 2, 2, (1, 1, 1, 1), 1, 1), (130, 96, 17, 15, 64, 3, 3, 2, 2, (1, 1, 1, 1), 1, 1),   # strided, odd planes
+    (256, 64, 32, 32, 128, 1, 1, 2, 2, (0, 0, 0, 0), 1, 1),    # classes that no tap reaches
+    (24, 32, 20, 44, 32, 5, 5, 1, 1, (4, 4, 4, 4), 2, 2), (160, 64, 32, 4, 128, 3, 2, 1, 2, (2, 0, 1, 1), 1, 1),
+    (128, 128, 4, 4, 256, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1)])
+def test_conv2d_from_channels_last_copies(ctx, case):
+    """Boxes of 128 and of 32 pixels over several images and rows, ragged boxes and channel blocks: TF32-valued operands, 2e-5 scaled."""
+    s, x, wt, b, g, y, dx, dw = conv_case(*case)
+    assert 2.0 * g.size * s.cin * s.kh * s.kw >= 1e9
+    ctx.set_flags(omb.OM_TF32)
+    try:
+        Y, DX, DW, DW2 = run_conv(ctx, s, x, wt, b, g)
+    finally:
+        ctx.set_flags(0)
+    for got, want in ((Y, y), (DX, dx), (DW, dw), (DW2, 2 * dw)):
+        assert scaled_diff(got, want) <= 2e-5
