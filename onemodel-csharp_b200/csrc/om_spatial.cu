@@ -194,19 +194,49 @@ cnhw_to_nchw_bias_kernel(const float* __restrict__ t, const float* __restrict__ 
 }
 
 // dbias[co] = sum over images of the plane sums of g[n][co][:], in double. Stage 1: CTA (co, slice) sums the planes of a
-// fixed slice of images (thread partials in a fixed tree); stage 2 adds the slices in order.
+// fixed slice of images (thread partials in a fixed tree); stage 2 adds the slices in order. VEC == 4: planes of a multiple of four
+// aligned floats. Each thread keeps its place in the plane by additions and four loads in flight: one load at a time behind two
+// divisions took 42 us for 64 channels of 256 planes of 32 x 32 (67 MB: 10 us).
 constexpr int kDbiasSlices = 16;
+template <int VEC>
 __global__ void __launch_bounds__(256)
 conv_dbias_partial_kernel(const float* __restrict__ g, int n, int cout, int plane, int per_slice, double* __restrict__ partial) {
   __shared__ double sm[256];
   const int co = blockIdx.x, slice = blockIdx.y;
   const int i0 = slice * per_slice, i1 = min(n, i0 + per_slice);
+  const int pv = plane / VEC;                                   // accesses of a plane
+  const int64_t image = (int64_t)cout * plane;
   double acc = 0.0;
-  const int64_t span = (int64_t)(i1 - i0) * plane;
-  for (int64_t e = threadIdx.x; e < span; e += 256) {
-    const int i = i0 + (int)(e / plane);
-    const int p = (int)(e % plane);
-    acc += (double)g[((int64_t)i * cout + co) * plane + p];
+  int i = i0 + (int)(threadIdx.x / (unsigned)pv), p = (int)(threadIdx.x % (unsigned)pv);
+  const int step_i = 256 / pv, step_p = 256 % pv;
+  const float* base = g + (int64_t)co * plane;
+  constexpr int LOADS = VEC == 4 ? 4 : 8;
+  while (i < i1) {
+    float v[LOADS][VEC];
+#pragma unroll
+    for (int l = 0; l < LOADS; l++) {
+#pragma unroll
+      for (int j = 0; j < VEC; j++) v[l][j] = 0.f;
+      if (i < i1) {
+        const float* src = base + (int64_t)i * image + (int64_t)p * VEC;
+        if (VEC == 4) {
+          const float4 t = __ldg(reinterpret_cast<const float4*>(src));
+          v[l][0] = t.x; v[l][VEC / 4] = t.y; v[l][VEC / 2] = t.z; v[l][VEC - 1] = t.w;
+        } else {
+          v[l][0] = __ldg(src);
+        }
+      }
+      p += step_p;
+      i += step_i;
+      if (p >= pv) {
+        p -= pv;
+        i++;
+      }
+    }
+#pragma unroll
+    for (int l = 0; l < LOADS; l++)
+#pragma unroll
+      for (int j = 0; j < VEC; j++) acc += (double)v[l][j];
   }
   sm[threadIdx.x] = acc;
   __syncthreads();
@@ -678,7 +708,11 @@ int32_t om_conv2d_dbias(om_ctx* ctx, const om_conv_shape* s, const float* gr, fl
   const int slices = g.n < kDbiasSlices ? g.n : kDbiasSlices, per_slice = (int)ceil_div(g.n, slices);
   double* partial = nullptr;
   OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)slices * g.cout, false, (void**)&partial));
-  conv_dbias_partial_kernel<<<dim3(g.cout, slices), 256, 0, ctx->stream>>>(gr, g.n, g.cout, g.oh * g.ow, per_slice, partial);
+  const int plane = g.oh * g.ow;
+  if ((plane & 3) == 0 && (reinterpret_cast<uintptr_t>(gr) & 15) == 0)
+    conv_dbias_partial_kernel<4><<<dim3(g.cout, slices), 256, 0, ctx->stream>>>(gr, g.n, g.cout, plane, per_slice, partial);
+  else
+    conv_dbias_partial_kernel<1><<<dim3(g.cout, slices), 256, 0, ctx->stream>>>(gr, g.n, g.cout, plane, per_slice, partial);
   conv_dbias_finish_kernel<<<(unsigned)ceil_div(g.cout, 128), 128, 0, ctx->stream>>>(partial, slices, g.cout, dbias, accumulate);
   pool_free(ctx, partial);
   OM_LAUNCH_CHECK(ctx, "om_conv2d_dbias");

@@ -258,3 +258,13 @@ def test_conv2d_from_channels_last_copies(ctx, case):
         ctx.set_flags(0)
     for got, want in ((Y, y), (DX, dx), (DW, dw), (DW2, 2 * dw)):
         assert scaled_diff(got, want) <= 2e-5
+
+
+@pytest.mark.parametrize("n,cout,h,w", [(1, 3, 2, 2), (5, 7, 4, 16), (17, 2, 33, 31), (3, 4, 1, 3), (40, 5, 40, 64)])
+def test_conv2d_bias_gradient_planes(ctx, n, cout, h, w):
+    """Planes smaller and larger than a CTA's stride, of a multiple of four floats or not: sums in double, 1e-6."""
+    s, g = ConvShape(n, 1, h, w, cout, 1, 1, 1, 1, 0, 0, 0, 0, 1, 1, 1), normal(n, n, cout, h, w)
+    G, DB = ctx.to_device(g), ctx.empty((cout,))
+    ctx.call("om_conv2d_dbias", ctx.handle, C.byref(s), G.ptr, DB.ptr, i32(0))
+    want = g.astype(np.float64).sum((0, 2, 3))
+    assert np.max(np.abs(DB.numpy() - want) / np.abs(g).astype(np.float64).sum((0, 2, 3))) <= 1e-6
