@@ -373,6 +373,85 @@ __global__ void maxpool_bwd_tiled_kernel(int h, int w, int oh, int ow, int kh, i
   }
 }
 
+// Windows of kh x KW that tile the plane (KW 1, 2 or 4; w a multiple of four, h one of kh; 16-byte aligned arrays): a thread owns the windows
+// under four adjacent inputs, 4 / KW of them, and reads or writes their kh rows 16 bytes at a time. The rule for the maximum is the one
+// above. One 4-byte access at a time, an output (forward) or four inputs (backward) a thread behind four divisions, 64 x 64 planes
+// of 32 x 256 through 2 x 2 windows took 78 us forward and 75 backward (201 MB: 30 us).
+template <int KW>
+__global__ void __launch_bounds__(256)
+maxpool_fwd_windows_kernel(int h, int w, int kh, const float* __restrict__ x, int groups, float* __restrict__ y, int32_t* __restrict__ idx) {
+  constexpr int OUT = 4 / KW;
+  const int wg = w / 4, oh = h / kh, ow = w / KW;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < groups; q += gridDim.x * blockDim.x) {
+    const int row = q / wg, xg = q - row * wg;          // row of windows over all planes
+    const int pl = row / oh, oy = row - pl * oh;
+    const int at = (pl * h + oy * kh) * w + 4 * xg;
+    float best[OUT];
+    int32_t where[OUT];
+    for (int ky = 0; ky < kh; ky++) {
+      const float4 t = __ldg(reinterpret_cast<const float4*>(x + at + ky * w));
+      const float v[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int o = j / KW;
+        const bool start = ky == 0 && j % KW == 0;
+        const bool wins = start || (!(best[o] != best[o]) && (v[j] > best[o] || v[j] != v[j]));
+        best[o] = wins ? v[j] : best[o];
+        where[o] = wins ? at + ky * w + j : where[o];
+      }
+    }
+    const int out = row * ow + OUT * xg;
+    if constexpr (OUT == 4) {
+      *reinterpret_cast<float4*>(y + out) = make_float4(best[0], best[1], best[2], best[3]);
+      if (idx) *reinterpret_cast<int4*>(idx + out) = make_int4(where[0], where[1], where[2], where[3]);
+    } else if constexpr (OUT == 2) {
+      *reinterpret_cast<float2*>(y + out) = make_float2(best[0], best[1]);
+      if (idx) *reinterpret_cast<int2*>(idx + out) = make_int2(where[0], where[1]);
+    } else {
+      y[out] = best[0];
+      if (idx) idx[out] = where[0];
+    }
+  }
+}
+template <int KW>
+__global__ void __launch_bounds__(256)
+maxpool_bwd_windows_kernel(int h, int w, int kh, const float* __restrict__ gr, const int32_t* __restrict__ idx, int groups, float* __restrict__ dx) {
+  constexpr int OUT = 4 / KW;
+  const int wg = w / 4, oh = h / kh, ow = w / KW;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < groups; q += gridDim.x * blockDim.x) {
+    const int row = q / wg, xg = q - row * wg;
+    const int pl = row / oh, oy = row - pl * oh;
+    const int at = (pl * h + oy * kh) * w + 4 * xg, out = row * ow + OUT * xg;
+    float g[OUT];
+    int32_t where[OUT];
+    if constexpr (OUT == 4) {
+      const float4 t = __ldg(reinterpret_cast<const float4*>(gr + out));
+      const int4 i = __ldg(reinterpret_cast<const int4*>(idx + out));
+      g[0] = t.x; g[1] = t.y; g[2] = t.z; g[3] = t.w;
+      where[0] = i.x; where[1] = i.y; where[2] = i.z; where[3] = i.w;
+    } else if constexpr (OUT == 2) {
+      const float2 t = __ldg(reinterpret_cast<const float2*>(gr + out));
+      const int2 i = __ldg(reinterpret_cast<const int2*>(idx + out));
+      g[0] = t.x; g[1] = t.y;
+      where[0] = i.x; where[1] = i.y;
+    } else {
+      g[0] = __ldg(gr + out);
+      where[0] = __ldg(idx + out);
+    }
+    for (int ky = 0; ky < kh; ky++) {
+      float v[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) v[j] = where[j / KW] == at + ky * w + j ? g[j / KW] : 0.f;
+      *reinterpret_cast<float4*>(dx + at + ky * w) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+  }
+}
+static bool pool_windows(const PoolGeom& g, int planes, const void* a, const void* b, const void* c) {
+  const uintptr_t any = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c);
+  return g.kh == g.sh && g.kw == g.sw && g.ph == 0 && g.pw == 0 && (g.kw == 1 || g.kw == 2 || g.kw == 4) && (g.w & 3) == 0 && g.h % g.kh == 0 &&
+         (any & 15) == 0 && (int64_t)planes * g.h * g.w < (int64_t)1 << 30;
+}
+
 // The in-bounds window of output (oy, ox) and its divisor (PoolWindow, BackwardNn.cs:490-506).
 __device__ __forceinline__ void pool_window(const PoolGeom& g, int include_pad, int oy, int ox, int* y0, int* y1, int* x0, int* x1, int* count) {
   int ys = oy * g.sh - g.ph, xs = ox * g.sw - g.pw;
@@ -762,7 +841,13 @@ int32_t om_maxpool_fwd(om_ctx* ctx, const float* x, int32_t planes, int32_t h, i
   int64_t total = (int64_t)planes * g.oh * g.ow;
   if (total <= 0) return OM_OK;
   ProfileScope prof(ctx, "om_maxpool_fwd", 0, 4.0 * planes * ((double)h * w + 2.0 * g.oh * g.ow));
-  if ((int64_t)planes * h * w < (int64_t)INT32_MAX) maxpool_fwd_kernel<int><<<grid_for(ctx, total, 256), 256, 0, ctx->stream>>>(g, x, total, y, idx);
+  if (pool_windows(g, planes, x, y, idx)) {
+    const int groups = (int)(total * kw / 4);
+    const int grid = grid_for(ctx, groups, 256);
+    if (kw == 1) maxpool_fwd_windows_kernel<1><<<grid, 256, 0, ctx->stream>>>(h, w, kh, x, groups, y, idx);
+    else if (kw == 2) maxpool_fwd_windows_kernel<2><<<grid, 256, 0, ctx->stream>>>(h, w, kh, x, groups, y, idx);
+    else maxpool_fwd_windows_kernel<4><<<grid, 256, 0, ctx->stream>>>(h, w, kh, x, groups, y, idx);
+  } else if ((int64_t)planes * h * w < (int64_t)INT32_MAX) maxpool_fwd_kernel<int><<<grid_for(ctx, total, 256), 256, 0, ctx->stream>>>(g, x, total, y, idx);
   else maxpool_fwd_kernel<int64_t><<<grid_for(ctx, total, 256), 256, 0, ctx->stream>>>(g, x, total, y, idx);
   OM_LAUNCH_CHECK(ctx, "om_maxpool_fwd");
   return OM_OK;
@@ -777,7 +862,13 @@ int32_t om_maxpool_bwd(om_ctx* ctx, const float* gr, const int32_t* idx, int32_t
   int64_t total = (int64_t)planes * h * w;
   if (total <= 0) return OM_OK;
   ProfileScope prof(ctx, "om_maxpool_bwd", 0, 4.0 * planes * ((double)h * w + 2.0 * oh * ow));
-  if (kh == sh && kw == sw && ph == 0 && pw == 0 && total < (int64_t)1 << 30) {
+  if (pool_windows(g, planes, gr, idx, dx)) {
+    const int groups = (int)(total / kh / 4);
+    const int grid = grid_for(ctx, groups, 256);
+    if (kw == 1) maxpool_bwd_windows_kernel<1><<<grid, 256, 0, ctx->stream>>>(h, w, kh, gr, idx, groups, dx);
+    else if (kw == 2) maxpool_bwd_windows_kernel<2><<<grid, 256, 0, ctx->stream>>>(h, w, kh, gr, idx, groups, dx);
+    else maxpool_bwd_windows_kernel<4><<<grid, 256, 0, ctx->stream>>>(h, w, kh, gr, idx, groups, dx);
+  } else if (kh == sh && kw == sw && ph == 0 && pw == 0 && total < (int64_t)1 << 30) {
     if ((w & 3) == 0 && (reinterpret_cast<uintptr_t>(dx) & 15) == 0)
       maxpool_bwd_tiled_kernel<4><<<grid_for(ctx, total / 4, 256), 256, 0, ctx->stream>>>(h, w, oh, ow, kh, kw, gr, idx, (int)(total / 4), dx);
     else

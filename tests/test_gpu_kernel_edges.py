@@ -268,3 +268,23 @@ def test_conv2d_bias_gradient_planes(ctx, n, cout, h, w):
     ctx.call("om_conv2d_dbias", ctx.handle, C.byref(s), G.ptr, DB.ptr, i32(0))
     want = g.astype(np.float64).sum((0, 2, 3))
     assert np.max(np.abs(DB.numpy() - want) / np.abs(g).astype(np.float64).sum((0, 2, 3))) <= 1e-6
+
+
+@pytest.mark.parametrize("planes,h,w,kh,kw", [(3, 4, 8, 2, 2), (2, 6, 12, 3, 1), (5, 4, 4, 4, 4), (1, 2, 4, 1, 2), (2, 5, 8, 2, 2), (300, 8, 20, 4, 1)])
+def test_max_pool_windows_are_bit_exact(ctx, K, planes, h, w, kh, kw):
+    """Windows that tile the plane: ties go to the first, NaN wins, all -inf; the bits and the indices of the oracle (a height that the window
+    does not divide keeps the general kernels)."""
+    x = np.round(normal(kh * 10 + kw, 1, planes, h, w) * 2) / 2
+    x.reshape(-1)[::17], x[0, 0, :kh, :kw] = np.nan, -np.inf
+    y, idx = K.maxpool_fwd(x, kh, kw, kh, kw, 0, 0)
+    X, Y, I = ctx.to_device(x), ctx.empty(y.shape), ctx.empty(y.shape, np.int32)
+    geometry = [i32(v) for v in (planes, h, w, kh, kw, kh, kw, 0, 0)]
+    ctx.call("om_maxpool_fwd", ctx.handle, X.ptr, *geometry, Y.ptr, I.ptr)
+    assert np.array_equal(Y.numpy(), y, equal_nan=True) and np.array_equal(I.numpy(), idx)
+    g = normal(3, *y.shape)
+    G, DX = ctx.to_device(g), ctx.empty(x.shape)
+    ctx.call("om_maxpool_bwd", ctx.handle, G.ptr, I.ptr, i32(planes), i32(h), i32(w), i32(y.shape[2]), i32(y.shape[3]), i32(kh), i32(kw), i32(kh), i32(kw), i32(0),
+             i32(0), DX.ptr)
+    want = np.zeros(x.size, np.float32)
+    want[idx.reshape(-1)] = g.reshape(-1)
+    assert np.array_equal(DX.numpy().reshape(-1), want)
