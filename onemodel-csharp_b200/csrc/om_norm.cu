@@ -4,6 +4,8 @@
 // partition that depends only on the shape and is combined in a fixed order.
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "om_common.cuh"
 
 namespace om {
@@ -344,19 +346,23 @@ layernorm_fwd_vec_kernel(const float* __restrict__ x, const float* __restrict__ 
   }
 }
 
-// Backward: a CTA owns kLnVecRows consecutive rows, a warp takes every eighth of them; otherwise as layernorm_bwd_fused_kernel.
+// Backward: a CTA owns cta_rows consecutive rows, a warp takes every eighth of them; otherwise as layernorm_bwd_fused_kernel. Eight to 56
+// rows, for about two CTAs an SM on 148 SMs: with 56 whatever the number of rows, 1407 rows were 26 CTAs whose warps walked
+// seven rows one after the other (320 columns: 12.6 us), 5120 were 92 (256 columns: 12.6 us).
 constexpr int kLnVecRows = 56;
+static int ln_cta_rows(int rows) { return std::min<int>(kLnVecRows, 8 * (int)ceil_div(std::max(rows, 1), 8 * 296)); }
 template <int NV>
 __global__ void __launch_bounds__(256, 2)
 layernorm_bwd_vec_kernel(const float* __restrict__ g, const float* __restrict__ x, const float* __restrict__ gamma,
                          const float* __restrict__ mean, const float* __restrict__ inv, int32_t rows, int32_t cols,
-                         float* __restrict__ dx, uint16_t* __restrict__ dx16, double* __restrict__ part_gamma, double* __restrict__ part_beta) {
+                         float* __restrict__ dx, uint16_t* __restrict__ dx16, double* __restrict__ part_gamma, double* __restrict__ part_beta,
+                         int32_t cta_rows) {
   pdl_enter();
   extern __shared__ double ln_smem[];            // [8][cols]
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nv = cols >> 2;
-  const int r0 = blockIdx.x * kLnVecRows;
-  const int r1 = min(rows, r0 + kLnVecRows);
+  const int r0 = blockIdx.x * cta_rows;
+  const int r1 = min(rows, r0 + cta_rows);
   float4 ag[NV], ab[NV];
 #pragma unroll
   for (int i = 0; i < NV; i++) ag[i] = ab[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -664,7 +670,8 @@ int32_t om_layernorm_bwd_b16(om_ctx* ctx, const float* g, const float* x, const 
   auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   const bool vec = (cols & 3) == 0 && al16(g) && al16(x) && al16(gamma) && (!dx || al16(dx)) && (!dx16 || (reinterpret_cast<uintptr_t>(dx16) & 7) == 0);
   // One pass: dx and the CTAs' column partials together; the partials are then added in CTA order.
-  const int used = (int)ceil_div(rows > 0 ? rows : 1, vec ? kLnVecRows : kLnFusedRows);
+  const int cta_rows = ln_cta_rows(rows);
+  const int used = (int)ceil_div(rows > 0 ? rows : 1, vec ? cta_rows : kLnFusedRows);
   double *pg = nullptr, *pb = nullptr;
   if (dgamma) OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)used * cols, false, (void**)&pg));
   if (dbeta) OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)used * cols, false, (void**)&pb));
@@ -685,7 +692,7 @@ int32_t om_layernorm_bwd_b16(om_ctx* ctx, const float* g, const float* x, const 
       OM_CUDA(ctx, cudaFuncSetAttribute(layernorm_bwd_vec_kernel<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 1024 * 8)); \
       attr_set = true;                                                                                                           \
     }                                                                                                                            \
-    launch_chained(ctx, layernorm_bwd_vec_kernel<NV>, used, 256, smem, g, x, gamma, mean, inv, rows, cols, dx, dx16, pg, pb);   \
+    launch_chained(ctx, layernorm_bwd_vec_kernel<NV>, used, 256, smem, g, x, gamma, mean, inv, rows, cols, dx, dx16, pg, pb, cta_rows); \
   } while (0)
   const int nvec = (int)ceil_div(cols, 128);
   if (vec && nvec <= 1) OM_LN_BWDV(1);

@@ -288,3 +288,19 @@ def test_max_pool_windows_are_bit_exact(ctx, K, planes, h, w, kh, kw):
     want = np.zeros(x.size, np.float32)
     want[idx.reshape(-1)] = g.reshape(-1)
     assert np.array_equal(DX.numpy().reshape(-1), want)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 320), (7, 64), (2367, 128), (2369, 256), (296 * 56 + 1, 32), (5000, 384)])
+def test_layer_norm_backward_rows_per_cta(ctx, K, rows, cols):
+    """Eight rows a CTA, the next step of eight, and the most: 1e-4, the gate of the layer norm tests; parameter sums in double."""
+    x, g, gamma = normal(1, rows, cols), normal(2, rows, cols), normal(3, cols)
+    beta = normal(4, cols)
+    X, G, GA, BE = (ctx.to_device(a) for a in (x, g, gamma, beta))
+    Y, M, I, DX, DG, DB = ctx.empty(x.shape), ctx.empty((rows,)), ctx.empty((rows,)), ctx.empty(x.shape), ctx.empty((cols,)), ctx.empty((cols,))
+    ctx.call("om_layernorm_fwd", ctx.handle, X.ptr, GA.ptr, BE.ptr, i32(rows), i32(cols), f32(1e-5), Y.ptr, M.ptr, I.ptr)
+    ctx.call("om_layernorm_bwd", ctx.handle, G.ptr, X.ptr, GA.ptr, M.ptr, I.ptr, i32(rows), i32(cols), DX.ptr, DG.ptr, DB.ptr, i32(0))
+    x64, g64 = x.astype(np.float64), g.astype(np.float64)
+    inv = 1.0 / np.sqrt(x64.var(1, keepdims=True) + 1e-5)
+    xh, dh = (x64 - x64.mean(1, keepdims=True)) * inv, g64 * gamma
+    assert scaled_diff(DX.numpy(), inv * (dh - dh.mean(1, keepdims=True) - xh * (dh * xh).mean(1, keepdims=True))) <= 1e-4
+    assert scaled_diff(DG.numpy(), (g64 * xh).sum(0)) <= 1e-4 and scaled_diff(DB.numpy(), g64.sum(0)) <= 1e-4
