@@ -29,6 +29,7 @@ __device__ __forceinline__ uint32_t taps_inside(const ConvGeom& g, int y0, int x
 
 __global__ void __launch_bounds__(128)
 conv_fma_fwd_kernel(const ConvGeom g, const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ y) {
+  pdl_enter();
   __shared__ __align__(16) float ws[CF_CHUNK][CF_CH];
   __shared__ int2 ks[CF_CHUNK];        // offset of k in the image, its tap's bit
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -100,6 +101,7 @@ conv_fma_fwd_kernel(const ConvGeom g, const float* __restrict__ x, const float* 
 
 __global__ void __launch_bounds__(128)
 conv_fma_dgrad_kernel(const ConvGeom g, const float* __restrict__ gr, const float* __restrict__ w, float* __restrict__ dx) {
+  pdl_enter();
   __shared__ __align__(16) float ws[CF_CHUNK][CF_CH];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int plane = g.oh * g.ow, hw = g.h * g.w, taps = g.kh * g.kw, kk = g.cin * taps;
@@ -180,6 +182,7 @@ conv_fma_dgrad_kernel(const ConvGeom g, const float* __restrict__ gr, const floa
 constexpr int CF_COLS = 128, CF_LD = 36;
 __global__ void __launch_bounds__(128)
 conv_fma_wgrad_kernel(const ConvGeom g, const float* __restrict__ gr, const float* __restrict__ x, int per_slice, float* __restrict__ part) {
+  pdl_enter();
   __shared__ __align__(16) float gs[CF_CH][CF_LD];
   __shared__ __align__(16) float xs[CF_COLS][CF_LD];
   __shared__ int2 ks[CF_COLS];
@@ -251,6 +254,7 @@ conv_fma_wgrad_kernel(const ConvGeom g, const float* __restrict__ gr, const floa
 
 // dw (+)= the slices in a fixed order: eight shares of a value's slices, each in increasing order, then the shares.
 __global__ void __launch_bounds__(256) conv_fma_finish_kernel(const float* __restrict__ part, int slices, int len, float* __restrict__ dw, int accumulate) {
+  pdl_enter();
   __shared__ float sums[8][32];
   const int lane = threadIdx.x & 31, share = threadIdx.x >> 5, at = blockIdx.x * 32 + lane;
   float acc = 0.f;
@@ -294,14 +298,14 @@ bool conv_fma_wgrad_fits(const ConvGeom& g) { return sizes_fit(g) && g.cin * g.k
 
 int32_t conv_fma_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y) {
   const dim3 grid((unsigned)ceil_div((int64_t)g.n * g.oh * g.ow, CF_TILE), (unsigned)ceil_div(g.cout, CF_CH));
-  conv_fma_fwd_kernel<<<grid, 128, 0, ctx->stream>>>(g, x, w, bias, y);
+  launch_chained(ctx, conv_fma_fwd_kernel, grid, 128, 0, g, x, w, bias, y);
   OM_LAUNCH_CHECK(ctx, "conv_fma_fwd");
   return OM_OK;
 }
 
 int32_t conv_fma_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx) {
   const dim3 grid((unsigned)ceil_div((int64_t)g.n * g.h * g.w, CF_TILE), (unsigned)ceil_div(g.cin, CF_CH));
-  conv_fma_dgrad_kernel<<<grid, 128, 0, ctx->stream>>>(g, gr, w, dx);
+  launch_chained(ctx, conv_fma_dgrad_kernel, grid, 128, 0, g, gr, w, dx);
   OM_LAUNCH_CHECK(ctx, "conv_fma_dgrad");
   return OM_OK;
 }
@@ -314,8 +318,8 @@ int32_t conv_fma_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const fl
   const int slices = (int)ceil_div(pixels, per_slice);
   float* part = nullptr;
   OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)slices * len, false, (void**)&part));
-  conv_fma_wgrad_kernel<<<dim3((unsigned)ceil_div(kk, CF_COLS), (unsigned)ceil_div(g.cout, CF_CH), (unsigned)slices), 128, 0, ctx->stream>>>(g, gr, x, per_slice, part);
-  conv_fma_finish_kernel<<<(unsigned)ceil_div(len, 32), 256, 0, ctx->stream>>>(part, slices, len, dw, accumulate);
+  launch_chained(ctx, conv_fma_wgrad_kernel, dim3((unsigned)ceil_div(kk, CF_COLS), (unsigned)ceil_div(g.cout, CF_CH), (unsigned)slices), 128, 0, g, gr, x, per_slice, part);
+  launch_chained(ctx, conv_fma_finish_kernel, (unsigned)ceil_div(len, 32), 256, 0, part, slices, len, dw, accumulate);
   pool_free(ctx, part);
   OM_LAUNCH_CHECK(ctx, "conv_fma_wgrad");
   return OM_OK;

@@ -205,6 +205,8 @@ conv_tc_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();   // tensor memory is held: later kernels may become resident
+  pdl_wait();      // everything below may depend on the previous kernel
 
   if (warp < CV_PRODUCERS) {
     // ---- gather: a thread owns a pixel and two of a stage's four units ----
@@ -341,6 +343,7 @@ struct ConvTurn {
 };
 template <int UNIT, int GROUP>
 __global__ void __launch_bounds__(256) conv_turn_weights_kernel(const float* __restrict__ w, float* __restrict__ wt, const __grid_constant__ ConvTurn t) {
+  pdl_enter();
   const int z = blockIdx.z, m = blockIdx.y;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < t.ld[z]; i += gridDim.x * blockDim.x) {
     int tap, c0;
@@ -401,6 +404,8 @@ conv_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();   // tensor memory is held: later kernels may become resident
+  pdl_wait();      // everything below may depend on the previous kernel
 
   if (warp < CV_PRODUCERS) {
     bool ok = true;
@@ -517,6 +522,7 @@ conv_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
 template <int SHARES, int UNIT, int GROUP>
 __global__ void __launch_bounds__(256)
 conv_wgrad_finish_kernel(const float* __restrict__ part, int splits, int cout, int units, int cin, int taps, float* __restrict__ dw, int accumulate) {
+  pdl_enter();
   constexpr int COLS = 256 / SHARES;
   __shared__ float sums[SHARES][COLS];
   const int ld = units * UNIT, lane = threadIdx.x % COLS, share = threadIdx.x / COLS;
@@ -575,6 +581,7 @@ struct ConvNhwcMaps {
 // t[q][c] = s[n][c][p] for pixel q = n * plane + p; rows of cp floats (c rounded up to a multiple of four, zero there).
 constexpr int CN_PX = 64;
 __global__ void __launch_bounds__(256) conv_channels_last_kernel(const float* __restrict__ src, float* __restrict__ t, int pixels, int plane, CvDiv div_plane, int c, int cp) {
+  pdl_enter();
   __shared__ float tile[32][CN_PX + 1];
   const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
   const int q0 = blockIdx.x * CN_PX, c0 = blockIdx.y * 32;
@@ -638,6 +645,8 @@ conv_nhwc_kernel(const __grid_constant__ ConvNhwcMaps maps, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();   // tensor memory is held: later kernels may become resident
+  pdl_wait();      // everything below may depend on the previous kernel
 
   if (warp == 0) {
     if (lane == 0) {
@@ -750,6 +759,8 @@ conv_nhwc_wgrad_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();   // tensor memory is held: later kernels may become resident
+  pdl_wait();      // everything below may depend on the previous kernel
 
   if (warp == 0) {
     if (lane == 0) {
@@ -865,7 +876,7 @@ static int32_t launch_conv_as(om_ctx* ctx, const ConvMaps& maps, const ConvTcPar
     OM_CUDA(ctx, cudaFuncSetAttribute(conv_tc_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     set = true;
   }
-  conv_tc_kernel<MT><<<grid, CV_THREADS, smem, ctx->stream>>>(maps, p);
+  launch_chained(ctx, conv_tc_kernel<MT>, grid, CV_THREADS, smem, maps, p);
   OM_LAUNCH_CHECK(ctx, "conv_tc");
   return OM_OK;
 }
@@ -898,7 +909,7 @@ static int32_t run_conv(om_ctx* ctx, ConvTcParams& p, ConvTurn& turn, int phases
       st = fail(ctx, OM_ERR_CUDA, "cuTensorMapEncodeTiled failed for a convolution's turned weights");
   if (st == OM_OK) {
     if (most_units > 0)
-      conv_turn_weights_kernel<CV_UNIT, CV_GROUP><<<dim3((unsigned)std::min<int64_t>(ceil_div(most_units * CV_UNIT, 256), 64), (unsigned)p.m, (unsigned)phases), 256, 0, ctx->stream>>>(
+      launch_chained(ctx, conv_turn_weights_kernel<CV_UNIT, CV_GROUP>, dim3((unsigned)std::min<int64_t>(ceil_div(most_units * CV_UNIT, 256), 64), (unsigned)p.m, (unsigned)phases), 256, 0, 
           w, wt, turn);
     // Two accumulators once that still leaves a CTA for every SM.
     const bool two = p.m > CV_TILE && all * ceil_div(p.m, 2 * CV_TILE) >= 148;
@@ -974,10 +985,10 @@ template <int UNIT, int GROUP>
 static void launch_finish(om_ctx* ctx, const float* part, int splits, const ConvGeom& g, int units, float* dw, int accumulate) {
   const int ld = units * UNIT;
   if (splits <= 8)
-    conv_wgrad_finish_kernel<1, UNIT, GROUP><<<dim3((unsigned)ceil_div(ld, 256), (unsigned)g.cout), 256, 0, ctx->stream>>>(part, splits, g.cout, units, g.cin,
+    launch_chained(ctx, conv_wgrad_finish_kernel<1, UNIT, GROUP>, dim3((unsigned)ceil_div(ld, 256), (unsigned)g.cout), 256, 0, part, splits, g.cout, units, g.cin,
                                                                                                                         g.kh * g.kw, dw, accumulate);
   else
-    conv_wgrad_finish_kernel<8, UNIT, GROUP><<<dim3((unsigned)ceil_div(ld, 32), (unsigned)g.cout), 256, 0, ctx->stream>>>(part, splits, g.cout, units, g.cin,
+    launch_chained(ctx, conv_wgrad_finish_kernel<8, UNIT, GROUP>, dim3((unsigned)ceil_div(ld, 32), (unsigned)g.cout), 256, 0, part, splits, g.cout, units, g.cin,
                                                                                                                        g.kh * g.kw, dw, accumulate);
 }
 
@@ -991,7 +1002,7 @@ static int32_t launch_wgrad(om_ctx* ctx, const CUtensorMap& map, const ConvWgrad
     OM_CUDA(ctx, cudaFuncSetAttribute(conv_wgrad_tc_kernel<A_TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     set = true;
   }
-  conv_wgrad_tc_kernel<A_TMA><<<grid, CV_THREADS, smem, ctx->stream>>>(map, p);
+  launch_chained(ctx, conv_wgrad_tc_kernel<A_TMA>, grid, CV_THREADS, smem, map, p);
   return OM_OK;
 }
 
@@ -1058,7 +1069,7 @@ static bool cn_map(CUtensorMap* map, const float* base, int c, int w, int h, int
 static int32_t cn_turn(om_ctx* ctx, const float* src, int n, int c, int plane, float** out) {
   const int pixels = n * plane, cp = cn_pitch(c);
   OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)pixels * cp, false, (void**)out));
-  conv_channels_last_kernel<<<dim3((unsigned)ceil_div(pixels, CN_PX), (unsigned)ceil_div(cp, 32)), 256, 0, ctx->stream>>>(src, *out, pixels, plane,
+  launch_chained(ctx, conv_channels_last_kernel, dim3((unsigned)ceil_div(pixels, CN_PX), (unsigned)ceil_div(cp, 32)), 256, 0, src, *out, pixels, plane,
                                                                                                                       cv_div((uint32_t)plane), c, cp);
   return OM_OK;
 }
@@ -1105,7 +1116,7 @@ static int32_t run_conv_nhwc(om_ctx* ctx, ConvNhwcParams& p, ConvTurn& turn, int
   }
   if (st == OM_OK && most > 0) {
     if (most_ld > 0)
-      conv_turn_weights_kernel<CV_BK, 1><<<dim3((unsigned)std::min<int64_t>(ceil_div(most_ld, 256), 64), (unsigned)p.m, (unsigned)phases), 256, 0, ctx->stream>>>(w, wt, turn);
+      launch_chained(ctx, conv_turn_weights_kernel<CV_BK, 1>, dim3((unsigned)std::min<int64_t>(ceil_div(most_ld, 256), 64), (unsigned)p.m, (unsigned)phases), 256, 0, w, wt, turn);
     const dim3 grid((unsigned)most, (unsigned)ceil_div(p.m, nt), (unsigned)phases);
     static bool set = false;
     constexpr size_t smem64 = (size_t)4 * (CV_BLOCK + 64 * 128) + 1024 + 128, smem128 = (size_t)3 * (CV_BLOCK + 128 * 128) + 1024 + 128;
@@ -1115,8 +1126,8 @@ static int32_t run_conv_nhwc(om_ctx* ctx, ConvNhwcParams& p, ConvTurn& turn, int
       set = st == OM_OK;
     }
     if (st == OM_OK) {
-      if (nt == 64) conv_nhwc_kernel<64><<<grid, CN_THREADS, smem64, ctx->stream>>>(maps, p);
-      else conv_nhwc_kernel<128><<<grid, CN_THREADS, smem128, ctx->stream>>>(maps, p);
+      if (nt == 64) launch_chained(ctx, conv_nhwc_kernel<64>, grid, CN_THREADS, smem64, maps, p);
+      else launch_chained(ctx, conv_nhwc_kernel<128>, grid, CN_THREADS, smem128, maps, p);
       st = check_cuda(ctx, cudaGetLastError(), "conv_nhwc");
     }
   }
@@ -1210,7 +1221,7 @@ int32_t conv_nhwc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const f
       set = st == OM_OK;
     }
     if (st == OM_OK) {
-      conv_nhwc_wgrad_kernel<<<dim3((unsigned)tn, (unsigned)tm, (unsigned)splits), CN_THREADS, smem, ctx->stream>>>(map_g, map_x, p);
+      launch_chained(ctx, conv_nhwc_wgrad_kernel, dim3((unsigned)tn, (unsigned)tm, (unsigned)splits), CN_THREADS, smem, map_g, map_x, p);
       launch_finish<CV_BK, 1>(ctx, p.part, splits, g, p.units, dw, accumulate);
       st = check_cuda(ctx, cudaGetLastError(), "conv_nhwc_wgrad");
     }

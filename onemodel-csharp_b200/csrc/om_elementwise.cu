@@ -521,6 +521,7 @@ __global__ void sum_to_generic_kernel(SumToShape s, const float* __restrict__ g,
 // Sum/Mean over the middle axis of [outer, n, inner] with a double accumulator in increasing order.
 __global__ void reduce_fwd_kernel(const float* __restrict__ x, int64_t outer, int64_t n, int64_t inner, int mean,
                                   float* __restrict__ y) {
+  pdl_enter();
   int64_t total = outer * inner;
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -548,6 +549,7 @@ __global__ void reduce_all_kernel(const float* __restrict__ x, int64_t n, int me
 
 __global__ void reduce_bwd_kernel(const float* __restrict__ g, int64_t outer, int64_t n, int64_t inner, int mean,
                                   float* __restrict__ dx) {
+  pdl_enter();
   int64_t total = outer * n * inner;
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -912,7 +914,7 @@ int32_t om_reduce_fwd(om_ctx* ctx, const float* x, int64_t outer, int64_t n, int
   if (outer * inner == 1 && n > 4096) {
     reduce_all_kernel<<<1, 1024, 0, ctx->stream>>>(x, n, mean, y);
   } else {
-    reduce_fwd_kernel<<<grid_for(ctx, outer * inner, 128), 128, 0, ctx->stream>>>(x, outer, n, inner, mean, y);
+    launch_chained(ctx, reduce_fwd_kernel, grid_for(ctx, outer * inner, 128), 128, 0, x, outer, n, inner, mean, y);
   }
   OM_LAUNCH_CHECK(ctx, "om_reduce_fwd");
   return OM_OK;
@@ -924,7 +926,7 @@ int32_t om_reduce_bwd(om_ctx* ctx, const float* g, int64_t outer, int64_t n, int
   int64_t total = outer * n * inner;
   if (total == 0) return OM_OK;
   ProfileScope prof(ctx, "om_reduce_bwd", 0, 4.0 * total);
-  reduce_bwd_kernel<<<grid_for(ctx, total, 256), 256, 0, ctx->stream>>>(g, outer, n, inner, mean, dx);
+  launch_chained(ctx, reduce_bwd_kernel, grid_for(ctx, total, 256), 256, 0, g, outer, n, inner, mean, dx);
   OM_LAUNCH_CHECK(ctx, "om_reduce_bwd");
   return OM_OK;
 }

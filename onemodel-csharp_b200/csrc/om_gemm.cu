@@ -21,6 +21,7 @@ int32_t gemm_tc_batched(om_ctx* ctx, int ta, int tb, int m, int n, int k, const 
                         int ldb, long long sB, float* C, int ldc, long long sC, int batch, int acc, const float* bias);
 
 __global__ void add_bias_rows_kernel(float* __restrict__ y, const float* __restrict__ bias, int64_t rows, int32_t cols, int64_t ld) {
+  pdl_enter();
   int64_t total = rows * cols;
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -79,7 +80,7 @@ int32_t gemm_dispatch(om_ctx* ctx, int ta, int tb, int m, int n, int k, const fl
   if (bias && gemm_simt_takes_bias(m, n)) return gemm_simt_bias(ctx, ta, tb, m, n, k, A, lda, B, ldb, C, ldc, acc, bias);
   OM_TRY(gemm_simt(ctx, ta, tb, m, n, k, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, acc));
   if (bias) {
-    add_bias_rows_kernel<<<grid_for(ctx, ((int64_t)m * n + 3) / 4, 256), 256, 0, ctx->stream>>>(C, bias, m, n, ldc);
+    launch_chained(ctx, add_bias_rows_kernel, grid_for(ctx, ((int64_t)m * n + 3) / 4, 256), 256, 0, C, bias, m, n, ldc);
     OM_LAUNCH_CHECK(ctx, "add_bias_rows");
   }
   return OM_OK;

@@ -13,6 +13,7 @@ gemm_simt_kernel(int m, int n, int k, const float* __restrict__ A, int lda, int6
                  const float* __restrict__ B, int ldb, int64_t strideB, float* __restrict__ C, int ldc,
                  int64_t strideC, int accumulate, int batch, int batch_per_z, int inner, int64_t innerA, int64_t innerB,
                  int64_t innerC) {
+  pdl_enter();
   constexpr int THREADS = (BM / TM) * (BN / TN);
   __shared__ float As[BK][BM + 4];
   __shared__ float Bs[BK][BN + 4];
@@ -129,6 +130,7 @@ __global__ void __launch_bounds__(kSmallTile * kSmallTile)
 gemm_small_kernel(int m, int n, int k, const float* __restrict__ A, int lda, int64_t strideA, const float* __restrict__ B, int ldb,
                   int64_t strideB, float* __restrict__ C, int ldc, int64_t strideC, int accumulate, int inner, int64_t innerA,
                   int64_t innerB, int64_t innerC, const float* __restrict__ bias) {
+  pdl_enter();
   __shared__ __align__(16) float As[kSmallTile][kSmallK + 4];
   __shared__ __align__(16) float Bs[kSmallTile][kSmallK + 4];
   constexpr int THREADS = kSmallTile * kSmallTile, LOADS = kSmallTile * kSmallK / THREADS;
@@ -194,10 +196,10 @@ static void launch_simt(om_ctx* ctx, int ta, int tb, int m, int n, int k, const 
                         int inner = 1, int64_t iA = 0, int64_t iB = 0, int64_t iC = 0) {
   dim3 grid((unsigned)ceil_div(n, BN), (unsigned)ceil_div(m, BM), (unsigned)(bpz ? ceil_div(batch, bpz) : batch));
   constexpr int T = (BM / TM) * (BN / TN);
-  if (!ta && !tb) gemm_simt_kernel<BM, BN, BK, TM, TN, false, false><<<grid, T, 0, ctx->stream>>>(m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, acc, batch, bpz, inner, iA, iB, iC);
-  else if (!ta && tb) gemm_simt_kernel<BM, BN, BK, TM, TN, false, true><<<grid, T, 0, ctx->stream>>>(m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, acc, batch, bpz, inner, iA, iB, iC);
-  else if (ta && !tb) gemm_simt_kernel<BM, BN, BK, TM, TN, true, false><<<grid, T, 0, ctx->stream>>>(m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, acc, batch, bpz, inner, iA, iB, iC);
-  else gemm_simt_kernel<BM, BN, BK, TM, TN, true, true><<<grid, T, 0, ctx->stream>>>(m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, acc, batch, bpz, inner, iA, iB, iC);
+  if (!ta && !tb) launch_chained(ctx, gemm_simt_kernel<BM, BN, BK, TM, TN, false, false>, grid, T, 0, m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, acc, batch, bpz, inner, iA, iB, iC);
+  else if (!ta && tb) launch_chained(ctx, gemm_simt_kernel<BM, BN, BK, TM, TN, false, true>, grid, T, 0, m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, acc, batch, bpz, inner, iA, iB, iC);
+  else if (ta && !tb) launch_chained(ctx, gemm_simt_kernel<BM, BN, BK, TM, TN, true, false>, grid, T, 0, m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, acc, batch, bpz, inner, iA, iB, iC);
+  else launch_chained(ctx, gemm_simt_kernel<BM, BN, BK, TM, TN, true, true>, grid, T, 0, m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, acc, batch, bpz, inner, iA, iB, iC);
 }
 
 static int32_t gemm_simt_any(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, int64_t sA, int64_t iA,
@@ -208,7 +210,7 @@ static int32_t gemm_simt_any(om_ctx* ctx, int ta, int tb, int m, int n, int k, c
   if ((int64_t)m * n * batch <= kSmallOutputs && batch <= 65535) {
     const dim3 grid((unsigned)ceil_div(n, kSmallTile), (unsigned)ceil_div(m, kSmallTile), (unsigned)batch);
 #define OM_SMALL(TA, TB) \
-  gemm_small_kernel<TA, TB><<<grid, kSmallTile * kSmallTile, 0, ctx->stream>>>(m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, acc, inner, iA, iB, iC, bias)
+  launch_chained(ctx, gemm_small_kernel<TA, TB>, grid, kSmallTile * kSmallTile, 0, m, n, k, A, lda, sA, B, ldb, sB, C, ldc, sC, acc, inner, iA, iB, iC, bias)
     if (!ta && !tb) OM_SMALL(false, false);
     else if (!ta) OM_SMALL(false, true);
     else if (!tb) OM_SMALL(true, false);

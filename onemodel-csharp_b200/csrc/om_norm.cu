@@ -448,6 +448,7 @@ __global__ void __launch_bounds__(kBnThreads)
 bn_partial_kernel(const float* __restrict__ x, const float* __restrict__ g, const double* __restrict__ mu64,
                   const float* __restrict__ mean, const float* __restrict__ inv, int32_t n, int32_t c, int32_t plane,
                   int32_t ipc, double* __restrict__ pa, double* __restrict__ pb) {
+  pdl_enter();
   __shared__ double sa[kBnThreads / 32], sb[kBnThreads / 32];
   const int ch = blockIdx.x, slice = blockIdx.y;
   const int i0 = slice * ipc, i1 = min(n, i0 + ipc);
@@ -504,6 +505,7 @@ bn_partial_kernel(const float* __restrict__ x, const float* __restrict__ g, cons
 }
 
 __global__ void bn_mean_kernel(const double* __restrict__ pa, int slices, int32_t c, double m, double* __restrict__ mu64) {
+  pdl_enter();
   int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
   double t = 0.0;
@@ -514,6 +516,7 @@ __global__ void bn_mean_kernel(const double* __restrict__ pa, int slices, int32_
 __global__ void bn_finish_stats_kernel(const double* __restrict__ pa, const double* __restrict__ mu64, int slices,
                                        int32_t c, double m, float momentum, float eps, float* __restrict__ mean,
                                        float* __restrict__ inv, float* __restrict__ rm, float* __restrict__ rv) {
+  pdl_enter();
   int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
   double ss = 0.0;
@@ -531,6 +534,7 @@ __global__ void bn_finish_stats_kernel(const double* __restrict__ pa, const doub
 
 __global__ void bn_eval_stats_kernel(const float* __restrict__ rm, const float* __restrict__ rv, int32_t c, float eps,
                                      float* __restrict__ mean, float* __restrict__ inv) {
+  pdl_enter();
   int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
   mean[ch] = rm[ch];
@@ -543,6 +547,7 @@ __global__ void __launch_bounds__(256)
 bn_apply_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
                 const float* __restrict__ mean, const float* __restrict__ inv, int64_t total, int32_t c, int32_t plane,
                 float* __restrict__ y) {
+  pdl_enter();
   int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * VEC;
   int64_t stride = (int64_t)gridDim.x * blockDim.x * VEC;
   for (int64_t e = i; e < total; e += stride) {
@@ -562,6 +567,7 @@ bn_apply_kernel(const float* __restrict__ x, const float* __restrict__ gamma, co
 // Per-channel scalars of the backward: k = gamma * inv, cb = mean(g), cg = mean(g * xhat), from the slice partials.
 __global__ void bn_bwd_coef_kernel(const float* __restrict__ gamma, const float* __restrict__ inv, const double* __restrict__ pa,
                                    const double* __restrict__ pb, int slices, double m, int32_t c, float* __restrict__ coef) {
+  pdl_enter();
   int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
   double sg = 0.0, sb = 0.0;
@@ -579,6 +585,7 @@ __global__ void __launch_bounds__(256)
 bn_bwd_apply_kernel(const float* __restrict__ g, const float* __restrict__ x, const float* __restrict__ mean,
                     const float* __restrict__ inv, const float* __restrict__ coef, int64_t total, int32_t c, int32_t plane,
                     int training, float* __restrict__ dx) {
+  pdl_enter();
   int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * VEC;
   int64_t stride = (int64_t)gridDim.x * blockDim.x * VEC;
   for (int64_t e = i; e < total; e += stride) {
@@ -741,20 +748,20 @@ int32_t om_batchnorm_fwd(om_ctx* ctx, const float* x, const float* gamma, const 
     OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)c, false, (void**)&mu64));
     double m = (double)n * plane;
     dim3 grid(c, slices);
-    bn_partial_kernel<0><<<grid, kBnThreads, 0, ctx->stream>>>(x, nullptr, nullptr, nullptr, nullptr, n, c, plane, ipc, pa, nullptr);
-    bn_mean_kernel<<<(unsigned)ceil_div(c, 128), 128, 0, ctx->stream>>>(pa, slices, c, m, mu64);
-    bn_partial_kernel<1><<<grid, kBnThreads, 0, ctx->stream>>>(x, nullptr, mu64, nullptr, nullptr, n, c, plane, ipc, pa, nullptr);
-    bn_finish_stats_kernel<<<(unsigned)ceil_div(c, 128), 128, 0, ctx->stream>>>(pa, mu64, slices, c, m, momentum, eps, mean, inv, running_mean, running_var);
+    launch_chained(ctx, bn_partial_kernel<0>, grid, kBnThreads, 0, x, nullptr, nullptr, nullptr, nullptr, n, c, plane, ipc, pa, nullptr);
+    launch_chained(ctx, bn_mean_kernel, (unsigned)ceil_div(c, 128), 128, 0, pa, slices, c, m, mu64);
+    launch_chained(ctx, bn_partial_kernel<1>, grid, kBnThreads, 0, x, nullptr, mu64, nullptr, nullptr, n, c, plane, ipc, pa, nullptr);
+    launch_chained(ctx, bn_finish_stats_kernel, (unsigned)ceil_div(c, 128), 128, 0, pa, mu64, slices, c, m, momentum, eps, mean, inv, running_mean, running_var);
     pool_free(ctx, pa);
     pool_free(ctx, mu64);
   } else {
-    bn_eval_stats_kernel<<<(unsigned)ceil_div(c, 128), 128, 0, ctx->stream>>>(running_mean, running_var, c, eps, mean, inv);
+    launch_chained(ctx, bn_eval_stats_kernel, (unsigned)ceil_div(c, 128), 128, 0, running_mean, running_var, c, eps, mean, inv);
   }
   int64_t planes = (int64_t)n * c;
   if (planes > 0 && plane > 0) {
     const int64_t total = planes * plane;
-    if ((plane & 3) == 0) bn_apply_kernel<4><<<grid_for(ctx, total / 4, 256), 256, 0, ctx->stream>>>(x, gamma, beta, mean, inv, total, c, plane, y);
-    else bn_apply_kernel<1><<<grid_for(ctx, total, 256), 256, 0, ctx->stream>>>(x, gamma, beta, mean, inv, total, c, plane, y);
+    if ((plane & 3) == 0) launch_chained(ctx, bn_apply_kernel<4>, grid_for(ctx, total / 4, 256), 256, 0, x, gamma, beta, mean, inv, total, c, plane, y);
+    else launch_chained(ctx, bn_apply_kernel<1>, grid_for(ctx, total, 256), 256, 0, x, gamma, beta, mean, inv, total, c, plane, y);
   }
   OM_LAUNCH_CHECK(ctx, "om_batchnorm_fwd");
   return OM_OK;
@@ -772,15 +779,15 @@ int32_t om_batchnorm_bwd(om_ctx* ctx, const float* g, const float* x, const floa
   double *pa = nullptr, *pb = nullptr;
   OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)slices * c, false, (void**)&pa));
   OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)slices * c, false, (void**)&pb));
-  bn_partial_kernel<2><<<dim3(c, slices), kBnThreads, 0, ctx->stream>>>(x, g, nullptr, mean, inv, n, c, plane, ipc, pa, pb);
+  launch_chained(ctx, bn_partial_kernel<2>, dim3(c, slices), kBnThreads, 0, x, g, nullptr, mean, inv, n, c, plane, ipc, pa, pb);
   int64_t planes = (int64_t)n * c;
   if (dx && planes > 0 && plane > 0) {
     float* coef = nullptr;
     OM_TRY(pool_alloc(ctx, sizeof(float) * 3 * (size_t)c, false, (void**)&coef));
-    bn_bwd_coef_kernel<<<(unsigned)ceil_div(c, 128), 128, 0, ctx->stream>>>(gamma, inv, pa, pb, slices, (double)n * plane, c, coef);
+    launch_chained(ctx, bn_bwd_coef_kernel, (unsigned)ceil_div(c, 128), 128, 0, gamma, inv, pa, pb, slices, (double)n * plane, c, coef);
     const int64_t total = planes * plane;
-    if ((plane & 3) == 0) bn_bwd_apply_kernel<4><<<grid_for(ctx, total / 4, 256), 256, 0, ctx->stream>>>(g, x, mean, inv, coef, total, c, plane, training, dx);
-    else bn_bwd_apply_kernel<1><<<grid_for(ctx, total, 256), 256, 0, ctx->stream>>>(g, x, mean, inv, coef, total, c, plane, training, dx);
+    if ((plane & 3) == 0) launch_chained(ctx, bn_bwd_apply_kernel<4>, grid_for(ctx, total / 4, 256), 256, 0, g, x, mean, inv, coef, total, c, plane, training, dx);
+    else launch_chained(ctx, bn_bwd_apply_kernel<1>, grid_for(ctx, total, 256), 256, 0, g, x, mean, inv, coef, total, c, plane, training, dx);
     pool_free(ctx, coef);
   }
   if (dgamma || dbeta)

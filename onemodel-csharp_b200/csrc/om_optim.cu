@@ -139,6 +139,7 @@ __device__ __forceinline__ void sgd_element(float& p, float g, float& buf, bool 
 // in visits of 16384 elements. On the first step the momentum buffer is written without being read, as before.
 __global__ void __launch_bounds__(256)
 sgd_kernel(TensorTable t, om_sgd_hyper hv, const om_sgd_hyper* __restrict__ hd) {
+  pdl_enter();
   const om_sgd_hyper h = hd ? *hd : hv;
   const float keep = __fsub_rn(1.0f, h.dampening);
   const int total = t.chunk_prefix[t.n];
@@ -445,7 +446,7 @@ int32_t om_optim_sgd_step(om_ctx* ctx, int32_t n_tensors, float* const* p, const
     int count = std::min(kMaxTensors, n_tensors - base);
     int chunks = fill_table(t, base, count, p, g, buf, nullptr, nullptr, first, len, update_chunk(table_total(base, count, len)));
     if (chunks == 0) continue;
-    sgd_kernel<<<grid_chunks(ctx, chunks), 256, 0, ctx->stream>>>(t, *hyper_host, hyper_dev);
+    launch_chained(ctx, sgd_kernel, grid_chunks(ctx, chunks), 256, 0, t, *hyper_host, hyper_dev);
     OM_LAUNCH_CHECK(ctx, "om_optim_sgd_step");
   }
   return OM_OK;

@@ -201,6 +201,7 @@ constexpr int kDbiasSlices = 16;
 template <int VEC>
 __global__ void __launch_bounds__(256)
 conv_dbias_partial_kernel(const float* __restrict__ g, int n, int cout, int plane, int per_slice, double* __restrict__ partial) {
+  pdl_enter();
   __shared__ double sm[256];
   const int co = blockIdx.x, slice = blockIdx.y;
   const int i0 = slice * per_slice, i1 = min(n, i0 + per_slice);
@@ -247,6 +248,7 @@ conv_dbias_partial_kernel(const float* __restrict__ g, int n, int cout, int plan
   if (threadIdx.x == 0) partial[(int64_t)slice * cout + co] = sm[0];
 }
 __global__ void conv_dbias_finish_kernel(const double* __restrict__ partial, int slices, int cout, float* __restrict__ dbias, int accumulate) {
+  pdl_enter();
   int co = blockIdx.x * blockDim.x + threadIdx.x;
   if (co >= cout) return;
   double t = 0.0;
@@ -281,6 +283,7 @@ static bool pool_out(int size, int kernel, int stride, int pad, int* out) {
 // IDX: int when the input has fewer than 2^31 elements (32-bit divisions).
 template <typename IDX>
 __global__ void maxpool_fwd_kernel(PoolGeom g, const float* __restrict__ x, int64_t total, float* __restrict__ y, int32_t* __restrict__ idx) {
+  pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t e = i; e < total; e += stride) {
@@ -314,6 +317,7 @@ __global__ void maxpool_fwd_kernel(PoolGeom g, const float* __restrict__ x, int6
 // dx[j] = sum of g[i] over the outputs i (in increasing i) whose saved index is j.
 __global__ void maxpool_bwd_kernel(PoolGeom g, const float* __restrict__ gr, const int32_t* __restrict__ idx, int64_t total,
                                    float* __restrict__ dx) {
+  pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t e = i; e < total; e += stride) {
@@ -337,6 +341,7 @@ __global__ void maxpool_bwd_kernel(PoolGeom g, const float* __restrict__ gr, con
 template <int VEC>
 __global__ void maxpool_bwd_tiled_kernel(int h, int w, int oh, int ow, int kh, int kw, const float* __restrict__ gr,
                                          const int32_t* __restrict__ idx, int groups, float* __restrict__ dx) {
+  pdl_enter();
   const int stride = gridDim.x * blockDim.x;
   const int wg = w / VEC;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < groups; q += stride) {
@@ -380,6 +385,7 @@ __global__ void maxpool_bwd_tiled_kernel(int h, int w, int oh, int ow, int kh, i
 template <int KW>
 __global__ void __launch_bounds__(256)
 maxpool_fwd_windows_kernel(int h, int w, int kh, const float* __restrict__ x, int groups, float* __restrict__ y, int32_t* __restrict__ idx) {
+  pdl_enter();
   constexpr int OUT = 4 / KW;
   const int wg = w / 4, oh = h / kh, ow = w / KW;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < groups; q += gridDim.x * blockDim.x) {
@@ -416,6 +422,7 @@ maxpool_fwd_windows_kernel(int h, int w, int kh, const float* __restrict__ x, in
 template <int KW>
 __global__ void __launch_bounds__(256)
 maxpool_bwd_windows_kernel(int h, int w, int kh, const float* __restrict__ gr, const int32_t* __restrict__ idx, int groups, float* __restrict__ dx) {
+  pdl_enter();
   constexpr int OUT = 4 / KW;
   const int wg = w / 4, oh = h / kh, ow = w / KW;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < groups; q += gridDim.x * blockDim.x) {
@@ -789,10 +796,10 @@ int32_t om_conv2d_dbias(om_ctx* ctx, const om_conv_shape* s, const float* gr, fl
   OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)slices * g.cout, false, (void**)&partial));
   const int plane = g.oh * g.ow;
   if ((plane & 3) == 0 && (reinterpret_cast<uintptr_t>(gr) & 15) == 0)
-    conv_dbias_partial_kernel<4><<<dim3(g.cout, slices), 256, 0, ctx->stream>>>(gr, g.n, g.cout, plane, per_slice, partial);
+    launch_chained(ctx, conv_dbias_partial_kernel<4>, dim3(g.cout, slices), 256, 0, gr, g.n, g.cout, plane, per_slice, partial);
   else
-    conv_dbias_partial_kernel<1><<<dim3(g.cout, slices), 256, 0, ctx->stream>>>(gr, g.n, g.cout, plane, per_slice, partial);
-  conv_dbias_finish_kernel<<<(unsigned)ceil_div(g.cout, 128), 128, 0, ctx->stream>>>(partial, slices, g.cout, dbias, accumulate);
+    launch_chained(ctx, conv_dbias_partial_kernel<1>, dim3(g.cout, slices), 256, 0, gr, g.n, g.cout, plane, per_slice, partial);
+  launch_chained(ctx, conv_dbias_finish_kernel, (unsigned)ceil_div(g.cout, 128), 128, 0, partial, slices, g.cout, dbias, accumulate);
   pool_free(ctx, partial);
   OM_LAUNCH_CHECK(ctx, "om_conv2d_dbias");
   return OM_OK;
@@ -844,11 +851,11 @@ int32_t om_maxpool_fwd(om_ctx* ctx, const float* x, int32_t planes, int32_t h, i
   if (pool_windows(g, planes, x, y, idx)) {
     const int groups = (int)(total * kw / 4);
     const int grid = grid_for(ctx, groups, 256);
-    if (kw == 1) maxpool_fwd_windows_kernel<1><<<grid, 256, 0, ctx->stream>>>(h, w, kh, x, groups, y, idx);
-    else if (kw == 2) maxpool_fwd_windows_kernel<2><<<grid, 256, 0, ctx->stream>>>(h, w, kh, x, groups, y, idx);
-    else maxpool_fwd_windows_kernel<4><<<grid, 256, 0, ctx->stream>>>(h, w, kh, x, groups, y, idx);
-  } else if ((int64_t)planes * h * w < (int64_t)INT32_MAX) maxpool_fwd_kernel<int><<<grid_for(ctx, total, 256), 256, 0, ctx->stream>>>(g, x, total, y, idx);
-  else maxpool_fwd_kernel<int64_t><<<grid_for(ctx, total, 256), 256, 0, ctx->stream>>>(g, x, total, y, idx);
+    if (kw == 1) launch_chained(ctx, maxpool_fwd_windows_kernel<1>, grid, 256, 0, h, w, kh, x, groups, y, idx);
+    else if (kw == 2) launch_chained(ctx, maxpool_fwd_windows_kernel<2>, grid, 256, 0, h, w, kh, x, groups, y, idx);
+    else launch_chained(ctx, maxpool_fwd_windows_kernel<4>, grid, 256, 0, h, w, kh, x, groups, y, idx);
+  } else if ((int64_t)planes * h * w < (int64_t)INT32_MAX) launch_chained(ctx, maxpool_fwd_kernel<int>, grid_for(ctx, total, 256), 256, 0, g, x, total, y, idx);
+  else launch_chained(ctx, maxpool_fwd_kernel<int64_t>, grid_for(ctx, total, 256), 256, 0, g, x, total, y, idx);
   OM_LAUNCH_CHECK(ctx, "om_maxpool_fwd");
   return OM_OK;
 }
@@ -865,16 +872,16 @@ int32_t om_maxpool_bwd(om_ctx* ctx, const float* gr, const int32_t* idx, int32_t
   if (pool_windows(g, planes, gr, idx, dx)) {
     const int groups = (int)(total / kh / 4);
     const int grid = grid_for(ctx, groups, 256);
-    if (kw == 1) maxpool_bwd_windows_kernel<1><<<grid, 256, 0, ctx->stream>>>(h, w, kh, gr, idx, groups, dx);
-    else if (kw == 2) maxpool_bwd_windows_kernel<2><<<grid, 256, 0, ctx->stream>>>(h, w, kh, gr, idx, groups, dx);
-    else maxpool_bwd_windows_kernel<4><<<grid, 256, 0, ctx->stream>>>(h, w, kh, gr, idx, groups, dx);
+    if (kw == 1) launch_chained(ctx, maxpool_bwd_windows_kernel<1>, grid, 256, 0, h, w, kh, gr, idx, groups, dx);
+    else if (kw == 2) launch_chained(ctx, maxpool_bwd_windows_kernel<2>, grid, 256, 0, h, w, kh, gr, idx, groups, dx);
+    else launch_chained(ctx, maxpool_bwd_windows_kernel<4>, grid, 256, 0, h, w, kh, gr, idx, groups, dx);
   } else if (kh == sh && kw == sw && ph == 0 && pw == 0 && total < (int64_t)1 << 30) {
     if ((w & 3) == 0 && (reinterpret_cast<uintptr_t>(dx) & 15) == 0)
-      maxpool_bwd_tiled_kernel<4><<<grid_for(ctx, total / 4, 256), 256, 0, ctx->stream>>>(h, w, oh, ow, kh, kw, gr, idx, (int)(total / 4), dx);
+      launch_chained(ctx, maxpool_bwd_tiled_kernel<4>, grid_for(ctx, total / 4, 256), 256, 0, h, w, oh, ow, kh, kw, gr, idx, (int)(total / 4), dx);
     else
-      maxpool_bwd_tiled_kernel<1><<<grid_for(ctx, total, 256), 256, 0, ctx->stream>>>(h, w, oh, ow, kh, kw, gr, idx, (int)total, dx);
+      launch_chained(ctx, maxpool_bwd_tiled_kernel<1>, grid_for(ctx, total, 256), 256, 0, h, w, oh, ow, kh, kw, gr, idx, (int)total, dx);
   } else
-    maxpool_bwd_kernel<<<grid_for(ctx, total, 256), 256, 0, ctx->stream>>>(g, gr, idx, total, dx);
+    launch_chained(ctx, maxpool_bwd_kernel, grid_for(ctx, total, 256), 256, 0, g, gr, idx, total, dx);
   OM_LAUNCH_CHECK(ctx, "om_maxpool_bwd");
   return OM_OK;
 }
