@@ -606,10 +606,9 @@ __global__ void __launch_bounds__(256) conv_channels_last_kernel(const float* __
 }
 
 constexpr int CN_THREADS = 192;      // warp 0: TMA, warp 1: products, warps 2-5: results
-template <int NT>
-__global__ void __launch_bounds__(CN_THREADS, 2)
+template <int NT, int STAGES>
+__global__ void __launch_bounds__(CN_THREADS, STAGES > 4 ? 1 : 2)
 conv_nhwc_kernel(const __grid_constant__ ConvNhwcMaps maps, const __grid_constant__ ConvNhwcParams p) {
-  constexpr int STAGES = NT == 64 ? 4 : 3;
   constexpr int STAGE_BYTES = CV_BLOCK + NT * 128;
   const ConvNhwcPhase& ph = p.phase[blockIdx.z];
   const ConvBox& box = ph.box;
@@ -1081,6 +1080,18 @@ static bool cn_worth(const ConvGeom& g) {
          (long long)g.n * g.oh * g.ow * cn_pitch(g.cout) < (1ll << 30);
 }
 
+template <int NT, int STAGES>
+static int32_t launch_nhwc(om_ctx* ctx, const ConvNhwcMaps& maps, const ConvNhwcParams& p, dim3 grid) {
+  constexpr size_t smem = (size_t)STAGES * (CV_BLOCK + NT * 128) + 1024 + 256;
+  static bool set = false;
+  if (!set) {
+    OM_CUDA(ctx, cudaFuncSetAttribute(conv_nhwc_kernel<NT, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    set = true;
+  }
+  launch_chained(ctx, conv_nhwc_kernel<NT, STAGES>, grid, CN_THREADS, smem, maps, p);
+  return check_cuda(ctx, cudaGetLastError(), "conv_nhwc");
+}
+
 // Runs the product of every phase from the turned source; the phases' grids, taps and output positions are set.
 static int32_t run_conv_nhwc(om_ctx* ctx, ConvNhwcParams& p, ConvTurn& turn, int phases, const float* src, int sc, int sh, int sw, const float* w) {
   ConvNhwcMaps maps = {};
@@ -1118,18 +1129,10 @@ static int32_t run_conv_nhwc(om_ctx* ctx, ConvNhwcParams& p, ConvTurn& turn, int
     if (most_ld > 0)
       launch_chained(ctx, conv_turn_weights_kernel<CV_BK, 1>, dim3((unsigned)std::min<int64_t>(ceil_div(most_ld, 256), 64), (unsigned)p.m, (unsigned)phases), 256, 0, w, wt, turn);
     const dim3 grid((unsigned)most, (unsigned)ceil_div(p.m, nt), (unsigned)phases);
-    static bool set = false;
-    constexpr size_t smem64 = (size_t)4 * (CV_BLOCK + 64 * 128) + 1024 + 128, smem128 = (size_t)3 * (CV_BLOCK + 128 * 128) + 1024 + 128;
-    if (!set) {
-      st = check_cuda(ctx, cudaFuncSetAttribute(conv_nhwc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem64), "conv_nhwc");
-      if (st == OM_OK) st = check_cuda(ctx, cudaFuncSetAttribute(conv_nhwc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem128), "conv_nhwc");
-      set = st == OM_OK;
-    }
-    if (st == OM_OK) {
-      if (nt == 64) launch_chained(ctx, conv_nhwc_kernel<64>, grid, CN_THREADS, smem64, maps, p);
-      else launch_chained(ctx, conv_nhwc_kernel<128>, grid, CN_THREADS, smem128, maps, p);
-      st = check_cuda(ctx, cudaGetLastError(), "conv_nhwc");
-    }
+    // Twice the stages where the grid gives an SM one CTA at most.
+    const bool alone = (int64_t)grid.x * grid.y * grid.z <= 148;
+    if (nt == 64) st = alone ? launch_nhwc<64, 8>(ctx, maps, p, grid) : launch_nhwc<64, 4>(ctx, maps, p, grid);
+    else st = alone ? launch_nhwc<128, 6>(ctx, maps, p, grid) : launch_nhwc<128, 3>(ctx, maps, p, grid);
   }
   pool_free(ctx, t);
   if (wt) pool_free(ctx, wt);

@@ -20,14 +20,17 @@
 namespace om {
 
 constexpr int BM = 128, BN = 128, BK = 32;       // BK fp32 elements = one 128-byte swizzle row
-constexpr int STAGES = 3;                        // 96 KiB of operand tiles: two CTAs per SM, one's epilogue under the other's MMAs
+// Operand stages. 96 KiB of them where two CTAs share an SM, one's epilogue under the other's MMAs; twice that where the grid gives an
+// SM one CTA at most, which then has the same bytes on their way alone: a stage is 32 KB a round trip to L2, so three of them
+// were waited for (STAGE_FIGURES).
+constexpr int kStagesShared = 3, kStagesAlone = 6;
 constexpr int UMMA_K = 8;                        // tf32: 32 bytes of k per instruction
 constexpr int A_TILE_BYTES = BM * BK * 4;        // 16 KiB
 constexpr int B_TILE_BYTES = BN * BK * 4;
 constexpr int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
 constexpr int TC_THREADS = 192;
 constexpr int TMEM_COLS = 128;
-constexpr size_t TC_SMEM = (size_t)STAGES * STAGE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
+constexpr size_t tc_smem(int stages) { return (size_t)stages * STAGE_BYTES + 1024 /* alignment slack */ + 256 /* barriers */; }
 
 struct TcParams {
   int tma_store;        // the epilogue writes C through map_c (C and its pitches are 16-byte aligned)
@@ -57,8 +60,8 @@ __host__ __device__ constexpr uint32_t make_idesc_tf32(bool a_mn, bool b_mn) {
 // MN-major tile in shared memory: 4 chunks of [BK k-rows x 128 bytes of m/n]; chunks BK*128 bytes apart (leading
 //                                 offset), 4-row k groups (the 32-byte-unit swizzle atom) 512 bytes apart (stride
 //                                 offset); one MMA consumes 8 k-rows = 1024 bytes.
-template <bool A_MN, bool B_MN>
-__global__ void __launch_bounds__(TC_THREADS, 2)
+template <bool A_MN, bool B_MN, int STAGES>
+__global__ void __launch_bounds__(TC_THREADS, STAGES == kStagesShared ? 2 : 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_c, TcParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -440,20 +443,28 @@ int32_t gemm_tc_heads(om_ctx* ctx, int ta, int tb, int m, int n, int k, const fl
                            : make_store_map(&map_c, C, n, m, ldc, inner, iC, outer, sC);
   if (!p.tma_store) map_c = map_a;   // never used, but the parameter must hold a valid map
   dim3 grid((unsigned)ceil_div(n, BN), (unsigned)ceil_div(m, BM), (unsigned)(batch > 1 ? batch : splits));
-#define OM_TC_LAUNCH(AMN, BMN)                                                                                         \
-  do {                                                                                                                 \
-    static bool attr_set = false;                                                                                      \
-    if (!attr_set) {                                                                                                   \
-      OM_CUDA(ctx, cudaFuncSetAttribute(gemm_tc_kernel<AMN, BMN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM)); \
-      attr_set = true;                                                                                                 \
-    }                                                                                                                  \
-    launch_chained(ctx, gemm_tc_kernel<AMN, BMN>, grid, TC_THREADS, TC_SMEM, map_a, map_b, map_c, p);                    \
+  // One CTA an SM of 148 at most, and more blocks of k than the short ring holds.
+  const bool alone = (int64_t)grid.x * grid.y * grid.z <= 148 && kb_per_split > kStagesShared;
+#define OM_TC_LAUNCH_AS(AMN, BMN, ST)                                                                                      \
+  do {                                                                                                                     \
+    static bool attr_set = false;                                                                                          \
+    if (!attr_set) {                                                                                                       \
+      OM_CUDA(ctx, cudaFuncSetAttribute(gemm_tc_kernel<AMN, BMN, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem(ST))); \
+      attr_set = true;                                                                                                     \
+    }                                                                                                                      \
+    launch_chained(ctx, gemm_tc_kernel<AMN, BMN, ST>, grid, TC_THREADS, tc_smem(ST), map_a, map_b, map_c, p);               \
+  } while (0)
+#define OM_TC_LAUNCH(AMN, BMN)                               \
+  do {                                                       \
+    if (alone) OM_TC_LAUNCH_AS(AMN, BMN, kStagesAlone);      \
+    else OM_TC_LAUNCH_AS(AMN, BMN, kStagesShared);           \
   } while (0)
   if (!a_mn && !b_mn) OM_TC_LAUNCH(false, false);
   else if (!a_mn && b_mn) OM_TC_LAUNCH(false, true);
   else if (a_mn && !b_mn) OM_TC_LAUNCH(true, false);
   else OM_TC_LAUNCH(true, true);
 #undef OM_TC_LAUNCH
+#undef OM_TC_LAUNCH_AS
   OM_LAUNCH_CHECK(ctx, "gemm_tc");
   if (splits > 1) {
     int64_t mn = (int64_t)m * n;
