@@ -22,7 +22,7 @@ namespace om {
 constexpr int BM = 128, BN = 128, BK = 32;       // BK fp32 elements = one 128-byte swizzle row
 // Operand stages. 96 KiB of them where two CTAs share an SM, one's epilogue under the other's MMAs; twice that where the grid gives an
 // SM one CTA at most, which then has the same bytes on their way alone: a stage is 32 KB a round trip to L2, so three of them
-// were waited for (STAGE_FIGURES).
+// were waited for.
 constexpr int kStagesShared = 3, kStagesAlone = 6;
 constexpr int UMMA_K = 8;                        // tf32: 32 bytes of k per instruction
 constexpr int A_TILE_BYTES = BM * BK * 4;        // 16 KiB

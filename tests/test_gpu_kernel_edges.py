@@ -304,3 +304,26 @@ def test_layer_norm_backward_rows_per_cta(ctx, K, rows, cols):
     xh, dh = (x64 - x64.mean(1, keepdims=True)) * inv, g64 * gamma
     assert scaled_diff(DX.numpy(), inv * (dh - dh.mean(1, keepdims=True) - xh * (dh * xh).mean(1, keepdims=True))) <= 1e-4
     assert scaled_diff(DG.numpy(), (g64 * xh).sum(0)) <= 1e-4 and scaled_diff(DB.numpy(), g64.sum(0)) <= 1e-4
+
+
+@pytest.mark.parametrize("rows,cols,ld", [(3, 4096, 4096), (2, 4099, 4100), (5, 8193, 8196), (300, 16385, 16392), (2, 30522, 30528), (2, 32768, 32768), (2, 32769, 32772),
+                                          (2, 4099, 4099)])
+def test_cross_entropy_of_wide_rows(ctx, rows, cols, ld):
+    """Rows held in registers and the widths on either side of them, ragged ends, pitched rows: against float64, 1e-6 of the largest value forward, 1e-5
+    backward (the log-softmax is rounded to fp32 before its exponential)."""
+    x = normal(cols, rows, ld, scale=3.0)
+    t = np.random.default_rng(1).integers(0, cols, rows)
+    t[-1] = -100
+    x64 = x[:, :cols].astype(np.float64)
+    lse = np.log(np.exp(x64 - x64.max(1, keepdims=True)).sum(1, keepdims=True)) + x64.max(1, keepdims=True)
+    X, T = ctx.to_device(x), ctx.to_device(t)
+    LP, L, N, D, G = ctx.to_device(np.zeros_like(x)), ctx.empty(()), ctx.empty((1,), np.int32), ctx.to_device(np.zeros_like(x)), ctx.to_device(np.ones(1, np.float32))
+    ctx.call("om_cross_entropy_fwd_ld", ctx.handle, X.ptr, T.ptr, i32(omb.OM_I64), i32(rows), i32(cols), i32(ld), i32(1), i64(-100), f32(0.0), LP.ptr, L.ptr, N.ptr)
+    ctx.call("om_cross_entropy_bwd_ld", ctx.handle, G.ptr, LP.ptr, T.ptr, i32(omb.OM_I64), i32(rows), i32(cols), i32(ld), i32(1), i64(-100), f32(0.0), D.ptr)
+    want = np.exp(x64 - lse)
+    want[np.arange(rows - 1), t[:-1]] -= 1.0
+    want[-1] = 0.0
+    assert scaled_diff(LP.numpy()[:, :cols], x64 - lse) <= 1e-6
+    assert scaled_diff(D.numpy()[:, :cols], want / (rows - 1)) <= 1e-5
+    assert abs(float(L.numpy()) - (lse[:-1, 0] - x64[np.arange(rows - 1), t[:-1]]).mean()) <= 1e-5 * 10
+    assert int(N.numpy()[0]) == rows - 1 and not LP.numpy()[:, cols:].any() and not D.numpy()[:, cols:].any()
