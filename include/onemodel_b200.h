@@ -548,6 +548,10 @@ int32_t om_conv2d_dgrad(om_ctx* ctx, const om_conv_shape* s, const float* g, con
 int32_t om_conv2d_wgrad(om_ctx* ctx, const om_conv_shape* s, const float* g, const float* x, float* dw,
                         int32_t accumulate);
 int32_t om_conv2d_dbias(om_ctx* ctx, const om_conv_shape* s, const float* g, float* dbias, int32_t accumulate);
+/* The three of them in one call, each left out where its result is NULL: what they share (a channels-last copy of the gradient
+ * under OM_TF32) is made once. */
+int32_t om_conv2d_bwd(om_ctx* ctx, const om_conv_shape* s, const float* g, const float* x, const float* w, float* dx, float* dw,
+                      int32_t accumulate_w, float* dbias, int32_t accumulate_b);
 
 /* Max pooling over NCHW planes; idx receives the Int32 flat NCHW index of each maximum (first wins ties,
  * NaN wins), bit-exact with ReferenceKernels.MaxPool2d (src/OneModel/Tensors/TensorKernels.cs:242-295). */

@@ -21,9 +21,11 @@ int32_t conv_tc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const flo
 bool conv_nhwc_fwd_fits(const ConvGeom& g);
 int32_t conv_nhwc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y);
 bool conv_nhwc_dgrad_fits(const ConvGeom& g);
-int32_t conv_nhwc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx);
+int32_t conv_nhwc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx, const float* turned_gr = nullptr);
 bool conv_nhwc_wgrad_fits(const ConvGeom& g);
-int32_t conv_nhwc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, float* dw, int accumulate);
+int32_t conv_nhwc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, float* dw, int accumulate, const float* turned_gr = nullptr);
+int32_t conv_nhwc_bwd(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, const float* w, float* dx, float* dw, int accumulate_w, float* dbias,
+                      int accumulate_b);
 
 // The fp32 products of small shapes without an unfolded matrix (om_conv_fma.cu).
 bool conv_fma_fwd_fits(const ConvGeom& g);

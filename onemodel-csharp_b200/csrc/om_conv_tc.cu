@@ -578,30 +578,65 @@ struct ConvNhwcMaps {
   CUtensorMap src[CV_MAX_PHASES], w[CV_MAX_PHASES];
 };
 
-// t[q][c] = s[n][c][p] for pixel q = n * plane + p; rows of cp floats (c rounded up to a multiple of four, zero there).
-constexpr int CN_PX = 64;
-__global__ void __launch_bounds__(256) conv_channels_last_kernel(const float* __restrict__ src, float* __restrict__ t, int pixels, int plane, CvDiv div_plane, int c, int cp) {
+// t[q][c] = s[n][c][p] for pixel q = n * plane + p; rows of cp floats (c rounded up to a multiple of four, zero there). SUMS: the pass also
+// leaves the channels' sums over this CTA's pixels in sums[blockIdx.x][c], in double (the bias gradient, which would otherwise be
+// another pass over the gradient: 118 us a step for the eight layers of the convolutional network).
+constexpr int CN_PX = 64, CN_SUM_CTAS = 512;
+template <bool SUMS>
+__global__ void __launch_bounds__(256) conv_channels_last_kernel(const float* __restrict__ src, float* __restrict__ t, int pixels, int plane, CvDiv div_plane, int c, int cp,
+                                                                 double* __restrict__ sums) {
   pdl_enter();
   __shared__ float tile[32][CN_PX + 1];
   const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
-  const int q0 = blockIdx.x * CN_PX, c0 = blockIdx.y * 32;
+  const int c0 = blockIdx.y * 32;
+  double acc = 0.0;
+  for (int q0 = blockIdx.x * CN_PX; q0 < pixels; q0 += gridDim.x * CN_PX) {
 #pragma unroll
-  for (int i = 0; i < CN_PX / 32; i++) {
-    const int q = q0 + 32 * i + lane;
-    const int n = cv_quot(q < pixels ? q : 0, div_plane), p = (q < pixels ? q : 0) - n * plane;
-    const float* base = src + (long long)n * c * plane + p;
+    for (int i = 0; i < CN_PX / 32; i++) {
+      const int q = q0 + 32 * i + lane;
+      const int n = cv_quot(q < pixels ? q : 0, div_plane), p = (q < pixels ? q : 0) - n * plane;
+      const float* base = src + (long long)n * c * plane + p;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int ch = c0 + row + 8 * j;
-      tile[row + 8 * j][32 * i + lane] = q < pixels && ch < c ? __ldg(base + (long long)ch * plane) : 0.f;
+      for (int j = 0; j < 4; j++) {
+        const int ch = c0 + row + 8 * j;
+        tile[row + 8 * j][32 * i + lane] = q < pixels && ch < c ? __ldg(base + (long long)ch * plane) : 0.f;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < CN_PX / 8; i++) {
+      const int q = q0 + row + 8 * i;
+      const float v = tile[lane][row + 8 * i];
+      if (SUMS) acc += (double)v;
+      if (c0 + lane < cp && q < pixels) t[(long long)q * cp + c0 + lane] = v;
+    }
+    __syncthreads();
+  }
+  if (SUMS) {
+    __shared__ double part[8][32];
+    part[row][lane] = acc;
+    __syncthreads();
+    if (row == 0 && c0 + lane < c) {
+      for (int i = 1; i < 8; i++) acc += part[i][lane];
+      sums[(long long)blockIdx.x * c + c0 + lane] = acc;
     }
   }
+}
+// dbias[co] (+)= the CTAs' sums: eight shares of them in increasing order, then the shares, in double.
+__global__ void __launch_bounds__(256) conv_sums_finish_kernel(const double* __restrict__ sums, int ctas, int c, float* __restrict__ dbias, int accumulate) {
+  pdl_enter();
+  __shared__ double part[8][32];
+  const int lane = threadIdx.x & 31, share = threadIdx.x >> 5, ch = blockIdx.x * 32 + lane;
+  double acc = 0.0;
+  if (ch < c) {
+#pragma unroll 8
+    for (int i = share; i < ctas; i += 8) acc += sums[(long long)i * c + ch];
+  }
+  part[share][lane] = acc;
   __syncthreads();
-  if (c0 + lane >= cp) return;
-#pragma unroll
-  for (int i = 0; i < CN_PX / 8; i++) {
-    const int q = q0 + row + 8 * i;
-    if (q < pixels) t[(long long)q * cp + c0 + lane] = tile[lane][row + 8 * i];
+  if (share == 0 && ch < c) {
+    for (int i = 1; i < 8; i++) acc += part[i][lane];
+    dbias[ch] = accumulate ? dbias[ch] + (float)acc : (float)acc;
   }
 }
 
@@ -1068,8 +1103,20 @@ static bool cn_map(CUtensorMap* map, const float* base, int c, int w, int h, int
 static int32_t cn_turn(om_ctx* ctx, const float* src, int n, int c, int plane, float** out) {
   const int pixels = n * plane, cp = cn_pitch(c);
   OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)pixels * cp, false, (void**)out));
-  launch_chained(ctx, conv_channels_last_kernel, dim3((unsigned)ceil_div(pixels, CN_PX), (unsigned)ceil_div(cp, 32)), 256, 0, src, *out, pixels, plane,
-                                                                                                                      cv_div((uint32_t)plane), c, cp);
+  launch_chained(ctx, conv_channels_last_kernel<false>, dim3((unsigned)ceil_div(pixels, CN_PX), (unsigned)ceil_div(cp, 32)), 256, 0, src, *out, pixels, plane,
+                 cv_div((uint32_t)plane), c, cp, nullptr);
+  return OM_OK;
+}
+// The same and the sums of the channels.
+static int32_t cn_turn_sums(om_ctx* ctx, const float* src, int n, int c, int plane, float** out, float* dbias, int accumulate) {
+  const int pixels = n * plane, cp = cn_pitch(c), ctas = (int)std::min<int64_t>(ceil_div(pixels, CN_PX), CN_SUM_CTAS);
+  double* sums = nullptr;
+  OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)pixels * cp, false, (void**)out));
+  OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)ctas * c, false, (void**)&sums));
+  launch_chained(ctx, conv_channels_last_kernel<true>, dim3((unsigned)ctas, (unsigned)ceil_div(cp, 32)), 256, 0, src, *out, pixels, plane, cv_div((uint32_t)plane), c,
+                 cp, sums);
+  launch_chained(ctx, conv_sums_finish_kernel, (unsigned)ceil_div(c, 32), 256, 0, sums, ctas, c, dbias, accumulate);
+  pool_free(ctx, sums);
   return OM_OK;
 }
 
@@ -1092,11 +1139,13 @@ static int32_t launch_nhwc(om_ctx* ctx, const ConvNhwcMaps& maps, const ConvNhwc
   return check_cuda(ctx, cudaGetLastError(), "conv_nhwc");
 }
 
-// Runs the product of every phase from the turned source; the phases' grids, taps and output positions are set.
-static int32_t run_conv_nhwc(om_ctx* ctx, ConvNhwcParams& p, ConvTurn& turn, int phases, const float* src, int sc, int sh, int sw, const float* w) {
+// Runs the product of every phase from the turned source (turned here when none is given); the phases' grids, taps and output
+// positions are set.
+static int32_t run_conv_nhwc(om_ctx* ctx, ConvNhwcParams& p, ConvTurn& turn, int phases, const float* src, const float* turned, int sc, int sh, int sw, const float* w) {
   ConvNhwcMaps maps = {};
-  float *t = nullptr, *wt = nullptr;
-  OM_TRY(cn_turn(ctx, src, p.images, sc, sh * sw, &t));
+  float *own = nullptr, *wt = nullptr;
+  if (!turned) OM_TRY(cn_turn(ctx, src, p.images, sc, sh * sw, &own));
+  const float* t = turned ? turned : own;
   const int nt = p.m <= 64 ? 64 : 128;
   long long floats = 0, most = 0;
   int most_ld = 0;
@@ -1134,7 +1183,7 @@ static int32_t run_conv_nhwc(om_ctx* ctx, ConvNhwcParams& p, ConvTurn& turn, int
     if (nt == 64) st = alone ? launch_nhwc<64, 8>(ctx, maps, p, grid) : launch_nhwc<64, 4>(ctx, maps, p, grid);
     else st = alone ? launch_nhwc<128, 6>(ctx, maps, p, grid) : launch_nhwc<128, 3>(ctx, maps, p, grid);
   }
-  pool_free(ctx, t);
+  if (own) pool_free(ctx, own);
   if (wt) pool_free(ctx, wt);
   return st;
 }
@@ -1162,14 +1211,14 @@ int32_t conv_nhwc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const floa
   }
   turn.m = g.cout; turn.sc = g.cin;
   turn.stride_m = (long long)g.cin * f.taps; turn.stride_sc = f.taps;
-  return run_conv_nhwc(ctx, p, turn, 1, x, g.cin, g.h, g.w, w);
+  return run_conv_nhwc(ctx, p, turn, 1, x, nullptr, g.cin, g.h, g.w, w);
 }
 
 bool conv_nhwc_dgrad_fits(const ConvGeom& g) {
   return encode_fn() && cv_sizes_fit(g) && cn_worth(g) && cn_channels_fit(g.cout) && cn_grid_fits((int)ceil_div(g.w, g.sw), (int)ceil_div(g.h, g.sh), g.n);
 }
 
-int32_t conv_nhwc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx) {
+int32_t conv_nhwc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx, const float* gt) {
   ConvNhwcParams p = {};
   ConvTurn turn = {};
   p.out = dx; p.status = ctx->status_dev;
@@ -1185,7 +1234,7 @@ int32_t conv_nhwc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const f
   }
   turn.m = g.cin; turn.sc = g.cout;
   turn.stride_m = g.kh * g.kw; turn.stride_sc = (long long)g.cin * g.kh * g.kw;
-  return run_conv_nhwc(ctx, p, turn, g.sh * g.sw, gr, g.cout, g.oh, g.ow, w);
+  return run_conv_nhwc(ctx, p, turn, g.sh * g.sw, gr, gt, g.cout, g.oh, g.ow, w);
 }
 
 // The pixel boxes have to tile the output exactly: a slot outside it would multiply its zero gradient with values of the input, which may
@@ -1196,7 +1245,7 @@ bool conv_nhwc_wgrad_fits(const ConvGeom& g) {
   return g.ow % b.w == 0 && g.oh % b.h == 0 && g.n % b.n == 0;
 }
 
-int32_t conv_nhwc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, float* dw, int accumulate) {
+int32_t conv_nhwc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, float* dw, int accumulate, const float* turned) {
   ConvNhwcWgradParams p = {};
   p.status = ctx->status_dev;
   p.cout = g.cout; p.cin = g.cin; p.kw = g.kw; p.taps = g.kh * g.kw; p.sh = g.sh; p.sw = g.sw; p.pt = g.pt; p.pl = g.pl; p.dh = g.dh; p.dw = g.dw;
@@ -1209,9 +1258,10 @@ int32_t conv_nhwc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const f
   int splits = (int)std::max<long long>(1, std::min<long long>(kSplitSlots / ((long long)tn * tm), p.blocks / 8));
   p.blocks_per_split = (int)ceil_div(p.blocks, splits);
   splits = (int)ceil_div(p.blocks, p.blocks_per_split);
-  float *gt = nullptr, *xt = nullptr;
+  float *own = nullptr, *xt = nullptr;
   CUtensorMap map_g = {}, map_x = {};
-  int32_t st = cn_turn(ctx, gr, g.n, g.cout, g.oh * g.ow, &gt);
+  int32_t st = turned ? OM_OK : cn_turn(ctx, gr, g.n, g.cout, g.oh * g.ow, &own);
+  const float* gt = turned ? turned : own;
   if (st == OM_OK) st = cn_turn(ctx, x, g.n, g.cin, g.h * g.w, &xt);
   if (st == OM_OK) st = pool_alloc(ctx, sizeof(float) * (size_t)splits * g.cout * ld, false, (void**)&p.part);
   if (st == OM_OK && (!cn_map(&map_g, gt, g.cout, g.ow, g.oh, g.n, p.box, 1, 1, true) || !cn_map(&map_x, xt, g.cin, g.w, g.h, g.n, p.box, g.sw, g.sh, true)))
@@ -1229,9 +1279,20 @@ int32_t conv_nhwc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const f
       st = check_cuda(ctx, cudaGetLastError(), "conv_nhwc_wgrad");
     }
   }
-  if (gt) pool_free(ctx, gt);
+  if (own) pool_free(ctx, own);
   if (xt) pool_free(ctx, xt);
   if (p.part) pool_free(ctx, p.part);
+  return st;
+}
+
+// Weight and input gradient (and the bias gradient, when asked for) from one channels-last copy of the output's gradient.
+int32_t conv_nhwc_bwd(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, const float* w, float* dx, float* dw, int accumulate_w, float* dbias,
+                      int accumulate_b) {
+  float* gt = nullptr;
+  int32_t st = dbias ? cn_turn_sums(ctx, gr, g.n, g.cout, g.oh * g.ow, &gt, dbias, accumulate_b) : cn_turn(ctx, gr, g.n, g.cout, g.oh * g.ow, &gt);
+  if (st == OM_OK) st = conv_nhwc_wgrad(ctx, g, gr, x, dw, accumulate_w, gt);
+  if (st == OM_OK) st = conv_nhwc_dgrad(ctx, g, gr, w, dx, gt);
+  if (gt) pool_free(ctx, gt);
   return st;
 }
 

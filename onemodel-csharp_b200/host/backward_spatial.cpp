@@ -35,17 +35,14 @@ static void ConvBackward(BackwardRecord& r, const Tensor& g) {
   s.pad_bottom = (int)r.Ints[4]; s.pad_right = (int)r.Ints[5]; s.dil_h = (int)r.Ints[6]; s.dil_w = (int)r.Ints[7]; s.groups = (int)r.Ints[8];
   Tensor gc = g.Contiguous();
   // Order of the reference: bias, weights, input.
-  GradSlot db(r, 2);
-  if (db.needed) Check(om_conv2d_dbias(C(), &s, gc.Data(), db.ptr, db.accumulate));
+  GradSlot db(r, 2), dw(r, 1);
+  Tensor dx;
+  if (r.NeedsInputGrad(0)) dx = Tensor::Create(DType::F32, x.GetShape());
+  Check(om_conv2d_bwd(C(), &s, gc.Data(), x.Data(), w.Data(), dx.IsEmpty() ? nullptr : dx.Data(), dw.needed ? dw.ptr : nullptr, dw.accumulate,
+                      db.needed ? db.ptr : nullptr, db.accumulate));
   db.Done(r, 2);
-  GradSlot dw(r, 1);
-  if (dw.needed) Check(om_conv2d_wgrad(C(), &s, gc.Data(), x.Data(), dw.ptr, dw.accumulate));
   dw.Done(r, 1);
-  if (r.NeedsInputGrad(0)) {
-    Tensor dx = Tensor::Create(DType::F32, x.GetShape());
-    Check(om_conv2d_dgrad(C(), &s, gc.Data(), w.Data(), dx.Data()));
-    Engine::Emit(r, 0, dx, true);
-  }
+  if (r.NeedsInputGrad(0)) Engine::Emit(r, 0, dx, true);
 }
 
 // The record of Ops::LstmBidirectional: inputs x, then (wIh, wHh, bIh, bHh) per direction; slots 0 x, then per direction

@@ -327,3 +327,27 @@ def test_cross_entropy_of_wide_rows(ctx, rows, cols, ld):
     assert scaled_diff(D.numpy()[:, :cols], want / (rows - 1)) <= 1e-5
     assert abs(float(L.numpy()) - (lse[:-1, 0] - x64[np.arange(rows - 1), t[:-1]]).mean()) <= 1e-5 * 10
     assert int(N.numpy()[0]) == rows - 1 and not LP.numpy()[:, cols:].any() and not D.numpy()[:, cols:].any()
+
+
+@pytest.mark.parametrize("tf32", [0, 1])
+@pytest.mark.parametrize("case", [(33, 64, 16, 16, 96, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1), (64, 64, 16, 16, 256, 3, 3, 2, 2, (1, 1, 1, 1), 1, 1),
+                                  (80, 32, 16, 16, 97, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1), (3, 5, 9, 7, 6, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1)])
+def test_conv2d_backward_in_one_call(ctx, case, tf32):
+    """Together and one by one: the same bits (the bias gradient, another order of sums in double, within 1e-6), each result left out too."""
+    s, x, wt, b, g, y, dx, dw = conv_case(*case)
+    ctx.set_flags(omb.OM_TF32 if tf32 else 0)
+    try:
+        X, W, G = (ctx.to_device(a) for a in (x, wt, g))
+        DX, DW, DB = (ctx.empty(a) for a in (x.shape, wt.shape, b.shape))
+        apart = run_conv(ctx, s, x, wt, b, g)
+        want = g.astype(np.float64).sum((0, 2, 3))
+        for skip in (None, 0, 1, 2):
+            out = [None if skip == i else a.ptr for i, a in enumerate((DX, DW, DB))]
+            ctx.call("om_conv2d_bwd", ctx.handle, C.byref(s), G.ptr, X.ptr, W.ptr, out[0], out[1], i32(0), out[2], i32(0))
+            assert skip == 0 or np.array_equal(DX.numpy(), apart[1])
+            assert skip == 1 or np.array_equal(DW.numpy(), apart[2])
+            assert skip == 2 or np.max(np.abs(DB.numpy() - want) / np.abs(g).astype(np.float64).sum((0, 2, 3))) <= 1e-6
+        ctx.call("om_conv2d_bwd", ctx.handle, C.byref(s), G.ptr, X.ptr, W.ptr, DX.ptr, DW.ptr, i32(1), DB.ptr, i32(1))
+        assert np.array_equal(DW.numpy(), apart[3]) and scaled_diff(DB.numpy(), 2 * want) <= 2e-6
+    finally:
+        ctx.set_flags(0)
