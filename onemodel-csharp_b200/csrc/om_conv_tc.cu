@@ -557,6 +557,30 @@ conv_wgrad_finish_kernel(const float* __restrict__ part, int splits, int cout, i
 //   forward, dgrad   D [128 pixels, NT channels] += x [pixels + tap, 32 c] W [NT, (32 c, tap)]      both K-major
 //   wgrad            D [128 co, 4 x (32 c, tap)] += g [32 pixels, co] x [32 pixels + tap, 32 c]      both MN-major
 // Accumulator rows are pixels, so a warp's store of one channel is 32 neighbouring pixels of the NCHW result.
+// The weights for these kernels: wt[phase][m][(32-channel block, tap), 32] as conv_turn_weights_kernel<32, 1> would order them, by tiles of
+// 8 m x 32 source channels through shared memory. Read and written in runs (element by element, the reads were 4 bytes a line:
+// 512 x 512 x 3 x 3 took 14 us).
+constexpr int CN_PACK_M = 8;
+__global__ void __launch_bounds__(256) conv_pack_weights_kernel(const float* __restrict__ w, float* __restrict__ wt, const __grid_constant__ ConvTurn t, int taps_all, int phases) {
+  pdl_enter();
+  extern __shared__ float pack[];       // [8 m][32 channels][taps, to an odd number]
+  const int m0 = blockIdx.y * CN_PACK_M, c0 = blockIdx.x * CV_BK, tp = taps_all | 1;
+  const bool by_m = t.stride_sc < t.stride_m;          // a run of memory is (channel, tap) of one m, or (m, tap) of one channel
+  const int run = (by_m ? CV_BK : CN_PACK_M) * taps_all;
+  for (int e = threadIdx.x; e < CN_PACK_M * CV_BK * taps_all; e += 256) {
+    const int outer = e / run, rem = e - outer * run, inner = rem / taps_all, tap = rem - inner * taps_all;
+    const int m = by_m ? outer : inner, c = by_m ? inner : outer;
+    pack[(m * CV_BK + c) * tp + tap] = m0 + m < t.m && c0 + c < t.sc ? __ldg(w + (m0 + m) * t.stride_m + (c0 + c) * t.stride_sc + tap) : 0.f;
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (m0 + warp >= t.m) return;
+  for (int z = 0; z < phases; z++) {
+    float* out = wt + t.start[z] + (long long)(m0 + warp) * t.ld[z] + (long long)blockIdx.x * t.taps[z] * CV_BK + lane;
+    for (int j = 0; j < t.taps[z]; j++) out[j * CV_BK] = pack[(warp * CV_BK + lane) * tp + t.tap[z][j]];
+  }
+}
+
 struct ConvBox {
   int w, h, n;                 // a tile of w x h x n pixels (powers of two)
   int tw, th, tn;              // tiles along each
@@ -1141,7 +1165,8 @@ static int32_t launch_nhwc(om_ctx* ctx, const ConvNhwcMaps& maps, const ConvNhwc
 
 // Runs the product of every phase from the turned source (turned here when none is given); the phases' grids, taps and output
 // positions are set.
-static int32_t run_conv_nhwc(om_ctx* ctx, ConvNhwcParams& p, ConvTurn& turn, int phases, const float* src, const float* turned, int sc, int sh, int sw, const float* w) {
+static int32_t run_conv_nhwc(om_ctx* ctx, ConvNhwcParams& p, ConvTurn& turn, int phases, int taps_all, const float* src, const float* turned, int sc, int sh, int sw,
+                             const float* w) {
   ConvNhwcMaps maps = {};
   float *own = nullptr, *wt = nullptr;
   if (!turned) OM_TRY(cn_turn(ctx, src, p.images, sc, sh * sw, &own));
@@ -1176,7 +1201,8 @@ static int32_t run_conv_nhwc(om_ctx* ctx, ConvNhwcParams& p, ConvTurn& turn, int
   }
   if (st == OM_OK && most > 0) {
     if (most_ld > 0)
-      launch_chained(ctx, conv_turn_weights_kernel<CV_BK, 1>, dim3((unsigned)std::min<int64_t>(ceil_div(most_ld, 256), 64), (unsigned)p.m, (unsigned)phases), 256, 0, w, wt, turn);
+      launch_chained(ctx, conv_pack_weights_kernel, dim3((unsigned)ceil_div(sc, CV_BK), (unsigned)ceil_div(p.m, CN_PACK_M)), 256,
+                     sizeof(float) * CN_PACK_M * CV_BK * (taps_all | 1), w, wt, turn, taps_all, phases);
     const dim3 grid((unsigned)most, (unsigned)ceil_div(p.m, nt), (unsigned)phases);
     // Twice the stages where the grid gives an SM one CTA at most.
     const bool alone = (int64_t)grid.x * grid.y * grid.z <= 148;
@@ -1211,7 +1237,7 @@ int32_t conv_nhwc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const floa
   }
   turn.m = g.cout; turn.sc = g.cin;
   turn.stride_m = (long long)g.cin * f.taps; turn.stride_sc = f.taps;
-  return run_conv_nhwc(ctx, p, turn, 1, x, nullptr, g.cin, g.h, g.w, w);
+  return run_conv_nhwc(ctx, p, turn, 1, f.taps, x, nullptr, g.cin, g.h, g.w, w);
 }
 
 bool conv_nhwc_dgrad_fits(const ConvGeom& g) {
@@ -1234,7 +1260,7 @@ int32_t conv_nhwc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const f
   }
   turn.m = g.cin; turn.sc = g.cout;
   turn.stride_m = g.kh * g.kw; turn.stride_sc = (long long)g.cin * g.kh * g.kw;
-  return run_conv_nhwc(ctx, p, turn, g.sh * g.sw, gr, gt, g.cout, g.oh, g.ow, w);
+  return run_conv_nhwc(ctx, p, turn, g.sh * g.sw, g.kh * g.kw, gr, gt, g.cout, g.oh, g.ow, w);
 }
 
 // The pixel boxes have to tile the output exactly: a slot outside it would multiply its zero gradient with values of the input, which may

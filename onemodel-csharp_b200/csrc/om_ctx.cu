@@ -449,6 +449,30 @@ int32_t om_stage_commit(om_ctx* ctx, int32_t slot) {
   return OM_OK;
 }
 
+int32_t om_stage_wait_ready(om_ctx* ctx, int32_t slot) {
+  OM_CHECK_CTX(ctx);
+  OM_TRY(stage_setup(ctx, slot));
+  OM_CUDA(ctx, cudaEventSynchronize(ctx->stage_ready[slot]));
+  return OM_OK;
+}
+
+int32_t om_host_is_pinned(om_ctx* ctx, const void* p, size_t bytes, int32_t* pinned) {
+  OM_CHECK_CTX(ctx);
+  *pinned = 0;
+  if (p == nullptr || bytes == 0) return OM_OK;
+  const char* ends[2] = {static_cast<const char*>(p), static_cast<const char*>(p) + bytes - 1};
+  cudaPointerAttributes a[2];
+  for (int i = 0; i < 2; i++)
+    if (cudaPointerGetAttributes(&a[i], ends[i]) != cudaSuccess) {
+      cudaGetLastError();      // memory the driver does not know
+      return OM_OK;
+    }
+  // both ends in page-locked memory, mapped as one range
+  *pinned = a[0].type == cudaMemoryTypeHost && a[1].type == cudaMemoryTypeHost &&
+            static_cast<const char*>(a[1].devicePointer) - static_cast<const char*>(a[0].devicePointer) == ends[1] - ends[0];
+  return OM_OK;
+}
+
 int32_t om_stage_acquire(om_ctx* ctx, int32_t slot) {
   OM_CHECK_CTX(ctx);
   OM_TRY(stage_setup(ctx, slot));
