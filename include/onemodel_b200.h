@@ -123,11 +123,15 @@ int32_t om_memset(om_ctx* ctx, void* dst, int32_t byte, size_t bytes);
  *   om_stage_commit(slot)         the slot's batch is complete (an event on the copy stream);
  *   om_stage_acquire(slot)        the compute stream waits for that event (no host wait);
  *   om_stage_release(slot)        the work queued so far on the compute stream has taken the batch: the slot may be refilled;
- *   om_stage_wait_taken(slot)     host wait for that point.
+ *   om_stage_wait_taken(slot)     host wait for that point;
+ *   om_stage_wait_ready(slot)     host wait until the slot's batch has landed (the source may be written again);
+ *   om_host_is_pinned(p, bytes)   whether that range is page-locked memory the driver knows.
  * Slots 0..15. The host memory must stay unchanged until the copy has run (keep it in the loader's ring). */
 int32_t om_stage_h2d(om_ctx* ctx, int32_t slot, void* dst, const void* src_pinned, size_t bytes);
 int32_t om_stage_commit(om_ctx* ctx, int32_t slot);
 int32_t om_stage_acquire(om_ctx* ctx, int32_t slot);
+int32_t om_stage_wait_ready(om_ctx* ctx, int32_t slot);
+int32_t om_host_is_pinned(om_ctx* ctx, const void* p, size_t bytes, int32_t* pinned);
 int32_t om_stage_release(om_ctx* ctx, int32_t slot);
 /* Host wait until the slot's last om_stage_release has been reached by the compute stream (the loader's back-pressure:
  * the pinned buffer behind the slot may be rewritten after it). Returns at once when the slot was never released. */
