@@ -393,10 +393,20 @@ void splitk_reduce_launch(om_ctx* ctx, const float* part, int splits, int64_t mn
   launch_chained(ctx, splitk_reduce_kernel, grid_for(ctx, mn, 256), 256, 0, part, splits, mn, n, ldc, bias, out, accumulate);
 }
 
+// Products for the persistent CTA-pair kernel with 256 x 256 tiles: those that give nearly every pair a tile, in columns nearly full, or half of
+// them one where the many blocks of k of a tile outweigh the idle pairs. us here / there (the kernel that served the shape):
+//   8192 x 1536 x 384: 28.4 / 24.1, 16384 x 768 x 768: 42.3 / 35.3, 16384 x 3072 x 768: 136 / 109, 16384 x 768 x 3072: 120 / 110 (CTA pairs),
+//   4096 x 2048 x 2048: 65.4 / 51.9, 8192 x 512 x 2048: 36.5 / 31.0 (this file); even at 8192 x 1152 x 384 and 8192 x 512 x 512; the
+//   other way at 5120 x 1024 x 256: 15.2 / 16.4, and with 384 columns: 30.0 / 35.8 at k = 1536.
+static bool persistent_tiles(int m, int n, int k) {
+  const int64_t tiles = ceil_div(m, 256) * ceil_div(n, 256);
+  return m >= 2048 && n >= 512 && 10 * (int64_t)n >= 9 * ceil_div(n, 256) * 256 && (tiles >= 128 || (tiles >= 64 && k >= 1024));
+}
+
 int32_t gemm_tc_heads(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, long long sA, long long iA,
                       const float* B, int ldb, long long sB, long long iB, float* C, int ldc, long long sC, long long iC, int batch,
                       int inner, int acc, const float* bias) {
-  if (batch == 1 && (ctx->flags & OM_PERSISTENT_TILES) && m >= 256 && n >= 64 && gemm_ws_supported(ctx, 0, m, n, k, A, lda, B, ldb, C, ldc))
+  if (batch == 1 && ((ctx->flags & OM_PERSISTENT_TILES) ? m >= 256 && n >= 64 : persistent_tiles(m, n, k)) && gemm_ws_supported(ctx, 0, m, n, k, A, lda, B, ldb, C, ldc))
     return gemm_ws(ctx, 0, ta, tb, m, n, k, A, lda, B, ldb, C, ldc, acc, bias, nullptr);
   if (batch == 1 && gemm_pair_supported(ctx, m, n, k)) return gemm_pair(ctx, ta, tb, m, n, k, A, lda, B, ldb, C, ldc, acc, bias);
   // op(A) is [m, k]. ta == 0: stored [m, k] (K-major tile, map inner = k). ta != 0: stored [k, m] (MN-major, inner = m).
