@@ -351,3 +351,27 @@ def test_conv2d_backward_in_one_call(ctx, case, tf32):
         assert np.array_equal(DW.numpy(), apart[3]) and scaled_diff(DB.numpy(), 2 * want) <= 2e-6
     finally:
         ctx.set_flags(0)
+
+
+@pytest.mark.parametrize("n,c,h,w,offset", [(2, 3, 1, 1, 0.0), (5, 2, 3, 1, 0.0), (17, 4, 7, 9, 1e4), (33, 3, 16, 16, -1e4), (3, 2, 128, 130, 100.0), (1, 5, 1, 4, 0.0)])
+def test_batch_norm_statistics_and_sums(ctx, n, c, h, w, offset):
+    """Empty and ragged slices, planes on and off four values, pieces smaller and larger than a CTA's registers, and channels whose mean is ten
+    thousand deviations away (nothing may cancel): the saved statistics within 1e-6 of float64, gradients within 1e-4."""
+    x, g = (normal(n + c, n, c, h, w) + np.float32(offset)).astype(np.float32), normal(7, n, c, h, w)
+    gamma, beta = normal(8, c), normal(9, c)
+    X, G, GA, BE, RM, RV = (ctx.to_device(a) for a in (x, g, gamma, beta, np.zeros(c, np.float32), np.ones(c, np.float32)))
+    Y, M, I, DX, DG, DB = ctx.empty(x.shape), ctx.empty((c,)), ctx.empty((c,)), ctx.empty(x.shape), ctx.empty((c,)), ctx.empty((c,))
+    ctx.call("om_batchnorm_fwd", ctx.handle, X.ptr, GA.ptr, BE.ptr, RM.ptr, RV.ptr, i32(n), i32(c), i32(h * w), i32(1), f32(0.1), f32(1e-5), Y.ptr, M.ptr, I.ptr)
+    ctx.call("om_batchnorm_bwd", ctx.handle, G.ptr, X.ptr, GA.ptr, M.ptr, I.ptr, i32(n), i32(c), i32(h * w), i32(1), DX.ptr, DG.ptr, DB.ptr, i32(0))
+    x64, g64 = x.astype(np.float64), g.astype(np.float64)
+    mu, var, m = x64.mean((0, 2, 3)), x64.var((0, 2, 3)), n * h * w
+    assert np.max(np.abs(M.numpy() - mu) / np.maximum(np.abs(mu), 1e-3)) <= 1e-6
+    assert np.max(np.abs(I.numpy() * np.sqrt(var + 1e-5) - 1)) <= 1e-6
+    assert np.max(np.abs(RV.numpy() - (0.9 + 0.1 * var * m / max(m - 1, 1)))) <= 1e-6 * (1 + np.max(var))
+    mean, inv = (a.numpy().astype(np.float64)[None, :, None, None] for a in (M, I))     # (the gradient is that of the saved statistics)
+    xh = (x64 - mean) * inv
+    sb, sg = g64.sum((0, 2, 3)), (g64 * xh).sum((0, 2, 3))
+    assert np.max(np.abs(DB.numpy() - sb)) <= 1e-5 * max(1.0, np.max(np.abs(sb)))
+    assert np.max(np.abs(DG.numpy() - sg)) <= 1e-4 * max(1.0, np.max(np.abs(sg)))
+    want = gamma[None, :, None, None] * inv * (g64 - sb[None, :, None, None] / m - xh * sg[None, :, None, None] / m)
+    assert np.max(np.abs(DX.numpy() - want)) <= 1e-4 * max(1.0, np.max(np.abs(want)))
