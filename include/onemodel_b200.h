@@ -67,7 +67,8 @@ typedef enum om_status {
  * OM_SEQ_KERNELS (with OM_TF32): an LSTM layer whose shape fits (hidden a multiple of 16, batch <= 256 for the backward)
  * runs all its time steps in one cooperative launch with fp32 recurrent products, instead of a product and a gate
  * kernel per step. OM_OVERLAP_LAUNCHES: the frequent kernels are launched as programmatic dependents of their
- * predecessor in the stream, so that launch latency and prologue overlap the predecessor's tail (same results).
+ * predecessor in the stream, so that launch latency and prologue overlap the predecessor's tail (same results); without
+ * it only those of up to 1184 CTAs are, or of up to 296 while a step is being captured.
  * OM_PERSISTENT_TILES (with OM_TF32): plain products run on the persistent CTA-pair kernel that the bfloat16 products
  * always use (two accumulator buffers in tensor memory: a tile's read-back and stores run under the next tile's MMAs). */
 #define OM_TF32 1u
@@ -441,6 +442,14 @@ int32_t om_batchnorm_fwd(om_ctx* ctx, const float* x, const float* gamma, const 
 int32_t om_batchnorm_bwd(om_ctx* ctx, const float* g, const float* x, const float* gamma, const float* mean,
                          const float* inv, int32_t n, int32_t c, int32_t plane, int32_t training, float* dx,
                          float* dgamma, float* dbeta, int32_t accumulate_params);
+/* The norm and a rectifier behind it in one call: the values of om_batchnorm_fwd followed by om_unary(OM_RELU), bit for bit. The forward keeps
+ * the beta it used for the backward (beta_used [c], may be NULL), which forms the rectifier's input again. */
+int32_t om_batchnorm_relu_fwd(om_ctx* ctx, const float* x, const float* gamma, const float* beta,
+                              float* running_mean, float* running_var, int32_t n, int32_t c, int32_t plane,
+                              int32_t training, float momentum, float eps, float* y, float* mean, float* inv, float* beta_used);
+int32_t om_batchnorm_relu_bwd(om_ctx* ctx, const float* g, const float* x, const float* gamma, const float* beta_used, const float* mean,
+                              const float* inv, int32_t n, int32_t c, int32_t plane, int32_t training, float* dx,
+                              float* dgamma, float* dbeta, int32_t accumulate_params);
 
 /* ---- embedding ------------------------------------------------------------------------------------------ */
 

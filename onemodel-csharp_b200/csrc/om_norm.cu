@@ -442,6 +442,10 @@ layernorm_bwd_vec_kernel(const float* __restrict__ g, const float* __restrict__ 
 // CTA (ch, slice) walks the planes of images [slice*ipc, (slice+1)*ipc) of channel ch, VEC values an access (VEC == 4: planes of a multiple of four
 // values). Each thread keeps its place by additions, with several loads in flight.
 constexpr int kBnThreads = 256;
+// RELU, in the kernels below: the rectifier behind the norm in the same pass. The backward forms its input again, in the same four
+// operations, to know where it was positive: two passes over the activation less forward, three less backward.
+__device__ __forceinline__ float bn_relu(float x) { return x > 0.0f ? x : (x == x ? 0.0f : x); }
+__device__ __forceinline__ float bn_norm(float x, float mm, float s, float gg, float bb) { return (((x - mm) * s) * gg) + bb; }
 struct BnWalk {
   int i, p, step_i, step_p, pv;
   __device__ BnWalk(int i0, int vectors) {
@@ -553,17 +557,17 @@ bn_stats_kernel(const float* __restrict__ x, int32_t n, int32_t c, int32_t plane
 }
 
 // Backward: sum of g * xhat and sum of g over the slice.
-template <int VEC>
+template <int VEC, bool RELU>
 __global__ void __launch_bounds__(kBnThreads)
-bn_bwd_partial_kernel(const float* __restrict__ x, const float* __restrict__ g, const float* __restrict__ mean, const float* __restrict__ inv, int32_t n,
-                      int32_t c, int32_t plane, int32_t ipc, double* __restrict__ pa, double* __restrict__ pb) {
+bn_bwd_partial_kernel(const float* __restrict__ x, const float* __restrict__ g, const float* __restrict__ mean, const float* __restrict__ inv,
+                      const float* __restrict__ gamma, const float* __restrict__ beta, int32_t n, int32_t c, int32_t plane, int32_t ipc, double* __restrict__ pa, double* __restrict__ pb) {
   pdl_enter();
   __shared__ double sm[kBnThreads / 32];
   constexpr int LOADS = VEC == 4 ? 4 : 8;
   const int ch = blockIdx.x, slice = blockIdx.y;
   const int i0 = slice * ipc, i1 = min(n, i0 + ipc);
   const int64_t image = (int64_t)c * plane, first = (int64_t)ch * plane;
-  const float mm = mean[ch], s = inv[ch];
+  const float mm = mean[ch], s = inv[ch], gg = RELU ? gamma[ch] : 0.f, bb = RELU ? beta[ch] : 0.f;
   double a = 0.0, b = 0.0;
   if (plane > 0) {
     BnWalk w(i0, plane / VEC);
@@ -585,8 +589,10 @@ bn_bwd_partial_kernel(const float* __restrict__ x, const float* __restrict__ g, 
         if (l < have)
 #pragma unroll
           for (int j = 0; j < VEC; j++) {
-            a += (double)(gv[l][j] * ((xv[l][j] - mm) * s));
-            b += (double)gv[l][j];
+            float gj = gv[l][j];
+            if (RELU && !(bn_norm(xv[l][j], mm, s, gg, bb) > 0.0f)) gj = 0.0f;
+            a += (double)(gj * ((xv[l][j] - mm) * s));
+            b += (double)gj;
           }
     }
   }
@@ -600,10 +606,11 @@ bn_bwd_partial_kernel(const float* __restrict__ x, const float* __restrict__ g, 
 
 __global__ void bn_finish_stats_kernel(const double* __restrict__ pmean, const double* __restrict__ pdev, int slices, int32_t n, int32_t ipc, int32_t plane,
                                        int32_t c, double m, float momentum, float eps, float* __restrict__ mean,
-                                       float* __restrict__ inv, float* __restrict__ rm, float* __restrict__ rv) {
+                                       float* __restrict__ inv, float* __restrict__ rm, float* __restrict__ rv, const float* __restrict__ beta, float* __restrict__ beta_out) {
   pdl_enter();
   int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
+  if (beta_out) beta_out[ch] = beta[ch];
   BnSet set = {0.0, 0.0, 0.0};
   for (int s = 0; s < slices; s++) set.add((double)max(0, min(n, (s + 1) * ipc) - s * ipc) * plane, pmean[(int64_t)s * c + ch], pdev[(int64_t)s * c + ch]);
   const double mu = set.mean;
@@ -618,16 +625,17 @@ __global__ void bn_finish_stats_kernel(const double* __restrict__ pmean, const d
 }
 
 __global__ void bn_eval_stats_kernel(const float* __restrict__ rm, const float* __restrict__ rv, int32_t c, float eps,
-                                     float* __restrict__ mean, float* __restrict__ inv) {
+                                     float* __restrict__ mean, float* __restrict__ inv, const float* __restrict__ beta, float* __restrict__ beta_out) {
   pdl_enter();
   int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
+  if (beta_out) beta_out[ch] = beta[ch];
   mean[ch] = rm[ch];
   inv[ch] = 1.0f / sqrtf(rv[ch] + eps);
 }
 
 // Element-wise over the whole tensor, VEC consecutive elements of one plane per thread (VEC == 4: plane % 4 == 0).
-template <int VEC>
+template <int VEC, bool RELU>
 __global__ void __launch_bounds__(256)
 bn_apply_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
                 const float* __restrict__ mean, const float* __restrict__ inv, int64_t total, int32_t c, int32_t plane,
@@ -640,11 +648,12 @@ bn_apply_kernel(const float* __restrict__ x, const float* __restrict__ gamma, co
     const float mm = mean[ch], s = inv[ch], gg = gamma[ch], bb = beta[ch];
     if (VEC == 4) {
       float4 v = __ldg(reinterpret_cast<const float4*>(x + e));
-      v.x = (((v.x - mm) * s) * gg) + bb; v.y = (((v.y - mm) * s) * gg) + bb;
-      v.z = (((v.z - mm) * s) * gg) + bb; v.w = (((v.w - mm) * s) * gg) + bb;
+      v.x = bn_norm(v.x, mm, s, gg, bb); v.y = bn_norm(v.y, mm, s, gg, bb); v.z = bn_norm(v.z, mm, s, gg, bb); v.w = bn_norm(v.w, mm, s, gg, bb);
+      if (RELU) { v.x = bn_relu(v.x); v.y = bn_relu(v.y); v.z = bn_relu(v.z); v.w = bn_relu(v.w); }
       *reinterpret_cast<float4*>(y + e) = v;
     } else {
-      y[e] = (((x[e] - mm) * s) * gg) + bb;
+      const float v = bn_norm(x[e], mm, s, gg, bb);
+      y[e] = RELU ? bn_relu(v) : v;
     }
   }
 }
@@ -665,10 +674,10 @@ __global__ void bn_bwd_coef_kernel(const float* __restrict__ gamma, const float*
   coef[2 * c + ch] = (float)(sg / m);
 }
 
-template <int VEC>
+template <int VEC, bool RELU>
 __global__ void __launch_bounds__(256)
 bn_bwd_apply_kernel(const float* __restrict__ g, const float* __restrict__ x, const float* __restrict__ mean,
-                    const float* __restrict__ inv, const float* __restrict__ coef, int64_t total, int32_t c, int32_t plane,
+                    const float* __restrict__ inv, const float* __restrict__ gamma, const float* __restrict__ beta, const float* __restrict__ coef, int64_t total, int32_t c, int32_t plane,
                     int training, float* __restrict__ dx) {
   pdl_enter();
   int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * VEC;
@@ -676,9 +685,16 @@ bn_bwd_apply_kernel(const float* __restrict__ g, const float* __restrict__ x, co
   for (int64_t e = i; e < total; e += stride) {
     const int ch = (int)((e / plane) % c);
     const float mm = mean[ch], s = inv[ch], k = coef[ch], cb = coef[c + ch], cg = coef[2 * c + ch];
+    const float gg = RELU ? gamma[ch] : 0.f, bb = RELU ? beta[ch] : 0.f;
     if (VEC == 4) {
-      const float4 gv = __ldg(reinterpret_cast<const float4*>(g + e));
+      float4 gv = __ldg(reinterpret_cast<const float4*>(g + e));
       const float4 xv = __ldg(reinterpret_cast<const float4*>(x + e));
+      if (RELU) {
+        if (!(bn_norm(xv.x, mm, s, gg, bb) > 0.0f)) gv.x = 0.0f;
+        if (!(bn_norm(xv.y, mm, s, gg, bb) > 0.0f)) gv.y = 0.0f;
+        if (!(bn_norm(xv.z, mm, s, gg, bb) > 0.0f)) gv.z = 0.0f;
+        if (!(bn_norm(xv.w, mm, s, gg, bb) > 0.0f)) gv.w = 0.0f;
+      }
       float4 o;
       if (training) {
         o.x = k * ((gv.x - cb) - (((xv.x - mm) * s) * cg)); o.y = k * ((gv.y - cb) - (((xv.y - mm) * s) * cg));
@@ -688,7 +704,9 @@ bn_bwd_apply_kernel(const float* __restrict__ g, const float* __restrict__ x, co
       }
       *reinterpret_cast<float4*>(dx + e) = o;
     } else {
-      dx[e] = training ? k * ((g[e] - cb) - (((x[e] - mm) * s) * cg)) : k * g[e];
+      float gv = g[e];
+      if (RELU && !(bn_norm(x[e], mm, s, gg, bb) > 0.0f)) gv = 0.0f;
+      dx[e] = training ? k * ((gv - cb) - (((x[e] - mm) * s) * cg)) : k * gv;
     }
   }
 }
@@ -822,9 +840,9 @@ static int bn_slices(int n, int c, int plane) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(std::min(n, 16), std::max(by_size, by_channels)));
 }
 
-int32_t om_batchnorm_fwd(om_ctx* ctx, const float* x, const float* gamma, const float* beta, float* running_mean,
-                         float* running_var, int32_t n, int32_t c, int32_t plane, int32_t training, float momentum,
-                         float eps, float* y, float* mean, float* inv) {
+static int32_t batchnorm_fwd(om_ctx* ctx, const float* x, const float* gamma, const float* beta, float* running_mean,
+                             float* running_var, int32_t n, int32_t c, int32_t plane, int32_t training, float momentum,
+                             float eps, float* y, float* mean, float* inv, bool relu, float* beta_out) {
   OM_CHECK_CTX(ctx);
   if (n < 0 || c < 0 || plane < 0) return fail(ctx, OM_ERR_SHAPE, "om_batchnorm_fwd: n %d c %d plane %d", n, c, plane);
   if (training && (int64_t)n * plane < 1) return fail(ctx, OM_ERR_SHAPE, "BatchNorm2d in training needs at least one value per channel.");
@@ -841,25 +859,40 @@ int32_t om_batchnorm_fwd(om_ctx* ctx, const float* x, const float* gamma, const 
     if ((plane & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) launch_chained(ctx, bn_stats_kernel<4>, grid, kBnThreads, 0, x, n, c, plane, ipc, pa, pb);
     else launch_chained(ctx, bn_stats_kernel<1>, grid, kBnThreads, 0, x, n, c, plane, ipc, pa, pb);
     launch_chained(ctx, bn_finish_stats_kernel, (unsigned)ceil_div(c, 128), 128, 0, pa, pb, slices, n, ipc, plane, c, m, momentum, eps, mean, inv, running_mean,
-                   running_var);
+                   running_var, beta, beta_out);
     pool_free(ctx, pa);
     pool_free(ctx, pb);
   } else {
-    launch_chained(ctx, bn_eval_stats_kernel, (unsigned)ceil_div(c, 128), 128, 0, running_mean, running_var, c, eps, mean, inv);
+    launch_chained(ctx, bn_eval_stats_kernel, (unsigned)ceil_div(c, 128), 128, 0, running_mean, running_var, c, eps, mean, inv, beta, beta_out);
   }
   int64_t planes = (int64_t)n * c;
   if (planes > 0 && plane > 0) {
     const int64_t total = planes * plane;
-    if ((plane & 3) == 0) launch_chained(ctx, bn_apply_kernel<4>, grid_for(ctx, total / 4, 256), 256, 0, x, gamma, beta, mean, inv, total, c, plane, y);
-    else launch_chained(ctx, bn_apply_kernel<1>, grid_for(ctx, total, 256), 256, 0, x, gamma, beta, mean, inv, total, c, plane, y);
+    auto apply = [&](auto kernel, int64_t accesses) {
+      launch_chained(ctx, kernel, grid_for(ctx, accesses, 256), 256, 0, x, gamma, beta, mean, inv, total, c, plane, y);
+    };
+    if ((plane & 3) == 0) relu ? apply(bn_apply_kernel<4, true>, total / 4) : apply(bn_apply_kernel<4, false>, total / 4);
+    else relu ? apply(bn_apply_kernel<1, true>, total) : apply(bn_apply_kernel<1, false>, total);
   }
   OM_LAUNCH_CHECK(ctx, "om_batchnorm_fwd");
   return OM_OK;
 }
 
-int32_t om_batchnorm_bwd(om_ctx* ctx, const float* g, const float* x, const float* gamma, const float* mean,
-                         const float* inv, int32_t n, int32_t c, int32_t plane, int32_t training, float* dx,
-                         float* dgamma, float* dbeta, int32_t accumulate_params) {
+int32_t om_batchnorm_fwd(om_ctx* ctx, const float* x, const float* gamma, const float* beta, float* running_mean,
+                         float* running_var, int32_t n, int32_t c, int32_t plane, int32_t training, float momentum,
+                         float eps, float* y, float* mean, float* inv) {
+  return batchnorm_fwd(ctx, x, gamma, beta, running_mean, running_var, n, c, plane, training, momentum, eps, y, mean, inv, false, nullptr);
+}
+
+int32_t om_batchnorm_relu_fwd(om_ctx* ctx, const float* x, const float* gamma, const float* beta, float* running_mean,
+                              float* running_var, int32_t n, int32_t c, int32_t plane, int32_t training, float momentum,
+                              float eps, float* y, float* mean, float* inv, float* beta_used) {
+  return batchnorm_fwd(ctx, x, gamma, beta, running_mean, running_var, n, c, plane, training, momentum, eps, y, mean, inv, true, beta_used);
+}
+
+static int32_t batchnorm_bwd(om_ctx* ctx, const float* g, const float* x, const float* gamma, const float* mean,
+                             const float* inv, int32_t n, int32_t c, int32_t plane, int32_t training, float* dx,
+                             float* dgamma, float* dbeta, int32_t accumulate_params, bool relu, const float* beta) {
   OM_CHECK_CTX(ctx);
   if (n < 0 || c < 0 || plane < 0) return fail(ctx, OM_ERR_SHAPE, "om_batchnorm_bwd: n %d c %d plane %d", n, c, plane);
   if (c == 0) return OM_OK;
@@ -869,18 +902,23 @@ int32_t om_batchnorm_bwd(om_ctx* ctx, const float* g, const float* x, const floa
   double *pa = nullptr, *pb = nullptr;
   OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)slices * c, false, (void**)&pa));
   OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)slices * c, false, (void**)&pb));
-  if ((plane & 3) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(g)) & 15) == 0)
-    launch_chained(ctx, bn_bwd_partial_kernel<4>, dim3(c, slices), kBnThreads, 0, x, g, mean, inv, n, c, plane, ipc, pa, pb);
-  else
-    launch_chained(ctx, bn_bwd_partial_kernel<1>, dim3(c, slices), kBnThreads, 0, x, g, mean, inv, n, c, plane, ipc, pa, pb);
+  const bool vec = (plane & 3) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(g)) & 15) == 0;
+  auto partial = [&](auto kernel) {
+    launch_chained(ctx, kernel, dim3(c, slices), kBnThreads, 0, x, g, mean, inv, gamma, beta, n, c, plane, ipc, pa, pb);
+  };
+  if (vec) relu ? partial(bn_bwd_partial_kernel<4, true>) : partial(bn_bwd_partial_kernel<4, false>);
+  else relu ? partial(bn_bwd_partial_kernel<1, true>) : partial(bn_bwd_partial_kernel<1, false>);
   int64_t planes = (int64_t)n * c;
   if (dx && planes > 0 && plane > 0) {
     float* coef = nullptr;
     OM_TRY(pool_alloc(ctx, sizeof(float) * 3 * (size_t)c, false, (void**)&coef));
     launch_chained(ctx, bn_bwd_coef_kernel, (unsigned)ceil_div(c, 128), 128, 0, gamma, inv, pa, pb, slices, (double)n * plane, c, coef);
     const int64_t total = planes * plane;
-    if ((plane & 3) == 0) launch_chained(ctx, bn_bwd_apply_kernel<4>, grid_for(ctx, total / 4, 256), 256, 0, g, x, mean, inv, coef, total, c, plane, training, dx);
-    else launch_chained(ctx, bn_bwd_apply_kernel<1>, grid_for(ctx, total, 256), 256, 0, g, x, mean, inv, coef, total, c, plane, training, dx);
+    auto apply = [&](auto kernel, int64_t accesses) {
+      launch_chained(ctx, kernel, grid_for(ctx, accesses, 256), 256, 0, g, x, mean, inv, gamma, beta, coef, total, c, plane, training, dx);
+    };
+    if ((plane & 3) == 0) relu ? apply(bn_bwd_apply_kernel<4, true>, total / 4) : apply(bn_bwd_apply_kernel<4, false>, total / 4);
+    else relu ? apply(bn_bwd_apply_kernel<1, true>, total) : apply(bn_bwd_apply_kernel<1, false>, total);
     pool_free(ctx, coef);
   }
   if (dgamma || dbeta)
@@ -889,6 +927,18 @@ int32_t om_batchnorm_bwd(om_ctx* ctx, const float* g, const float* x, const floa
   pool_free(ctx, pb);
   OM_LAUNCH_CHECK(ctx, "om_batchnorm_bwd");
   return OM_OK;
+}
+
+int32_t om_batchnorm_bwd(om_ctx* ctx, const float* g, const float* x, const float* gamma, const float* mean,
+                         const float* inv, int32_t n, int32_t c, int32_t plane, int32_t training, float* dx,
+                         float* dgamma, float* dbeta, int32_t accumulate_params) {
+  return batchnorm_bwd(ctx, g, x, gamma, mean, inv, n, c, plane, training, dx, dgamma, dbeta, accumulate_params, false, nullptr);
+}
+
+int32_t om_batchnorm_relu_bwd(om_ctx* ctx, const float* g, const float* x, const float* gamma, const float* beta, const float* mean,
+                              const float* inv, int32_t n, int32_t c, int32_t plane, int32_t training, float* dx,
+                              float* dgamma, float* dbeta, int32_t accumulate_params) {
+  return batchnorm_bwd(ctx, g, x, gamma, mean, inv, n, c, plane, training, dx, dgamma, dbeta, accumulate_params, true, beta);
 }
 
 }  // extern "C"

@@ -465,8 +465,12 @@ static void BatchNormBackward(BackwardRecord& r, const Tensor& g) {
   bool acc, gleaf, bleaf;
   Tensor tg, tb;
   NormParamGrads(r, &dg, &db, &acc, &tg, &tb, &gleaf, &bleaf);
-  Check(om_batchnorm_bwd(C(), gc.Data(), x.Data(), gamma.Data(), mean.Data(), inv.Data(), n, c, plane, r.Ints[0] != 0,
-                         dx.IsEmpty() ? nullptr : dx.Data(), dg, db, acc));
+  if (r.Ints[1] != 0)
+    Check(om_batchnorm_relu_bwd(C(), gc.Data(), x.Data(), gamma.Data(), r.Saved(4).Data(), mean.Data(), inv.Data(), n, c, plane, r.Ints[0] != 0,
+                                dx.IsEmpty() ? nullptr : dx.Data(), dg, db, acc));
+  else
+    Check(om_batchnorm_bwd(C(), gc.Data(), x.Data(), gamma.Data(), mean.Data(), inv.Data(), n, c, plane, r.Ints[0] != 0,
+                           dx.IsEmpty() ? nullptr : dx.Data(), dg, db, acc));
   if (!dx.IsEmpty()) Engine::Emit(r, 0, dx, true);
   EmitNormParams(r, tg, tb, gleaf, bleaf);
 }

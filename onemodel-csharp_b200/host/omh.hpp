@@ -368,7 +368,7 @@ struct Ops {
   // LayerNorm(Add(a, b), gamma, beta) in one pass over a and b (the residual connection in front of a layer norm).
   static Tensor AddLayerNorm(const Tensor& a, const Tensor& b, const Tensor& gamma, const Tensor& beta, float epsilon = 1e-5f);
   static Tensor BatchNorm2d(const Tensor& x, const Tensor& gamma, const Tensor& beta, const Tensor& runningMean,
-                            const Tensor& runningVar, bool training, float momentum = 0.1f, float epsilon = 1e-5f);
+                            const Tensor& runningVar, bool training, float momentum = 0.1f, float epsilon = 1e-5f, bool relu = false);
   static Tensor Conv2d(const Tensor& x, const Tensor& weight, const Tensor& bias, const Conv2dParams& p);
   static Tensor MaxPool2d(const Tensor& x, int kh, int kw, int sh, int sw, int ph = 0, int pw = 0);
   static Tensor AvgPool2d(const Tensor& x, int kh, int kw, int sh, int sw, int ph = 0, int pw = 0, bool countIncludePad = false);
@@ -549,7 +549,12 @@ struct ConvTranspose2d : NnModule {
 struct Lambda : NnModule {
   std::function<Tensor(const Tensor&)> Fn;
   explicit Lambda(std::function<Tensor(const Tensor&)> fn) : Fn(std::move(fn)) {}
-  static Lambda* Relu() { return new Lambda([](const Tensor& x) { return Ops::Relu(x); }); }
+  bool IsRelu = false;
+  static Lambda* Relu() {
+    Lambda* l = new Lambda([](const Tensor& x) { return Ops::Relu(x); });
+    l->IsRelu = true;
+    return l;
+  }
   static Lambda* Gelu(bool approximateTanh = false) { return new Lambda([=](const Tensor& x) { return Ops::Gelu(x, approximateTanh); }); }
   static Lambda* Sigmoid() { return new Lambda([](const Tensor& x) { return Ops::Sigmoid(x); }); }
   static Lambda* Tanh() { return new Lambda([](const Tensor& x) { return Ops::Tanh(x); }); }
@@ -572,22 +577,35 @@ struct Lambda : NnModule {
   Tensor Forward(const Tensor& x) override { return Fn(x); }
 };
 // Children named "0", "1", ... applied in order; takes ownership of the layers (Layers.cs:428-453).
-struct Sequential : NnModule {
-  explicit Sequential(std::vector<NnModule*> layers) {
-    for (size_t i = 0; i < layers.size(); i++) RegisterModule(std::to_string(i), layers[i]);
-  }
-  Tensor Forward(const Tensor& x) override {
-    Tensor h = x;
-    for (auto& c : children_) h = c.second->Forward(h);
-    return h;
-  }
-};
 struct BatchNorm2d : NnModule {
   Tensor Gamma, Beta, RunningMean, RunningVar;
   float Momentum, Epsilon;
   explicit BatchNorm2d(int channels, float momentum = 0.1f, float eps = 1e-5f);
   Tensor Forward(const Tensor& x) override {
     return Ops::BatchNorm2d(x, Gamma, Beta, RunningMean, RunningVar, Training, Momentum, Epsilon);
+  }
+  // Relu(Forward(x)) in the norm's own passes.
+  Tensor ForwardRelu(const Tensor& x) {
+    return Ops::BatchNorm2d(x, Gamma, Beta, RunningMean, RunningVar, Training, Momentum, Epsilon, true);
+  }
+};
+struct Sequential : NnModule {
+  explicit Sequential(std::vector<NnModule*> layers) {
+    for (size_t i = 0; i < layers.size(); i++) RegisterModule(std::to_string(i), layers[i]);
+  }
+  Tensor Forward(const Tensor& x) override {
+    Tensor h = x;
+    for (size_t i = 0; i < children_.size(); i++) {
+      BatchNorm2d* norm = i + 1 < children_.size() ? dynamic_cast<BatchNorm2d*>(&*children_[i].second) : nullptr;
+      Lambda* next = norm ? dynamic_cast<Lambda*>(&*children_[i + 1].second) : nullptr;
+      if (next && next->IsRelu) {
+        h = norm->ForwardRelu(h);      // the rectifier behind a batch norm rides in it
+        i++;
+      } else {
+        h = children_[i].second->Forward(h);
+      }
+    }
+    return h;
   }
 };
 struct MultiHeadAttention : NnModule {

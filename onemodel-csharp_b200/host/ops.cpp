@@ -262,7 +262,7 @@ Tensor Ops::AddLayerNorm(const Tensor& a, const Tensor& b, const Tensor& gamma, 
 }
 
 Tensor Ops::BatchNorm2d(const Tensor& x, const Tensor& gamma, const Tensor& beta, const Tensor& runningMean,
-                        const Tensor& runningVar, bool training, float momentum, float eps) {
+                        const Tensor& runningVar, bool training, float momentum, float eps, bool relu) {
   RequireFloat32(x);
   if (x.Rank() != 4) throw TensorShapeException("BatchNorm2d needs an (N,C,H,W) input, not " + x.GetShape().ToString() + ".");
   int n = x.GetShape()[0], c = x.GetShape()[1], plane = x.GetShape()[2] * x.GetShape()[3];
@@ -272,15 +272,23 @@ Tensor Ops::BatchNorm2d(const Tensor& x, const Tensor& gamma, const Tensor& beta
   Tensor xc = x.Contiguous(), gc = gamma.Contiguous(), bc = beta.Contiguous();
   Tensor mean = Tensor::Create(DType::F32, Shape{c}), inv = Tensor::Create(DType::F32, Shape{c});
   Tensor r = NewOut(x.GetShape());
-  Check(om_batchnorm_fwd(C(), xc.Data(), gc.Data(), bc.Data(), runningMean.Data(), runningVar.Data(), n, c, plane,
-                         training, momentum, eps, r.Data(), mean.Data(), inv.Data()));
+  Tensor used;
+  if (relu) {
+    used = Tensor::Create(DType::F32, Shape{c});
+    Check(om_batchnorm_relu_fwd(C(), xc.Data(), gc.Data(), bc.Data(), runningMean.Data(), runningVar.Data(), n, c, plane,
+                                training, momentum, eps, r.Data(), mean.Data(), inv.Data(), used.Data()));
+  } else {
+    Check(om_batchnorm_fwd(C(), xc.Data(), gc.Data(), bc.Data(), runningMean.Data(), runningVar.Data(), n, c, plane,
+                           training, momentum, eps, r.Data(), mean.Data(), inv.Data()));
+  }
   if (!Recording({&x, &gamma, &beta})) return r;
-  auto br = BackwardRecord::Create(OpKind::BatchNorm, 4, {&x, &gamma, &beta});
+  auto br = BackwardRecord::Create(OpKind::BatchNorm, relu ? 5 : 4, {&x, &gamma, &beta});
+  if (relu) br->Save(4, used);
   br->Save(0, xc.Detach());
   br->Save(1, gc.Detach());
   br->Save(2, mean);
   br->Save(3, inv);
-  br->Ints = {training ? 1 : 0};
+  br->Ints = {training ? 1 : 0, relu ? 1 : 0};
   br->Floats = {eps};
   return br->Attach(r);
 }

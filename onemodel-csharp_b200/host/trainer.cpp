@@ -120,7 +120,7 @@ struct SmallCnn : NnModule {
   }
   Tensor Forward(const Tensor& x) override {
     Tensor h = x;
-    for (size_t i = 0; i < convs.size(); i++) h = Ops::Relu(norms[i]->Forward(convs[i]->Forward(h)));
+    for (size_t i = 0; i < convs.size(); i++) h = norms[i]->ForwardRelu(convs[i]->Forward(h));
     Tensor pooled = Ops::GlobalAvgPool2d(h);
     return Fc->Forward(pooled.Reshape(Shape{pooled.GetShape()[0], pooled.GetShape()[1]}));
   }

@@ -375,3 +375,33 @@ def test_batch_norm_statistics_and_sums(ctx, n, c, h, w, offset):
     assert np.max(np.abs(DG.numpy() - sg)) <= 1e-4 * max(1.0, np.max(np.abs(sg)))
     want = gamma[None, :, None, None] * inv * (g64 - sb[None, :, None, None] / m - xh * sg[None, :, None, None] / m)
     assert np.max(np.abs(DX.numpy() - want)) <= 1e-4 * max(1.0, np.max(np.abs(want)))
+
+
+@pytest.mark.parametrize("n,c,h,w,training", [(5, 3, 4, 4, 1), (3, 2, 3, 5, 1), (17, 4, 16, 20, 1), (4, 3, 7, 4, 0)])
+def test_batch_norm_with_its_rectifier(ctx, n, c, h, w, training):
+    """One call against the norm followed by the rectifier: the same bits forward and backward, negative and zero inputs and a NaN among them."""
+    x, g = normal(1, n, c, h, w), normal(2, n, c, h, w)
+    gamma, beta = normal(3, c), normal(4, c)
+    gamma[0] = 0.0                       # a channel whose rectifier sees beta alone
+    if not training:
+        x[0, 1, 0, 0] = np.nan
+    X, G, GA, BE = (ctx.to_device(a) for a in (x, g, gamma, beta))
+    geometry = [i32(n), i32(c), i32(h * w)]
+    out = {}
+    for fused in (0, 1):
+        RM, RV = ctx.to_device(np.full(c, 0.1, np.float32)), ctx.to_device(np.full(c, 2.0, np.float32))
+        Y, M, I, DX, DG, DB, U = ctx.empty(x.shape), ctx.empty((c,)), ctx.empty((c,)), ctx.empty(x.shape), ctx.empty((c,)), ctx.empty((c,)), ctx.empty((c,))
+        args = [X.ptr, GA.ptr, BE.ptr, RM.ptr, RV.ptr, *geometry, i32(training), f32(0.1), f32(1e-5)]
+        if fused:
+            ctx.call("om_batchnorm_relu_fwd", ctx.handle, *args, Y.ptr, M.ptr, I.ptr, U.ptr)
+            ctx.call("om_batchnorm_relu_bwd", ctx.handle, G.ptr, X.ptr, GA.ptr, U.ptr, M.ptr, I.ptr, *geometry, i32(training), DX.ptr, DG.ptr, DB.ptr, i32(0))
+            assert np.array_equal(U.numpy(), beta)
+        else:
+            Z, GZ = ctx.empty(x.shape), ctx.empty(x.shape)
+            ctx.call("om_batchnorm_fwd", ctx.handle, *args, Z.ptr, M.ptr, I.ptr)
+            ctx.call("om_unary", ctx.handle, i32(1), Z.ptr, Y.ptr, i64(x.size))
+            ctx.call("om_unary_bwd", ctx.handle, i32(1), G.ptr, Y.ptr, GZ.ptr, i64(x.size))
+            ctx.call("om_batchnorm_bwd", ctx.handle, GZ.ptr, X.ptr, GA.ptr, M.ptr, I.ptr, *geometry, i32(training), DX.ptr, DG.ptr, DB.ptr, i32(0))
+        out[fused] = [a.numpy().copy() for a in (Y, M, I, RM, RV, DX, DG, DB)]
+    for a, b in zip(out[0], out[1]):
+        assert np.array_equal(a, b, equal_nan=True)
