@@ -137,7 +137,18 @@ static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 // Without the launch attribute both instructions do nothing.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// What follows the wait depends on a value that comes out of it (the grid's width, never zero): the compiler takes loads through
+// `const __restrict__` pointers and __ldg as loads of constants and moves them above the bare instruction, its memory clobber
+// notwithstanding. In a chain of small resident kernels such a load read what was there before the chain (a count written
+// three kernels earlier: stale in 100 of 100 runs, none with the dependence).
+__device__ __forceinline__ void pdl_wait() {
+  uint32_t grid;
+  asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, %%nctaid.x;" : "=r"(grid) :: "memory");
+  if (grid == 0) {
+    asm volatile("exit;");
+    __builtin_unreachable();
+  }
+}
 __device__ __forceinline__ void pdl_enter() {
   pdl_trigger();
   pdl_wait();

@@ -405,3 +405,25 @@ def test_batch_norm_with_its_rectifier(ctx, n, c, h, w, training):
         out[fused] = [a.numpy().copy() for a in (Y, M, I, RM, RV, DX, DG, DB)]
     for a, b in zip(out[0], out[1]):
         assert np.array_equal(a, b, equal_nan=True)
+
+
+@pytest.mark.parametrize("v,dim,n", [(50, 16, 20), (7, 3, 5), (300, 8, 64)])
+def test_kernels_of_a_chain_read_what_the_chain_wrote(ctx, v, dim, n):
+    """A count that one kernel of a chain leaves and others read, while a slow kernel in front lets the whole chain queue up: every round has
+    another number of rows, and the dense form is that of float32 additions in position order."""
+    r = np.random.default_rng(v)
+    slow, S = ctx.to_device(normal(1, 4096)), ctx.empty((1,))
+    cap = min(n, v)
+    rows, values, count = ctx.empty((cap,), np.int32), ctx.empty((cap, dim)), ctx.to_device(np.zeros(1, np.int32))
+    for distinct in (cap, 1, cap // 2, 2, cap):
+        ids = r.permutation(v)[:distinct][r.integers(0, distinct, n)].astype(np.int32)
+        g = normal(distinct, n, dim)
+        I, G, D = ctx.to_device(ids), ctx.to_device(g), ctx.to_device(np.zeros((v, dim), np.float32))
+        for _ in range(4):
+            ctx.call("om_reduce_fwd", ctx.handle, slow.ptr, i64(1), i64(4096), i64(1), i32(0), S.ptr)
+        ctx.call("om_embedding_bwd_sparse", ctx.handle, G.ptr, I.ptr, i32(1), i64(n), i32(v), i32(dim), i64(-1), rows.ptr, values.ptr, i32(cap), count.ptr)
+        ctx.call("om_rowsparse_add_to", ctx.handle, rows.ptr, values.ptr, count.ptr, i32(cap), i32(dim), D.ptr, i32(v))
+        want = np.zeros((v, dim), np.float32)
+        np.add.at(want, ids, g)
+        assert count.numpy()[0] == np.unique(ids).size
+        assert np.array_equal(D.numpy(), want)
