@@ -485,12 +485,14 @@ __device__ __forceinline__ double bn_cta_sum(double v, double* sm) {
   return t;
 }
 
-// Count, mean and sum of squared deviations of a set of values; two sets combine by the rule of Chan, Golub and LeVeque ("Updating
-// formulae and a pairwise algorithm for computing sample variances", 1979), so nothing cancels.
+// Count, sum, mean and sum of squared deviations of a set of values; two sets combine by the rule of Chan, Golub and LeVeque ("Updating
+// formulae and a pairwise algorithm for computing sample variances", 1979), so nothing cancels. The mean that leaves is the sum's: one
+// infinite value makes the combined mean inf - inf, and the channel's mean is infinite.
 struct BnSet {
-  double n, mean, dev;
-  __device__ void add(double nb, double mb, double db) {
+  double n, sum, mean, dev;
+  __device__ void add(double nb, double sb, double mb, double db) {
     if (nb == 0.0) return;
+    sum += sb;
     const double all = n + nb, d = mb - mean, share = nb / all;
     mean += d * share;
     dev += db + d * d * (n * share);
@@ -503,7 +505,7 @@ struct BnSet {
 // the tensor again for the deviations took 157 us a step for the eight layers of the convolutional network.
 template <int VEC>
 __global__ void __launch_bounds__(kBnThreads)
-bn_stats_kernel(const float* __restrict__ x, int32_t n, int32_t c, int32_t plane, int32_t ipc, double* __restrict__ pmean, double* __restrict__ pdev) {
+bn_stats_kernel(const float* __restrict__ x, int32_t n, int32_t c, int32_t plane, int32_t ipc, double* __restrict__ psum, double* __restrict__ pdev) {
   pdl_enter();
   __shared__ BnSet sm[kBnThreads / 32];
   constexpr int LOADS = VEC == 4 ? 8 : 16;
@@ -512,7 +514,7 @@ bn_stats_kernel(const float* __restrict__ x, int32_t n, int32_t c, int32_t plane
   const int64_t image = (int64_t)c * plane;
   const float* base = x + (int64_t)ch * plane;
   BnWalk w(i0, plane / VEC);
-  BnSet set = {0.0, 0.0, 0.0};
+  BnSet set = {0.0, 0.0, 0.0, 0.0};
   while (w.i < i1) {
     float v[LOADS][VEC];
     int have = 0;
@@ -540,18 +542,19 @@ bn_stats_kernel(const float* __restrict__ x, int32_t n, int32_t c, int32_t plane
           const double d = (double)v[l][j] - mb;
           q += d * d;
         }
-    set.add(nb, mb, q);
+    set.add(nb, s, mb, q);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    const double nb = __shfl_down_sync(0xffffffffu, set.n, o), mb = __shfl_down_sync(0xffffffffu, set.mean, o), db = __shfl_down_sync(0xffffffffu, set.dev, o);
-    set.add(nb, mb, db);
+    const double nb = __shfl_down_sync(0xffffffffu, set.n, o), sb = __shfl_down_sync(0xffffffffu, set.sum, o);
+    const double mb = __shfl_down_sync(0xffffffffu, set.mean, o), db = __shfl_down_sync(0xffffffffu, set.dev, o);
+    set.add(nb, sb, mb, db);
   }
   if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = set;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int k = 1; k < kBnThreads / 32; k++) set.add(sm[k].n, sm[k].mean, sm[k].dev);
-    pmean[(int64_t)slice * c + ch] = set.mean;
+    for (int k = 1; k < kBnThreads / 32; k++) set.add(sm[k].n, sm[k].sum, sm[k].mean, sm[k].dev);
+    psum[(int64_t)slice * c + ch] = set.sum;
     pdev[(int64_t)slice * c + ch] = set.dev;
   }
 }
@@ -604,16 +607,19 @@ bn_bwd_partial_kernel(const float* __restrict__ x, const float* __restrict__ g, 
   }
 }
 
-__global__ void bn_finish_stats_kernel(const double* __restrict__ pmean, const double* __restrict__ pdev, int slices, int32_t n, int32_t ipc, int32_t plane,
+__global__ void bn_finish_stats_kernel(const double* __restrict__ psum, const double* __restrict__ pdev, int slices, int32_t n, int32_t ipc, int32_t plane,
                                        int32_t c, double m, float momentum, float eps, float* __restrict__ mean,
                                        float* __restrict__ inv, float* __restrict__ rm, float* __restrict__ rv, const float* __restrict__ beta, float* __restrict__ beta_out) {
   pdl_enter();
   int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
   if (beta_out) beta_out[ch] = beta[ch];
-  BnSet set = {0.0, 0.0, 0.0};
-  for (int s = 0; s < slices; s++) set.add((double)max(0, min(n, (s + 1) * ipc) - s * ipc) * plane, pmean[(int64_t)s * c + ch], pdev[(int64_t)s * c + ch]);
-  const double mu = set.mean;
+  BnSet set = {0.0, 0.0, 0.0, 0.0};
+  for (int s = 0; s < slices; s++) {
+    const double nb = (double)max(0, min(n, (s + 1) * ipc) - s * ipc) * plane, sb = psum[(int64_t)s * c + ch];
+    set.add(nb, sb, sb / nb, pdev[(int64_t)s * c + ch]);
+  }
+  const double mu = set.sum / m;
   double var = set.dev / m;
   mean[ch] = (float)mu;
   inv[ch] = 1.0f / sqrtf((float)var + eps);

@@ -427,3 +427,18 @@ def test_kernels_of_a_chain_read_what_the_chain_wrote(ctx, v, dim, n):
         np.add.at(want, ids, g)
         assert count.numpy()[0] == np.unique(ids).size
         assert np.array_equal(D.numpy(), want)
+
+
+@pytest.mark.parametrize("n,c,h,w", [(6, 3, 4, 4), (5, 3, 3, 5), (70, 3, 16, 8)])
+def test_batch_norm_statistics_with_infinities(ctx, n, c, h, w):
+    """An infinite value makes its channel's mean infinite (and the running mean), both signs make it NaN; the other channel is unharmed."""
+    x = normal(1, n, c, h, w)
+    x[1, 0, 1, 2] = np.inf
+    x[0, 1, 0, 0], x[n - 1, 1, 2, 1] = np.inf, -np.inf
+    X, GA, BE, RM, RV = (ctx.to_device(a) for a in (x, np.ones(c, np.float32), np.zeros(c, np.float32), np.zeros(c, np.float32), np.ones(c, np.float32)))
+    Y, M, I = ctx.empty(x.shape), ctx.empty((c,)), ctx.empty((c,))
+    ctx.call("om_batchnorm_fwd", ctx.handle, X.ptr, GA.ptr, BE.ptr, RM.ptr, RV.ptr, i32(n), i32(c), i32(h * w), i32(1), f32(0.1), f32(1e-5), Y.ptr, M.ptr, I.ptr)
+    mean, running = M.numpy(), RM.numpy()
+    assert mean[0] == np.inf and running[0] == np.inf and np.isnan(mean[1]) and np.isnan(running[1])
+    assert np.isnan(I.numpy()[:2]).all() and np.isfinite(Y.numpy()[:, 2]).all()
+    assert abs(mean[2] - x[:, 2].astype(np.float64).mean()) <= 1e-6
