@@ -16,6 +16,7 @@
 #include <stdexcept>
 #include <string>
 #include <utility>
+#include <typeinfo>
 #include <vector>
 
 #include "onemodel_b200.h"
@@ -549,12 +550,11 @@ struct ConvTranspose2d : NnModule {
 struct Lambda : NnModule {
   std::function<Tensor(const Tensor&)> Fn;
   explicit Lambda(std::function<Tensor(const Tensor&)> fn) : Fn(std::move(fn)) {}
-  bool IsRelu = false;
-  static Lambda* Relu() {
-    Lambda* l = new Lambda([](const Tensor& x) { return Ops::Relu(x); });
-    l->IsRelu = true;
-    return l;
-  }
+  struct Rectifier {
+    Tensor operator()(const Tensor& x) const { return Ops::Relu(x); }
+  };
+  static Lambda* Relu() { return new Lambda(Rectifier()); }
+  bool IsRelu() const { return Fn.target<Rectifier>() != nullptr; }
   static Lambda* Gelu(bool approximateTanh = false) { return new Lambda([=](const Tensor& x) { return Ops::Gelu(x, approximateTanh); }); }
   static Lambda* Sigmoid() { return new Lambda([](const Tensor& x) { return Ops::Sigmoid(x); }); }
   static Lambda* Tanh() { return new Lambda([](const Tensor& x) { return Ops::Tanh(x); }); }
@@ -576,7 +576,6 @@ struct Lambda : NnModule {
   static Lambda* Mean(int axis) { return new Lambda([=](const Tensor& x) { return Ops::Mean(x, axis); }); }
   Tensor Forward(const Tensor& x) override { return Fn(x); }
 };
-// Children named "0", "1", ... applied in order; takes ownership of the layers (Layers.cs:428-453).
 struct BatchNorm2d : NnModule {
   Tensor Gamma, Beta, RunningMean, RunningVar;
   float Momentum, Epsilon;
@@ -589,6 +588,7 @@ struct BatchNorm2d : NnModule {
     return Ops::BatchNorm2d(x, Gamma, Beta, RunningMean, RunningVar, Training, Momentum, Epsilon, true);
   }
 };
+// Children named "0", "1", ... applied in order; takes ownership of the layers (Layers.cs:428-453).
 struct Sequential : NnModule {
   explicit Sequential(std::vector<NnModule*> layers) {
     for (size_t i = 0; i < layers.size(); i++) RegisterModule(std::to_string(i), layers[i]);
@@ -596,14 +596,17 @@ struct Sequential : NnModule {
   Tensor Forward(const Tensor& x) override {
     Tensor h = x;
     for (size_t i = 0; i < children_.size(); i++) {
-      BatchNorm2d* norm = i + 1 < children_.size() ? dynamic_cast<BatchNorm2d*>(&*children_[i].second) : nullptr;
-      Lambda* next = norm ? dynamic_cast<Lambda*>(&*children_[i + 1].second) : nullptr;
-      if (next && next->IsRelu) {
-        h = norm->ForwardRelu(h);      // the rectifier behind a batch norm rides in it
-        i++;
-      } else {
-        h = children_[i].second->Forward(h);
+      NnModule& layer = *children_[i].second;
+      // A rectifier behind a batch norm rides in it. Exactly these two types: one derived from them may have a Forward of its own.
+      if (i + 1 < children_.size() && typeid(layer) == typeid(BatchNorm2d)) {
+        NnModule& next = *children_[i + 1].second;
+        if (typeid(next) == typeid(Lambda) && static_cast<Lambda&>(next).IsRelu()) {
+          h = static_cast<BatchNorm2d&>(layer).ForwardRelu(h);
+          i++;
+          continue;
+        }
       }
+      h = layer.Forward(h);
     }
     return h;
   }
