@@ -16,7 +16,8 @@
 // What bounds the kernels is the load/store unit: 128 x 32 gathered elements a 128 x 128 x 32 product.
 //
 // dgrad with stride s works on the s * s classes of input positions modulo the stride (grid z): each is a stride-1
-// problem over the taps that reach it, so no product is formed with the zeros between the strides.
+// problem over the taps that reach it, so no product is formed with the zeros between the strides. Positions of the gradient outside its
+// plane count as zeros (folding left them out), so a weight that is infinite or NaN reaches the border pixels of dx also through those.
 #include "om_conv.cuh"
 #include "om_tc.cuh"
 
