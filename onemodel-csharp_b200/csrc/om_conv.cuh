@@ -12,8 +12,6 @@ struct ConvGeom {
 // has already decided that the product runs on the tensor pipe.
 bool conv_tc_fwd_fits(const ConvGeom& g);
 int32_t conv_tc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y);
-bool conv_tc_dgrad_fits(const ConvGeom& g);
-int32_t conv_tc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx);
 bool conv_tc_wgrad_fits(const ConvGeom& g);
 int32_t conv_tc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, float* dw, int accumulate);
 

@@ -2,7 +2,7 @@
 // BackwardNn.cs:317-462 of the reference), TF32 operands, fp32 accumulators in tensor memory.
 //
 //   forward  y[co, pixel]  = sum over k = (c, tap)    W[co, k]          x[c, pixel's input position of the tap]
-//   dgrad    dx[c, pixel]  = sum over k = (co, tap)   W[co, c, tap]     g[co, pixel's output position of the tap]
+//   dgrad    dx[c, pixel]  = sum over taps of the sum over co of   W[co, c, tap]     g[co, pixel's output position of the tap]
 //   wgrad    dW[co, n]     = sum over k = pixels      g[co, pixel]      x[n's channel, pixel's input position of n's tap]
 //
 // The operand that an unfolded matrix would hold is gathered by eight warps straight into the K-major, 128-byte-swizzled
@@ -15,9 +15,8 @@
 // taps of a window find each other's lines in L1. The weights are turned into the order of the units by a small kernel.
 // What bounds the kernels is the load/store unit: 128 x 32 gathered elements a 128 x 128 x 32 product.
 //
-// dgrad with stride s works on the s * s classes of input positions modulo the stride (grid z): each is a stride-1
-// problem over the taps that reach it, so no product is formed with the zeros between the strides. Positions of the gradient outside its
-// plane count as zeros (folding left them out), so a weight that is infinite or NaN reaches the border pixels of dx also through those.
+// dgrad (channels-last only) with stride s works on the s * s classes of input positions modulo the stride (grid z): each is a stride-1
+// problem over the taps that reach it, so no product is formed with the zeros between the strides.
 #include "om_conv.cuh"
 #include "om_tc.cuh"
 
@@ -33,7 +32,6 @@ constexpr int CV_THREADS = 32 * (CV_PRODUCERS + 2);   // + one warp issuing prod
 constexpr int CV_MAX_TAPS = 32;                   // a thread keeps the taps that lie inside the image as a bit mask
 constexpr int CV_MAX_PHASES = 4;
 constexpr int CV_STG_LD = CV_TILE + 4;            // floats per staged result row
-constexpr double CN_MIN_FLOPS = 1e9;              // below, turning the source costs more than it gives
 
 // n / d for 0 <= n < 2^31 by a multiplication (Granlund and Montgomery, "Division by invariant integers using
 // multiplication", 1994): s = ceil(log2 d), mul = floor(2^32 (2^s - d) / d) + 1, n / d = (mulhi(n, mul) + n) >> s.
@@ -61,14 +59,6 @@ __host__ __device__ __forceinline__ void cv_unit(int u, int channels, int taps, 
 }
 static int cv_units(int channels, int taps, int unit) { return (channels + unit - 1) / unit * taps; }
 
-struct ConvPhase {
-  int ph, pw;                  // grid of pixels
-  CvDiv div_plane, div_w;
-  int oy0, ox0;                // output position of pixel (0, 0)
-  int taps, units;
-  int dy[CV_MAX_TAPS], dx[CV_MAX_TAPS];
-};
-
 struct ConvTcParams {
   const float* src;
   float* out;
@@ -76,14 +66,12 @@ struct ConvTcParams {
   int32_t* status;
   int images, m;               // output channels
   int sc, sh, sw;              // source channels and plane
-  int out_w, out_plane;
+  int pw, plane;               // width and size of the output plane
+  CvDiv div_plane, div_w;
   int step_y, step_x, base_y, base_x;   // source position of pixel (y, x) and tap t: y * step_y + base_y + dy[t], likewise x
-  int ostep_y, ostep_x;        // output position of pixel (y, x): y * ostep_y + oy0, likewise x
   int vec;                     // four consecutive pixels are 16 aligned bytes of the output
-  ConvPhase phase[CV_MAX_PHASES];
-};
-struct ConvMaps {
-  CUtensorMap a[CV_MAX_PHASES];
+  int taps, units;
+  int dy[CV_MAX_TAPS], dx[CV_MAX_TAPS];
 };
 
 __device__ __forceinline__ uint32_t rn_tf32(float x) {
@@ -112,19 +100,14 @@ __device__ __forceinline__ void cv_issue(uint32_t tmem, uint32_t a_addr, uint32_
 }
 
 // Turns this CTA's 128 x 128 accumulator into rows of CV_STG_LD floats in shared memory (the dead operand stages).
-__device__ __forceinline__ void cv_stage_rows(float* stg, uint32_t tmem, int warp, int lane, bool any) {
+__device__ __forceinline__ void cv_stage_rows(float* stg, uint32_t tmem, int warp, int lane) {
   const int quad = warp & 3, half = warp >> 2;
 #pragma unroll
   for (int c = 0; c < 2; c++) {
     uint32_t r[32];
     const int col = half * 64 + c * 32;
-    if (any) {
-      tmem_ld_32x32b_x32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)col, r);
-      tmem_ld_wait();
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; j++) r[j] = 0u;
-    }
+    tmem_ld_32x32b_x32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)col, r);
+    tmem_ld_wait();
     float* dst = stg + (quad * 32 + lane) * CV_STG_LD + col;
 #pragma unroll
     for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(dst + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
@@ -151,20 +134,18 @@ __device__ __forceinline__ void cv_load_unit(float* v, const float* __restrict__
   }
 }
 
-// ---- forward and input gradient ------------------------------------------------------------------------------------------
+// ---- forward ---------------------------------------------------------------------------------------------------------------
 // MT: 128-row accumulators per CTA; two (three stages become two, so that two CTAs still share an SM) halve the gathering
 // per product where there are more than 128 output channels and pixels enough to fill the device.
 template <int MT>
 __global__ void __launch_bounds__(CV_THREADS, 2)
-conv_tc_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvTcParams p) {
+conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ ConvTcParams p) {
   constexpr int STAGES = MT == 1 ? 3 : 2;
   constexpr int STAGE_BYTES = (MT + 1) * CV_BLOCK;
   constexpr uint32_t TMEM_COLS = MT * CV_TILE;
-  const ConvPhase& ph = p.phase[blockIdx.z];
-  const int plane = ph.ph * ph.pw;
+  const int plane = p.plane;
   const int pixels = p.images * plane;
   const int q0 = blockIdx.x * CV_TILE;
-  if (q0 >= pixels) return;       // the classes of a strided gradient differ in size
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
@@ -177,7 +158,7 @@ conv_tc_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.y * (MT * CV_TILE);
   const int mts = min(MT, (p.m - m0 + CV_TILE - 1) / CV_TILE);
-  const int k_blocks = (ph.units * CV_UNIT + CV_BK - 1) / CV_BK;
+  const int k_blocks = (p.units * CV_UNIT + CV_BK - 1) / CV_BK;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) {
@@ -190,10 +171,10 @@ conv_tc_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
   }
   for (int u = threadIdx.x; u < k_blocks * (CV_BK / CV_UNIT); u += CV_THREADS) {
     int2 e = make_int2(0, 0);
-    if (u < ph.units) {
+    if (u < p.units) {
       int t, c0;
-      cv_unit<CV_UNIT, CV_GROUP>(u, p.sc, ph.taps, &t, &c0);
-      e.x = (int)(4u * (uint32_t)(c0 * p.sh * p.sw + ph.dy[t] * p.sw + ph.dx[t]));
+      cv_unit<CV_UNIT, CV_GROUP>(u, p.sc, p.taps, &t, &c0);
+      e.x = (int)(4u * (uint32_t)(c0 * p.sh * p.sw + p.dy[t] * p.sw + p.dx[t]));
       e.y = t | (min(CV_UNIT, p.sc - c0) << 8);
     }
     units[u] = e;
@@ -216,11 +197,11 @@ conv_tc_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
     const int q = q0 + px;
     uint32_t mask = 0, base = 0;
     if (q < pixels) {
-      const int n = cv_quot(q, ph.div_plane), r = q - n * plane;
-      const int y = cv_quot(r, ph.div_w), x = r - y * ph.pw;
+      const int n = cv_quot(q, p.div_plane), r = q - n * plane;
+      const int y = cv_quot(r, p.div_w), x = r - y * p.pw;
       const int y0 = y * p.step_y + p.base_y, x0 = x * p.step_x + p.base_x;
-      for (int t = 0; t < ph.taps; t++)
-        if ((unsigned)(y0 + ph.dy[t]) < (unsigned)p.sh && (unsigned)(x0 + ph.dx[t]) < (unsigned)p.sw) mask |= 1u << t;
+      for (int t = 0; t < p.taps; t++)
+        if ((unsigned)(y0 + p.dy[t]) < (unsigned)p.sh && (unsigned)(x0 + p.dx[t]) < (unsigned)p.sw) mask |= 1u << t;
       base = 4u * ((uint32_t)n * (uint32_t)(p.sc * p.sh * p.sw) + (uint32_t)(y0 * p.sw + x0));
     }
     const uint32_t step = 4u * (uint32_t)(p.sh * p.sw);
@@ -260,10 +241,7 @@ conv_tc_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
       deposit(v2, kb + 2);
     }
     // ---- results: accumulator rows through shared memory to rows of consecutive pixels ----
-    if (k_blocks > 0) {
-      const bool done = mbar_wait(acc_full, 0, abort_flag, p.status, 72);
-      ok = __all_sync(0xffffffffu, done) && ok;
-    }
+    ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, p.status, 72)) && ok;
     tc_fence_after();
     float* stg = reinterpret_cast<float*>(smem);
     long long at[4];               // output positions of this lane's pixels relative to their image's first channel; -1 past the end
@@ -272,13 +250,12 @@ conv_tc_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
       const int qi = q0 + (p.vec ? 4 * lane : lane + 32 * i);
       at[i] = -1;
       if (qi < pixels) {
-        const int n = cv_quot(qi, ph.div_plane), r = qi - n * plane;
-        const int y = cv_quot(r, ph.div_w), x = r - y * ph.pw;
-        at[i] = (long long)n * p.m * p.out_plane + (y * p.ostep_y + ph.oy0) * p.out_w + x * p.ostep_x + ph.ox0;
+        const int n = cv_quot(qi, p.div_plane);
+        at[i] = (long long)n * p.m * plane + (qi - n * plane);
       }
     }
     for (int mt = 0; mt < mts; mt++) {
-      if (ok) cv_stage_rows(stg, tmem_base + mt * CV_TILE, warp, lane, k_blocks > 0);
+      if (ok) cv_stage_rows(stg, tmem_base + mt * CV_TILE, warp, lane);
       asm volatile("bar.sync 1, 256;" ::: "memory");
       if (ok) {
 #pragma unroll 4
@@ -286,7 +263,7 @@ conv_tc_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
           const int row = warp * 16 + i, co = m0 + mt * CV_TILE + row;
           if (co >= p.m) break;
           const float bv = p.bias ? __ldg(p.bias + co) : 0.f;
-          float* out = p.out + (long long)co * p.out_plane;
+          float* out = p.out + (long long)co * plane;
           const float* sr = stg + row * CV_STG_LD;
           if (p.vec) {
             if (at[0] >= 0) {
@@ -304,7 +281,7 @@ conv_tc_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
       asm volatile("bar.sync 1, 256;" ::: "memory");
     }
   } else if (warp == CV_PRODUCERS) {
-    if (lane == 0 && k_blocks > 0) {
+    if (lane == 0) {
       for (int kb = 0; kb < k_blocks; kb++) {
         const int s = kb % STAGES;
         if (!mbar_wait(&full[s], (kb / STAGES) & 1, abort_flag, p.status, 73)) break;
@@ -322,7 +299,7 @@ conv_tc_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
       if (round > 0 && !mbar_wait(&empty[s], (round - 1) & 1, abort_flag, p.status, 74)) break;
       mbar_expect_tx(&full[s], (uint32_t)(mts * CV_BLOCK));
       for (int mt = 0; mt < mts; mt++)
-        tma_load_4d(smem + (size_t)s * STAGE_BYTES + mt * CV_BLOCK, &maps.a[blockIdx.z], kb * CV_BK, m0 + mt * CV_TILE, 0, 0, &full[s]);
+        tma_load_4d(smem + (size_t)s * STAGE_BYTES + mt * CV_BLOCK, &map_a, kb * CV_BK, m0 + mt * CV_TILE, 0, 0, &full[s]);
     }
   }
   tc_fence_before();
@@ -333,24 +310,16 @@ conv_tc_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ Co
   }
 }
 
-// The weights in the order of the units, one K-major row per output channel of the product: wt[phase][m][UNIT u + i] is the weight of
-// tap(u) and source channel c0(u) + i, zero past the last channel. Weights are addressed by their strides over (m, source channel).
-struct ConvTurn {
-  int m, sc;
-  long long stride_m, stride_sc;
-  int taps[CV_MAX_PHASES], ld[CV_MAX_PHASES];
-  long long start[CV_MAX_PHASES];
-  int tap[CV_MAX_PHASES][CV_MAX_TAPS];
-};
-template <int UNIT, int GROUP>
-__global__ void __launch_bounds__(256) conv_turn_weights_kernel(const float* __restrict__ w, float* __restrict__ wt, const __grid_constant__ ConvTurn t) {
+// The weights in the order of the units, one K-major row per output channel: wt[m][CV_UNIT u + i] is the weight of tap(u) and source channel
+// c0(u) + i, zero past the last channel.
+__global__ void __launch_bounds__(256) conv_turn_weights_kernel(const float* __restrict__ w, float* __restrict__ wt, int channels, int taps, int ld) {
   pdl_enter();
-  const int z = blockIdx.z, m = blockIdx.y;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < t.ld[z]; i += gridDim.x * blockDim.x) {
+  const int m = blockIdx.y;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ld; i += gridDim.x * blockDim.x) {
     int tap, c0;
-    cv_unit<UNIT, GROUP>(i / UNIT, t.sc, t.taps[z], &tap, &c0);
-    const int c = c0 + i % UNIT;
-    wt[t.start[z] + (long long)m * t.ld[z] + i] = c < t.sc ? __ldg(w + m * t.stride_m + c * t.stride_sc + t.tap[z][tap]) : 0.f;
+    cv_unit<CV_UNIT, CV_GROUP>(i / CV_UNIT, channels, taps, &tap, &c0);
+    const int c = c0 + i % CV_UNIT;
+    wt[(long long)m * ld + i] = c < channels ? __ldg(w + ((long long)m * channels + c) * taps + tap) : 0.f;
   }
 }
 
@@ -475,7 +444,7 @@ conv_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
     ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, p.status, 76)) && ok;
     tc_fence_after();
     float* stg = reinterpret_cast<float*>(smem);
-    if (ok) cv_stage_rows(stg, tmem_base, warp, lane, true);
+    if (ok) cv_stage_rows(stg, tmem_base, warp, lane);
     asm volatile("bar.sync 1, 256;" ::: "memory");
     if (ok) {
       const int ld = p.units * CV_UNIT, col = n0 + 4 * lane;
@@ -558,7 +527,15 @@ conv_wgrad_finish_kernel(const float* __restrict__ part, int splits, int cout, i
 //   forward, dgrad   D [128 pixels, NT channels] += x [pixels + tap, 32 c] W [NT, (32 c, tap)]      both K-major
 //   wgrad            D [128 co, 4 x (32 c, tap)] += g [32 pixels, co] x [32 pixels + tap, 32 c]      both MN-major
 // Accumulator rows are pixels, so a warp's store of one channel is 32 neighbouring pixels of the NCHW result.
-// The weights for these kernels: wt[phase][m][(32-channel block, tap), 32] as conv_turn_weights_kernel<32, 1> would order them, by tiles of
+struct ConvTurn {               // weights addressed by their strides over (m, source channel)
+  int m, sc;
+  long long stride_m, stride_sc;
+  int by_tap;                  // all channels of a tap before the next tap
+  int taps[CV_MAX_PHASES], ld[CV_MAX_PHASES];
+  long long start[CV_MAX_PHASES];
+  int tap[CV_MAX_PHASES][CV_MAX_TAPS];
+};
+// The weights for these kernels: wt[phase][m][(32-channel block, tap), 32], or (tap, 32-channel block) for dgrad, by tiles of
 // 8 m x 32 source channels through shared memory. Read and written in runs (element by element, the reads were 4 bytes a line:
 // 512 x 512 x 3 x 3 took 14 us).
 constexpr int CN_PACK_M = 8;
@@ -577,8 +554,11 @@ __global__ void __launch_bounds__(256) conv_pack_weights_kernel(const float* __r
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (m0 + warp >= t.m) return;
   for (int z = 0; z < phases; z++) {
-    float* out = wt + t.start[z] + (long long)(m0 + warp) * t.ld[z] + (long long)blockIdx.x * t.taps[z] * CV_BK + lane;
-    for (int j = 0; j < t.taps[z]; j++) out[j * CV_BK] = pack[(warp * CV_BK + lane) * tp + t.tap[z][j]];
+    float* out = wt + t.start[z] + (long long)(m0 + warp) * t.ld[z] + lane;
+    for (int j = 0; j < t.taps[z]; j++) {
+      const int block = t.by_tap ? j * (int)gridDim.x + (int)blockIdx.x : (int)blockIdx.x * t.taps[z] + j;
+      out[(long long)block * CV_BK] = pack[(warp * CV_BK + lane) * tp + t.tap[z][j]];
+    }
   }
 }
 
@@ -587,7 +567,7 @@ struct ConvBox {
   int tw, th, tn;              // tiles along each
 };
 struct ConvNhwcPhase {
-  int ph, pw, oy0, ox0, taps, k_blocks;
+  int ph, pw, oy0, ox0, taps, k_blocks, chain;
   ConvBox box;
   int dy[CV_MAX_TAPS], dx[CV_MAX_TAPS];
 };
@@ -597,6 +577,7 @@ struct ConvNhwcParams {
   int32_t* status;
   int images, m, out_w, out_plane;
   int step_y, step_x, base_y, base_x, ostep_y, ostep_x;
+  int by_tap, sh, sw;          // by_tap: chain t is tap t, and counts for the pixels whose position of it lies in the sh x sw source plane
   ConvNhwcPhase phase[CV_MAX_PHASES];
 };
 struct ConvNhwcMaps {
@@ -665,11 +646,44 @@ __global__ void __launch_bounds__(256) conv_sums_finish_kernel(const double* __r
   }
 }
 
-constexpr int CN_THREADS = 192;      // warp 0: TMA, warp 1: products, warps 2-5: results
-template <int NT, int STAGES>
-__global__ void __launch_bounds__(CN_THREADS, STAGES > 4 ? 1 : 2)
+// Warp 0: TMA, warp 1: products, the others: results. With chains there are two result warps for a quarter of the rows, half of the columns each.
+constexpr int CN_THREADS = 192, CN_CHAIN_THREADS = 320;
+__host__ __device__ constexpr int cn_threads(bool chains) { return chains ? CN_CHAIN_THREADS : CN_THREADS; }
+// What the result warps do with a tile that arrives in chains of `chain` k blocks (see conv_nhwc_kernel): add chain c, in accumulator c % 2 (`pitch` columns
+// apart), to their registers while the other accumulator is being filled. `take(c)`: whether the lane's row counts it.
+template <int COLS, typename Take>
+__device__ __forceinline__ bool cn_add_chains(float (&acc)[COLS], uint32_t tmem, int pitch, int chains, uint64_t* full, uint64_t* empty, volatile int* abort_flag,
+                                              int32_t* status, int where, Take take) {
+#pragma unroll
+  for (int j = 0; j < COLS; j++) acc[j] = 0.f;
+  for (int c = 0; c < chains; c++) {
+    const bool on = take(c);
+    if (!__all_sync(0xffffffffu, mbar_wait(&full[c & 1], (uint32_t)(c >> 1) & 1, abort_flag, status, where))) return false;
+    tc_fence_after();
+#pragma unroll
+    for (int col = 0; col < COLS; col += 16) {
+      uint32_t r[16];
+      tmem_ld_32x32b_x16(tmem + (uint32_t)((c & 1) * pitch + col), r);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; j++) acc[col + j] += on ? __uint_as_float(r[j]) : 0.f;
+    }
+    tc_fence_before();
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) cv_arrive(&empty[c & 1]);
+  }
+  return true;
+}
+// CHAINS: the sum over k in several accumulator chains that are added in fp32 in increasing order. The tensor core cuts what a step of its accumulator
+// cannot hold instead of rounding it, an error that grows with the number of steps (1.8e-8 of the result a step of eight k's: 4.9e-6 at k
+// = 2304). With a chain a tap, dx has the bits of the product on the unfolded matrix and its fold, and a tap outside the gradient's plane
+// is left out whatever its weight is; in one chain over all taps it was 7 times as far from the exact sums. Reading an accumulator back takes the
+// result warps about as long as a block of k takes the products, and goes on beside them.
+template <int NT, int STAGES, bool CHAINS>
+__global__ void __launch_bounds__(cn_threads(CHAINS), STAGES > 4 ? 1 : 2)
 conv_nhwc_kernel(const __grid_constant__ ConvNhwcMaps maps, const __grid_constant__ ConvNhwcParams p) {
   constexpr int STAGE_BYTES = CV_BLOCK + NT * 128;
+  constexpr int ACCS = CHAINS ? 2 : 1;
   const ConvNhwcPhase& ph = p.phase[blockIdx.z];
   const ConvBox& box = ph.box;
   const int tile = blockIdx.x;
@@ -679,7 +693,8 @@ conv_nhwc_kernel(const __grid_constant__ ConvNhwcMaps maps, const __grid_constan
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
   uint64_t* empty = full + STAGES;
   uint64_t* acc_full = empty + STAGES;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+  uint64_t* acc_empty = acc_full + ACCS;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + ACCS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -692,12 +707,15 @@ conv_nhwc_kernel(const __grid_constant__ ConvNhwcMaps maps, const __grid_constan
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(acc_full, 1);
+    for (int a = 0; a < ACCS; a++) {
+      mbar_init(&acc_full[a], 1);
+      mbar_init(&acc_empty[a], 8);
+    }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, NT);
+    tmem_alloc(tmem_slot, ACCS * NT);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -709,6 +727,7 @@ conv_nhwc_kernel(const __grid_constant__ ConvNhwcMaps maps, const __grid_constan
 
   if (warp == 0) {
     if (lane == 0) {
+      const int blocks = ph.taps > 0 ? k_blocks / ph.taps : 0;
       int t = 0, c0 = 0;
       for (int kb = 0; kb < k_blocks; kb++) {
         const int s = kb % STAGES;
@@ -718,7 +737,13 @@ conv_nhwc_kernel(const __grid_constant__ ConvNhwcMaps maps, const __grid_constan
         mbar_expect_tx(&full[s], STAGE_BYTES);
         tma_load_4d(a, &maps.src[blockIdx.z], c0, x0 * p.step_x + p.base_x + ph.dx[t], y0 * p.step_y + p.base_y + ph.dy[t], n0, &full[s]);
         tma_load_4d(a + CV_BLOCK, &maps.w[blockIdx.z], kb * CV_BK, m0, 0, 0, &full[s]);
-        if (++t == ph.taps) {
+        if (p.by_tap) {
+          c0 += CV_BK;
+          if (c0 == blocks * CV_BK) {
+            c0 = 0;
+            t++;
+          }
+        } else if (++t == ph.taps) {
           t = 0;
           c0 += CV_BK;
         }
@@ -727,17 +752,25 @@ conv_nhwc_kernel(const __grid_constant__ ConvNhwcMaps maps, const __grid_constan
   } else if (warp == 1) {
     if (lane == 0 && k_blocks > 0) {
       constexpr uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(CV_TILE >> 4) << 24);
+      int c = 0, at = 0;           // the chain, and the block of it
       for (int kb = 0; kb < k_blocks; kb++) {
         const int s = kb % STAGES;
+        if (CHAINS && at == 0 && c >= ACCS && !mbar_wait(&acc_empty[c & 1], (uint32_t)((c >> 1) - 1) & 1, abort_flag, p.status, 87)) break;
         if (!mbar_wait(&full[s], (kb / STAGES) & 1, abort_flag, p.status, 82)) break;
         tc_fence_after();
         const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES), b = a + CV_BLOCK;
 #pragma unroll
         for (int ks = 0; ks < CV_BK / 8; ks++)
-          umma_tf32(tmem_base, make_desc(a + ks * 32, 16, 1024, 2), make_desc(b + ks * 32, 16, 1024, 2), idesc, (kb > 0 || ks > 0) ? 1u : 0u);
+          umma_tf32(tmem_base + (CHAINS ? (c & 1) * NT : 0), make_desc(a + ks * 32, 16, 1024, 2), make_desc(b + ks * 32, 16, 1024, 2), idesc,
+                    ((CHAINS ? at : kb) > 0 || ks > 0) ? 1u : 0u);
         umma_commit(&empty[s]);
+        if (CHAINS && (++at == ph.chain || kb == k_blocks - 1)) {
+          umma_commit(&acc_full[c & 1]);
+          at = 0;
+          c++;
+        }
       }
-      umma_commit(acc_full);
+      if (!CHAINS) umma_commit(acc_full);
     }
   } else {
     const int quad = warp & 3, slot = quad * 32 + lane;
@@ -745,25 +778,35 @@ conv_nhwc_kernel(const __grid_constant__ ConvNhwcMaps maps, const __grid_constan
     const int x = x0 + ix, y = y0 + iy, n = n0 + in;
     const bool valid = x < ph.pw && y < ph.ph && n < p.images;
     float* out = p.out + ((long long)n * p.m + m0) * p.out_plane + (long long)(y * p.ostep_y + ph.oy0) * p.out_w + x * p.ostep_x + ph.ox0;
-    bool ok = true;
-    if (k_blocks > 0) ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, p.status, 83));
-    tc_fence_after();
-    if (ok) {
+    const uint32_t rows = tmem_base + ((uint32_t)(quad * 32) << 16);
+    if constexpr (CHAINS) {
+      const int sy = y * p.step_y + p.base_y, sx = x * p.step_x + p.base_x;
+      constexpr int COLS = NT / 2;
+      const int col0 = (warp - 2) / 4 * COLS;
+      float acc[COLS];
+      const bool ok = cn_add_chains<COLS>(acc, rows + (uint32_t)col0, NT, (k_blocks + ph.chain - 1) / ph.chain, acc_full, acc_empty, abort_flag, p.status, 83, [&](int c) {
+        return !p.by_tap || ((unsigned)(sy + ph.dy[c]) < (unsigned)p.sh && (unsigned)(sx + ph.dx[c]) < (unsigned)p.sw);
+      });
+      if (ok && valid) {
+#pragma unroll
+        for (int j = 0; j < COLS; j++)
+          if (m0 + col0 + j < p.m) out[(long long)(col0 + j) * p.out_plane] = p.bias ? acc[j] + __ldg(p.bias + m0 + col0 + j) : acc[j];
+      }
+    } else {
+      const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, p.status, 83));
+      tc_fence_after();
+      if (ok) {
 #pragma unroll 1
-      for (int c = 0; c < NT && m0 + c < p.m; c += 32) {
-        uint32_t r[32];
-        if (k_blocks > 0) {
-          tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c, r);
+        for (int c = 0; c < NT && m0 + c < p.m; c += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(rows + (uint32_t)c, r);
           tmem_ld_wait();
-        } else {
+          if (p.bias) add_bias32(r, p.bias, m0 + c, p.m);
+          if (valid) {
 #pragma unroll
-          for (int j = 0; j < 32; j++) r[j] = 0u;
-        }
-        if (p.bias) add_bias32(r, p.bias, m0 + c, p.m);
-        if (valid) {
-#pragma unroll
-          for (int j = 0; j < 32; j++)
-            if (m0 + c + j < p.m) out[(long long)(c + j) * p.out_plane] = __uint_as_float(r[j]);
+            for (int j = 0; j < 32; j++)
+              if (m0 + c + j < p.m) out[(long long)(c + j) * p.out_plane] = __uint_as_float(r[j]);
+          }
         }
       }
     }
@@ -772,7 +815,7 @@ conv_nhwc_kernel(const __grid_constant__ ConvNhwcMaps maps, const __grid_constan
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, NT);
+    tmem_dealloc(tmem_base, ACCS * NT);
   }
 }
 
@@ -923,121 +966,55 @@ static bool cv_sizes_fit(const ConvGeom& g) {
 }
 
 template <int MT>
-static int32_t launch_conv_as(om_ctx* ctx, const ConvMaps& maps, const ConvTcParams& p, dim3 grid, int units) {
+static int32_t launch_conv_as(om_ctx* ctx, const CUtensorMap& map, const ConvTcParams& p, dim3 grid) {
   constexpr int STAGES = MT == 1 ? 3 : 2;
   constexpr size_t stages = (size_t)STAGES * (MT + 1) * CV_BLOCK;
   constexpr int most = 227 * 1024;
   static_assert(stages >= (size_t)CV_TILE * CV_STG_LD * 4, "the result rows are staged in the operand stages");
   static_assert(stages + 1024 + 128 + (65535 + CV_MAX_TAPS * CV_UNIT) / CV_UNIT * sizeof(int2) + 64 <= most, "every table of units fits");
-  const size_t smem = stages + 1024 + 128 + (size_t)((units + 3) & ~3) * sizeof(int2);
+  const size_t smem = stages + 1024 + 128 + (size_t)((p.units + 3) & ~3) * sizeof(int2);
   static bool set = false;
   if (!set) {
     OM_CUDA(ctx, cudaFuncSetAttribute(conv_tc_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     set = true;
   }
-  launch_chained(ctx, conv_tc_kernel<MT>, grid, CV_THREADS, smem, maps, p);
+  launch_chained(ctx, conv_tc_kernel<MT>, grid, CV_THREADS, smem, map, p);
   OM_LAUNCH_CHECK(ctx, "conv_tc");
   return OM_OK;
-}
-
-// Turns the weights and runs the product of every phase. p holds all but the phases' divisors and units, turn the taps.
-static int32_t run_conv(om_ctx* ctx, ConvTcParams& p, ConvTurn& turn, int phases, const float* w) {
-  ConvMaps maps = {};
-  long long floats = 0, most = 0, all = 0;
-  int most_units = 0;
-  for (int z = 0; z < phases; z++) {
-    ConvPhase& f = p.phase[z];
-    f.div_plane = cv_div((uint32_t)std::max(1, f.ph * f.pw));
-    f.div_w = cv_div((uint32_t)std::max(1, f.pw));
-    f.units = cv_units(p.sc, f.taps, CV_UNIT);
-    turn.taps[z] = f.taps;
-    turn.ld[z] = f.units * CV_UNIT;
-    turn.start[z] = floats;
-    floats += (long long)turn.ld[z] * p.m;
-    most_units = std::max(most_units, f.units);
-    const long long tiles = ceil_div((long long)p.images * f.ph * f.pw, CV_TILE);
-    most = std::max(most, tiles);
-    all += tiles;
-  }
-  if (most == 0) return OM_OK;
-  float* wt = nullptr;
-  OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)std::max<long long>(floats, 4), false, (void**)&wt));
-  int32_t st = OM_OK;
-  for (int z = 0; z < phases && st == OM_OK; z++)
-    if (turn.ld[z] > 0 && !cv_map(&maps.a[z], wt + turn.start[z], turn.ld[z], p.m, turn.ld[z], 1, 0))
-      st = fail(ctx, OM_ERR_CUDA, "cuTensorMapEncodeTiled failed for a convolution's turned weights");
-  if (st == OM_OK) {
-    if (most_units > 0)
-      launch_chained(ctx, conv_turn_weights_kernel<CV_UNIT, CV_GROUP>, dim3((unsigned)std::min<int64_t>(ceil_div(most_units * CV_UNIT, 256), 64), (unsigned)p.m, (unsigned)phases), 256, 0, 
-          w, wt, turn);
-    // Two accumulators once that still leaves a CTA for every SM.
-    const bool two = p.m > CV_TILE && all * ceil_div(p.m, 2 * CV_TILE) >= 148;
-    const dim3 grid((unsigned)most, (unsigned)ceil_div(p.m, two ? 2 * CV_TILE : CV_TILE), (unsigned)phases);
-    st = two ? launch_conv_as<2>(ctx, maps, p, grid, most_units) : launch_conv_as<1>(ctx, maps, p, grid, most_units);
-  }
-  pool_free(ctx, wt);
-  return st;
 }
 
 bool conv_tc_fwd_fits(const ConvGeom& g) { return encode_fn() && cv_sizes_fit(g); }
 
 int32_t conv_tc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y) {
   ConvTcParams p = {};
-  ConvTurn turn = {};
-  const int plane = g.oh * g.ow;
   p.src = x; p.out = y; p.bias = bias; p.status = ctx->status_dev;
   p.images = g.n; p.m = g.cout; p.sc = g.cin; p.sh = g.h; p.sw = g.w;
-  p.out_w = g.ow; p.out_plane = plane;
+  p.pw = g.ow; p.plane = g.oh * g.ow;
+  p.div_plane = cv_div((uint32_t)p.plane);
+  p.div_w = cv_div((uint32_t)p.pw);
   p.step_y = g.sh; p.step_x = g.sw; p.base_y = -g.pt; p.base_x = -g.pl;
-  p.ostep_y = p.ostep_x = 1;
-  p.vec = (plane & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
-  ConvPhase& f = p.phase[0];
-  f.ph = g.oh; f.pw = g.ow; f.taps = g.kh * g.kw;
-  for (int t = 0; t < f.taps; t++) {
-    f.dy[t] = (t / g.kw) * g.dh;
-    f.dx[t] = (t % g.kw) * g.dw;
-    turn.tap[0][t] = t;
+  p.vec = (p.plane & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+  p.taps = g.kh * g.kw;
+  p.units = cv_units(g.cin, p.taps, CV_UNIT);
+  for (int t = 0; t < p.taps; t++) {
+    p.dy[t] = (t / g.kw) * g.dh;
+    p.dx[t] = (t % g.kw) * g.dw;
   }
-  turn.m = g.cout; turn.sc = g.cin;
-  turn.stride_m = (long long)g.cin * f.taps; turn.stride_sc = f.taps;
-  return run_conv(ctx, p, turn, 1, w);
-}
-
-bool conv_tc_dgrad_fits(const ConvGeom& g) { return encode_fn() && cv_sizes_fit(g) && g.sh * g.sw <= CV_MAX_PHASES; }
-
-// The taps that reach the input positions (oy0, ox0) modulo the stride, and where in the gradient from a pixel of that class.
-static int class_taps(const ConvGeom& g, int oy0, int ox0, int* dy, int* dx, int* tap) {
-  int n = 0;
-  for (int t = 0; t < g.kh * g.kw; t++) {
-    const int ty = oy0 + g.pt - (t / g.kw) * g.dh, tx = ox0 + g.pl - (t % g.kw) * g.dw;
-    if (ty % g.sh || tx % g.sw) continue;      // (exact for negative values too)
-    dy[n] = ty / g.sh;
-    dx[n] = tx / g.sw;
-    tap[n++] = t;
+  const int ld = p.units * CV_UNIT;
+  float* wt = nullptr;
+  CUtensorMap map;
+  OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)ld * p.m, false, (void**)&wt));
+  int32_t st = cv_map(&map, wt, ld, p.m, ld, 1, 0) ? OM_OK : fail(ctx, OM_ERR_CUDA, "cuTensorMapEncodeTiled failed for a convolution's turned weights");
+  if (st == OM_OK) {
+    launch_chained(ctx, conv_turn_weights_kernel, dim3((unsigned)std::min<int64_t>(ceil_div(ld, 256), 64), (unsigned)p.m), 256, 0, w, wt, g.cin, p.taps, ld);
+    // Two accumulators once that still leaves a CTA for every SM.
+    const int64_t tiles = ceil_div((int64_t)g.n * p.plane, CV_TILE);
+    const bool two = p.m > CV_TILE && tiles * ceil_div(p.m, 2 * CV_TILE) >= 148;
+    const dim3 grid((unsigned)tiles, (unsigned)ceil_div(p.m, two ? 2 * CV_TILE : CV_TILE));
+    st = two ? launch_conv_as<2>(ctx, map, p, grid) : launch_conv_as<1>(ctx, map, p, grid);
   }
-  return n;
-}
-
-int32_t conv_tc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx) {
-  ConvTcParams p = {};
-  ConvTurn turn = {};
-  p.src = gr; p.out = dx; p.status = ctx->status_dev;
-  p.images = g.n; p.m = g.cin; p.sc = g.cout; p.sh = g.oh; p.sw = g.ow;
-  p.out_w = g.w; p.out_plane = g.h * g.w;
-  p.step_y = p.step_x = 1;
-  p.ostep_y = g.sh; p.ostep_x = g.sw;
-  p.vec = g.sh == 1 && g.sw == 1 && (p.out_plane & 3) == 0 && (reinterpret_cast<uintptr_t>(dx) & 15) == 0;
-  for (int z = 0; z < g.sh * g.sw; z++) {
-    ConvPhase& f = p.phase[z];
-    f.oy0 = z / g.sw;
-    f.ox0 = z % g.sw;
-    f.ph = f.oy0 < g.h ? (g.h - f.oy0 + g.sh - 1) / g.sh : 0;
-    f.pw = f.ox0 < g.w ? (g.w - f.ox0 + g.sw - 1) / g.sw : 0;
-    f.taps = class_taps(g, f.oy0, f.ox0, f.dy, f.dx, turn.tap[z]);
-  }
-  turn.m = g.cin; turn.sc = g.cout;
-  turn.stride_m = g.kh * g.kw; turn.stride_sc = (long long)g.cin * g.kh * g.kw;
-  return run_conv(ctx, p, turn, g.sh * g.sw, w);
+  pool_free(ctx, wt);
+  return st;
 }
 
 template <int UNIT, int GROUP>
@@ -1147,20 +1124,30 @@ static int32_t cn_turn_sums(om_ctx* ctx, const float* src, int n, int c, int pla
 
 // A block of 32 channels may be partly empty, and a box partly outside the grid: at least two thirds of the work has to be real.
 static bool cn_channels_fit(int c) { return 3 * c >= 2 * (int)ceil_div(c, 32) * 32; }
-static bool cn_worth(const ConvGeom& g) {
-  return 2.0 * g.n * g.oh * g.ow * (double)g.cout * g.cin * g.kh * g.kw >= CN_MIN_FLOPS && g.sh <= 2 && g.sw <= 2 && (long long)g.n * g.h * g.w * cn_pitch(g.cin) < (1ll << 30) &&
+static bool cn_sizes_fit(const ConvGeom& g) {
+  return encode_fn() && cv_sizes_fit(g) && g.sh <= 2 && g.sw <= 2 && (long long)g.n * g.h * g.w * cn_pitch(g.cin) < (1ll << 30) &&
          (long long)g.n * g.oh * g.ow * cn_pitch(g.cout) < (1ll << 30);
 }
+// The lines between the channels-last form and the others, 3 x 3 windows, us channels last / unfolded; a forward product or a weight
+// gradient needs CN_MIN_FLOPS, below which turning the source costs more than it gives:
+//   input gradient  by the size of the unfolded matrix, the zeros between strides counted: 37 x 24 x 22 x 28 from 48 (4.9 M) 32 / 32, 16 x 256 x 12 x 12
+//                   from 256 (5.3 M) 50 / 36, 8 x 512 x 8 x 8 from 512 (2.4 M) 79 / 36; 37 x 128 x 11 x 12 from 128 (5.6 M) 36 / 40, 64 x 16 x 20 x 32
+//                   from 16 (5.9 M) 30 / 34, 37 x 132 x 11 x 12 from 36 (5.8 M) 30 / 36, 128 x 16 x 24 x 24 from 16 (10.6 M) 36 / 50, with stride 2 24 / 36.
+//                   A deep k makes the few CTAs of a small plane long: 32 x 512 x 7 x 7 from 512 (7.2 M, 144 blocks of k) 81 / 56, 256 x 512 x 4 x 4 from
+//                   512 (18.9 M) 83 / 104. 1 x 1 windows always: 64 x 64 x 16 x 16 15 / 22, 16 x 128 x 14 x 14 from 256 17 / 22.
+constexpr long long CN_MIN_UNFOLDED = 5500000, CN_MIN_UNFOLDED_A_BLOCK = 80000;
+constexpr double CN_MIN_FLOPS = 1e9;
+static double cn_flops(const ConvGeom& g) { return 2.0 * g.n * g.oh * g.ow * (double)g.cout * g.cin * g.kh * g.kw; }
 
-template <int NT, int STAGES>
+template <int NT, int STAGES, bool CHAINS>
 static int32_t launch_nhwc(om_ctx* ctx, const ConvNhwcMaps& maps, const ConvNhwcParams& p, dim3 grid) {
   constexpr size_t smem = (size_t)STAGES * (CV_BLOCK + NT * 128) + 1024 + 256;
   static bool set = false;
   if (!set) {
-    OM_CUDA(ctx, cudaFuncSetAttribute(conv_nhwc_kernel<NT, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    OM_CUDA(ctx, cudaFuncSetAttribute(conv_nhwc_kernel<NT, STAGES, CHAINS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     set = true;
   }
-  launch_chained(ctx, conv_nhwc_kernel<NT, STAGES>, grid, CN_THREADS, smem, maps, p);
+  launch_chained(ctx, conv_nhwc_kernel<NT, STAGES, CHAINS>, grid, cn_threads(CHAINS), smem, maps, p);
   return check_cuda(ctx, cudaGetLastError(), "conv_nhwc");
 }
 
@@ -1175,11 +1162,18 @@ static int32_t run_conv_nhwc(om_ctx* ctx, ConvNhwcParams& p, ConvTurn& turn, int
   const int nt = p.m <= 64 ? 64 : 128;
   long long floats = 0, most = 0;
   int most_ld = 0;
+  bool chains = false;
+  turn.by_tap = p.by_tap;
+  p.sh = sh;
+  p.sw = sw;
   for (int z = 0; z < phases; z++) {
     ConvNhwcPhase& f = p.phase[z];
     f.box = cn_box(CV_TILE, f.pw, f.ph, p.images);
     const int units = cv_units(sc, f.taps, CV_BK);
     f.k_blocks = units;
+    if (p.by_tap) f.chain = units / std::max(1, f.taps);
+    f.chain = std::max(1, f.chain);
+    chains = chains || f.chain < units || units == 0;
     turn.taps[z] = f.taps;
     turn.ld[z] = units * CV_BK;
     turn.start[z] = floats;
@@ -1207,12 +1201,27 @@ static int32_t run_conv_nhwc(om_ctx* ctx, ConvNhwcParams& p, ConvTurn& turn, int
     const dim3 grid((unsigned)most, (unsigned)ceil_div(p.m, nt), (unsigned)phases);
     // Twice the stages where the grid gives an SM one CTA at most.
     const bool alone = (int64_t)grid.x * grid.y * grid.z <= 148;
-    if (nt == 64) st = alone ? launch_nhwc<64, 8>(ctx, maps, p, grid) : launch_nhwc<64, 4>(ctx, maps, p, grid);
-    else st = alone ? launch_nhwc<128, 6>(ctx, maps, p, grid) : launch_nhwc<128, 3>(ctx, maps, p, grid);
+    if (chains && nt == 64) st = alone ? launch_nhwc<64, 8, true>(ctx, maps, p, grid) : launch_nhwc<64, 4, true>(ctx, maps, p, grid);
+    else if (chains) st = alone ? launch_nhwc<128, 6, true>(ctx, maps, p, grid) : launch_nhwc<128, 3, true>(ctx, maps, p, grid);
+    else if (nt == 64) st = alone ? launch_nhwc<64, 8, false>(ctx, maps, p, grid) : launch_nhwc<64, 4, false>(ctx, maps, p, grid);
+    else st = alone ? launch_nhwc<128, 6, false>(ctx, maps, p, grid) : launch_nhwc<128, 3, false>(ctx, maps, p, grid);
   }
   if (own) pool_free(ctx, own);
   if (wt) pool_free(ctx, wt);
   return st;
+}
+
+// The taps that reach the input positions (oy0, ox0) modulo the stride, and where in the gradient from a pixel of that class.
+static int class_taps(const ConvGeom& g, int oy0, int ox0, int* dy, int* dx, int* tap) {
+  int n = 0;
+  for (int t = 0; t < g.kh * g.kw; t++) {
+    const int ty = oy0 + g.pt - (t / g.kw) * g.dh, tx = ox0 + g.pl - (t % g.kw) * g.dw;
+    if (ty % g.sh || tx % g.sw) continue;      // (exact for negative values too)
+    dy[n] = ty / g.sh;
+    dx[n] = tx / g.sw;
+    tap[n++] = t;
+  }
+  return n;
 }
 
 static bool cn_grid_fits(int w, int h, int n) {
@@ -1220,7 +1229,7 @@ static bool cn_grid_fits(int w, int h, int n) {
   return 3 * (long long)w * h * n >= 2 * (long long)b.tw * b.th * b.tn * CV_TILE;
 }
 bool conv_nhwc_fwd_fits(const ConvGeom& g) {
-  return encode_fn() && cv_sizes_fit(g) && cn_worth(g) && cn_channels_fit(g.cin) && cn_grid_fits(g.ow, g.oh, g.n);
+  return cn_sizes_fit(g) && cn_channels_fit(g.cin) && cn_grid_fits(g.ow, g.oh, g.n) && cn_flops(g) >= CN_MIN_FLOPS;
 }
 
 int32_t conv_nhwc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y) {
@@ -1231,6 +1240,7 @@ int32_t conv_nhwc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const floa
   p.step_y = g.sh; p.step_x = g.sw; p.base_y = -g.pt; p.base_x = -g.pl; p.ostep_y = p.ostep_x = 1;
   ConvNhwcPhase& f = p.phase[0];
   f.ph = g.oh; f.pw = g.ow; f.taps = g.kh * g.kw;
+  f.chain = cv_units(g.cin, f.taps, CV_BK);
   for (int t = 0; t < f.taps; t++) {
     f.dy[t] = (t / g.kw) * g.dh;
     f.dx[t] = (t % g.kw) * g.dw;
@@ -1241,8 +1251,14 @@ int32_t conv_nhwc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const floa
   return run_conv_nhwc(ctx, p, turn, 1, f.taps, x, nullptr, g.cin, g.h, g.w, w);
 }
 
+// (what a box holds outside the grid counts against the size of the unfolded matrix: three times the time, at a quarter of the pixels)
 bool conv_nhwc_dgrad_fits(const ConvGeom& g) {
-  return encode_fn() && cv_sizes_fit(g) && cn_worth(g) && cn_channels_fit(g.cout) && cn_grid_fits((int)ceil_div(g.w, g.sw), (int)ceil_div(g.h, g.sh), g.n);
+  if (!cn_sizes_fit(g)) return false;
+  if (g.kh * g.kw == 1) return true;
+  const int cw = (int)ceil_div(g.w, g.sw), ch = (int)ceil_div(g.h, g.sh);
+  const ConvBox b = cn_box(CV_TILE, cw, ch, g.n);
+  const double unfolded = (double)g.n * g.oh * g.ow * g.sh * g.sw * g.cin * g.kh * g.kw, filled = (double)cw * ch * g.n / ((double)b.tw * b.th * b.tn * CV_TILE);
+  return unfolded * filled >= (double)std::max(CN_MIN_UNFOLDED, CN_MIN_UNFOLDED_A_BLOCK * cv_units(g.cout, g.kh * g.kw, CV_BK));
 }
 
 int32_t conv_nhwc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx, const float* gt) {
@@ -1250,7 +1266,7 @@ int32_t conv_nhwc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const f
   ConvTurn turn = {};
   p.out = dx; p.status = ctx->status_dev;
   p.images = g.n; p.m = g.cin; p.out_w = g.w; p.out_plane = g.h * g.w;
-  p.step_y = p.step_x = 1; p.ostep_y = g.sh; p.ostep_x = g.sw;
+  p.step_y = p.step_x = 1; p.by_tap = 1; p.ostep_y = g.sh; p.ostep_x = g.sw;
   for (int z = 0; z < g.sh * g.sw; z++) {
     ConvNhwcPhase& f = p.phase[z];
     f.oy0 = z / g.sw;
@@ -1267,7 +1283,7 @@ int32_t conv_nhwc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const f
 // The pixel boxes have to tile the output exactly: a slot outside it would multiply its zero gradient with values of the input, which may
 // be infinite.
 bool conv_nhwc_wgrad_fits(const ConvGeom& g) {
-  if (!encode_fn() || !cv_sizes_fit(g) || !cn_worth(g) || !cn_channels_fit(g.cin)) return false;
+  if (!cn_sizes_fit(g) || !cn_channels_fit(g.cin) || cn_flops(g) < CN_MIN_FLOPS) return false;
   const ConvBox b = cn_box(CV_BK, g.ow, g.oh, g.n);
   return g.ow % b.w == 0 && g.oh % b.h == 0 && g.n % b.n == 0;
 }

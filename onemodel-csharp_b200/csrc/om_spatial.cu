@@ -624,11 +624,21 @@ static bool conv_on_tensor_pipe(om_ctx* ctx, const ConvGeom& g, bool need_w_kmaj
   return (double)g.cout * kk * (double)np >= 32.0 * 32 * 32;
 }
 
+// Weights that TMA can read: themselves, or a copy (*own) where a view starts off the 16-byte grid.
+static int32_t on_grid(om_ctx* ctx, const float** w, size_t floats, float** own) {
+  if ((reinterpret_cast<uintptr_t>(*w) & 15) == 0) return OM_OK;
+  OM_TRY(pool_alloc(ctx, sizeof(float) * floats, false, (void**)own));
+  const cudaError_t e = cudaMemcpyAsync(*own, *w, sizeof(float) * floats, cudaMemcpyDeviceToDevice, ctx->stream);
+  if (e != cudaSuccess) return check_cuda(ctx, e, "a copy of a convolution's weights");
+  *w = *own;
+  return OM_OK;
+}
+
 static int32_t to_cnhw(om_ctx* ctx, const ConvGeom& g, const float* gr, float** out) {
   const int plane = g.oh * g.ow;
   int64_t total = (int64_t)g.n * g.cout * plane;
   OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)total, false, (void**)out));
-  if ((plane & 3) == 0) nchw_to_cnhw_kernel<4><<<grid_for(ctx, total / 4, 256), 256, 0, ctx->stream>>>(gr, *out, g.n, g.cout, plane, total);
+  if ((plane & 3) == 0 && (reinterpret_cast<uintptr_t>(gr) & 15) == 0) nchw_to_cnhw_kernel<4><<<grid_for(ctx, total / 4, 256), 256, 0, ctx->stream>>>(gr, *out, g.n, g.cout, plane, total);
   else nchw_to_cnhw_kernel<1><<<grid_for(ctx, total, 256), 256, 0, ctx->stream>>>(gr, *out, g.n, g.cout, plane, total);
   return OM_OK;
 }
@@ -656,10 +666,13 @@ int32_t om_conv2d_fwd(om_ctx* ctx, const om_conv_shape* s, const float* x, const
     float *cols = nullptr, *yt = nullptr;
     OM_TRY(unfold(ctx, g, x, &cols, true));
     int32_t st = pool_alloc(ctx, sizeof(float) * (size_t)g.cout * np, false, (void**)&yt);
+    float* own = nullptr;
+    if (st == OM_OK) st = on_grid(ctx, &w, (size_t)g.cout * kk, &own);
     if (st == OM_OK) st = gemm_tc(ctx, 0, 0, g.cout, np, kk, w, kk, cols, np, yt, np, 0, nullptr);
+    if (own) pool_free(ctx, own);
     if (st == OM_OK) {
       int64_t total = (int64_t)g.cout * np;
-      if ((plane & 3) == 0) cnhw_to_nchw_bias_kernel<4><<<grid_for(ctx, total / 4, 256), 256, 0, ctx->stream>>>(yt, bias, y, g.n, g.cout, plane, total);
+      if ((plane & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0) cnhw_to_nchw_bias_kernel<4><<<grid_for(ctx, total / 4, 256), 256, 0, ctx->stream>>>(yt, bias, y, g.n, g.cout, plane, total);
       else cnhw_to_nchw_bias_kernel<1><<<grid_for(ctx, total, 256), 256, 0, ctx->stream>>>(yt, bias, y, g.n, g.cout, plane, total);
     }
     pool_free(ctx, cols);
@@ -696,7 +709,6 @@ int32_t om_conv2d_dgrad(om_ctx* ctx, const om_conv_shape* s, const float* gr, co
   ProfileScope prof(ctx, "om_conv2d_dgrad", 2.0 * g.n * g.cout * (double)kk * plane, 4.0 * ((double)g.n * g.cin * g.h * g.w + (double)g.n * g.cout * plane));
   const bool tensor_pipe = conv_on_tensor_pipe(ctx, g, true);
   if (tensor_pipe && conv_nhwc_dgrad_fits(g)) return conv_nhwc_dgrad(ctx, g, gr, w, dx);
-  if (tensor_pipe && conv_tc_dgrad_fits(g)) return conv_tc_dgrad(ctx, g, gr, w, dx);
   if (!tensor_pipe && conv_fma_dgrad_fits(g)) return conv_fma_dgrad(ctx, g, gr, w, dx);
   float* dcols = nullptr;
   int64_t total_cols = (int64_t)g.n * g.groups * kk * plane;
@@ -706,7 +718,10 @@ int32_t om_conv2d_dgrad(om_ctx* ctx, const om_conv_shape* s, const float* gr, co
     float* gt = nullptr;
     int32_t st = to_cnhw(ctx, g, gr, &gt);
     // dcols [K, N*P] = W^T [K, Cout] * g_t [Cout, N*P]
+    float* own = nullptr;
+    if (st == OM_OK) st = on_grid(ctx, &w, (size_t)g.cout * kk, &own);
     if (st == OM_OK) st = gemm_tc(ctx, 1, 0, kk, np, g.cout, w, kk, gt, np, dcols, np, 0, nullptr);
+    if (own) pool_free(ctx, own);
     if (st == OM_OK) {
       launch_col2im(ctx, g, dcols, dx, np, plane);
     }

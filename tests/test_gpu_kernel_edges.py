@@ -260,6 +260,58 @@ def test_conv2d_from_channels_last_copies(ctx, case):
         assert scaled_diff(got, want) <= 2e-5
 
 
+@pytest.mark.parametrize("case", [
+    (33, 64, 16, 16, 96, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1), (64, 64, 16, 16, 256, 3, 3, 2, 2, (1, 1, 1, 1), 1, 1),
+    (40, 72, 17, 15, 160, 3, 3, 2, 2, (1, 1, 1, 1), 1, 1), (256, 64, 32, 32, 128, 1, 1, 2, 2, (0, 0, 0, 0), 1, 1),
+    (24, 32, 20, 44, 32, 5, 5, 1, 1, (4, 4, 4, 4), 2, 2), (160, 64, 32, 4, 128, 3, 2, 1, 2, (2, 0, 1, 1), 1, 1), (37, 48, 11, 12, 96, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1)])
+def test_conv2d_input_gradient_has_the_bits_of_product_and_fold(ctx, case):
+    """The TF32 product W^T g on its own (k = output channels) and its fold, one tap after the other in float32: the same bits, so the sums are no
+    less exact than those, whatever the kernel. An infinite and a NaN weight reach exactly the values whose taps lie inside the gradient's plane."""
+    s, x, wt, b, g, y, dx, dw = conv_case(*case)
+    n, cin, h, w, cout, kh, kw, sh, sw, (pt, pl, pb, pr), dh, dw_ = case
+    oh, ow = g.shape[2:]
+    kk, pixels = cin * kh * kw, n * oh * ow
+    assert cout < 512 and pixels % 4 == 0 and kk % 4 == 0      # (the product does not split k)
+    wt[3, 5, 0, 0], wt[1, cin - 1, kh - 1, kw - 1] = np.inf, np.nan
+    G, W, DX, D = ctx.to_device(g), ctx.to_device(wt), ctx.empty(x.shape), ctx.empty((kk, pixels))
+    GT = ctx.to_device(np.ascontiguousarray(g.transpose(1, 0, 2, 3).reshape(cout, pixels)))
+    ctx.set_flags(omb.OM_TF32)
+    try:
+        ctx.call("om_conv2d_dgrad", ctx.handle, C.byref(s), G.ptr, W.ptr, DX.ptr)
+        ctx.call("om_matmul", ctx.handle, i32(1), i32(0), i32(kk), i32(pixels), i32(cout), W.ptr, i32(kk), GT.ptr, i32(pixels), D.ptr, i32(pixels), i32(0))
+        cols, got = D.numpy().reshape(cin, kh, kw, n, oh, ow).transpose(3, 0, 1, 2, 4, 5), DX.numpy()
+    finally:
+        ctx.set_flags(0)
+    want = np.zeros((n, cin, h + pt + pb + dh * kh, w + pl + pr + dw_ * kw), np.float32)
+    for ky in range(kh):
+        for kx in range(kw):
+            want[:, :, ky * dh:ky * dh + oh * sh:sh, kx * dw_:kx * dw_ + ow * sw:sw] += cols[:, :, ky, kx]
+    want = want[:, :, pt:pt + h, pl:pl + w]
+    assert np.array_equal(got, want, equal_nan=True)
+    assert np.isfinite(want[:, 5]).any() and not np.isfinite(want[:, 5]).all() and np.isnan(want[:, cin - 1]).any()
+
+
+@pytest.mark.parametrize("tf32", [0, 1])
+@pytest.mark.parametrize("case", [(4, 8, 8, 8, 12, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1), (4, 4, 14, 14, 9, 3, 3, 3, 3, (1, 1, 1, 1), 1, 1), (4, 4, 12, 12, 9, 6, 6, 1, 1, (2, 2, 2, 2), 1, 1),
+                                  (33, 64, 16, 16, 96, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1), (8, 64, 8, 8, 64, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1)])
+def test_conv2d_of_arrays_off_the_16_byte_grid(ctx, case, tf32):
+    """Every array one float past a 16-byte boundary, as a slice of a larger tensor may be: the values of the aligned call (2e-5, another order of sums)."""
+    s, x, wt, b, g, y, dx, dw = conv_case(*case)
+    ctx.set_flags(omb.OM_TF32 if tf32 else 0)
+    off = lambda a: C.c_void_p(a.ptr.value + 4)  # noqa: E731
+    try:
+        X, W, B, G = (ctx.to_device(np.concatenate([np.zeros(1, np.float32), a.ravel()])) for a in (x, wt, b, g))
+        Y, DX, DW = (ctx.empty((a.size + 1,)) for a in (g, x, wt))
+        ctx.call("om_conv2d_fwd", ctx.handle, C.byref(s), off(X), off(W), off(B), off(Y))
+        ctx.call("om_conv2d_dgrad", ctx.handle, C.byref(s), off(G), off(W), off(DX))
+        ctx.call("om_conv2d_wgrad", ctx.handle, C.byref(s), off(G), off(X), off(DW), i32(0))
+        ctx.sync()
+        for got, want in ((Y, y), (DX, dx), (DW, dw)):
+            assert scaled_diff(got.numpy()[1:].reshape(want.shape), want) <= 2e-5
+    finally:
+        ctx.set_flags(0)
+
+
 @pytest.mark.parametrize("n,cout,h,w", [(1, 3, 2, 2), (5, 7, 4, 16), (17, 2, 33, 31), (3, 4, 1, 3), (40, 5, 40, 64)])
 def test_conv2d_bias_gradient_planes(ctx, n, cout, h, w):
     """Planes smaller and larger than a CTA's stride, of a multiple of four floats or not: sums in double, 1e-6."""
