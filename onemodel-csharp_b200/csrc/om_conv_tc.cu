@@ -825,18 +825,22 @@ struct ConvNhwcWgradParams {
   int cout, units, cin, kw, taps, sh, sw, pt, pl, dh, dw;
   ConvBox box;                 // 32 pixels, tiling the output exactly
   int blocks, blocks_per_split;
+  int chain;                   // pixel boxes an accumulator adds up
 };
-// One CTA: 128 output channels x four units of 32 channels of a tap, over a slice of the pixel boxes.
-__global__ void __launch_bounds__(CN_THREADS, 2)
+// One CTA: 128 output channels x four units of 32 channels of a tap, over a slice of the pixel boxes. CHAINS: a slice in several accumulator
+// chains, as in conv_nhwc_kernel, where the product on the unfolded matrix has shorter slices.
+template <bool CHAINS>
+__global__ void __launch_bounds__(cn_threads(CHAINS), 2)
 conv_nhwc_wgrad_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ ConvNhwcWgradParams p) {
-  constexpr int STAGES = 3;
+  constexpr int STAGES = 3, ACCS = CHAINS ? 2 : 1;
   constexpr int STAGE_BYTES = 2 * CV_BLOCK, CHUNK = CV_BK * 128;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
   uint64_t* empty = full + STAGES;
   uint64_t* acc_full = empty + STAGES;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+  uint64_t* acc_empty = acc_full + ACCS;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + ACCS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -849,12 +853,15 @@ conv_nhwc_wgrad_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_c
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(acc_full, 1);
+    for (int a = 0; a < ACCS; a++) {
+      mbar_init(&acc_full[a], 1);
+      mbar_init(&acc_empty[a], 8);
+    }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, CV_TILE);
+    tmem_alloc(tmem_slot, ACCS * CV_TILE);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -896,42 +903,68 @@ conv_nhwc_wgrad_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_c
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(CV_TILE >> 3) << 17) | ((uint32_t)(CV_TILE >> 4) << 24);
+      int c = 0, at = 0;           // the chain, and the box of it
       for (int kb = 0; kb < k_blocks; kb++) {
         const int s = kb % STAGES;
+        if (CHAINS && at == 0 && c >= ACCS && !mbar_wait(&acc_empty[c & 1], (uint32_t)((c >> 1) - 1) & 1, abort_flag, p.status, 88)) break;
         if (!mbar_wait(&full[s], (kb / STAGES) & 1, abort_flag, p.status, 85)) break;
         tc_fence_after();
         const uint32_t a = smem_u32(smem + (size_t)s * STAGE_BYTES), b = a + CV_BLOCK;
 #pragma unroll
         for (int ks = 0; ks < CV_BK / 8; ks++)
-          umma_tf32(tmem_base, make_desc(a + ks * 1024, CHUNK, 512, 1), make_desc(b + ks * 1024, CHUNK, 512, 1), idesc, (kb > 0 || ks > 0) ? 1u : 0u);
+          umma_tf32(tmem_base + (CHAINS ? (c & 1) * CV_TILE : 0), make_desc(a + ks * 1024, CHUNK, 512, 1), make_desc(b + ks * 1024, CHUNK, 512, 1), idesc,
+                    ((CHAINS ? at : kb) > 0 || ks > 0) ? 1u : 0u);
         umma_commit(&empty[s]);
+        if (CHAINS && (++at == p.chain || kb == k_blocks - 1)) {
+          umma_commit(&acc_full[c & 1]);
+          at = 0;
+          c++;
+        }
       }
-      umma_commit(acc_full);
+      if (!CHAINS) umma_commit(acc_full);
     }
   } else {
     const int quad = warp & 3;
-    const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, p.status, 86));
-    tc_fence_after();
-    // Accumulator rows through the dead operand stages, then whole rows of 128 columns.
-    float* stg = reinterpret_cast<float*>(smem) + quad * 32 * CV_STG_LD;
-    if (ok) {
-#pragma unroll 1
-      for (int c = 0; c < 4; c++) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 32), r);
-        tmem_ld_wait();
+    const uint32_t rows = tmem_base + ((uint32_t)(quad * 32) << 16);
+    // Accumulator rows through shared memory, then rows of whole 128-byte lines (COLS columns a warp). The last chain is complete only after every product,
+    // and nothing more is loaded: the operand stages are dead.
+    constexpr int COLS = CHAINS ? CV_TILE / 2 : CV_TILE, LD = COLS + 4;
+    float* stg = reinterpret_cast<float*>(smem) + (warp - 2) * 32 * LD;
+    const int col0 = (warp - 2) / 4 * COLS;
+    bool ok;
+    if constexpr (CHAINS) {
+      float acc[COLS];
+      ok = cn_add_chains<COLS>(acc, rows + (uint32_t)col0, CV_TILE, (k_blocks + p.chain - 1) / p.chain, acc_full, acc_empty, abort_flag, p.status, 86,
+                               [](int) { return true; });
+      if (ok) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(stg + lane * CV_STG_LD + c * 32 + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+        for (int j = 0; j < COLS; j += 4) *reinterpret_cast<float4*>(stg + lane * LD + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
       }
+    } else {
+      ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, p.status, 86));
+      tc_fence_after();
+      if (ok) {
+#pragma unroll 1
+        for (int c = 0; c < 4; c++) {
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(rows + (uint32_t)(c * 32), r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(stg + lane * LD + c * 32 + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+        }
+      }
+    }
+    if (ok) {
       __syncwarp();
-      const int ld = p.units * CV_BK, col = u0 * CV_BK + 4 * lane;
+      constexpr int LANES = COLS / 4;                  // of a row
+      const int ld = p.units * CV_BK, col = u0 * CV_BK + col0 + 4 * (lane % LANES);
       float* out = p.part + (long long)blockIdx.z * p.cout * ld + col;
       if (col < ld) {
 #pragma unroll 4
-        for (int i = 0; i < 32; i++) {
+        for (int i = lane / LANES; i < 32; i += 32 / LANES) {
           const int co = m0 + quad * 32 + i;
           if (co >= p.cout) break;
-          *reinterpret_cast<float4*>(out + (long long)co * ld) = *reinterpret_cast<const float4*>(stg + i * CV_STG_LD + 4 * lane);
+          *reinterpret_cast<float4*>(out + (long long)co * ld) = *reinterpret_cast<const float4*>(stg + i * LD + 4 * (lane % LANES));
         }
       }
     }
@@ -940,7 +973,7 @@ conv_nhwc_wgrad_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_c
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, CV_TILE);
+    tmem_dealloc(tmem_base, ACCS * CV_TILE);
   }
 }
 
@@ -983,7 +1016,11 @@ static int32_t launch_conv_as(om_ctx* ctx, const CUtensorMap& map, const ConvTcP
   return OM_OK;
 }
 
-bool conv_tc_fwd_fits(const ConvGeom& g) { return encode_fn() && cv_sizes_fit(g); }
+// Where the product on the unfolded matrix would add up k in several slices, one accumulator for all of it would lose bits.
+bool conv_tc_fwd_fits(const ConvGeom& g) {
+  const int kk = g.cin * g.kh * g.kw;
+  return encode_fn() && cv_sizes_fit(g) && product_chain_blocks(g.cout, g.n * g.oh * g.ow, kk) >= (int)ceil_div(kk, CV_BK);
+}
 
 int32_t conv_tc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y) {
   ConvTcParams p = {};
@@ -1055,12 +1092,13 @@ int32_t conv_tc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const flo
   CUtensorMap map = {};
   if (a_tma && !cv_map(&map, gr, p.plane, g.cout, p.plane, g.n, (long long)g.cout * p.plane))
     return fail(ctx, OM_ERR_CUDA, "cuTensorMapEncodeTiled failed for a convolution's gradient");
-  // Slices of the pixels for one round of two CTAs an SM, each at least eight stages long: a function of the shape alone.
+  // Slices of the pixels for one round of two CTAs an SM, each at least eight stages long, and none longer than those of the product on the
+  // unfolded matrix (what one accumulator adds up loses bits with its length): a function of the shape alone.
   const int ld = p.units * CV_UNIT;
   const int tn = (int)ceil_div(ld, CV_TILE), tm = (int)ceil_div(g.cout, CV_TILE);
   const long long blocks = ceil_div(p.pixels, CV_BK);
   int splits = (int)std::max<long long>(1, std::min<long long>(kSplitSlots / ((long long)tn * tm), blocks / 8));
-  p.blocks_per_split = (int)ceil_div(blocks, splits);
+  p.blocks_per_split = std::min((int)ceil_div(blocks, splits), product_chain_blocks(g.cout, g.cin * p.taps, p.pixels));
   splits = (int)ceil_div(blocks, p.blocks_per_split);
   OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)splits * g.cout * ld, false, (void**)&p.part));
   const dim3 grid((unsigned)tn, (unsigned)tm, (unsigned)splits);
@@ -1241,6 +1279,8 @@ int32_t conv_nhwc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const floa
   ConvNhwcPhase& f = p.phase[0];
   f.ph = g.oh; f.pw = g.ow; f.taps = g.kh * g.kw;
   f.chain = cv_units(g.cin, f.taps, CV_BK);
+  const int plain = product_chain_blocks(g.cout, g.n * g.oh * g.ow, g.cin * f.taps);
+  if (plain < (int)ceil_div(g.cin * f.taps, CV_BK)) f.chain = plain;     // (a chain no longer than the product on the unfolded matrix has)
   for (int t = 0; t < f.taps; t++) {
     f.dy[t] = (t / g.kw) * g.dh;
     f.dx[t] = (t % g.kw) * g.dw;
@@ -1288,6 +1328,19 @@ bool conv_nhwc_wgrad_fits(const ConvGeom& g) {
   return g.ow % b.w == 0 && g.oh % b.h == 0 && g.n % b.n == 0;
 }
 
+template <bool CHAINS>
+static int32_t launch_nhwc_wgrad(om_ctx* ctx, const CUtensorMap& map_g, const CUtensorMap& map_x, const ConvNhwcWgradParams& p, dim3 grid) {
+  constexpr size_t smem = (size_t)3 * 2 * CV_BLOCK + 1024 + 128;
+  static_assert(3 * 2 * CV_BLOCK >= (cn_threads(CHAINS) - 64) * (CV_TILE / (CHAINS ? 2 : 1) + 4) * 4, "the result rows are staged in the operand stages");
+  static bool set = false;
+  if (!set) {
+    OM_CUDA(ctx, cudaFuncSetAttribute(conv_nhwc_wgrad_kernel<CHAINS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    set = true;
+  }
+  launch_chained(ctx, conv_nhwc_wgrad_kernel<CHAINS>, grid, cn_threads(CHAINS), smem, map_g, map_x, p);
+  return OM_OK;
+}
+
 int32_t conv_nhwc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, float* dw, int accumulate, const float* turned) {
   ConvNhwcWgradParams p = {};
   p.status = ctx->status_dev;
@@ -1301,6 +1354,7 @@ int32_t conv_nhwc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const f
   int splits = (int)std::max<long long>(1, std::min<long long>(kSplitSlots / ((long long)tn * tm), p.blocks / 8));
   p.blocks_per_split = (int)ceil_div(p.blocks, splits);
   splits = (int)ceil_div(p.blocks, p.blocks_per_split);
+  p.chain = std::min(p.blocks_per_split, product_chain_blocks(g.cout, g.cin * p.taps, g.n * g.oh * g.ow));
   float *own = nullptr, *xt = nullptr;
   CUtensorMap map_g = {}, map_x = {};
   int32_t st = turned ? OM_OK : cn_turn(ctx, gr, g.n, g.cout, g.oh * g.ow, &own);
@@ -1310,14 +1364,9 @@ int32_t conv_nhwc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const f
   if (st == OM_OK && (!cn_map(&map_g, gt, g.cout, g.ow, g.oh, g.n, p.box, 1, 1, true) || !cn_map(&map_x, xt, g.cin, g.w, g.h, g.n, p.box, g.sw, g.sh, true)))
     st = fail(ctx, OM_ERR_CUDA, "cuTensorMapEncodeTiled failed for a convolution's operands");
   if (st == OM_OK) {
-    constexpr size_t smem = (size_t)3 * 2 * CV_BLOCK + 1024 + 128;
-    static bool set = false;
-    if (!set) {
-      st = check_cuda(ctx, cudaFuncSetAttribute(conv_nhwc_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "conv_nhwc_wgrad");
-      set = st == OM_OK;
-    }
+    const dim3 grid((unsigned)tn, (unsigned)tm, (unsigned)splits);
+    st = p.chain < p.blocks_per_split ? launch_nhwc_wgrad<true>(ctx, map_g, map_x, p, grid) : launch_nhwc_wgrad<false>(ctx, map_g, map_x, p, grid);
     if (st == OM_OK) {
-      launch_chained(ctx, conv_nhwc_wgrad_kernel, dim3((unsigned)tn, (unsigned)tm, (unsigned)splits), CN_THREADS, smem, map_g, map_x, p);
       launch_finish<CV_BK, 1>(ctx, p.part, splits, g, p.units, dw, accumulate);
       st = check_cuda(ctx, cudaGetLastError(), "conv_nhwc_wgrad");
     }

@@ -382,6 +382,8 @@ int32_t gemm_tc_batched(om_ctx* ctx, int ta, int tb, int m, int n, int k, const 
 }
 
 bool gemm_pair_supported(om_ctx* ctx, int m, int n, int k);
+bool gemm_pair_shape(int m, int n, int k);
+PairPlan pair_plan(int m, int n, int k);
 bool gemm_ws_supported(om_ctx* ctx, int elem, int m, int n, int k, const void* A, long long lda, const void* B, long long ldb, const float* C,
                        long long ldc);
 int32_t gemm_ws(om_ctx* ctx, int elem, int ta, int tb, int m, int n, int k, const void* A, long long lda, const void* B, long long ldb, float* C,
@@ -403,6 +405,21 @@ static bool persistent_tiles(int m, int n, int k) {
   return m >= 2048 && n >= 512 && 10 * (int64_t)n >= 9 * ceil_div(n, 256) * 256 && (tiles >= 128 || (tiles >= 64 && k >= 1024));
 }
 
+// Blocks of k a CTA adds up in its accumulator. Fixed slices of k for one full round of CTAs, each at least 8 k-blocks deep: a function of
+// the shape only, so results do not depend on the device or on timing.
+static int blocks_per_split(int m, int n, int k) {
+  const int tiles = (int)(ceil_div(m, BM) * ceil_div(n, BN)), k_blocks = (int)ceil_div(k, BK);
+  if (tiles >= 148 || k_blocks < 16) return k_blocks;
+  // As many slices as still run in one round of two CTAs per SM on a 148-SM device (a constant, not the device's count).
+  return (int)ceil_div(k_blocks, std::min(32, std::max(1, std::min(kSplitSlots / tiles, k_blocks / 8))));
+}
+
+// The same of the kernel that om_matmul gives a product of this shape, without a scheduling flag.
+int product_chain_blocks(int m, int n, int k) {
+  if (persistent_tiles(m, n, k)) return (int)ceil_div(k, BK);
+  return gemm_pair_shape(m, n, k) ? pair_plan(m, n, k).kb_per_split : blocks_per_split(m, n, k);
+}
+
 int32_t gemm_tc_heads(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, long long sA, long long iA,
                       const float* B, int ldb, long long sB, long long iB, float* C, int ldc, long long sC, long long iC, int batch,
                       int inner, int acc, const float* bias) {
@@ -418,19 +435,8 @@ int32_t gemm_tc_heads(om_ctx* ctx, int ta, int tb, int m, int n, int k, const fl
   ok = ok && (b_mn ? make_map(&map_b, B, n, k, ldb, BK, true, outer, sB, inner, iB) : make_map(&map_b, B, k, n, ldb, BN, false, outer, sB, inner, iB));
   if (!ok) return fail(ctx, OM_ERR_CUDA, "cuTensorMapEncodeTiled failed (m %d n %d k %d lda %d ldb %d)", m, n, k, lda, ldb);
 
-  const int tiles = (int)(ceil_div(m, BM) * ceil_div(n, BN));
-  const int k_blocks = (int)ceil_div(k, BK);
-  // Fixed split of k: slices for one full round of CTAs, each slice at least 8 k-blocks deep. The split count is
-  // a function of the shape only, so results do not depend on the device or on timing.
-  int splits = 1;
-  if (batch == 1 && tiles < 148 && k_blocks >= 16) {
-    // As many slices as still run in one round of two CTAs per SM on a 148-SM device (a constant, not the device's count).
-    splits = (int)std::min<int64_t>(kSplitSlots / tiles, k_blocks / 8);
-    if (splits < 1) splits = 1;
-    if (splits > 32) splits = 32;
-  }
-  const int kb_per_split = (int)ceil_div(k_blocks, splits);
-  splits = (int)ceil_div(k_blocks, kb_per_split);
+  const int k_blocks = (int)ceil_div(k, BK), kb_per_split = batch == 1 ? blocks_per_split(m, n, k) : k_blocks;
+  const int splits = (int)ceil_div(k_blocks, kb_per_split);
 
   TcParams p;
   p.m = m; p.n = n; p.k = k;

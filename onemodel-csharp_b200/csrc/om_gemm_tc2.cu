@@ -308,9 +308,9 @@ static bool pair_map(CUtensorMap* map, const float* base, int inner, int outer, 
 // with several rounds of tiles over the device and no split of k (measured: 3 to 10 % faster on the widest products of a
 // 768-wide encoder, 1.44x at 4096^3, slower on products of one or two rounds, where the larger tile leaves SMs idle);
 // OM_PAIR_TILES sends every product it can take to it.
-bool gemm_pair_supported(om_ctx* ctx, int m, int n, int k) {
-  if (m < 256 || n < 128 || k < 64 || m > 65535 * 256) return false;
-  if (ctx->flags & OM_PAIR_TILES) return true;
+static bool pair_takes(int m, int n, int k) { return m >= 256 && n >= 128 && k >= 64 && m <= 65535 * 256; }
+bool gemm_pair_shape(int m, int n, int k) {
+  if (!pair_takes(m, n, k)) return false;
   const int64_t tiles = ceil_div(m, P_BM) * ceil_div(n, 128);
   if (tiles >= 4 * (int64_t)148 && m >= 1024 && n >= 256) return true;
   // One round of pairs over wide rows with a short k: 5120 x 1024 x 256 12.5 us against 15.2, 2048 x 2560 x 640 18.6 against 24.5.
@@ -319,6 +319,9 @@ bool gemm_pair_supported(om_ctx* ctx, int m, int n, int k) {
   // Deep-k products with few tiles (the weight gradients of a wide layer): measured 1.3-1.4x at 768-wide layers, about
   // even at 384.
   return tiles < 148 && k >= 128 * P_BK && m >= 512 && m % 256 == 0 && n >= 512 && n % 256 == 0;
+}
+bool gemm_pair_supported(om_ctx* ctx, int m, int n, int k) {
+  return (ctx->flags & OM_PAIR_TILES) ? pair_takes(m, n, k) : gemm_pair_shape(m, n, k);
 }
 
 template <int BN>
@@ -343,9 +346,7 @@ static int32_t launch_pair(om_ctx* ctx, bool a_mn, bool b_mn, const CUtensorMap&
   return OM_OK;
 }
 
-int32_t gemm_pair(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, const float* B, int ldb, float* C, int ldc,
-                  int acc, const float* bias) {
-  const bool a_mn = ta != 0, b_mn = tb == 0;
+PairPlan pair_plan(int m, int n, int k) {
   // Tile width 128, 192 or 256: the one with the shortest estimated time, counted as rounds of CTAs over the device (two
   // CTAs per SM) times the work of a CTA (its tile width plus a fixed part for prologue and epilogue). Wide tiles bring in
   // fewer operand bytes per output but leave small products with too few CTAs.
@@ -365,20 +366,23 @@ int32_t gemm_pair(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float*
     // divides the width (fewest operand bytes per output).
     if (2 * ceil_div(m, 2 * P_BM) * ceil_div(n, 128) < 148 && k >= 64 * P_BK) bn = n % 256 == 0 ? 256 : n % 192 == 0 ? 192 : 128;
   }
+  const int ctas = (int)(2 * ceil_div(m, 2 * P_BM) * ceil_div(n, bn)), k_blocks = (int)ceil_div(k, P_BK);
+  int splits = 1;
+  if (ctas < 148 && k_blocks >= 16) splits = std::min(32, std::max(1, std::min(kSplitSlots / ctas, k_blocks / 8)));
+  return {bn, (int)ceil_div(k_blocks, splits)};
+}
+
+int32_t gemm_pair(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, const float* B, int ldb, float* C, int ldc,
+                  int acc, const float* bias) {
+  const bool a_mn = ta != 0, b_mn = tb == 0;
+  const PairPlan plan = pair_plan(m, n, k);
+  const int bn = plan.bn, kb_per_split = plan.kb_per_split;
   CUtensorMap map_a, map_b;
   bool ok = a_mn ? pair_map(&map_a, A, m, k, lda, P_BK, true) : pair_map(&map_a, A, k, m, lda, P_BM, false);
   ok = ok && (b_mn ? pair_map(&map_b, B, n, k, ldb, P_BK, true) : pair_map(&map_b, B, k, n, ldb, bn / 2, false));
   if (!ok) return fail(ctx, OM_ERR_CUDA, "cuTensorMapEncodeTiled failed (pair kernel, m %d n %d k %d)", m, n, k);
   const int pairs = (int)ceil_div(m, 2 * P_BM), n_tiles = (int)ceil_div(n, bn);
-  const int ctas = 2 * pairs * n_tiles, k_blocks = (int)ceil_div(k, P_BK);
-  int splits = 1;
-  if (ctas < 148 && k_blocks >= 16) {
-    splits = (int)std::min<int64_t>(kSplitSlots / ctas, k_blocks / 8);
-    if (splits < 1) splits = 1;
-    if (splits > 32) splits = 32;
-  }
-  const int kb_per_split = (int)ceil_div(k_blocks, splits);
-  splits = (int)ceil_div(k_blocks, kb_per_split);
+  const int splits = (int)ceil_div(ceil_div(k, P_BK), kb_per_split);
   PairParams p;
   p.m = m; p.n = n; p.k = k; p.k_per_split = kb_per_split * P_BK; p.splits = splits; p.status = ctx->status_dev;
   float* workspace = nullptr;

@@ -8,6 +8,12 @@
 namespace om {
 
 constexpr int kSplitSlots = 296;   // CTAs of one round at two per SM on 148 SMs: the k-split target of the product kernels
+// How the CTA-pair kernel cuts a product: its tile width, and the blocks of 32 k's that one of its slices of k adds up.
+struct PairPlan {
+  int bn, kb_per_split;
+};
+// Blocks of 32 k's that the plain TF32 product of this shape adds up in one accumulator (om_gemm_tc.cu).
+int product_chain_blocks(int m, int n, int k);
 constexpr long long WAIT_CYCLES = 2000000000LL;   // about one second of SM clock: the bound of every mbarrier wait
 
 // ---- PTX wrappers -----------------------------------------------------------------------------------------------------

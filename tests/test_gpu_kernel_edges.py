@@ -291,6 +291,31 @@ def test_conv2d_input_gradient_has_the_bits_of_product_and_fold(ctx, case):
     assert np.isfinite(want[:, 5]).any() and not np.isfinite(want[:, 5]).all() and np.isnan(want[:, cin - 1]).any()
 
 
+@pytest.mark.parametrize("n,cin,h,w,cout", [(128, 128, 8, 8, 128), (64, 256, 8, 8, 512), (16, 64, 20, 32, 64), (61, 40, 20, 32, 40), (37, 48, 11, 12, 96), (7, 24, 30, 28, 200)])
+def test_conv2d_sums_are_no_less_exact_than_the_plain_products(ctx, n, cin, h, w, cout):
+    """Forward and weight gradient against float64, beside om_matmul on the unfolded input, which splits k (the tensor core's accumulator loses bits
+    with the length of a sum): values of one sign on one side, as behind a rectifier, and 5 % for the order of the sums."""
+    s, x, wt, b, g, y, dx, dw = conv_case(n, cin, h, w, cout, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1)
+    x = np.maximum(x, 0)
+    pad, kk, pixels = np.pad(x, ((0, 0), (0, 0), (1, 1), (1, 1))), cin * 9, n * h * w
+    cols = np.stack([pad[:, :, i:i + h, j:j + w] for i in range(3) for j in range(3)], 2).transpose(1, 2, 0, 3, 4).reshape(kk, pixels)
+    gt, wm = np.ascontiguousarray(g.transpose(1, 0, 2, 3).reshape(cout, pixels)), wt.reshape(cout, kk)
+    CO, GT, W, PY, PW = ctx.to_device(cols), ctx.to_device(gt), ctx.to_device(wm), ctx.empty((cout, pixels)), ctx.empty((cout, kk))
+    ctx.set_flags(omb.OM_TF32)
+    try:
+        Y, DX, DW, DW2 = run_conv(ctx, s, x, wt, np.zeros_like(b), g)
+        ctx.call("om_matmul", ctx.handle, i32(0), i32(0), i32(cout), i32(pixels), i32(kk), W.ptr, i32(kk), CO.ptr, i32(pixels), PY.ptr, i32(pixels), i32(0))
+        ctx.call("om_matmul", ctx.handle, i32(0), i32(1), i32(cout), i32(kk), i32(pixels), GT.ptr, i32(pixels), CO.ptr, i32(pixels), PW.ptr, i32(kk), i32(0))
+        py, pw = PY.numpy(), PW.numpy()
+    finally:
+        ctx.set_flags(0)
+    far = lambda got, want: np.linalg.norm(got.astype(np.float64) - want)  # noqa: E731
+    want = wm.astype(np.float64) @ cols.astype(np.float64)
+    assert far(Y.transpose(1, 0, 2, 3).reshape(cout, pixels), want) <= 1.05 * far(py, want)
+    want = gt.astype(np.float64) @ cols.T.astype(np.float64)
+    assert far(DW.reshape(cout, kk), want) <= 1.05 * far(pw, want)
+
+
 @pytest.mark.parametrize("tf32", [0, 1])
 @pytest.mark.parametrize("case", [(4, 8, 8, 8, 12, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1), (4, 4, 14, 14, 9, 3, 3, 3, 3, (1, 1, 1, 1), 1, 1), (4, 4, 12, 12, 9, 6, 6, 1, 1, (2, 2, 2, 2), 1, 1),
                                   (33, 64, 16, 16, 96, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1), (8, 64, 8, 8, 64, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1)])
