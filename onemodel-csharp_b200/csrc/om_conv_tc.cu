@@ -1065,7 +1065,14 @@ static void launch_finish(om_ctx* ctx, const float* part, int splits, const Conv
                                                                                                                        g.kh * g.kw, dw, accumulate);
 }
 
-bool conv_tc_wgrad_fits(const ConvGeom& g) { return encode_fn() && cv_sizes_fit(g); }
+// Planes of whole stages always. With others the warps gather both operands, and the few pixels of a small product are too long a chain of loads; us
+// unfolded / here: 37 x 64 x 11 x 12 by 64 (4884 pixels, 2.8 M floats unfolded) 26 / 34, 37 x 256 x 11 x 12 by 256 (4884, 11 M) 63 / 75, 32 x 256 x 14 x 14 by
+// 256 (6272, 14 M) 77 / 89, 37 x 16 x 22 x 28 by 32 (22792, 3.3 M) 32 / 38, 128 x 32 x 24 x 24 by 32 with stride 2 (18432, 5.3 M) 34 / 38; 37 x 32 x 22 x 28
+// by 32 (22792, 6.6 M) 40 / 38, 16 x 32 x 30 x 30 by 32 with 5 x 5 (14400, 11.5 M) 56 / 42.
+bool conv_tc_wgrad_fits(const ConvGeom& g) {
+  const long long pixels = (long long)g.n * g.oh * g.ow;
+  return encode_fn() && cv_sizes_fit(g) && ((g.oh * g.ow) % CV_BK == 0 || (pixels >= 12288 && pixels * g.cin * g.kh * g.kw >= 6500000));
+}
 
 template <bool A_TMA>
 static int32_t launch_wgrad(om_ctx* ctx, const CUtensorMap& map, const ConvWgradParams& p, dim3 grid) {
@@ -1166,8 +1173,11 @@ static bool cn_sizes_fit(const ConvGeom& g) {
   return encode_fn() && cv_sizes_fit(g) && g.sh <= 2 && g.sw <= 2 && (long long)g.n * g.h * g.w * cn_pitch(g.cin) < (1ll << 30) &&
          (long long)g.n * g.oh * g.ow * cn_pitch(g.cout) < (1ll << 30);
 }
-// The lines between the channels-last form and the others, 3 x 3 windows, us channels last / unfolded; a forward product or a weight
-// gradient needs CN_MIN_FLOPS, below which turning the source costs more than it gives:
+// The lines between the channels-last form and the others, 3 x 3 windows, us channels last / unfolded / gathered:
+//   forward         against the unfolded matrix by its size, np x k floats: 16 x 256 x 12 x 12 to 256 (5.3 M) 52 / 38, 8 x 512 x 8 x 8 to 512 (2.4 M)
+//                   83 / 32, 37 x 64 x 11 x 12 to 64 (2.8 M) 28 / 26; 37 x 128 x 11 x 12 to 128 (5.6 M) 39 / 38, 32 x 96 x 16 x 16 to 96 (7.1 M)
+//                   34 / 40, 37 x 256 x 11 x 12 to 256 (11 M) 54 / 63. Against the gathering kernel by its products: 64 x 40 x 20 x 32 to 40
+//                   (1.2 GFLOP) 38 / 65 / 34, 64 x 24 x 20 x 32 to 48 (0.8) 30 / 46 / 26, 37 x 64 x 22 x 28 to 64 (1.7) 26 / 52.
 //   input gradient  by the size of the unfolded matrix, the zeros between strides counted: 37 x 24 x 22 x 28 from 48 (4.9 M) 32 / 32, 16 x 256 x 12 x 12
 //                   from 256 (5.3 M) 50 / 36, 8 x 512 x 8 x 8 from 512 (2.4 M) 79 / 36; 37 x 128 x 11 x 12 from 128 (5.6 M) 36 / 40, 64 x 16 x 20 x 32
 //                   from 16 (5.9 M) 30 / 34, 37 x 132 x 11 x 12 from 36 (5.8 M) 30 / 36, 128 x 16 x 24 x 24 from 16 (10.6 M) 36 / 50, with stride 2 24 / 36.
@@ -1267,7 +1277,8 @@ static bool cn_grid_fits(int w, int h, int n) {
   return 3 * (long long)w * h * n >= 2 * (long long)b.tw * b.th * b.tn * CV_TILE;
 }
 bool conv_nhwc_fwd_fits(const ConvGeom& g) {
-  return cn_sizes_fit(g) && cn_channels_fit(g.cin) && cn_grid_fits(g.ow, g.oh, g.n) && cn_flops(g) >= CN_MIN_FLOPS;
+  return cn_sizes_fit(g) && cn_channels_fit(g.cin) && cn_grid_fits(g.ow, g.oh, g.n) && (long long)g.n * g.oh * g.ow * g.cin * g.kh * g.kw >= CN_MIN_UNFOLDED &&
+         (cn_flops(g) >= CN_MIN_FLOPS || !conv_tc_fwd_fits(g));
 }
 
 int32_t conv_nhwc_fwd(om_ctx* ctx, const ConvGeom& g, const float* x, const float* w, const float* bias, float* y) {
