@@ -400,9 +400,12 @@ void splitk_reduce_launch(om_ctx* ctx, const float* part, int splits, int64_t mn
 //   8192 x 1536 x 384: 28.4 / 24.1, 16384 x 768 x 768: 42.3 / 35.3, 16384 x 3072 x 768: 136 / 109, 16384 x 768 x 3072: 120 / 110 (CTA pairs),
 //   4096 x 2048 x 2048: 65.4 / 51.9, 8192 x 512 x 2048: 36.5 / 31.0 (this file); even at 8192 x 1152 x 384 and 8192 x 512 x 512; the
 //   other way at 5120 x 1024 x 256: 15.2 / 16.4, and with 384 columns: 30.0 / 35.8 at k = 1536.
-static bool persistent_tiles(int m, int n, int k) {
+// The lines of k: with 128 tiles and more, 4096 x 2048 at k = 64 15.4 / 17.4, 128 17.8 / 19.5, 256 20.6 / 21.5, 384 24.6 / 23.5, 16384 x 512 at 128 18.4 / 19.5, 256 22.5 /
+//   21.5, 12288 x 1024 at 64 20.6 / 23.6, 256 28.7 / 25.6; with 64, 2048 x 2048 at 1024 24.6 / 23.6, 1536 31.7 / 29.7, but with A stored [k, m] at 1024
+//   26.6 / 27.6, 2048 41.0 / 39.9.
+static bool persistent_tiles(bool a_mn, int m, int n, int k) {
   const int64_t tiles = ceil_div(m, 256) * ceil_div(n, 256);
-  return m >= 2048 && n >= 512 && 10 * (int64_t)n >= 9 * ceil_div(n, 256) * 256 && (tiles >= 128 || (tiles >= 64 && k >= 1024));
+  return m >= 2048 && n >= 512 && 10 * (int64_t)n >= 9 * ceil_div(n, 256) * 256 && ((tiles >= 128 && k >= 256) || (tiles >= 64 && k >= (a_mn ? 2048 : 1024)));
 }
 
 // Blocks of k a CTA adds up in its accumulator. Fixed slices of k for one full round of CTAs, each at least 8 k-blocks deep: a function of
@@ -416,14 +419,14 @@ static int blocks_per_split(int m, int n, int k) {
 
 // The same of the kernel that om_matmul gives a product of this shape, without a scheduling flag.
 int product_chain_blocks(int m, int n, int k) {
-  if (persistent_tiles(m, n, k)) return (int)ceil_div(k, BK);
+  if (persistent_tiles(false, m, n, k)) return (int)ceil_div(k, BK);
   return gemm_pair_shape(m, n, k) ? pair_plan(m, n, k).kb_per_split : blocks_per_split(m, n, k);
 }
 
 int32_t gemm_tc_heads(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, long long sA, long long iA,
                       const float* B, int ldb, long long sB, long long iB, float* C, int ldc, long long sC, long long iC, int batch,
                       int inner, int acc, const float* bias) {
-  if (batch == 1 && ((ctx->flags & OM_PERSISTENT_TILES) ? m >= 256 && n >= 64 : persistent_tiles(m, n, k)) && gemm_ws_supported(ctx, 0, m, n, k, A, lda, B, ldb, C, ldc))
+  if (batch == 1 && ((ctx->flags & OM_PERSISTENT_TILES) ? m >= 256 && n >= 64 : persistent_tiles(ta != 0, m, n, k)) && gemm_ws_supported(ctx, 0, m, n, k, A, lda, B, ldb, C, ldc))
     return gemm_ws(ctx, 0, ta, tb, m, n, k, A, lda, B, ldb, C, ldc, acc, bias, nullptr);
   if (batch == 1 && gemm_pair_supported(ctx, m, n, k)) return gemm_pair(ctx, ta, tb, m, n, k, A, lda, B, ldb, C, ldc, acc, bias);
   // op(A) is [m, k]. ta == 0: stored [m, k] (K-major tile, map inner = k). ta != 0: stored [k, m] (MN-major, inner = m).

@@ -313,9 +313,10 @@ bool gemm_pair_shape(int m, int n, int k) {
   if (!pair_takes(m, n, k)) return false;
   const int64_t tiles = ceil_div(m, P_BM) * ceil_div(n, 128);
   if (tiles >= 4 * (int64_t)148 && m >= 1024 && n >= 256) return true;
-  // One round of pairs over wide rows with a short k: 5120 x 1024 x 256 12.5 us against 15.2, 2048 x 2560 x 640 18.6 against 24.5.
-  const int64_t wide = ceil_div(m, 256) * ceil_div(n, 256);
-  if (wide >= 64 && wide < 128 && m >= 2048 && n >= 1024 && k < 1024) return true;
+  // One round of pairs over wide rows with a short k, where the tiles of 128 x 128 no longer make one round of two CTAs an SM; us there / here:
+  // 80 pairs, 5120 x 1024 at k = 128 16.5 / 14.4, 512 25.8 / 21.5, 896 36.9 / 27.6; 120 pairs, 7680 x 1024 at 128 17.5 / 16.5, 640 31.7 / 26.7; but 72 pairs,
+  // 3072 x 1536 at 128 12.3 / 13.3, 512 17.4 / 19.4, 896 23.4 / 24.6, and 64, 2048 x 2048 at 128 12.3 / 14.3, 640 19.5 / 20.5.
+  if (tiles > kSplitSlots && ceil_div(m, 256) * ceil_div(n, 256) < 128 && m >= 2048 && n >= 1024 && k < 1024) return true;
   // Deep-k products with few tiles (the weight gradients of a wide layer): measured 1.3-1.4x at 768-wide layers, about
   // even at 384.
   return tiles < 148 && k >= 128 * P_BK && m >= 512 && m % 256 == 0 && n >= 512 && n % 256 == 0;
