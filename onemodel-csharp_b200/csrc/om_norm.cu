@@ -641,6 +641,7 @@ __global__ void bn_eval_stats_kernel(const float* __restrict__ rm, const float* 
 }
 
 // Element-wise over the whole tensor, VEC consecutive elements of one plane per thread (VEC == 4: plane % 4 == 0).
+// (VEC == 4: and x and y, backward g, x and dx, on the 16-byte grid)
 template <int VEC, bool RELU>
 __global__ void __launch_bounds__(256)
 bn_apply_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
@@ -855,6 +856,8 @@ static int32_t batchnorm_fwd(om_ctx* ctx, const float* x, const float* gamma, co
   if (c == 0) return OM_OK;
   double total = (double)n * c * plane;
   ProfileScope prof(ctx, "om_batchnorm_fwd", 0, (training ? 16.0 : 8.0) * total);
+  // 16-byte accesses: planes of whole float4s, and every array that is accessed so on the 16-byte grid (a view may start off it).
+  const bool vec_x = (plane & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0, vec = vec_x && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
   if (training) {
     int slices = bn_slices(n, c, plane), ipc = (int)ceil_div(n, slices);
     double *pa = nullptr, *pb = nullptr;
@@ -862,7 +865,7 @@ static int32_t batchnorm_fwd(om_ctx* ctx, const float* x, const float* gamma, co
     OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)slices * c, false, (void**)&pb));
     double m = (double)n * plane;
     dim3 grid(c, slices);
-    if ((plane & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) launch_chained(ctx, bn_stats_kernel<4>, grid, kBnThreads, 0, x, n, c, plane, ipc, pa, pb);
+    if (vec_x) launch_chained(ctx, bn_stats_kernel<4>, grid, kBnThreads, 0, x, n, c, plane, ipc, pa, pb);
     else launch_chained(ctx, bn_stats_kernel<1>, grid, kBnThreads, 0, x, n, c, plane, ipc, pa, pb);
     launch_chained(ctx, bn_finish_stats_kernel, (unsigned)ceil_div(c, 128), 128, 0, pa, pb, slices, n, ipc, plane, c, m, momentum, eps, mean, inv, running_mean,
                    running_var, beta, beta_out);
@@ -877,7 +880,7 @@ static int32_t batchnorm_fwd(om_ctx* ctx, const float* x, const float* gamma, co
     auto apply = [&](auto kernel, int64_t accesses) {
       launch_chained(ctx, kernel, grid_for(ctx, accesses, 256), 256, 0, x, gamma, beta, mean, inv, total, c, plane, y);
     };
-    if ((plane & 3) == 0) relu ? apply(bn_apply_kernel<4, true>, total / 4) : apply(bn_apply_kernel<4, false>, total / 4);
+    if (vec) relu ? apply(bn_apply_kernel<4, true>, total / 4) : apply(bn_apply_kernel<4, false>, total / 4);
     else relu ? apply(bn_apply_kernel<1, true>, total) : apply(bn_apply_kernel<1, false>, total);
   }
   OM_LAUNCH_CHECK(ctx, "om_batchnorm_fwd");
@@ -908,11 +911,12 @@ static int32_t batchnorm_bwd(om_ctx* ctx, const float* g, const float* x, const 
   double *pa = nullptr, *pb = nullptr;
   OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)slices * c, false, (void**)&pa));
   OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)slices * c, false, (void**)&pb));
-  const bool vec = (plane & 3) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(g)) & 15) == 0;
+  const bool vec_xg = (plane & 3) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(g)) & 15) == 0;
+  const bool vec = vec_xg && (reinterpret_cast<uintptr_t>(dx) & 15) == 0;
   auto partial = [&](auto kernel) {
     launch_chained(ctx, kernel, dim3(c, slices), kBnThreads, 0, x, g, mean, inv, gamma, beta, n, c, plane, ipc, pa, pb);
   };
-  if (vec) relu ? partial(bn_bwd_partial_kernel<4, true>) : partial(bn_bwd_partial_kernel<4, false>);
+  if (vec_xg) relu ? partial(bn_bwd_partial_kernel<4, true>) : partial(bn_bwd_partial_kernel<4, false>);
   else relu ? partial(bn_bwd_partial_kernel<1, true>) : partial(bn_bwd_partial_kernel<1, false>);
   int64_t planes = (int64_t)n * c;
   if (dx && planes > 0 && plane > 0) {
@@ -923,7 +927,7 @@ static int32_t batchnorm_bwd(om_ctx* ctx, const float* g, const float* x, const 
     auto apply = [&](auto kernel, int64_t accesses) {
       launch_chained(ctx, kernel, grid_for(ctx, accesses, 256), 256, 0, g, x, mean, inv, gamma, beta, coef, total, c, plane, training, dx);
     };
-    if ((plane & 3) == 0) relu ? apply(bn_bwd_apply_kernel<4, true>, total / 4) : apply(bn_bwd_apply_kernel<4, false>, total / 4);
+    if (vec) relu ? apply(bn_bwd_apply_kernel<4, true>, total / 4) : apply(bn_bwd_apply_kernel<4, false>, total / 4);
     else relu ? apply(bn_bwd_apply_kernel<1, true>, total) : apply(bn_bwd_apply_kernel<1, false>, total);
     pool_free(ctx, coef);
   }

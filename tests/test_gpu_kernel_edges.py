@@ -484,6 +484,30 @@ def test_batch_norm_with_its_rectifier(ctx, n, c, h, w, training):
         assert np.array_equal(a, b, equal_nan=True)
 
 
+@pytest.mark.parametrize("relu", [0, 1])
+@pytest.mark.parametrize("off", [(1, 1, 1, 1), (1, 0, 0, 0), (0, 1, 0, 0), (0, 0, 1, 0), (0, 0, 0, 1)])
+def test_batch_norm_of_planes_off_the_16_byte_grid(ctx, relu, off):
+    """x, y, g and dx one float past a 16-byte boundary, together and alone, planes of whole float4s: the bits of the aligned calls where the statistics'
+    own accesses are the same, and 1e-6 where their double sums run in another order."""
+    n, c, h, w = 5, 3, 4, 8
+    x, g, gamma, beta = normal(1, n, c, h, w), normal(2, n, c, h, w), normal(3, c), normal(4, c)
+    out = []
+    for shift in ((0, 0, 0, 0), off):
+        X, G = (ctx.to_device(np.concatenate([np.zeros(k, np.float32), a.ravel()])) for a, k in ((x, shift[0]), (g, shift[2])))
+        Y, DX = (ctx.empty((x.size + k,)) for k in (shift[1], shift[3]))
+        GA, BE, RM, RV = (ctx.to_device(a) for a in (gamma, beta, np.zeros(c, np.float32), np.ones(c, np.float32)))
+        M, I, DG, DB, U = (ctx.empty((c,)) for _ in range(5))
+        px, py, pg, pd = (C.c_void_p(a.ptr.value + 4 * k) for a, k in zip((X, Y, G, DX), shift))
+        geometry, last = [i32(n), i32(c), i32(h * w)], [i32(1), pd, DG.ptr, DB.ptr, i32(0)]
+        ctx.call("om_batchnorm_relu_fwd" if relu else "om_batchnorm_fwd", ctx.handle, px, GA.ptr, BE.ptr, RM.ptr, RV.ptr, *geometry, i32(1), f32(0.1), f32(1e-5), py, M.ptr, I.ptr,
+                 *([U.ptr] if relu else []))
+        ctx.call("om_batchnorm_relu_bwd" if relu else "om_batchnorm_bwd", ctx.handle, pg, px, GA.ptr, *([U.ptr] if relu else []), M.ptr, I.ptr, *geometry, *last)
+        ctx.sync()
+        out.append([Y.numpy()[shift[1]:], DX.numpy()[shift[3]:], M.numpy(), I.numpy(), DG.numpy(), DB.numpy()])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b) if not (off[0] or off[2]) else np.max(np.abs(a - b)) <= 1e-6 * np.max(np.abs(a))
+
+
 @pytest.mark.parametrize("v,dim,n", [(50, 16, 20), (7, 3, 5), (300, 8, 64)])
 def test_kernels_of_a_chain_read_what_the_chain_wrote(ctx, v, dim, n):
     """A count that one kernel of a chain leaves and others read, while a slow kernel in front lets the whole chain queue up: every round has
