@@ -443,7 +443,8 @@ int32_t om_batchnorm_bwd(om_ctx* ctx, const float* g, const float* x, const floa
                          const float* inv, int32_t n, int32_t c, int32_t plane, int32_t training, float* dx,
                          float* dgamma, float* dbeta, int32_t accumulate_params);
 /* The norm and a rectifier behind it in one call: the values of om_batchnorm_fwd followed by om_unary(OM_RELU), bit for bit. The forward keeps
- * the beta it used for the backward (beta_used [c], may be NULL), which forms the rectifier's input again. */
+ * the beta it used for the backward (beta_used [c], may be NULL where no backward follows), which forms the rectifier's input again
+ * (OM_ERR_ARG without it). */
 int32_t om_batchnorm_relu_fwd(om_ctx* ctx, const float* x, const float* gamma, const float* beta,
                               float* running_mean, float* running_var, int32_t n, int32_t c, int32_t plane,
                               int32_t training, float momentum, float eps, float* y, float* mean, float* inv, float* beta_used);

@@ -948,6 +948,7 @@ int32_t om_batchnorm_bwd(om_ctx* ctx, const float* g, const float* x, const floa
 int32_t om_batchnorm_relu_bwd(om_ctx* ctx, const float* g, const float* x, const float* gamma, const float* beta, const float* mean,
                               const float* inv, int32_t n, int32_t c, int32_t plane, int32_t training, float* dx,
                               float* dgamma, float* dbeta, int32_t accumulate_params) {
+  if (ctx && !beta && c > 0) return fail(ctx, OM_ERR_ARG, "om_batchnorm_relu_bwd: the forward's beta is needed to form the rectifier's input again");
   return batchnorm_bwd(ctx, g, x, gamma, mean, inv, n, c, plane, training, dx, dgamma, dbeta, accumulate_params, true, beta);
 }
 

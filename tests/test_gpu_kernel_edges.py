@@ -484,6 +484,15 @@ def test_batch_norm_with_its_rectifier(ctx, n, c, h, w, training):
         assert np.array_equal(a, b, equal_nan=True)
 
 
+def test_batch_norm_relu_backward_needs_the_beta_of_the_forward(ctx):
+    """The forward may leave it out (no gradient wanted); the backward without it is refused on the host."""
+    X, V = ctx.to_device(normal(1, 2, 3, 2, 2)), ctx.to_device(np.ones(3, np.float32))
+    with pytest.raises(omb.OmError) as e:
+        ctx.call("om_batchnorm_relu_bwd", ctx.handle, X.ptr, X.ptr, V.ptr, None, V.ptr, V.ptr, i32(2), i32(3), i32(4), i32(1), None, None, None, i32(0))
+    assert e.value.code == 8      # OM_ERR_ARG
+    ctx.sync()
+
+
 @pytest.mark.parametrize("relu", [0, 1])
 @pytest.mark.parametrize("off", [(1, 1, 1, 1), (1, 0, 0, 0), (0, 1, 0, 0), (0, 0, 1, 0), (0, 0, 0, 1)])
 def test_batch_norm_of_planes_off_the_16_byte_grid(ctx, relu, off):
