@@ -655,20 +655,17 @@ int32_t om_ctc_grad(om_ctx* ctx, const float* g, const float* lp, int32_t t, int
   if (b == 0 || t == 0) return OM_OK;
   ProfileScope prof(ctx, "om_ctc_grad", 0, 8.0 * t * b * (double)c);
   const int max_ext = 2 * t + 1;
+  const size_t rows_bytes = 4 * sizeof(double) * (size_t)max_ext;
+  constexpr size_t most = 80 * 1024;
+  const int use_rows = rows_bytes <= most;
+  // (before anything is allocated, and for each call: the attribute belongs to the device)
+  if (use_rows) OM_CUDA(ctx, cudaFuncSetAttribute(ctc_chains_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
   double *alpha = nullptr, *beta = nullptr, *ends = nullptr;
   OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)b * t * max_ext, false, (void**)&alpha));
   int32_t st = pool_alloc(ctx, sizeof(double) * (size_t)b * t * max_ext, false, (void**)&beta);
   if (st == OM_OK) st = pool_alloc(ctx, (sizeof(double) + sizeof(int32_t)) * (size_t)b, false, (void**)&ends);
   if (st == OM_OK) {
     int32_t* offsets = reinterpret_cast<int32_t*>(ends + b);
-    const size_t rows_bytes = 4 * sizeof(double) * (size_t)max_ext;
-    constexpr size_t most = 80 * 1024;
-    const int use_rows = rows_bytes <= most;
-    static bool set = false;
-    if (!set) {
-      OM_CUDA(ctx, cudaFuncSetAttribute(ctc_chains_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
-      set = true;
-    }
     ctc_chains_kernel<<<b, 2 * kCtcThreads, use_rows ? rows_bytes : 0, ctx->stream>>>(lp, t, b, c, targets, target_lengths, input_lengths, blank, max_ext, alpha,
                                                                                    beta, ends, offsets, use_rows);
     // grid y holds 65535 sequences
