@@ -126,7 +126,7 @@ int32_t om_memset(om_ctx* ctx, void* dst, int32_t byte, size_t bytes);
  *   om_stage_release(slot)        the work queued so far on the compute stream has taken the batch: the slot may be refilled;
  *   om_stage_wait_taken(slot)     host wait for that point;
  *   om_stage_wait_ready(slot)     host wait until the slot's batch has landed (the source may be written again);
- *   om_host_is_pinned(p, bytes)   whether that range is page-locked memory the driver knows.
+ *   om_host_is_pinned(p, bytes)   whether that range lies in one page-locked allocation or registration.
  * Slots 0..15. The host memory must stay unchanged until the copy has run (keep it in the loader's ring). */
 int32_t om_stage_h2d(om_ctx* ctx, int32_t slot, void* dst, const void* src_pinned, size_t bytes);
 int32_t om_stage_commit(om_ctx* ctx, int32_t slot);

@@ -1,4 +1,5 @@
 // Context, pooled device memory, copies, graph capture and the per-entry-point profiler.
+#include <cuda.h>
 #include <stdarg.h>
 
 #include <algorithm>
@@ -227,6 +228,18 @@ static void profile_drain(om_ctx* ctx) {
     }
     kv.second.pending.clear();
   }
+}
+
+// cuPointerGetAttribute through the driver's entry points (no link against libcuda); null where there is none.
+typedef CUresult (*PointerAttributeFn)(void*, CUpointer_attribute, CUdeviceptr);
+static PointerAttributeFn pointer_attribute_fn() {
+  static const PointerAttributeFn fn = [] {
+    void* sym = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const bool found = cudaGetDriverEntryPoint("cuPointerGetAttribute", &sym, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
+    return found ? reinterpret_cast<PointerAttributeFn>(sym) : nullptr;
+  }();
+  return fn;
 }
 
 }  // namespace om
@@ -460,16 +473,21 @@ int32_t om_host_is_pinned(om_ctx* ctx, const void* p, size_t bytes, int32_t* pin
   OM_CHECK_CTX(ctx);
   *pinned = 0;
   if (p == nullptr || bytes == 0) return OM_OK;
-  const char* ends[2] = {static_cast<const char*>(p), static_cast<const char*>(p) + bytes - 1};
-  cudaPointerAttributes a[2];
-  for (int i = 0; i < 2; i++)
-    if (cudaPointerGetAttributes(&a[i], ends[i]) != cudaSuccess) {
-      cudaGetLastError();      // memory the driver does not know
-      return OM_OK;
-    }
-  // both ends in page-locked memory, mapped as one range
-  *pinned = a[0].type == cudaMemoryTypeHost && a[1].type == cudaMemoryTypeHost &&
-            static_cast<const char*>(a[1].devicePointer) - static_cast<const char*>(a[0].devicePointer) == ends[1] - ends[0];
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();      // memory the driver does not know
+    return OM_OK;
+  }
+  if (a.type != cudaMemoryTypeHost) return OM_OK;
+  // The whole range has to lie in the one allocation or registration that p belongs to: its ends may lie in two with pageable memory between.
+  // Where the driver does not say, the answer is no.
+  const PointerAttributeFn attribute = pointer_attribute_fn();
+  CUdeviceptr start = 0;
+  size_t length = 0;
+  const CUdeviceptr at = (CUdeviceptr)(uintptr_t)p;
+  if (!attribute || attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS || attribute(&length, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS)
+    return OM_OK;
+  *pinned = start <= at && bytes <= length && at - start <= length - bytes;
   return OM_OK;
 }
 

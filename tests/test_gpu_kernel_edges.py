@@ -489,7 +489,7 @@ def test_batch_norm_relu_backward_needs_the_beta_of_the_forward(ctx):
     X, V = ctx.to_device(normal(1, 2, 3, 2, 2)), ctx.to_device(np.ones(3, np.float32))
     with pytest.raises(omb.OmError) as e:
         ctx.call("om_batchnorm_relu_bwd", ctx.handle, X.ptr, X.ptr, V.ptr, None, V.ptr, V.ptr, i32(2), i32(3), i32(4), i32(1), None, None, None, i32(0))
-    assert e.value.code == 8      # OM_ERR_ARG
+    assert e.value.status == 8      # OM_ERR_ARG
     ctx.sync()
 
 

@@ -1,5 +1,8 @@
 """The benchmark configurations' training steps (host/trainer.cpp, the path bench.py times) against the CPU oracle
 running the same model on the same weights and batches, at sizes the oracle finishes in seconds."""
+import ctypes as C
+import mmap
+
 import numpy as np
 import pytest
 
@@ -254,6 +257,76 @@ def test_batches_staged_ahead_give_the_same_run(ctx, depth):
     assert np.array_equal(np.array(la), np.array(lb))
     for a, b in zip(pa, pb):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("depth", [1, 2])
+def test_staged_arrays_may_be_written_when_the_call_returns(ctx, depth, graph):
+    """Batches of more than the 128 KiB from which page-locked arrays are transferred from where they are: page-locked, pageable and mixed (labels), each
+    array overwritten as soon as it is staged. Losses and parameters of the plain loop, bit for bit."""
+    torch = pytest.importorskip("torch")
+    ctx.set_flags(0)
+    ctx.make_current()
+    cfg = [64, 3, 16, 16, 10, 2, 8, 8, 1, 2]
+    batches = [synth.cnn_batch(64, 3, 16, 16, 10, s) for s in range(7)]
+    assert batches[0][0].nbytes >= 128 * 1024
+
+    def run(staged):
+        tr = omb.Trainer("cnn", cfg, lr=0.05, weight_decay=0.0, seed=0)
+        images = [torch.empty(batches[0][0].size, dtype=torch.float32, pin_memory=pin) for pin in (True, False)]
+        labels = np.empty_like(batches[0][1])
+        pinned = C.c_int32()
+        for t in images:
+            ctx.call("om_host_is_pinned", ctx.handle, C.c_void_p(t.data_ptr()), C.c_size_t(batches[0][0].nbytes), C.byref(pinned))
+            assert pinned.value == int(t.is_pinned())
+        losses, nxt = [], 0
+        if staged:
+            tr.prefetch_depth(depth)
+        for s in range(len(batches)):
+            if graph and s == 2:
+                tr.enable_graph()
+            if not staged:
+                losses.append(np.float32(tr.step(list(batches[s]))))
+                continue
+            while nxt < len(batches) and nxt - s < depth:
+                image = images[nxt % 3 == 2]
+                image.numpy()[:] = batches[nxt][0].ravel()
+                labels[:] = batches[nxt][1]
+                tr.prefetch_ptrs((C.c_void_p * 2)(image.data_ptr(), labels.ctypes.data))
+                image.numpy()[:] = np.nan
+                labels[:] = -7
+                nxt += 1
+            losses.append(np.float32(tr.step_prefetched()))
+        params = [tr.get_param(i, sh) for i, (_, sh) in enumerate(tr.named_parameters())]
+        tr.close()
+        return losses, params
+
+    (la, pa), (lb, pb) = run(False), run(True)
+    assert np.array_equal(np.array(la), np.array(lb))
+    for a, b in zip(pa, pb):
+        assert np.array_equal(a, b)
+
+
+def test_a_range_across_two_page_locked_registrations_is_not_page_locked(ctx):
+    """Two registered ranges with pageable memory between them: each alone is page-locked, what reaches over an end or from one into the other is not."""
+    torch = pytest.importorskip("torch")
+    size = 1 << 20
+    buf = mmap.mmap(-1, 3 * size)
+    base = np.frombuffer(buf, np.uint8)
+    base[:] = 1
+    at, rt, pinned = base.ctypes.data, torch.cuda.cudart(), C.c_int32()
+
+    def asked(offset, nbytes):
+        ctx.call("om_host_is_pinned", ctx.handle, C.c_void_p(at + offset), C.c_size_t(nbytes), C.byref(pinned))
+        return pinned.value
+
+    assert asked(0, 3 * size) == 0
+    assert int(rt.cudaHostRegister(at, size, 0)) == 0 and int(rt.cudaHostRegister(at + 2 * size, size, 0)) == 0
+    try:
+        assert asked(0, size) == 1 and asked(2 * size, size) == 1 and asked(4096, size - 4096) == 1
+        assert asked(0, 3 * size) == 0 and asked(0, size + 1) == 0 and asked(4096, size) == 0 and asked(size, size) == 0
+    finally:
+        assert int(rt.cudaHostUnregister(at)) == 0 and int(rt.cudaHostUnregister(at + 2 * size)) == 0
 
 
 @pytest.mark.parametrize("graph", [False, True])
