@@ -566,6 +566,13 @@ int32_t om_conv2d_dbias(om_ctx* ctx, const om_conv_shape* s, const float* g, flo
  * under OM_TF32) is made once. */
 int32_t om_conv2d_bwd(om_ctx* ctx, const om_conv_shape* s, const float* g, const float* x, const float* w, float* dx, float* dw,
                       int32_t accumulate_w, float* dbias, int32_t accumulate_b);
+/* The same in two calls, so that what waits for the parameter gradients (their exchange between ranks) starts under the input gradient: first the weight and
+ * bias gradient (each left out where NULL), then the input gradient. om_conv2d_bwd_workspace gives the size of what they share in floats, 0 where that is
+ * nothing under the context's present flags; the caller allocates it (16-byte aligned) and hands it to both calls unchanged, or NULL to both. */
+int32_t om_conv2d_bwd_workspace(om_ctx* ctx, const om_conv_shape* s, int64_t* floats);
+int32_t om_conv2d_bwd_params(om_ctx* ctx, const om_conv_shape* s, const float* g, const float* x, float* dw, int32_t accumulate_w, float* dbias,
+                             int32_t accumulate_b, float* workspace);
+int32_t om_conv2d_bwd_input(om_ctx* ctx, const om_conv_shape* s, const float* g, const float* w, float* dx, const float* workspace);
 
 /* Max pooling over NCHW planes; idx receives the Int32 flat NCHW index of each maximum (first wins ties,
  * NaN wins), bit-exact with ReferenceKernels.MaxPool2d (src/OneModel/Tensors/TensorKernels.cs:242-295). */

@@ -22,8 +22,10 @@ bool conv_nhwc_dgrad_fits(const ConvGeom& g);
 int32_t conv_nhwc_dgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* w, float* dx, const float* turned_gr = nullptr);
 bool conv_nhwc_wgrad_fits(const ConvGeom& g);
 int32_t conv_nhwc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, float* dw, int accumulate, const float* turned_gr = nullptr);
-int32_t conv_nhwc_bwd(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, const float* w, float* dx, float* dw, int accumulate_w, float* dbias,
-                      int accumulate_b);
+// The channels-last copy of the output's gradient that weight and input gradient take (turned_gr above): its floats, and the pass that writes it and, when asked
+// for, the bias gradient.
+long long conv_nhwc_turned_floats(const ConvGeom& g);
+int32_t conv_nhwc_turn_gradient(om_ctx* ctx, const ConvGeom& g, const float* gr, float* turned, float* dbias, int accumulate_b);
 
 // The fp32 products of small shapes without an unfolded matrix (om_conv_fma.cu).
 bool conv_fma_fwd_fits(const ConvGeom& g);

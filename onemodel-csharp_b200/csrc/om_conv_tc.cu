@@ -1154,18 +1154,6 @@ static int32_t cn_turn(om_ctx* ctx, const float* src, int n, int c, int plane, f
                  cv_div((uint32_t)plane), c, cp, nullptr);
   return OM_OK;
 }
-// The same and the sums of the channels.
-static int32_t cn_turn_sums(om_ctx* ctx, const float* src, int n, int c, int plane, float** out, float* dbias, int accumulate) {
-  const int pixels = n * plane, cp = cn_pitch(c), ctas = (int)std::min<int64_t>(ceil_div(pixels, CN_PX), CN_SUM_CTAS);
-  double* sums = nullptr;
-  OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)pixels * cp, false, (void**)out));
-  OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)ctas * c, false, (void**)&sums));
-  launch_chained(ctx, conv_channels_last_kernel<true>, dim3((unsigned)ctas, (unsigned)ceil_div(cp, 32)), 256, 0, src, *out, pixels, plane, cv_div((uint32_t)plane), c,
-                 cp, sums);
-  launch_chained(ctx, conv_sums_finish_kernel, (unsigned)ceil_div(c, 32), 256, 0, sums, ctas, c, dbias, accumulate);
-  pool_free(ctx, sums);
-  return OM_OK;
-}
 
 // A block of 32 channels may be partly empty, and a box partly outside the grid: at least two thirds of the work has to be real.
 static bool cn_channels_fit(int c) { return 3 * c >= 2 * (int)ceil_div(c, 32) * 32; }
@@ -1388,15 +1376,23 @@ int32_t conv_nhwc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const f
   return st;
 }
 
-// Weight and input gradient (and the bias gradient, when asked for) from one channels-last copy of the output's gradient.
-int32_t conv_nhwc_bwd(om_ctx* ctx, const ConvGeom& g, const float* gr, const float* x, const float* w, float* dx, float* dw, int accumulate_w, float* dbias,
-                      int accumulate_b) {
-  float* gt = nullptr;
-  int32_t st = dbias ? cn_turn_sums(ctx, gr, g.n, g.cout, g.oh * g.ow, &gt, dbias, accumulate_b) : cn_turn(ctx, gr, g.n, g.cout, g.oh * g.ow, &gt);
-  if (st == OM_OK) st = conv_nhwc_wgrad(ctx, g, gr, x, dw, accumulate_w, gt);
-  if (st == OM_OK) st = conv_nhwc_dgrad(ctx, g, gr, w, dx, gt);
-  if (gt) pool_free(ctx, gt);
-  return st;
+long long conv_nhwc_turned_floats(const ConvGeom& g) { return (long long)g.n * g.oh * g.ow * cn_pitch(g.cout); }
+
+int32_t conv_nhwc_turn_gradient(om_ctx* ctx, const ConvGeom& g, const float* gr, float* turned, float* dbias, int accumulate_b) {
+  const int plane = g.oh * g.ow, pixels = g.n * plane, cp = cn_pitch(g.cout);
+  const unsigned columns = (unsigned)ceil_div(cp, 32), tiles = (unsigned)ceil_div(pixels, CN_PX);
+  if (!dbias) {
+    launch_chained(ctx, conv_channels_last_kernel<false>, dim3(tiles, columns), 256, 0, gr, turned, pixels, plane, cv_div((uint32_t)plane), g.cout, cp, nullptr);
+  } else {
+    const int ctas = std::min((int)tiles, CN_SUM_CTAS);
+    double* sums = nullptr;
+    OM_TRY(pool_alloc(ctx, sizeof(double) * (size_t)ctas * g.cout, false, (void**)&sums));
+    launch_chained(ctx, conv_channels_last_kernel<true>, dim3((unsigned)ctas, columns), 256, 0, gr, turned, pixels, plane, cv_div((uint32_t)plane), g.cout, cp, sums);
+    launch_chained(ctx, conv_sums_finish_kernel, (unsigned)ceil_div(g.cout, 32), 256, 0, sums, ctas, g.cout, dbias, accumulate_b);
+    pool_free(ctx, sums);
+  }
+  OM_LAUNCH_CHECK(ctx, "conv_nhwc_turn_gradient");
+  return OM_OK;
 }
 
 }  // namespace om

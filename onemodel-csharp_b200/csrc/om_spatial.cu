@@ -820,20 +820,52 @@ int32_t om_conv2d_dbias(om_ctx* ctx, const om_conv_shape* s, const float* gr, fl
   return OM_OK;
 }
 
-int32_t om_conv2d_bwd(om_ctx* ctx, const om_conv_shape* s, const float* gr, const float* x, const float* w, float* dx, float* dw,
-                      int32_t accumulate_w, float* dbias, int32_t accumulate_b) {
+int32_t om_conv2d_bwd_workspace(om_ctx* ctx, const om_conv_shape* s, int64_t* floats) {
   OM_CHECK_CTX(ctx);
   ConvGeom g;
   if (!s || !conv_geom(s, &g)) return fail(ctx, OM_ERR_SHAPE, "Invalid convolution geometry.");
-  if (dx && dw && g.n > 0 && g.n <= 65535 && conv_on_tensor_pipe(ctx, g, true) && conv_nhwc_wgrad_fits(g) && conv_nhwc_dgrad_fits(g)) {
-    const double flops = 2.0 * g.n * g.cout * (double)g.cin * g.kh * g.kw * g.oh * g.ow;
-    ProfileScope prof(ctx, "om_conv2d_bwd", 2.0 * flops, 4.0 * g.n * (2.0 * g.cin * g.h * g.w + 2.0 * g.cout * (double)g.oh * g.ow));
-    return conv_nhwc_bwd(ctx, g, gr, x, w, dx, dw, accumulate_w, dbias, accumulate_b);
+  const bool shared = g.n > 0 && g.n <= 65535 && conv_on_tensor_pipe(ctx, g, true) && conv_nhwc_wgrad_fits(g) && conv_nhwc_dgrad_fits(g);
+  *floats = shared ? conv_nhwc_turned_floats(g) : 0;
+  return OM_OK;
+}
+
+int32_t om_conv2d_bwd_params(om_ctx* ctx, const om_conv_shape* s, const float* gr, const float* x, float* dw, int32_t accumulate_w, float* dbias,
+                             int32_t accumulate_b, float* workspace) {
+  OM_CHECK_CTX(ctx);
+  ConvGeom g;
+  if (!s || !conv_geom(s, &g)) return fail(ctx, OM_ERR_SHAPE, "Invalid convolution geometry.");
+  if (workspace) {
+    ProfileScope prof(ctx, "om_conv2d_bwd_params", dw ? 2.0 * g.n * g.cout * (double)g.cin * g.kh * g.kw * g.oh * g.ow : 0.0,
+                      4.0 * g.n * ((double)g.cin * g.h * g.w + (double)g.cout * g.oh * g.ow));
+    OM_TRY(conv_nhwc_turn_gradient(ctx, g, gr, workspace, dbias, accumulate_b));
+    return dw ? conv_nhwc_wgrad(ctx, g, gr, x, dw, accumulate_w, workspace) : OM_OK;
   }
   if (dbias) OM_TRY(om_conv2d_dbias(ctx, s, gr, dbias, accumulate_b));
   if (dw) OM_TRY(om_conv2d_wgrad(ctx, s, gr, x, dw, accumulate_w));
-  if (dx) OM_TRY(om_conv2d_dgrad(ctx, s, gr, w, dx));
   return OM_OK;
+}
+
+int32_t om_conv2d_bwd_input(om_ctx* ctx, const om_conv_shape* s, const float* gr, const float* w, float* dx, const float* workspace) {
+  OM_CHECK_CTX(ctx);
+  if (!workspace) return om_conv2d_dgrad(ctx, s, gr, w, dx);
+  ConvGeom g;
+  if (!s || !conv_geom(s, &g)) return fail(ctx, OM_ERR_SHAPE, "Invalid convolution geometry.");
+  ProfileScope prof(ctx, "om_conv2d_dgrad", 2.0 * g.n * g.cout * (double)g.cin * g.kh * g.kw * g.oh * g.ow,
+                    4.0 * g.n * ((double)g.cin * g.h * g.w + (double)g.cout * g.oh * g.ow));
+  return conv_nhwc_dgrad(ctx, g, gr, w, dx, workspace);
+}
+
+int32_t om_conv2d_bwd(om_ctx* ctx, const om_conv_shape* s, const float* gr, const float* x, const float* w, float* dx, float* dw,
+                      int32_t accumulate_w, float* dbias, int32_t accumulate_b) {
+  OM_CHECK_CTX(ctx);
+  int64_t floats = 0;
+  float* turned = nullptr;
+  OM_TRY(om_conv2d_bwd_workspace(ctx, s, &floats));
+  if (dx && dw && floats > 0) OM_TRY(pool_alloc(ctx, sizeof(float) * (size_t)floats, false, (void**)&turned));
+  int32_t st = om_conv2d_bwd_params(ctx, s, gr, x, dw, accumulate_w, dbias, accumulate_b, turned);
+  if (st == OM_OK && dx) st = om_conv2d_bwd_input(ctx, s, gr, w, dx, turned);
+  if (turned) pool_free(ctx, turned);
+  return st;
 }
 
 int32_t om_resize2d_fwd(om_ctx* ctx, const float* x, int64_t planes, int32_t h, int32_t w, int32_t out_h, int32_t out_w, int32_t mode,

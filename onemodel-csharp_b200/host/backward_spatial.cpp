@@ -34,15 +34,24 @@ static void ConvBackward(BackwardRecord& r, const Tensor& g) {
   s.stride_h = (int)r.Ints[0]; s.stride_w = (int)r.Ints[1]; s.pad_top = (int)r.Ints[2]; s.pad_left = (int)r.Ints[3];
   s.pad_bottom = (int)r.Ints[4]; s.pad_right = (int)r.Ints[5]; s.dil_h = (int)r.Ints[6]; s.dil_w = (int)r.Ints[7]; s.groups = (int)r.Ints[8];
   Tensor gc = g.Contiguous();
-  // Order of the reference: bias, weights, input.
+  // Order of the reference: bias, weights, input. The parameters' gradients are reported before the input's is queued, so that their exchange runs under it.
   GradSlot db(r, 2), dw(r, 1);
-  Tensor dx;
-  if (r.NeedsInputGrad(0)) dx = Tensor::Create(DType::F32, x.GetShape());
-  Check(om_conv2d_bwd(C(), &s, gc.Data(), x.Data(), w.Data(), dx.IsEmpty() ? nullptr : dx.Data(), dw.needed ? dw.ptr : nullptr, dw.accumulate,
-                      db.needed ? db.ptr : nullptr, db.accumulate));
+  Tensor shared;
+  if (dw.needed && r.NeedsInputGrad(0)) {
+    int64_t floats = 0;
+    Check(om_conv2d_bwd_workspace(C(), &s, &floats));
+    if (floats > 0) shared = Tensor::Create(DType::F32, Shape{(int)floats});
+  }
+  float* ws = shared.IsEmpty() ? nullptr : shared.Data();
+  if (db.needed || dw.needed)
+    Check(om_conv2d_bwd_params(C(), &s, gc.Data(), x.Data(), dw.needed ? dw.ptr : nullptr, dw.accumulate, db.needed ? db.ptr : nullptr, db.accumulate, ws));
   db.Done(r, 2);
   dw.Done(r, 1);
-  if (r.NeedsInputGrad(0)) Engine::Emit(r, 0, dx, true);
+  if (r.NeedsInputGrad(0)) {
+    Tensor dx = Tensor::Create(DType::F32, x.GetShape());
+    Check(om_conv2d_bwd_input(C(), &s, gc.Data(), w.Data(), dx.Data(), ws));
+    Engine::Emit(r, 0, dx, true);
+  }
 }
 
 // The record of Ops::LstmBidirectional: inputs x, then (wIh, wHh, bIh, bHh) per direction; slots 0 x, then per direction

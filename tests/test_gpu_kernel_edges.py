@@ -261,7 +261,7 @@ def test_conv2d_from_channels_last_copies(ctx, case):
 
 
 @pytest.mark.parametrize("case", [
-    (33, 64, 16, 16, 96, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1), (64, 64, 16, 16, 256, 3, 3, 2, 2, (1, 1, 1, 1), 1, 1),
+    (33, 64, 16, 16, 96, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1), (72, 64, 16, 16, 96, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1), (64, 64, 16, 16, 256, 3, 3, 2, 2, (1, 1, 1, 1), 1, 1),
     (40, 72, 17, 15, 160, 3, 3, 2, 2, (1, 1, 1, 1), 1, 1), (256, 64, 32, 32, 128, 1, 1, 2, 2, (0, 0, 0, 0), 1, 1),
     (24, 32, 20, 44, 32, 5, 5, 1, 1, (4, 4, 4, 4), 2, 2), (160, 64, 32, 4, 128, 3, 2, 1, 2, (2, 0, 1, 1), 1, 1), (37, 48, 11, 12, 96, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1)])
 def test_conv2d_input_gradient_has_the_bits_of_product_and_fold(ctx, case):
@@ -426,6 +426,30 @@ def test_conv2d_backward_in_one_call(ctx, case, tf32):
             assert skip == 2 or np.max(np.abs(DB.numpy() - want) / np.abs(g).astype(np.float64).sum((0, 2, 3))) <= 1e-6
         ctx.call("om_conv2d_bwd", ctx.handle, C.byref(s), G.ptr, X.ptr, W.ptr, DX.ptr, DW.ptr, i32(1), DB.ptr, i32(1))
         assert np.array_equal(DW.numpy(), apart[3]) and scaled_diff(DB.numpy(), 2 * want) <= 2e-6
+    finally:
+        ctx.set_flags(0)
+
+
+@pytest.mark.parametrize("tf32", [0, 1])
+@pytest.mark.parametrize("case", [(48, 64, 16, 16, 96, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1), (64, 64, 16, 16, 256, 3, 3, 2, 2, (1, 1, 1, 1), 1, 1), (3, 5, 9, 7, 6, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1)])
+def test_conv2d_parameter_gradients_before_the_input_gradient(ctx, case, tf32):
+    """The two calls give the bits of the one; after the first the parameters' gradients are there and nothing of the input gradient is."""
+    s, x, wt, b, g, y, dx, dw = conv_case(*case)
+    ctx.set_flags(omb.OM_TF32 if tf32 else 0)
+    try:
+        X, W, G = (ctx.to_device(a) for a in (x, wt, g))
+        DX, DW, DB, DX2, DW2, DB2 = (ctx.empty(a) for a in (x.shape, wt.shape, b.shape) * 2)
+        floats = C.c_int64()
+        ctx.call("om_conv2d_bwd_workspace", ctx.handle, C.byref(s), C.byref(floats))
+        assert (floats.value > 0) == bool(tf32 and g.size > 1e5)
+        ws = ctx.empty((max(1, floats.value),)) if floats.value else None
+        ctx.call("om_conv2d_bwd", ctx.handle, C.byref(s), G.ptr, X.ptr, W.ptr, DX.ptr, DW.ptr, i32(0), DB.ptr, i32(0))
+        ctx.call("om_memset", ctx.handle, DX2.ptr, i32(0x2b), C.c_size_t(x.nbytes))
+        ctx.call("om_conv2d_bwd_params", ctx.handle, C.byref(s), G.ptr, X.ptr, DW2.ptr, i32(0), DB2.ptr, i32(0), ws.ptr if ws else None)
+        assert np.array_equal(DW2.numpy(), DW.numpy()) and np.array_equal(DB2.numpy(), DB.numpy())
+        assert (DX2.numpy().view(np.uint32) == 0x2b2b2b2b).all()
+        ctx.call("om_conv2d_bwd_input", ctx.handle, C.byref(s), G.ptr, W.ptr, DX2.ptr, ws.ptr if ws else None)
+        assert np.array_equal(DX2.numpy(), DX.numpy())
     finally:
         ctx.set_flags(0)
 
