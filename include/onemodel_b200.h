@@ -68,7 +68,8 @@ typedef enum om_status {
  * runs all its time steps in one cooperative launch with fp32 recurrent products, instead of a product and a gate
  * kernel per step. OM_OVERLAP_LAUNCHES: the frequent kernels are launched as programmatic dependents of their
  * predecessor in the stream, so that launch latency and prologue overlap the predecessor's tail (same results); without
- * it only those of up to 1184 CTAs are, or of up to 296 while a step is being captured.
+ * it only those of up to 1184 CTAs are, or of up to 296 while a step is being captured. OM_SERIAL_LAUNCHES: none is, whatever the other flags say:
+ * what overlapped runs are compared with, and what a profiler's durations of single kernels need.
  * OM_PERSISTENT_TILES (with OM_TF32): plain products run on the persistent CTA-pair kernel that the bfloat16 products
  * always use (two accumulator buffers in tensor memory: a tile's read-back and stores run under the next tile's MMAs). */
 #define OM_TF32 1u
@@ -79,6 +80,7 @@ typedef enum om_status {
 #define OM_SEQ_KERNELS 32u
 #define OM_OVERLAP_LAUNCHES 64u
 #define OM_PERSISTENT_TILES 128u
+#define OM_SERIAL_LAUNCHES 256u
 
 typedef enum om_dtype { OM_F32 = 0, OM_I32 = 1, OM_I64 = 2 } om_dtype;
 

@@ -171,7 +171,8 @@ static inline void launch_chained(om_ctx* ctx, void (*kernel)(KArgs...), dim3 gr
   // (a captured classifier step of 128 x 784: 6 % faster, the encoder steps unchanged); outside, the eight CTAs an SM that the
   // element-wise kernels launch at most.
   const int64_t ctas = (int64_t)grid.x * grid.y * grid.z;
-  cfg.numAttrs = (ctx->flags & OM_OVERLAP_LAUNCHES) || ctas <= (ctx->capturing ? 2 * 148 : 8 * 148) ? 1 : 0;
+  const bool overlap = (ctx->flags & OM_OVERLAP_LAUNCHES) || ctas <= (ctx->capturing ? 2 * 148 : 8 * 148);
+  cfg.numAttrs = overlap && !(ctx->flags & OM_SERIAL_LAUNCHES) ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 #endif

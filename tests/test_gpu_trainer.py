@@ -111,14 +111,14 @@ def test_full_size_encoder_step_is_deterministic_and_graph_equals_eager(ctx, tf3
 
 
 def test_scheduling_flags_do_not_change_the_bits(ctx):
-    """Config 3 at full size with overlapped launches (programmatic dependent launch), the two-stream linear backward and
+    """Config 3 at full size with overlapped launches (programmatic dependent launch: the small ones, then all), the two-stream linear backward and
     both together, eager and replayed from a captured graph: scheduling only, so the losses and every parameter after
-    four steps equal the plain run bit for bit."""
+    four steps equal the run in which no launch overlaps another bit for bit."""
     ctx.make_current()
     try:
-        ctx.set_flags(omb.OM_TF32)
+        ctx.set_flags(omb.OM_TF32 | omb.OM_SERIAL_LAUNCHES)
         la, pa = _run_c3(4, 2, True)
-        for extra in (omb.OM_OVERLAP_LAUNCHES, omb.OM_TWO_STREAMS, omb.OM_OVERLAP_LAUNCHES | omb.OM_TWO_STREAMS):
+        for extra in (0, omb.OM_OVERLAP_LAUNCHES, omb.OM_TWO_STREAMS, omb.OM_OVERLAP_LAUNCHES | omb.OM_TWO_STREAMS):
             ctx.set_flags(omb.OM_TF32 | extra)
             for graph_at in (None, 2):
                 lb, pb = _run_c3(4, graph_at, True)
@@ -127,6 +127,35 @@ def test_scheduling_flags_do_not_change_the_bits(ctx):
                     assert np.array_equal(a, b), (extra, graph_at)
     finally:
         ctx.set_flags(0)
+
+
+@pytest.mark.parametrize("graph_at", [None, 2])
+@pytest.mark.parametrize("kind,flags", [("cnn", omb.OM_TF32), ("cnn", 0), ("mlp", 0), ("mlp", omb.OM_TF32), ("crnn", omb.OM_TF32 | omb.OM_SEQ_KERNELS)])
+def test_overlapped_small_launches_do_not_change_the_bits(ctx, kind, flags, graph_at):
+    """Chains of small kernels (convolutions and batch norm, small fp32 products, recurrent layers), every step's batch another: the losses and parameters
+    of the run in which no launch overlaps another, bit for bit."""
+    ctx.make_current()
+    cfg = {"cnn": [64, 3, 16, 16, 10, 4, 16, 32, 64, 64, 1, 2, 1, 2], "mlp": [16, 64, 128, 128, 10], "crnn": [8, 32, 48, 11, 32, 5, 4, 6, 8, 8]}[kind]
+    batch = {"cnn": lambda s: synth.cnn_batch(64, 3, 16, 16, 10, s), "mlp": lambda s: synth.mlp_batch(16, 64, 10, s),
+             "crnn": lambda s: synth.crnn_batch(8, 32, 48, 11, 5, 2, s)}[kind]
+    runs = []
+    try:
+        for extra in (omb.OM_SERIAL_LAUNCHES, 0, omb.OM_OVERLAP_LAUNCHES):
+            ctx.set_flags(flags | extra)
+            tr = omb.Trainer(kind, cfg, lr=1e-3, weight_decay=0.0, seed=0)
+            losses = []
+            for step in range(6):
+                if step == graph_at:
+                    tr.enable_graph()
+                losses.append(tr.step(list(batch(step))))
+            runs.append((losses, [tr.get_param(i, s) for i, (_, s) in enumerate(tr.named_parameters())]))
+            tr.close()
+    finally:
+        ctx.set_flags(0)
+    for losses, params in runs[1:]:
+        assert losses == runs[0][0]
+        for a, b in zip(params, runs[0][1]):
+            assert np.array_equal(a, b)
 
 
 def test_cnn_config_small(ctx, configs):
