@@ -174,6 +174,25 @@ def test_conv2d_on_the_fma_pipe(ctx, case, tf32):
     assert scaled_diff(DW2, 2 * dw) <= (2e-5 if tc else 1e-5)
 
 
+@pytest.mark.parametrize("n,cin,h,w,cout,k,stride", [
+    (3, 8, 20, 24, 40, 3, 1), (3, 9, 20, 24, 40, 3, 1), (36, 8, 20, 24, 40, 3, 1), (36, 9, 20, 24, 40, 3, 1),       # 72 and 81 terms, few and many CTAs
+    (36, 32, 20, 24, 48, 3, 1), (36, 33, 20, 24, 48, 3, 1), (31, 32, 20, 24, 48, 3, 1), (32, 32, 20, 24, 32, 3, 2),  # 288 and 297 terms, either side of 120 CTAs
+    (36, 28, 20, 24, 64, 3, 1), (36, 27, 20, 24, 64, 3, 1), (36, 64, 10, 24, 65, 1, 1), (2, 1, 33, 31, 3, 5, 2)])
+def test_conv2d_fp32_bits_do_not_depend_on_the_kernel(ctx, K, n, cin, h, w, cout, k, stride):
+    """Either side of the lines between the kernels without an unfolded matrix and the product on one, the forward and the input gradient have the
+    bits of the reference's order: one chain over (channel, ky, kx), and tap by tap one chain over the output channels."""
+    ctx.set_flags(0)
+    pad = k // 2
+    x, wt, b = normal(1, n, cin, h, w), normal(2, cout, cin, k, k, scale=0.2), normal(3, cout)
+    y = K.conv2d_fwd(x, wt, b, stride, pad)
+    g = normal(4, *y.shape)
+    dx = K.conv2d_bwd(g, x, wt, stride, pad)[0]
+    s = ConvShape(n, cin, h, w, cout, k, k, stride, stride, pad, pad, pad, pad, 1, 1, 1)
+    Y, DX, _, _ = run_conv(ctx, s, x, wt, b, g)
+    assert np.array_equal(Y, y)
+    assert np.array_equal(DX, dx)
+
+
 def test_ctc_chains_and_classes_are_bit_exact(ctx, K):
     """Extended targets of more positions than a CTA has threads, repeated labels, an empty target, more labels than steps, no steps, and a
     number of steps whose rows no longer fit on the chip: the reference's doubles bit for bit."""
