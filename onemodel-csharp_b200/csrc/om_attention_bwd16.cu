@@ -120,7 +120,7 @@ __device__ __forceinline__ void ab_slot_free(int lane) {
 // Rows are taken in the order (batch, query, head), the order of memory for activations stored [batch, query, head * 64], so
 // that the warps of a CTA read one contiguous stretch.
 __global__ void __launch_bounds__(256)
-attention_dots_kernel(const float* __restrict__ g, const float* __restrict__ out, long long g_batch, long long g_head, long long g_row,
+attention_dots_kernel(const float* g, const float* out, long long g_batch, long long g_head, long long g_row,
                       long long o_batch, long long o_head, long long o_row, int heads, int lq, long long rows, float* __restrict__ dots) {
   pdl_enter();
   const int lane = threadIdx.x & 31;
@@ -162,7 +162,7 @@ attention_dots_kernel(const float* __restrict__ g, const float* __restrict__ out
 // one (batch, head); a thread owns two of them and has four parts of each in flight. No division per element: the head
 // is the CTA's y index and a row of 64 columns is 16 groups.
 __global__ void __launch_bounds__(256)
-attention_dq_reduce_kernel(const float* __restrict__ parts, int nk, long long part_stride, int heads, int lq, float* __restrict__ dq,
+attention_dq_reduce_kernel(const float* parts, int nk, long long part_stride, int heads, int lq, float* __restrict__ dq,
                            uint16_t* __restrict__ dq16, long long dq_batch, long long dq_head, long long dq_row) {
   pdl_enter();
   const int bh = blockIdx.y, bi = bh / heads, hi = bh - bi * heads;
@@ -380,8 +380,8 @@ attention_bwd16_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const int qrow = i * AB_TILE + row;
       const bool row_ok = qrow < p.lq;
       const bool edge = key_edge || (i + 1) * AB_TILE > p.lq;
-      const float dot = row_ok ? __ldg(p.dots + (long long)bh * p.lq + qrow) : 0.f;
-      const float lse_l = row_ok ? __ldg(p.lse + (long long)bh * p.lq + qrow) * LOG2E : 0.f;
+      const float dot = row_ok ? ld_global(p.dots + (long long)bh * p.lq + qrow) : 0.f;
+      const float lse_l = row_ok ? ld_global(p.lse + (long long)bh * p.lq + qrow) * LOG2E : 0.f;
       const float* mrow = (p.mask && row_ok) ? p.mask + (long long)bi * p.mask_batch_stride + (long long)qrow * p.lk : nullptr;
       for (int h = 0; h < 2 && ok; h++) {
         ok = mbar_wait(&bar_sdp[h], (uint32_t)i & 1, abort_flag, p.status, 57);

@@ -82,7 +82,7 @@ constexpr float AF_BOUND_LIMIT = 40.f;
 
 // kmax2[b, h] = max over the keys of |k|^2 (fp32 sum of the squares of the bfloat16 values). One CTA per (batch, head).
 __global__ void __launch_bounds__(256)
-attention_kmax_kernel(const uint16_t* __restrict__ k16, long long s_batch, long long s_head, long long s_row, int heads, int lk,
+attention_kmax_kernel(const uint16_t* k16, long long s_batch, long long s_head, long long s_row, int heads, int lk,
                       float* __restrict__ kmax2) {
   pdl_enter();
   __shared__ float wmax[8];
@@ -94,7 +94,7 @@ attention_kmax_kernel(const uint16_t* __restrict__ k16, long long s_batch, long 
     float ss = 0.f;
 #pragma unroll
     for (int c = 0; c < AF_D / 8; c++) {
-      const uint4 v = __ldg(rowp + c);
+      const uint4 v = ld_global(rowp + c);
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int q = 0; q < 4; q++) {

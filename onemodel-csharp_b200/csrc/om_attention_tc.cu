@@ -61,16 +61,16 @@ __device__ __forceinline__ uint32_t att_idesc(int n, bool a_mn, bool b_mn) {
 // layer, most of it those loads; 61 and 59 us this way). Instead the warp reads the block by rows (eight lanes cover the 128
 // bytes of one, before the wait for the scores) and turns it through 4 KB of shared memory whose 16-byte chunk c of row r
 // sits at c ^ (r & 7). Rows and columns outside the mask read as zero.
-__device__ __forceinline__ void mask_fetch(float4 (&m)[8], const float* __restrict__ mask, int row0, int lq, int col0, int lk, int lane) {
+__device__ __forceinline__ void mask_fetch(float4 (&m)[8], const float* mask, int row0, int lq, int col0, int lk, int lane) {
   const int col = col0 + (lane & 7) * 4;
 #pragma unroll
   for (int i = 0; i < 8; i++) {
     const int row = row0 + i * 4 + (lane >> 3);
-    m[i] = row < lq && col < lk ? __ldg(reinterpret_cast<const float4*>(mask + (long long)row * lk + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    m[i] = row < lq && col < lk ? ld_global(reinterpret_cast<const float4*>(mask + (long long)row * lk + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
 // Without 16-byte rows (vec == false) the warp fetches here, a row per step.
-__device__ __forceinline__ void mask_deposit(uint8_t* blk, const float4 (&m)[8], bool vec, const float* __restrict__ mask, int row0, int lq, int col0,
+__device__ __forceinline__ void mask_deposit(uint8_t* blk, const float4 (&m)[8], bool vec, const float* mask, int row0, int lq, int col0,
                                              int lk, int lane) {
   if (vec) {
 #pragma unroll
@@ -82,7 +82,7 @@ __device__ __forceinline__ void mask_deposit(uint8_t* blk, const float4 (&m)[8],
 #pragma unroll 8
     for (int r = 0; r < 32; r++)
       *reinterpret_cast<float*>(blk + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4) =
-          row0 + r < lq && col0 + lane < lk ? __ldg(mask + (long long)(row0 + r) * lk + col0 + lane) : 0.f;
+          row0 + r < lq && col0 + lane < lk ? ld_global(mask + (long long)(row0 + r) * lk + col0 + lane) : 0.f;
   }
   __syncwarp();
 }

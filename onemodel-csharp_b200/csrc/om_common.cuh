@@ -137,10 +137,12 @@ static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 // Without the launch attribute both instructions do nothing.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// What follows the wait depends on a value that comes out of it (the grid's width, never zero): the compiler takes loads through
-// `const __restrict__` pointers and __ldg as loads of constants and moves them above the bare instruction, its memory clobber
-// notwithstanding. In a chain of small resident kernels such a load read what was there before the chain (a count written
-// three kernels earlier: stale in 100 of 100 runs, none with the dependence).
+// The memory clobber orders every ordinary access behind the wait. Not so __ldg and loads through pointers marked const __restrict__: they are for data
+// that is constant while the grid runs, which under an overlapped launch it is not (the grid is resident while its predecessor still writes),
+// and the compiler moved one above the wait: in a chain of small kernels a count written three kernels earlier was stale in 100 of 100
+// runs. Kernels that begin with the wait therefore load with ordinary loads (ld_global, unmarked pointers; __restrict__ stays on what is
+// only written). What follows depends on a value that comes out of the wait (the grid's width, never zero) all the same: nothing is to
+// move above it on the grounds of a mark on some pointer.
 __device__ __forceinline__ void pdl_wait() {
   uint32_t grid;
   asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, %%nctaid.x;" : "=r"(grid) :: "memory");
@@ -148,6 +150,10 @@ __device__ __forceinline__ void pdl_wait() {
     asm volatile("exit;");
     __builtin_unreachable();
   }
+}
+template <typename T>
+__device__ __forceinline__ T ld_global(const T* p) {
+  return *p;
 }
 __device__ __forceinline__ void pdl_enter() {
   pdl_trigger();

@@ -28,7 +28,7 @@ __device__ __forceinline__ uint32_t taps_inside(const ConvGeom& g, int y0, int x
 }
 
 __global__ void __launch_bounds__(128)
-conv_fma_fwd_kernel(const ConvGeom g, const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ y) {
+conv_fma_fwd_kernel(const ConvGeom g, const float* x, const float* w, const float* bias, float* __restrict__ y) {
   pdl_enter();
   __shared__ __align__(16) float ws[CF_CHUNK][CF_CH];
   __shared__ int2 ks[CF_CHUNK];        // offset of k in the image, its tap's bit
@@ -59,7 +59,7 @@ conv_fma_fwd_kernel(const ConvGeom g, const float* __restrict__ x, const float* 
     __syncthreads();
     for (int i = threadIdx.x; i < CF_CHUNK * CF_CH; i += 128) {
       const int k = i % CF_CHUNK, c = i / CF_CHUNK;
-      if (k < kn) ws[k][c] = co0 + c < g.cout ? __ldg(w + (long long)(co0 + c) * kk + k0 + k) : 0.f;
+      if (k < kn) ws[k][c] = co0 + c < g.cout ? ld_global(w + (long long)(co0 + c) * kk + k0 + k) : 0.f;
     }
     if (threadIdx.x < kn) {
       const int k = k0 + threadIdx.x, c = k / taps, t = k - c * taps;
@@ -71,7 +71,7 @@ conv_fma_fwd_kernel(const ConvGeom g, const float* __restrict__ x, const float* 
       const int2 e = ks[k];
       float v[CF_PX];
 #pragma unroll
-      for (int j = 0; j < CF_PX; j++) v[j] = (mask[j] & (uint32_t)e.y) ? __ldg(base[j] + e.x) : 0.f;
+      for (int j = 0; j < CF_PX; j++) v[j] = (mask[j] & (uint32_t)e.y) ? ld_global(base[j] + e.x) : 0.f;
 #pragma unroll
       for (int i = 0; i < 8; i += 4) {
         const float4 a = *reinterpret_cast<const float4*>(&ws[k][warp * 8 + i]);
@@ -94,13 +94,13 @@ conv_fma_fwd_kernel(const ConvGeom g, const float* __restrict__ x, const float* 
 #pragma unroll
     for (int i = 0; i < 8; i++) {
       const int co = co0 + warp * 8 + i;
-      if (co < g.cout) out[(long long)i * plane] = bias ? acc[i][j] + __ldg(bias + co) : acc[i][j];
+      if (co < g.cout) out[(long long)i * plane] = bias ? acc[i][j] + ld_global(bias + co) : acc[i][j];
     }
   }
 }
 
 __global__ void __launch_bounds__(128)
-conv_fma_dgrad_kernel(const ConvGeom g, const float* __restrict__ gr, const float* __restrict__ w, float* __restrict__ dx) {
+conv_fma_dgrad_kernel(const ConvGeom g, const float* gr, const float* w, float* __restrict__ dx) {
   pdl_enter();
   __shared__ __align__(16) float ws[CF_CHUNK][CF_CH];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -142,14 +142,14 @@ conv_fma_dgrad_kernel(const ConvGeom g, const float* __restrict__ gr, const floa
       __syncthreads();
       for (int i = threadIdx.x; i < CF_CHUNK * CF_CH; i += 128) {
         const int c = i % CF_CH, k = i / CF_CH;
-        if (k < kn) ws[k][c] = c0 + c < g.cin ? __ldg(w + (long long)(k0 + k) * kk + (c0 + c) * taps + t) : 0.f;
+        if (k < kn) ws[k][c] = c0 + c < g.cin ? ld_global(w + (long long)(k0 + k) * kk + (c0 + c) * taps + t) : 0.f;
       }
       __syncthreads();
 #pragma unroll 4
       for (int k = 0; k < kn; k++) {
         float v[CF_PX];
 #pragma unroll
-        for (int j = 0; j < CF_PX; j++) v[j] = on[j] ? __ldg(src[j] + (long long)(k0 + k) * plane) : 0.f;
+        for (int j = 0; j < CF_PX; j++) v[j] = on[j] ? ld_global(src[j] + (long long)(k0 + k) * plane) : 0.f;
         const float4 a = *reinterpret_cast<const float4*>(&ws[k][warp * 8]), b = *reinterpret_cast<const float4*>(&ws[k][warp * 8 + 4]);
         const float wv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
@@ -181,7 +181,7 @@ conv_fma_dgrad_kernel(const ConvGeom g, const float* __restrict__ gr, const floa
 // operands as rows of pixels, read four pixels at a time (rows of 36 floats: no bank conflicts).
 constexpr int CF_COLS = 128, CF_LD = 36;
 __global__ void __launch_bounds__(128)
-conv_fma_wgrad_kernel(const ConvGeom g, const float* __restrict__ gr, const float* __restrict__ x, int per_slice, float* __restrict__ part) {
+conv_fma_wgrad_kernel(const ConvGeom g, const float* gr, const float* x, int per_slice, float* __restrict__ part) {
   pdl_enter();
   __shared__ __align__(16) float gs[CF_CH][CF_LD];
   __shared__ __align__(16) float xs[CF_COLS][CF_LD];
@@ -216,12 +216,12 @@ conv_fma_wgrad_kernel(const ConvGeom g, const float* __restrict__ gr, const floa
 #pragma unroll
     for (int i = 0; i < CF_CH / 4; i++) {
       const int c = warp + 4 * i;
-      gs[c][lane] = inside && co0 + c < g.cout ? __ldg(gb + (long long)c * plane) : 0.f;
+      gs[c][lane] = inside && co0 + c < g.cout ? ld_global(gb + (long long)c * plane) : 0.f;
     }
 #pragma unroll 8
     for (int k = warp; k < cols; k += 4) {
       const int2 e = ks[k];
-      xs[k][lane] = (mask & (uint32_t)e.y) ? __ldg(xb + e.x) : 0.f;
+      xs[k][lane] = (mask & (uint32_t)e.y) ? ld_global(xb + e.x) : 0.f;
     }
     __syncthreads();
 #pragma unroll
@@ -253,7 +253,7 @@ conv_fma_wgrad_kernel(const ConvGeom g, const float* __restrict__ gr, const floa
 }
 
 // dw (+)= the slices in a fixed order: eight shares of a value's slices, each in increasing order, then the shares.
-__global__ void __launch_bounds__(256) conv_fma_finish_kernel(const float* __restrict__ part, int slices, int len, float* __restrict__ dw, int accumulate) {
+__global__ void __launch_bounds__(256) conv_fma_finish_kernel(const float* part, int slices, int len, float* dw, int accumulate) {
   pdl_enter();
   __shared__ float sums[8][32];
   const int lane = threadIdx.x & 31, share = threadIdx.x >> 5, at = blockIdx.x * 32 + lane;

@@ -115,20 +115,20 @@ __device__ __forceinline__ void cv_stage_rows(float* stg, uint32_t tmem, int war
 }
 
 // Eight channels of one tap for this lane's pixel. o: byte offset of the first (modulo 2^32), step: bytes of a plane.
-__device__ __forceinline__ void cv_load_unit(float* v, const float* __restrict__ src, uint32_t o, uint32_t step, int count) {
+__device__ __forceinline__ void cv_load_unit(float* v, const float* src, uint32_t o, uint32_t step, int count) {
 #pragma unroll
   for (int j = 0; j < CV_UNIT; j++) v[j] = 0.f;
   const char* base = reinterpret_cast<const char*>(src);
   if (count == CV_UNIT) {
 #pragma unroll
     for (int j = 0; j < CV_UNIT; j++) {
-      v[j] = __ldg(reinterpret_cast<const float*>(base + o));
+      v[j] = ld_global(reinterpret_cast<const float*>(base + o));
       o += step;
     }
   } else if (count > 0) {        // the last channels
 #pragma unroll
     for (int j = 0; j < CV_UNIT; j++) {
-      if (j < count) v[j] = __ldg(reinterpret_cast<const float*>(base + o));
+      if (j < count) v[j] = ld_global(reinterpret_cast<const float*>(base + o));
       o += step;
     }
   }
@@ -262,7 +262,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int i = 0; i < 16; i++) {
           const int row = warp * 16 + i, co = m0 + mt * CV_TILE + row;
           if (co >= p.m) break;
-          const float bv = p.bias ? __ldg(p.bias + co) : 0.f;
+          const float bv = p.bias ? ld_global(p.bias + co) : 0.f;
           float* out = p.out + (long long)co * plane;
           const float* sr = stg + row * CV_STG_LD;
           if (p.vec) {
@@ -312,14 +312,14 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
 // The weights in the order of the units, one K-major row per output channel: wt[m][CV_UNIT u + i] is the weight of tap(u) and source channel
 // c0(u) + i, zero past the last channel.
-__global__ void __launch_bounds__(256) conv_turn_weights_kernel(const float* __restrict__ w, float* __restrict__ wt, int channels, int taps, int ld) {
+__global__ void __launch_bounds__(256) conv_turn_weights_kernel(const float* w, float* __restrict__ wt, int channels, int taps, int ld) {
   pdl_enter();
   const int m = blockIdx.y;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ld; i += gridDim.x * blockDim.x) {
     int tap, c0;
     cv_unit<CV_UNIT, CV_GROUP>(i / CV_UNIT, channels, taps, &tap, &c0);
     const int c = c0 + i % CV_UNIT;
-    wt[(long long)m * ld + i] = c < channels ? __ldg(w + ((long long)m * channels + c) * taps + tap) : 0.f;
+    wt[(long long)m * ld + i] = c < channels ? ld_global(w + ((long long)m * channels + c) * taps + tap) : 0.f;
   }
 }
 
@@ -491,7 +491,7 @@ conv_wgrad_tc_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
 // with eight, most of whose threads had nothing to add.
 template <int SHARES, int UNIT, int GROUP>
 __global__ void __launch_bounds__(256)
-conv_wgrad_finish_kernel(const float* __restrict__ part, int splits, int cout, int units, int cin, int taps, float* __restrict__ dw, int accumulate) {
+conv_wgrad_finish_kernel(const float* part, int splits, int cout, int units, int cin, int taps, float* dw, int accumulate) {
   pdl_enter();
   constexpr int COLS = 256 / SHARES;
   __shared__ float sums[SHARES][COLS];
@@ -539,7 +539,7 @@ struct ConvTurn {               // weights addressed by their strides over (m, s
 // 8 m x 32 source channels through shared memory. Read and written in runs (element by element, the reads were 4 bytes a line:
 // 512 x 512 x 3 x 3 took 14 us).
 constexpr int CN_PACK_M = 8;
-__global__ void __launch_bounds__(256) conv_pack_weights_kernel(const float* __restrict__ w, float* __restrict__ wt, const __grid_constant__ ConvTurn t, int taps_all, int phases) {
+__global__ void __launch_bounds__(256) conv_pack_weights_kernel(const float* w, float* __restrict__ wt, const __grid_constant__ ConvTurn t, int taps_all, int phases) {
   pdl_enter();
   extern __shared__ float pack[];       // [8 m][32 channels][taps, to an odd number]
   const int m0 = blockIdx.y * CN_PACK_M, c0 = blockIdx.x * CV_BK, tp = taps_all | 1;
@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(256) conv_pack_weights_kernel(const float* __r
   for (int e = threadIdx.x; e < CN_PACK_M * CV_BK * taps_all; e += 256) {
     const int outer = e / run, rem = e - outer * run, inner = rem / taps_all, tap = rem - inner * taps_all;
     const int m = by_m ? outer : inner, c = by_m ? inner : outer;
-    pack[(m * CV_BK + c) * tp + tap] = m0 + m < t.m && c0 + c < t.sc ? __ldg(w + (m0 + m) * t.stride_m + (c0 + c) * t.stride_sc + tap) : 0.f;
+    pack[(m * CV_BK + c) * tp + tap] = m0 + m < t.m && c0 + c < t.sc ? ld_global(w + (m0 + m) * t.stride_m + (c0 + c) * t.stride_sc + tap) : 0.f;
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -589,7 +589,7 @@ struct ConvNhwcMaps {
 // another pass over the gradient: 118 us a step for the eight layers of the convolutional network).
 constexpr int CN_PX = 64, CN_SUM_CTAS = 512;
 template <bool SUMS>
-__global__ void __launch_bounds__(256) conv_channels_last_kernel(const float* __restrict__ src, float* __restrict__ t, int pixels, int plane, CvDiv div_plane, int c, int cp,
+__global__ void __launch_bounds__(256) conv_channels_last_kernel(const float* src, float* __restrict__ t, int pixels, int plane, CvDiv div_plane, int c, int cp,
                                                                  double* __restrict__ sums) {
   pdl_enter();
   __shared__ float tile[32][CN_PX + 1];
@@ -605,7 +605,7 @@ __global__ void __launch_bounds__(256) conv_channels_last_kernel(const float* __
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const int ch = c0 + row + 8 * j;
-        tile[row + 8 * j][32 * i + lane] = q < pixels && ch < c ? __ldg(base + (long long)ch * plane) : 0.f;
+        tile[row + 8 * j][32 * i + lane] = q < pixels && ch < c ? ld_global(base + (long long)ch * plane) : 0.f;
       }
     }
     __syncthreads();
@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(256) conv_channels_last_kernel(const float* __
   }
 }
 // dbias[co] (+)= the CTAs' sums: eight shares of them in increasing order, then the shares, in double.
-__global__ void __launch_bounds__(256) conv_sums_finish_kernel(const double* __restrict__ sums, int ctas, int c, float* __restrict__ dbias, int accumulate) {
+__global__ void __launch_bounds__(256) conv_sums_finish_kernel(const double* sums, int ctas, int c, float* dbias, int accumulate) {
   pdl_enter();
   __shared__ double part[8][32];
   const int lane = threadIdx.x & 31, share = threadIdx.x >> 5, ch = blockIdx.x * 32 + lane;
@@ -790,7 +790,7 @@ conv_nhwc_kernel(const __grid_constant__ ConvNhwcMaps maps, const __grid_constan
       if (ok && valid) {
 #pragma unroll
         for (int j = 0; j < COLS; j++)
-          if (m0 + col0 + j < p.m) out[(long long)(col0 + j) * p.out_plane] = p.bias ? acc[j] + __ldg(p.bias + m0 + col0 + j) : acc[j];
+          if (m0 + col0 + j < p.m) out[(long long)(col0 + j) * p.out_plane] = p.bias ? acc[j] + ld_global(p.bias + m0 + col0 + j) : acc[j];
       }
     } else {
       const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, p.status, 83));

@@ -27,8 +27,8 @@ __device__ __forceinline__ float keep_factor(unsigned long long stream, int64_t 
 // MODE 0: mask only; 1: y = x * mask (mask also stored when `mask` is not null); 2: backward, dx = g * mask.
 template <int MODE>
 __global__ void __launch_bounds__(256)
-dropout_kernel(const float* __restrict__ x, int64_t n, float p, float scale, unsigned long long seed,
-               const int64_t* __restrict__ draw_src, int64_t* __restrict__ draw_used, float* __restrict__ y,
+dropout_kernel(const float* x, int64_t n, float p, float scale, unsigned long long seed,
+               const int64_t* draw_src, int64_t* __restrict__ draw_used, float* __restrict__ y,
                float* __restrict__ mask) {
   pdl_enter();
   const unsigned long long draw = (unsigned long long)draw_src[0];

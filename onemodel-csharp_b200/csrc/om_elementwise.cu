@@ -27,7 +27,7 @@ __device__ __forceinline__ float binary_apply(int op, float a, float b) {
 }
 
 template <int OP>
-__global__ void binary_same_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out,
+__global__ void binary_same_kernel(const float* a, const float* b, float* out,
                                    int64_t n4, int64_t n) {
   pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -49,7 +49,7 @@ __global__ void binary_same_kernel(const float* __restrict__ a, const float* __r
 // out[r, c] = a[r, c] (op) b[c]: the bias-add pattern; also a b that spans several trailing axes (a position table added to
 // every batch element), the trailing axes then counting as one row of `cols` elements.
 template <int OP>
-__global__ void binary_rowb_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out,
+__global__ void binary_rowb_kernel(const float* a, const float* b, float* out,
                                    int64_t rows, int32_t cols) {
   pdl_enter();
   int64_t total = rows * cols;
@@ -88,8 +88,8 @@ __global__ void binary_rowb_kernel(const float* __restrict__ a, const float* __r
   }
 }
 
-__global__ void binary_strided_kernel(int op, Strided2 s, const float* __restrict__ a, const float* __restrict__ b,
-                                      float* __restrict__ out, int64_t n) {
+__global__ void binary_strided_kernel(int op, Strided2 s, const float* a, const float* b,
+                                      float* out, int64_t n) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t j = i; j < n; j += stride) {
@@ -118,7 +118,7 @@ __device__ __forceinline__ uint16_t bf16_of(float v) {
 
 // y16 (may be null): the bfloat16 copy of y, written in the same pass for the product that reads y next.
 template <int OP>
-__global__ void unary_kernel(const float* __restrict__ x, float* __restrict__ y, uint16_t* __restrict__ y16, int64_t n4, int64_t n) {
+__global__ void unary_kernel(const float* x, float* __restrict__ y, uint16_t* __restrict__ y16, int64_t n4, int64_t n) {
   pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -141,7 +141,7 @@ __global__ void unary_kernel(const float* __restrict__ x, float* __restrict__ y,
 }
 
 template <int OP>
-__global__ void unary_bwd_kernel(const float* __restrict__ g, const float* __restrict__ s, float* __restrict__ dx,
+__global__ void unary_bwd_kernel(const float* g, const float* s, float* __restrict__ dx,
                                  uint16_t* __restrict__ dx16, int64_t n4, int64_t n) {
   pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -165,7 +165,7 @@ __global__ void unary_bwd_kernel(const float* __restrict__ g, const float* __res
   }
 }
 
-__global__ void add_into_kernel(float* dst, const float* __restrict__ src, int64_t n4, int64_t n) {
+__global__ void add_into_kernel(float* dst, const float* src, int64_t n4, int64_t n) {
   pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -179,14 +179,14 @@ __global__ void add_into_kernel(float* dst, const float* __restrict__ src, int64
   for (int64_t j = n4 * 4 + i; j < n; j += stride) dst[j] += src[j];
 }
 
-__global__ void div_scalar_kernel(const float* __restrict__ x, float d, float* __restrict__ y, int64_t n) {
+__global__ void div_scalar_kernel(const float* x, float d, float* __restrict__ y, int64_t n) {
   pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t j = i; j < n; j += stride) y[j] = x[j] / d;
 }
 
-__global__ void fill_kernel(float* __restrict__ dst, float v, int64_t n) {
+__global__ void fill_kernel(float* dst, float v, int64_t n) {
   pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -220,7 +220,7 @@ __global__ void multi_zero_kernel(ZeroTable t) {
 
 // ---- strided copy -------------------------------------------------------------------------------------------------
 
-__global__ void strided_copy_kernel(Strided2 s, const float* __restrict__ src, float* __restrict__ dst, int64_t n) {
+__global__ void strided_copy_kernel(Strided2 s, const float* src, float* dst, int64_t n) {
   pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -238,7 +238,7 @@ __global__ void strided_copy_kernel(Strided2 s, const float* __restrict__ src, f
 
 // Same with the innermost axis contiguous on both sides and a multiple of 4 elements, 16-byte aligned: one float4
 // per thread-iteration.
-__global__ void strided_copy_vec4_kernel(Strided2 s, const float* __restrict__ src, float* __restrict__ dst,
+__global__ void strided_copy_vec4_kernel(Strided2 s, const float* src, float* dst,
                                          int64_t n4) {
   pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -259,7 +259,7 @@ __global__ void strided_copy_vec4_kernel(Strided2 s, const float* __restrict__ s
 }
 
 // 2-D transpose through a padded shared tile: dst[c, r] = src[r, c].
-__global__ void transpose2d_kernel(const float* __restrict__ src, float* __restrict__ dst, int32_t rows, int32_t cols,
+__global__ void transpose2d_kernel(const float* src, float* dst, int32_t rows, int32_t cols,
                                    int64_t src_ld, int64_t dst_ld) {
   pdl_enter();
   __shared__ float tile[32][33];
@@ -285,7 +285,7 @@ constexpr int kColsumLanes = 32;
 // adds them in increasing chunk order, exactly as colsum_stage2_kernel does, and resets the arrival counter for the next
 // launch. Which CTA arrives last does not matter for the result. `tid` is the thread's linear index in the CTA.
 template <int COLS = 32>
-__device__ __forceinline__ void colsum_finish(const double* __restrict__ partial, unsigned* __restrict__ arrival, float* __restrict__ out,
+__device__ __forceinline__ void colsum_finish(const double* partial, unsigned* arrival, float* out,
                                               int accumulate, int32_t cols, int tid, int* is_last) {
   __syncthreads();
   if (tid == 0) *is_last = atomicAdd(&arrival[blockIdx.x], 1u) == gridDim.y - 1;
@@ -317,8 +317,8 @@ __device__ __forceinline__ void colsum_finish(const double* __restrict__ partial
 // 32 row-lanes per column accumulate in double over rows lane, lane+32, ...; the 32 lane sums are combined in lane
 // order. partial[chunk, col] is written in double.
 __global__ void __launch_bounds__(1024)
-colsum_stage1_kernel(const float* __restrict__ g, int32_t rows, int32_t cols, int64_t ld, double* __restrict__ partial,
-                     unsigned* __restrict__ arrival, float* __restrict__ out, int accumulate) {
+colsum_stage1_kernel(const float* g, int32_t rows, int32_t cols, int64_t ld, double* partial,
+                     unsigned* arrival, float* out, int accumulate) {
   pdl_enter();
   __shared__ double sm[kColsumLanes][33];
   __shared__ int is_last;
@@ -345,8 +345,8 @@ colsum_stage1_kernel(const float* __restrict__ g, int32_t rows, int32_t cols, in
 // colsum_stage1_kernel, but each thread owns four adjacent columns (one 16-byte load per row) and has all of its 16
 // rows in flight at once. A CTA is 8 column groups x 32 row lanes and covers 32 columns of one chunk.
 __global__ void __launch_bounds__(256)
-colsum_stage1_vec4_kernel(const float* __restrict__ g, int32_t rows, int32_t cols, int64_t ld, double* __restrict__ partial,
-                          unsigned* __restrict__ arrival, float* __restrict__ out, int accumulate) {
+colsum_stage1_vec4_kernel(const float* g, int32_t rows, int32_t cols, int64_t ld, double* partial,
+                          unsigned* arrival, float* out, int accumulate) {
   pdl_enter();
   __shared__ double sm[kColsumLanes][33];
   __shared__ int is_last;
@@ -361,7 +361,7 @@ colsum_stage1_vec4_kernel(const float* __restrict__ g, int32_t rows, int32_t col
 #pragma unroll
     for (int u = 0; u < PER_LANE; u++) {
       const int r = r0 + ty + kColsumLanes * u;
-      v[u] = r < r1 ? __ldg(reinterpret_cast<const float4*>(g + (int64_t)r * ld + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[u] = r < r1 ? ld_global(reinterpret_cast<const float4*>(g + (int64_t)r * ld + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
     for (int u = 0; u < PER_LANE; u++) {
@@ -406,8 +406,8 @@ __device__ __forceinline__ void add_bf16x8(float (&a)[8], const uint4& v) {
   }
 }
 __global__ void __launch_bounds__(256, 3)
-colsum16_stage1_kernel(const uint16_t* __restrict__ g, int32_t rows, int32_t cols, int64_t ld, double* __restrict__ partial,
-                       unsigned* __restrict__ arrival, float* __restrict__ out, int accumulate) {
+colsum16_stage1_kernel(const uint16_t* g, int32_t rows, int32_t cols, int64_t ld, double* partial,
+                       unsigned* arrival, float* out, int accumulate) {
   pdl_enter();
   __shared__ float sm[kColsumLanes][65];
   __shared__ int is_last;
@@ -424,7 +424,7 @@ colsum16_stage1_kernel(const uint16_t* __restrict__ g, int32_t rows, int32_t col
 #pragma unroll
     for (int u = 0; u < PER_LANE; u++) {
       const int r = r0 + ty + kColsumLanes * u;
-      v[u] = r < r1 ? __ldg(reinterpret_cast<const uint4*>(g + (int64_t)r * ld + col)) : make_uint4(0u, 0u, 0u, 0u);
+      v[u] = r < r1 ? ld_global(reinterpret_cast<const uint4*>(g + (int64_t)r * ld + col)) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int u = 0; u < PER_LANE; u++)
@@ -449,8 +449,8 @@ colsum16_stage1_kernel(const uint16_t* __restrict__ g, int32_t rows, int32_t col
   if (arrival != nullptr) colsum_finish<64>(partial, arrival, out, accumulate, cols, threadIdx.x, &is_last);
 }
 
-__global__ void colsum_stage2_kernel(const double* __restrict__ partial, int32_t chunks, int32_t cols,
-                                     float* __restrict__ out, int accumulate) {
+__global__ void colsum_stage2_kernel(const double* partial, int32_t chunks, int32_t cols,
+                                     float* out, int accumulate) {
   pdl_enter();
   int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= cols) return;
@@ -462,7 +462,7 @@ __global__ void colsum_stage2_kernel(const double* __restrict__ partial, int32_t
 
 // Row sums: out[r] = sum_c g[r, c]; one warp per row, lanes stride the row, lane sums combined by a fixed
 // butterfly (xor shuffle) so every lane ends with the same bits.
-__global__ void rowsum_kernel(const float* __restrict__ g, int64_t rows, int32_t cols, float* __restrict__ out) {
+__global__ void rowsum_kernel(const float* g, int64_t rows, int32_t cols, float* out) {
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int lane = threadIdx.x & 31;
   int warps = (gridDim.x * blockDim.x) >> 5;
@@ -484,7 +484,7 @@ struct SumToShape {
 
 // Generic fallback: one thread per output element walks every source element that maps to it in increasing source
 // order (the reference's order) with a double accumulator.
-__global__ void sum_to_generic_kernel(SumToShape s, const float* __restrict__ g, float* __restrict__ out,
+__global__ void sum_to_generic_kernel(SumToShape s, const float* g, float* out,
                                       int64_t out_len) {
   int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (o >= out_len) return;
@@ -519,7 +519,7 @@ __global__ void sum_to_generic_kernel(SumToShape s, const float* __restrict__ g,
 }
 
 // Sum/Mean over the middle axis of [outer, n, inner] with a double accumulator in increasing order.
-__global__ void reduce_fwd_kernel(const float* __restrict__ x, int64_t outer, int64_t n, int64_t inner, int mean,
+__global__ void reduce_fwd_kernel(const float* x, int64_t outer, int64_t n, int64_t inner, int mean,
                                   float* __restrict__ y) {
   pdl_enter();
   int64_t total = outer * inner;
@@ -534,7 +534,7 @@ __global__ void reduce_fwd_kernel(const float* __restrict__ x, int64_t outer, in
 }
 
 // Whole-tensor sum with one CTA (used for rank-0 results): fixed partition over 1024 threads, fixed tree.
-__global__ void reduce_all_kernel(const float* __restrict__ x, int64_t n, int mean, float* __restrict__ y) {
+__global__ void reduce_all_kernel(const float* x, int64_t n, int mean, float* __restrict__ y) {
   __shared__ double sm[1024];
   double acc = 0.0;
   for (int64_t j = threadIdx.x; j < n; j += 1024) acc += (double)x[j];
@@ -547,7 +547,7 @@ __global__ void reduce_all_kernel(const float* __restrict__ x, int64_t n, int me
   if (threadIdx.x == 0) y[0] = mean ? (float)(sm[0] / (double)n) : (float)sm[0];
 }
 
-__global__ void reduce_bwd_kernel(const float* __restrict__ g, int64_t outer, int64_t n, int64_t inner, int mean,
+__global__ void reduce_bwd_kernel(const float* g, int64_t outer, int64_t n, int64_t inner, int mean,
                                   float* __restrict__ dx) {
   pdl_enter();
   int64_t total = outer * n * inner;

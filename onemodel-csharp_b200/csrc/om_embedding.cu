@@ -17,7 +17,7 @@ __device__ __forceinline__ void report_index(int32_t* status, int32_t detail) {
   if (atomicCAS(status, 0, (int32_t)OM_ERR_INDEX) == 0) status[1] = detail;
 }
 
-__global__ void embedding_fwd_kernel(const float* __restrict__ table, int32_t v, int32_t dim, const void* __restrict__ ids,
+__global__ void embedding_fwd_kernel(const float* table, int32_t v, int32_t dim, const void* ids,
                                      int dtype, int64_t n, float* __restrict__ out, int32_t* status) {
   pdl_enter();
   int lane = threadIdx.x & 31;
@@ -43,8 +43,8 @@ __global__ void embedding_fwd_kernel(const float* __restrict__ table, int32_t v,
   }
 }
 
-__global__ void embedding_count_kernel(const void* __restrict__ ids, int dtype, int64_t n, int32_t v, int64_t pad,
-                                       int32_t* __restrict__ count, int32_t* status) {
+__global__ void embedding_count_kernel(const void* ids, int dtype, int64_t n, int32_t v, int64_t pad,
+                                       int32_t* count, int32_t* status) {
   pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -60,7 +60,7 @@ __global__ void embedding_count_kernel(const void* __restrict__ ids, int dtype, 
 }
 
 // Exclusive prefix sum of count[0..v) by one CTA of 1024 threads (each thread scans a contiguous span).
-__global__ void embedding_scan_kernel(const int32_t* __restrict__ count, int32_t v, int32_t* __restrict__ offset) {
+__global__ void embedding_scan_kernel(const int32_t* count, int32_t v, int32_t* offset) {
   pdl_enter();
   __shared__ int32_t totals[1024];
   int span = (v + 1023) / 1024;
@@ -83,8 +83,8 @@ __global__ void embedding_scan_kernel(const int32_t* __restrict__ count, int32_t
   }
 }
 
-__global__ void embedding_fill_kernel(const void* __restrict__ ids, int dtype, int64_t n, int32_t v, int64_t pad,
-                                      const int32_t* __restrict__ offset, int32_t* __restrict__ cursor,
+__global__ void embedding_fill_kernel(const void* ids, int dtype, int64_t n, int32_t v, int64_t pad,
+                                      const int32_t* offset, int32_t* cursor,
                                       int32_t* __restrict__ bucket) {
   pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -99,10 +99,10 @@ __global__ void embedding_fill_kernel(const void* __restrict__ ids, int dtype, i
 
 // One warp per table row: order the row's bucket by position (rank = number of smaller entries; positions are unique),
 // then add g rows in that order.
-__global__ void embedding_bwd_rows_kernel(const float* __restrict__ g, int32_t v, int32_t dim,
-                                          const int32_t* __restrict__ count, const int32_t* __restrict__ offset,
-                                          const int32_t* __restrict__ bucket, int32_t* __restrict__ sorted,
-                                          float* __restrict__ dtable, int accumulate) {
+__global__ void embedding_bwd_rows_kernel(const float* g, int32_t v, int32_t dim,
+                                          const int32_t* count, const int32_t* offset,
+                                          const int32_t* bucket, int32_t* sorted,
+                                          float* dtable, int accumulate) {
   pdl_enter();
   int lane = threadIdx.x & 31;
   int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -163,7 +163,7 @@ __global__ void embedding_bwd_rows_kernel(const float* __restrict__ g, int32_t v
 // normed as a plain [capacity, width] tensor.
 
 // slot[i] = number of rows below i with flag[i] != 0 (the position of row i among the touched rows); *total = their count.
-__global__ void rowsparse_slot_scan_kernel(const int32_t* __restrict__ flag, int32_t v, int32_t* __restrict__ slot, int32_t* __restrict__ total) {
+__global__ void rowsparse_slot_scan_kernel(const int32_t* flag, int32_t v, int32_t* slot, int32_t* __restrict__ total) {
   pdl_enter();
   __shared__ int32_t totals[1024];
   int span = (v + 1023) / 1024;
@@ -187,10 +187,10 @@ __global__ void rowsparse_slot_scan_kernel(const int32_t* __restrict__ flag, int
 }
 
 // One warp per table row that was looked up: its bucket put into position order, its sum written to values[slot[row]].
-__global__ void embedding_bwd_sparse_rows_kernel(const float* __restrict__ g, int32_t v, int32_t dim, const int32_t* __restrict__ count,
-                                                 const int32_t* __restrict__ offset, const int32_t* __restrict__ bucket,
-                                                 int32_t* __restrict__ sorted, const int32_t* __restrict__ slot,
-                                                 int32_t* __restrict__ rows_out, float* __restrict__ values) {
+__global__ void embedding_bwd_sparse_rows_kernel(const float* g, int32_t v, int32_t dim, const int32_t* count,
+                                                 const int32_t* offset, const int32_t* bucket,
+                                                 int32_t* sorted, const int32_t* slot,
+                                                 int32_t* __restrict__ rows_out, float* values) {
   pdl_enter();
   int lane = threadIdx.x & 31;
   int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -220,7 +220,7 @@ __global__ void embedding_bwd_sparse_rows_kernel(const float* __restrict__ g, in
 }
 
 // Entries behind the row count: row -1, zero values.
-__global__ void rowsparse_tail_kernel(int32_t* __restrict__ rows, float* __restrict__ values, const int32_t* __restrict__ row_count,
+__global__ void rowsparse_tail_kernel(int32_t* rows, float* values, const int32_t* row_count,
                                       int32_t capacity, int32_t dim) {
   pdl_enter();
   int lane = threadIdx.x & 31;
@@ -234,8 +234,8 @@ __global__ void rowsparse_tail_kernel(int32_t* __restrict__ rows, float* __restr
 }
 
 // dense[rows[k]] += values[k] (RowSparseGradient.AddTo): the rows are distinct, so no two warps meet.
-__global__ void rowsparse_add_to_kernel(const int32_t* __restrict__ rows, const float* __restrict__ values, const int32_t* __restrict__ row_count,
-                                        int32_t capacity, int32_t dim, float* __restrict__ dense, int32_t v, int32_t* status) {
+__global__ void rowsparse_add_to_kernel(const int32_t* rows, const float* values, const int32_t* row_count,
+                                        int32_t capacity, int32_t dim, float* dense, int32_t v, int32_t* status) {
   pdl_enter();
   int lane = threadIdx.x & 31;
   int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -254,7 +254,7 @@ __global__ void rowsparse_add_to_kernel(const int32_t* __restrict__ rows, const 
 }
 
 // Merge, step one: where[row] = k + 1 for the k-th entry of a list, present[row] = 1.
-__global__ void rowsparse_mark_kernel(const int32_t* __restrict__ rows, const int32_t* __restrict__ row_count, int32_t capacity, int32_t v,
+__global__ void rowsparse_mark_kernel(const int32_t* rows, const int32_t* row_count, int32_t capacity, int32_t v,
                                       int32_t* __restrict__ where, int32_t* __restrict__ present, int32_t* status) {
   pdl_enter();
   const int n = min(*row_count, capacity);
@@ -270,10 +270,10 @@ __global__ void rowsparse_mark_kernel(const int32_t* __restrict__ rows, const in
 }
 
 // Merge, step two: one warp per table row in either list; a's values (or zero), then b's added (RowSparseGradient.Merge: a first).
-__global__ void rowsparse_merge_rows_kernel(const int32_t* __restrict__ where_a, const float* __restrict__ values_a,
-                                            const int32_t* __restrict__ where_b, const float* __restrict__ values_b,
-                                            const int32_t* __restrict__ present, const int32_t* __restrict__ slot, int32_t v, int32_t dim,
-                                            int32_t* __restrict__ rows_out, float* __restrict__ values_out) {
+__global__ void rowsparse_merge_rows_kernel(const int32_t* where_a, const float* values_a,
+                                            const int32_t* where_b, const float* values_b,
+                                            const int32_t* present, const int32_t* slot, int32_t v, int32_t dim,
+                                            int32_t* __restrict__ rows_out, float* values_out) {
   pdl_enter();
   int lane = threadIdx.x & 31;
   int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;

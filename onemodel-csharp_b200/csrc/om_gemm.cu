@@ -20,7 +20,7 @@ bool gemm_tc_batched_supported(om_ctx* ctx, int ta, int tb, int m, int n, int k,
 int32_t gemm_tc_batched(om_ctx* ctx, int ta, int tb, int m, int n, int k, const float* A, int lda, long long sA, const float* B,
                         int ldb, long long sB, float* C, int ldc, long long sC, int batch, int acc, const float* bias);
 
-__global__ void add_bias_rows_kernel(float* __restrict__ y, const float* __restrict__ bias, int64_t rows, int32_t cols, int64_t ld) {
+__global__ void add_bias_rows_kernel(float* y, const float* bias, int64_t rows, int32_t cols, int64_t ld) {
   pdl_enter();
   int64_t total = rows * cols;
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;

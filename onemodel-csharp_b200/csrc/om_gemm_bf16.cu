@@ -19,13 +19,13 @@ int32_t colsum_ld(om_ctx* ctx, const float* g, int32_t rows, int32_t cols, int64
 int32_t colsum16_ld(om_ctx* ctx, const uint16_t* g16, int32_t rows, int32_t cols, int64_t ld, float* out, int32_t accumulate);
 
 // Eight elements per thread: two 16-byte loads, one 16-byte store.
-__global__ void cast_bf16_kernel(const float* __restrict__ src, uint16_t* __restrict__ dst, int64_t n) {
+__global__ void cast_bf16_kernel(const float* src, uint16_t* __restrict__ dst, int64_t n) {
   pdl_enter();
   const int64_t n8 = n >> 3;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n8; i += stride) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(src) + 2 * i);
-    const float4 b = __ldg(reinterpret_cast<const float4*>(src) + 2 * i + 1);
+    const float4 a = ld_global(reinterpret_cast<const float4*>(src) + 2 * i);
+    const float4 b = ld_global(reinterpret_cast<const float4*>(src) + 2 * i + 1);
     __nv_bfloat162 p0 = __floats2bfloat162_rn(a.x, a.y), p1 = __floats2bfloat162_rn(a.z, a.w);
     __nv_bfloat162 p2 = __floats2bfloat162_rn(b.x, b.y), p3 = __floats2bfloat162_rn(b.z, b.w);
     uint4 o;

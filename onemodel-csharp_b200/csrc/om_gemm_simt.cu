@@ -9,8 +9,8 @@ namespace om {
 
 template <int BM, int BN, int BK, int TM, int TN, bool TA, bool TB>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
-gemm_simt_kernel(int m, int n, int k, const float* __restrict__ A, int lda, int64_t strideA,
-                 const float* __restrict__ B, int ldb, int64_t strideB, float* __restrict__ C, int ldc,
+gemm_simt_kernel(int m, int n, int k, const float* A, int lda, int64_t strideA,
+                 const float* B, int ldb, int64_t strideB, float* C, int ldc,
                  int64_t strideC, int accumulate, int batch, int batch_per_z, int inner, int64_t innerA, int64_t innerB,
                  int64_t innerC) {
   pdl_enter();
@@ -127,9 +127,9 @@ constexpr int64_t kSmallOutputs = (int64_t)4 * 148 * kSmallTile * kSmallTile;
 
 template <bool TA, bool TB>
 __global__ void __launch_bounds__(kSmallTile * kSmallTile)
-gemm_small_kernel(int m, int n, int k, const float* __restrict__ A, int lda, int64_t strideA, const float* __restrict__ B, int ldb,
-                  int64_t strideB, float* __restrict__ C, int ldc, int64_t strideC, int accumulate, int inner, int64_t innerA,
-                  int64_t innerB, int64_t innerC, const float* __restrict__ bias) {
+gemm_small_kernel(int m, int n, int k, const float* A, int lda, int64_t strideA, const float* B, int ldb,
+                  int64_t strideB, float* C, int ldc, int64_t strideC, int accumulate, int inner, int64_t innerA,
+                  int64_t innerB, int64_t innerC, const float* bias) {
   pdl_enter();
   __shared__ __align__(16) float As[kSmallTile][kSmallK + 4];
   __shared__ __align__(16) float Bs[kSmallTile][kSmallK + 4];
@@ -148,8 +148,8 @@ gemm_small_kernel(int m, int n, int k, const float* __restrict__ A, int lda, int
       // consecutive threads walk the index that is contiguous in memory
       const int am = m0 + (TA ? e % kSmallTile : e / kSmallK), ak = k0 + (TA ? e / kSmallTile : e % kSmallK);
       const int bn = n0 + (TB ? e / kSmallK : e % kSmallTile), bk = k0 + (TB ? e % kSmallK : e / kSmallTile);
-      ra[i] = am < m && ak < k ? __ldg(A + (TA ? (int64_t)ak * lda + am : (int64_t)am * lda + ak)) : 0.f;
-      rb[i] = bn < n && bk < k ? __ldg(B + (TB ? (int64_t)bn * ldb + bk : (int64_t)bk * ldb + bn)) : 0.f;
+      ra[i] = am < m && ak < k ? ld_global(A + (TA ? (int64_t)ak * lda + am : (int64_t)am * lda + ak)) : 0.f;
+      rb[i] = bn < n && bk < k ? ld_global(B + (TB ? (int64_t)bn * ldb + bk : (int64_t)bk * ldb + bn)) : 0.f;
     }
   };
   float acc = 0.f;
@@ -183,7 +183,7 @@ gemm_small_kernel(int m, int n, int k, const float* __restrict__ A, int lda, int
   if (gm < m && gn < n) {
     float* c = C + (int64_t)gm * ldc + gn;
     float v = accumulate ? *c + acc : acc;
-    if (bias) v += __ldg(bias + gn);
+    if (bias) v += ld_global(bias + gn);
     *c = v;
   }
 }

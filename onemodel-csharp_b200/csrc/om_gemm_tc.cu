@@ -278,8 +278,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
 // out = (accumulate ? out : 0) + part[0] + part[1] + ... in increasing split order.
 // The split sums are formed first, then bias and the previous contents are added, as the unsplit epilogue does.
-__global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits, int64_t mn, int n, int64_t ldc,
-                                     const float* __restrict__ bias, float* __restrict__ out, int accumulate) {
+__global__ void splitk_reduce_kernel(const float* part, int splits, int64_t mn, int n, int64_t ldc,
+                                     const float* bias, float* out, int accumulate) {
   pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;

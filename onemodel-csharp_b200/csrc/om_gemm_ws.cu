@@ -305,7 +305,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int64_t at = (int64_t)(in ? row : 0) * p.ld_aux + (in ? c0 : 0);
         const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const char*>(p.aux) + at * (ACT == 4 ? 2 : 4));
 #pragma unroll
-        for (int c4 = 0; c4 < AUXN; c4++) dst[c4] = (in && c0 + AUX_PER * c4 < p.n) ? __ldg(src + c4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int c4 = 0; c4 < AUXN; c4++) dst[c4] = (in && c0 + AUX_PER * c4 < p.n) ? ld_global(src + c4) : make_float4(0.f, 0.f, 0.f, 0.f);
       };
       if (AHEAD) load_aux(aux, part * CB_PER);
       ok = mbar_wait(&acc_full[a], use & 1, abort_flag, p.status, 44);

@@ -55,7 +55,7 @@ enum RowOp { SOFTMAX_FWD, LOGSOFTMAX_FWD, SOFTMAX_BWD, LOGSOFTMAX_BWD };
 // a = x (fwd) or g (bwd); b = y (bwd only).
 template <int G, int OP>
 __global__ void __launch_bounds__(kRowThreads)
-row_kernel(const float* __restrict__ a, const float* __restrict__ b, int32_t rows, int32_t cols, int64_t ld, float* __restrict__ out) {
+row_kernel(const float* a, const float* b, int32_t rows, int32_t cols, int64_t ld, float* __restrict__ out) {
   pdl_enter();
   __shared__ double sm[kRowThreads / 32];
   const int lane = G == 32 ? (threadIdx.x & 31) : threadIdx.x;
@@ -100,7 +100,7 @@ row_kernel(const float* __restrict__ a, const float* __restrict__ b, int32_t row
 constexpr int kWideThreads = 1024;
 template <int NV>
 __global__ void __launch_bounds__(kWideThreads)
-logsoftmax_wide_kernel(const float* __restrict__ a, int32_t rows, int32_t cols, int64_t ld, float* __restrict__ out) {
+logsoftmax_wide_kernel(const float* a, int32_t rows, int32_t cols, int64_t ld, float* __restrict__ out) {
   pdl_enter();
   __shared__ double sm[kWideThreads / 32];
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -111,7 +111,7 @@ logsoftmax_wide_kernel(const float* __restrict__ a, int32_t rows, int32_t cols, 
     for (int i = 0; i < NV; i++) {
       const int j = 4 * (i * kWideThreads + (int)threadIdx.x);
       v[i] = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
-      if (j + 3 < cols) v[i] = __ldg(reinterpret_cast<const float4*>(ar + j));
+      if (j + 3 < cols) v[i] = ld_global(reinterpret_cast<const float4*>(ar + j));
       else if (j < cols) {
         v[i].x = ar[j];
         if (j + 1 < cols) v[i].y = ar[j + 1];
@@ -180,7 +180,7 @@ __device__ __forceinline__ void report(int32_t* status, int32_t code, int32_t de
 }
 
 // One CTA of 1024 threads: loss = -(sum of logp[i, t_i]) over counted rows (double, fixed tree), count of counted rows.
-__global__ void nll_fwd_kernel(const float* __restrict__ logp, const void* __restrict__ targets, int dtype, int32_t rows,
+__global__ void nll_fwd_kernel(const float* logp, const void* targets, int dtype, int32_t rows,
                                int32_t cols, int64_t ld, int mean, int64_t ignore, float denominator, float* __restrict__ loss,
                                int32_t* __restrict__ count_out, int32_t* status) {
   pdl_enter();
@@ -216,7 +216,7 @@ __global__ void nll_fwd_kernel(const float* __restrict__ logp, const void* __res
   }
 }
 
-__global__ void count_targets_kernel(const void* __restrict__ targets, int dtype, int32_t rows, int64_t ignore,
+__global__ void count_targets_kernel(const void* targets, int dtype, int32_t rows, int64_t ignore,
                                      int32_t* __restrict__ count_out) {
   pdl_enter();
   __shared__ int scount[1024];
@@ -231,7 +231,7 @@ __global__ void count_targets_kernel(const void* __restrict__ targets, int dtype
   if (threadIdx.x == 0) count_out[0] = scount[0];
 }
 
-__global__ void target_mask_kernel(const void* __restrict__ targets, int dtype, int32_t rows, int64_t ignore, float* __restrict__ mask) {
+__global__ void target_mask_kernel(const void* targets, int dtype, int32_t rows, int64_t ignore, float* __restrict__ mask) {
   pdl_enter();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x)
     mask[i] = target_at(targets, dtype, i) != ignore ? 1.f : 0.f;
@@ -244,8 +244,8 @@ __device__ __forceinline__ float nll_scale(const float* g, int mean, const int32
   return gv / div;
 }
 
-__global__ void nll_bwd_kernel(const float* __restrict__ g, const void* __restrict__ targets, int dtype, int32_t rows,
-                               int32_t cols, int mean, int64_t ignore, const int32_t* __restrict__ count,
+__global__ void nll_bwd_kernel(const float* g, const void* targets, int dtype, int32_t rows,
+                               int32_t cols, int mean, int64_t ignore, const int32_t* count,
                                float* __restrict__ dx) {
   float scale = nll_scale(g, mean, count, 0.f);
   int64_t total = (int64_t)rows * cols;
@@ -264,9 +264,9 @@ __global__ void nll_bwd_kernel(const float* __restrict__ g, const void* __restri
 // with 4-byte accesses: 121 us for 600 MB).
 template <bool VEC>
 __global__ void __launch_bounds__(kRowThreads)
-cross_entropy_bwd_kernel(const float* __restrict__ g, const float* __restrict__ logp, const void* __restrict__ targets,
+cross_entropy_bwd_kernel(const float* g, const float* logp, const void* targets,
                          int dtype, int32_t rows, int32_t cols, int64_t ld, int mean, int64_t ignore, float denominator,
-                         const int32_t* __restrict__ count, float* __restrict__ dx) {
+                         const int32_t* count, float* __restrict__ dx) {
   pdl_enter();
   float scale = nll_scale(g, mean, count, denominator);
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -278,7 +278,7 @@ cross_entropy_bwd_kernel(const float* __restrict__ g, const float* __restrict__ 
     int j = threadIdx.x;
     if (VEC) {
       for (int q = 4 * threadIdx.x; q + 3 < cols; q += 4 * kRowThreads) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(y + q));
+        const float4 v = ld_global(reinterpret_cast<const float4*>(y + q));
         float4 o;
         o.x = ((counted && q == t) ? -scale : 0.f) - (expf(v.x) * s);
         o.y = ((counted && q + 1 == t) ? -scale : 0.f) - (expf(v.y) * s);

@@ -23,7 +23,7 @@ __device__ __forceinline__ float wsum_f(float v) {
 
 // ---- layer norm forward: one warp per row -------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-layernorm_fwd_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
+layernorm_fwd_kernel(const float* x, const float* gamma, const float* beta,
                      int32_t rows, int32_t cols, float eps, float* __restrict__ y, float* __restrict__ mean_out,
                      float* __restrict__ inv_out) {
   pdl_enter();
@@ -56,8 +56,8 @@ layernorm_fwd_kernel(const float* __restrict__ x, const float* __restrict__ gamm
 // the kernel is a chain of memory round trips and nothing else), then the lane sums are added in lane order: a fixed
 // order, so the result does not depend on the launch.
 __global__ void __launch_bounds__(1024)
-column_partials_finish_kernel(const double* __restrict__ pa, const double* __restrict__ pb, int chunks, int32_t cols,
-                              float* __restrict__ oa, float* __restrict__ ob, int accumulate) {
+column_partials_finish_kernel(const double* pa, const double* pb, int chunks, int32_t cols,
+                              float* oa, float* ob, int accumulate) {
   pdl_enter();
   __shared__ double sa[32][33], sb[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -111,8 +111,8 @@ __device__ __forceinline__ uint16_t bf16_bits(float v) {
 
 template <int NC>
 __global__ void __launch_bounds__(256)
-layernorm_fwd_reg_kernel(const float* __restrict__ x, const float* __restrict__ addend, float* __restrict__ sum_out,
-                         const float* __restrict__ gamma, const float* __restrict__ beta, int32_t rows, int32_t cols, float eps,
+layernorm_fwd_reg_kernel(const float* x, const float* addend, float* __restrict__ sum_out,
+                         const float* gamma, const float* beta, int32_t rows, int32_t cols, float eps,
                          float* __restrict__ y, uint16_t* __restrict__ y16, float* __restrict__ mean_out, float* __restrict__ inv_out) {
   pdl_enter();
   const int lane = threadIdx.x & 31;
@@ -184,8 +184,8 @@ layernorm_fwd_reg_kernel(const float* __restrict__ x, const float* __restrict__ 
 constexpr int kLnFusedRows = 64;
 template <int NC>
 __global__ void __launch_bounds__(256, 2)
-layernorm_bwd_fused_kernel(const float* __restrict__ g, const float* __restrict__ x, const float* __restrict__ gamma,
-                           const float* __restrict__ mean, const float* __restrict__ inv, int32_t rows, int32_t cols,
+layernorm_bwd_fused_kernel(const float* g, const float* x, const float* gamma,
+                           const float* mean, const float* inv, int32_t rows, int32_t cols,
                            float* __restrict__ dx, uint16_t* __restrict__ dx16, double* __restrict__ part_gamma,
                            double* __restrict__ part_beta) {
   pdl_enter();
@@ -211,7 +211,7 @@ layernorm_bwd_fused_kernel(const float* __restrict__ g, const float* __restrict_
       const float gv = in ? gr[j] : 0.f;
       const float xv = in ? xr[j] : m;
       xh[i] = (xv - m) * s;
-      dh[i] = gv * (in ? __ldg(gamma + j) : 0.f);   // gamma stays in L1: keeping it in registers would not fit two CTAs per SM
+      dh[i] = gv * (in ? ld_global(gamma + j) : 0.f);   // gamma stays in L1: keeping it in registers would not fit two CTAs per SM
       ag[i] += gv * xh[i];
       ab[i] += gv;
     }
@@ -272,8 +272,8 @@ __device__ __forceinline__ uint2 bf16x4_bits(float4 v) {
 
 template <int NV>
 __global__ void __launch_bounds__(256)
-layernorm_fwd_vec_kernel(const float* __restrict__ x, const float* __restrict__ addend, float* __restrict__ sum_out,
-                         const float* __restrict__ gamma, const float* __restrict__ beta, int32_t rows, int32_t cols, float eps,
+layernorm_fwd_vec_kernel(const float* x, const float* addend, float* __restrict__ sum_out,
+                         const float* gamma, const float* beta, int32_t rows, int32_t cols, float eps,
                          float* __restrict__ y, uint16_t* __restrict__ y16, float* __restrict__ mean_out, float* __restrict__ inv_out) {
   pdl_enter();
   const int lane = threadIdx.x & 31;
@@ -284,8 +284,8 @@ layernorm_fwd_vec_kernel(const float* __restrict__ x, const float* __restrict__ 
 #pragma unroll
   for (int i = 0; i < NV; i++) {
     const int j = lane + 32 * i;
-    gam[i] = j < nv ? __ldg(reinterpret_cast<const float4*>(gamma) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-    bet[i] = j < nv ? __ldg(reinterpret_cast<const float4*>(beta) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    gam[i] = j < nv ? ld_global(reinterpret_cast<const float4*>(gamma) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    bet[i] = j < nv ? ld_global(reinterpret_cast<const float4*>(beta) + j) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   for (int64_t r = warp; r < rows; r += warps) {
     const float4* xr = reinterpret_cast<const float4*>(x + r * cols);
@@ -353,8 +353,8 @@ constexpr int kLnVecRows = 56;
 static int ln_cta_rows(int rows) { return std::min<int>(kLnVecRows, 8 * (int)ceil_div(std::max(rows, 1), 8 * 296)); }
 template <int NV>
 __global__ void __launch_bounds__(256, 2)
-layernorm_bwd_vec_kernel(const float* __restrict__ g, const float* __restrict__ x, const float* __restrict__ gamma,
-                         const float* __restrict__ mean, const float* __restrict__ inv, int32_t rows, int32_t cols,
+layernorm_bwd_vec_kernel(const float* g, const float* x, const float* gamma,
+                         const float* mean, const float* inv, int32_t rows, int32_t cols,
                          float* __restrict__ dx, uint16_t* __restrict__ dx16, double* __restrict__ part_gamma, double* __restrict__ part_beta,
                          int32_t cta_rows) {
   pdl_enter();
@@ -382,7 +382,7 @@ layernorm_bwd_vec_kernel(const float* __restrict__ g, const float* __restrict__ 
     for (int i = 0; i < NV; i++) {
       const int j = lane + 32 * i;
       if (j < nv) {
-        const float4 gm = __ldg(reinterpret_cast<const float4*>(gamma) + j);   // gamma stays in L1: registers would not fit two CTAs per SM
+        const float4 gm = ld_global(reinterpret_cast<const float4*>(gamma) + j);   // gamma stays in L1: registers would not fit two CTAs per SM
         const float4 gv = dh[i];
         xh[i].x = (xh[i].x - m) * s; xh[i].y = (xh[i].y - m) * s; xh[i].z = (xh[i].z - m) * s; xh[i].w = (xh[i].w - m) * s;
         dh[i].x = gv.x * gm.x; dh[i].y = gv.y * gm.y; dh[i].z = gv.z * gm.z; dh[i].w = gv.w * gm.w;
@@ -465,12 +465,12 @@ struct BnWalk {
   }
 };
 template <int VEC>
-__device__ __forceinline__ void bn_load(float (&v)[VEC], const float* __restrict__ src) {
+__device__ __forceinline__ void bn_load(float (&v)[VEC], const float* src) {
   if constexpr (VEC == 4) {
-    const float4 t = __ldg(reinterpret_cast<const float4*>(src));
+    const float4 t = ld_global(reinterpret_cast<const float4*>(src));
     v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
   } else {
-    v[0] = __ldg(src);
+    v[0] = ld_global(src);
   }
 }
 // The CTA's sum, in every thread: lanes by a butterfly, warps in order.
@@ -505,7 +505,7 @@ struct BnSet {
 // the tensor again for the deviations took 157 us a step for the eight layers of the convolutional network.
 template <int VEC>
 __global__ void __launch_bounds__(kBnThreads)
-bn_stats_kernel(const float* __restrict__ x, int32_t n, int32_t c, int32_t plane, int32_t ipc, double* __restrict__ psum, double* __restrict__ pdev) {
+bn_stats_kernel(const float* x, int32_t n, int32_t c, int32_t plane, int32_t ipc, double* __restrict__ psum, double* __restrict__ pdev) {
   pdl_enter();
   __shared__ BnSet sm[kBnThreads / 32];
   constexpr int LOADS = VEC == 4 ? 8 : 16;
@@ -562,8 +562,8 @@ bn_stats_kernel(const float* __restrict__ x, int32_t n, int32_t c, int32_t plane
 // Backward: sum of g * xhat and sum of g over the slice.
 template <int VEC, bool RELU>
 __global__ void __launch_bounds__(kBnThreads)
-bn_bwd_partial_kernel(const float* __restrict__ x, const float* __restrict__ g, const float* __restrict__ mean, const float* __restrict__ inv,
-                      const float* __restrict__ gamma, const float* __restrict__ beta, int32_t n, int32_t c, int32_t plane, int32_t ipc, double* __restrict__ pa, double* __restrict__ pb) {
+bn_bwd_partial_kernel(const float* x, const float* g, const float* mean, const float* inv,
+                      const float* gamma, const float* beta, int32_t n, int32_t c, int32_t plane, int32_t ipc, double* __restrict__ pa, double* __restrict__ pb) {
   pdl_enter();
   __shared__ double sm[kBnThreads / 32];
   constexpr int LOADS = VEC == 4 ? 4 : 8;
@@ -607,9 +607,9 @@ bn_bwd_partial_kernel(const float* __restrict__ x, const float* __restrict__ g, 
   }
 }
 
-__global__ void bn_finish_stats_kernel(const double* __restrict__ psum, const double* __restrict__ pdev, int slices, int32_t n, int32_t ipc, int32_t plane,
+__global__ void bn_finish_stats_kernel(const double* psum, const double* pdev, int slices, int32_t n, int32_t ipc, int32_t plane,
                                        int32_t c, double m, float momentum, float eps, float* __restrict__ mean,
-                                       float* __restrict__ inv, float* __restrict__ rm, float* __restrict__ rv, const float* __restrict__ beta, float* __restrict__ beta_out) {
+                                       float* __restrict__ inv, float* rm, float* rv, const float* beta, float* __restrict__ beta_out) {
   pdl_enter();
   int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
@@ -630,8 +630,8 @@ __global__ void bn_finish_stats_kernel(const double* __restrict__ psum, const do
   rv[ch] = (float)(((double)(keep * rv[ch])) + ((double)momentum * unbiased));
 }
 
-__global__ void bn_eval_stats_kernel(const float* __restrict__ rm, const float* __restrict__ rv, int32_t c, float eps,
-                                     float* __restrict__ mean, float* __restrict__ inv, const float* __restrict__ beta, float* __restrict__ beta_out) {
+__global__ void bn_eval_stats_kernel(const float* rm, const float* rv, int32_t c, float eps,
+                                     float* __restrict__ mean, float* __restrict__ inv, const float* beta, float* __restrict__ beta_out) {
   pdl_enter();
   int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
@@ -644,8 +644,8 @@ __global__ void bn_eval_stats_kernel(const float* __restrict__ rm, const float* 
 // (VEC == 4: and x and y, backward g, x and dx, on the 16-byte grid)
 template <int VEC, bool RELU>
 __global__ void __launch_bounds__(256)
-bn_apply_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
-                const float* __restrict__ mean, const float* __restrict__ inv, int64_t total, int32_t c, int32_t plane,
+bn_apply_kernel(const float* x, const float* gamma, const float* beta,
+                const float* mean, const float* inv, int64_t total, int32_t c, int32_t plane,
                 float* __restrict__ y) {
   pdl_enter();
   int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * VEC;
@@ -654,7 +654,7 @@ bn_apply_kernel(const float* __restrict__ x, const float* __restrict__ gamma, co
     const int ch = (int)((e / plane) % c);
     const float mm = mean[ch], s = inv[ch], gg = gamma[ch], bb = beta[ch];
     if (VEC == 4) {
-      float4 v = __ldg(reinterpret_cast<const float4*>(x + e));
+      float4 v = ld_global(reinterpret_cast<const float4*>(x + e));
       v.x = bn_norm(v.x, mm, s, gg, bb); v.y = bn_norm(v.y, mm, s, gg, bb); v.z = bn_norm(v.z, mm, s, gg, bb); v.w = bn_norm(v.w, mm, s, gg, bb);
       if (RELU) { v.x = bn_relu(v.x); v.y = bn_relu(v.y); v.z = bn_relu(v.z); v.w = bn_relu(v.w); }
       *reinterpret_cast<float4*>(y + e) = v;
@@ -666,8 +666,8 @@ bn_apply_kernel(const float* __restrict__ x, const float* __restrict__ gamma, co
 }
 
 // Per-channel scalars of the backward: k = gamma * inv, cb = mean(g), cg = mean(g * xhat), from the slice partials.
-__global__ void bn_bwd_coef_kernel(const float* __restrict__ gamma, const float* __restrict__ inv, const double* __restrict__ pa,
-                                   const double* __restrict__ pb, int slices, double m, int32_t c, float* __restrict__ coef) {
+__global__ void bn_bwd_coef_kernel(const float* gamma, const float* inv, const double* pa,
+                                   const double* pb, int slices, double m, int32_t c, float* __restrict__ coef) {
   pdl_enter();
   int ch = blockIdx.x * blockDim.x + threadIdx.x;
   if (ch >= c) return;
@@ -683,8 +683,8 @@ __global__ void bn_bwd_coef_kernel(const float* __restrict__ gamma, const float*
 
 template <int VEC, bool RELU>
 __global__ void __launch_bounds__(256)
-bn_bwd_apply_kernel(const float* __restrict__ g, const float* __restrict__ x, const float* __restrict__ mean,
-                    const float* __restrict__ inv, const float* __restrict__ gamma, const float* __restrict__ beta, const float* __restrict__ coef, int64_t total, int32_t c, int32_t plane,
+bn_bwd_apply_kernel(const float* g, const float* x, const float* mean,
+                    const float* inv, const float* gamma, const float* beta, const float* coef, int64_t total, int32_t c, int32_t plane,
                     int training, float* __restrict__ dx) {
   pdl_enter();
   int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * VEC;
@@ -694,8 +694,8 @@ bn_bwd_apply_kernel(const float* __restrict__ g, const float* __restrict__ x, co
     const float mm = mean[ch], s = inv[ch], k = coef[ch], cb = coef[c + ch], cg = coef[2 * c + ch];
     const float gg = RELU ? gamma[ch] : 0.f, bb = RELU ? beta[ch] : 0.f;
     if (VEC == 4) {
-      float4 gv = __ldg(reinterpret_cast<const float4*>(g + e));
-      const float4 xv = __ldg(reinterpret_cast<const float4*>(x + e));
+      float4 gv = ld_global(reinterpret_cast<const float4*>(g + e));
+      const float4 xv = ld_global(reinterpret_cast<const float4*>(x + e));
       if (RELU) {
         if (!(bn_norm(xv.x, mm, s, gg, bb) > 0.0f)) gv.x = 0.0f;
         if (!(bn_norm(xv.y, mm, s, gg, bb) > 0.0f)) gv.y = 0.0f;

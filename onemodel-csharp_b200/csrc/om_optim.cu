@@ -70,7 +70,7 @@ __device__ __forceinline__ float adam_element(float& p, float g, float& m, float
 }
 
 __global__ void __launch_bounds__(256)
-adam_kernel(TensorTable t, om_adam_hyper hv, const om_adam_hyper* __restrict__ hd) {
+adam_kernel(TensorTable t, om_adam_hyper hv, const om_adam_hyper* hd) {
   pdl_enter();
   const om_adam_hyper h = hd ? *hd : hv;
   const float omb1 = __fsub_rn(1.0f, h.beta1), omb2 = __fsub_rn(1.0f, h.beta2);
@@ -138,7 +138,7 @@ __device__ __forceinline__ void sgd_element(float& p, float g, float& buf, bool 
 // 16-byte accesses where the three arrays allow them: 4.7 M parameters with momentum (94 MB) took 44 us with 4-byte ones
 // in visits of 16384 elements. On the first step the momentum buffer is written without being read, as before.
 __global__ void __launch_bounds__(256)
-sgd_kernel(TensorTable t, om_sgd_hyper hv, const om_sgd_hyper* __restrict__ hd) {
+sgd_kernel(TensorTable t, om_sgd_hyper hv, const om_sgd_hyper* hd) {
   pdl_enter();
   const om_sgd_hyper h = hd ? *hd : hv;
   const float keep = __fsub_rn(1.0f, h.dampening);
@@ -209,7 +209,7 @@ sumsq_kernel(TensorTable t, int infinity, double* __restrict__ partial, int chun
 }
 
 // Stage 2: one CTA combines the chunk partials in chunk order and writes {norm, coef}.
-__global__ void norm_finish_kernel(const double* __restrict__ partial, int chunks, int infinity, float max_norm,
+__global__ void norm_finish_kernel(const double* partial, int chunks, int infinity, float max_norm,
                                    float* __restrict__ total_norm, float* __restrict__ coef_out) {
   pdl_enter();
   __shared__ double sm[1024];
@@ -238,7 +238,7 @@ __global__ void norm_finish_kernel(const double* __restrict__ partial, int chunk
 }
 
 __global__ void __launch_bounds__(256)
-scale_by_coef_kernel(TensorTable t, const float* __restrict__ coef_ptr) {
+scale_by_coef_kernel(TensorTable t, const float* coef_ptr) {
   pdl_enter();
   const float coef = coef_ptr[0];
   if (!(coef < 1.0f)) return;
@@ -305,7 +305,7 @@ static int grid_chunks(om_ctx* ctx, int chunks) {
 // touched[row] = how many positions of this step's id list name the row (0 = untouched, its parameters AND moments stay
 // as they are: SparseAdam does not decay the moments of absent rows). grad is the dense-format table gradient of
 // om_embedding_bwd, whose touched rows hold the coalesced sums the reference's RowSparseGradient holds.
-__global__ void rows_touched_kernel(const void* __restrict__ ids, int dtype, int64_t n, int32_t rows, int64_t pad,
+__global__ void rows_touched_kernel(const void* ids, int dtype, int64_t n, int32_t rows, int64_t pad,
                                     int32_t* __restrict__ touched, int32_t* status) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
   for (; i < n; i += stride) {
@@ -321,8 +321,8 @@ __global__ void rows_touched_kernel(const void* __restrict__ ids, int dtype, int
 
 // One warp per row. SparseAdam.UpdateSparse (Optimizers.cs:696-722), this rounding sequence, no fused multiply-add:
 //   m = b1*m + (1-b1)*g;  v = b2*v + ((1-b2)*g)*g;  p -= (stepSize*m) / (sqrt(v) + eps)
-__global__ void sparse_adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                                   const int32_t* __restrict__ touched, int32_t rows, int32_t width, float b1, float b2, float eps,
+__global__ void sparse_adam_kernel(float* __restrict__ p, const float* g, float* __restrict__ m, float* __restrict__ v,
+                                   const int32_t* touched, int32_t rows, int32_t width, float b1, float b2, float eps,
                                    float step_size) {
   const int lane = threadIdx.x & 31;
   const float omb1 = __fsub_rn(1.f, b1), omb2 = __fsub_rn(1.f, b2);
@@ -342,7 +342,7 @@ __global__ void sparse_adam_kernel(float* __restrict__ p, const float* __restric
 }
 
 // Sgd.UpdateSparse (Optimizers.cs:377-397): p -= lr * g on the touched rows; no momentum, no weight decay.
-__global__ void sparse_sgd_kernel(float* __restrict__ p, const float* __restrict__ g, const int32_t* __restrict__ touched, int32_t rows,
+__global__ void sparse_sgd_kernel(float* __restrict__ p, const float* g, const int32_t* touched, int32_t rows,
                                   int32_t width, float lr) {
   const int lane = threadIdx.x & 31;
   int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -356,8 +356,8 @@ __global__ void sparse_sgd_kernel(float* __restrict__ p, const float* __restrict
 // The same two updates from a row list (the row-sparse gradient of om_embedding_bwd_sparse: rows[k] ascending, values[k, :],
 // the count on the device): one warp per listed row, the same rounding sequence as above, so a table updated from the row
 // list has the bits of one updated from the dense-format gradient.
-__global__ void sparse_adam_rows_kernel(float* __restrict__ p, const int32_t* __restrict__ rows, const float* __restrict__ g,
-                                        const int32_t* __restrict__ row_count, int32_t capacity, float* __restrict__ m, float* __restrict__ v,
+__global__ void sparse_adam_rows_kernel(float* __restrict__ p, const int32_t* rows, const float* g,
+                                        const int32_t* row_count, int32_t capacity, float* __restrict__ m, float* __restrict__ v,
                                         int32_t table_rows, int32_t width, float b1, float b2, float eps, float step_size, int32_t* status) {
   const int lane = threadIdx.x & 31;
   const float omb1 = __fsub_rn(1.f, b1), omb2 = __fsub_rn(1.f, b2);
@@ -381,8 +381,8 @@ __global__ void sparse_adam_rows_kernel(float* __restrict__ p, const int32_t* __
   }
 }
 
-__global__ void sparse_sgd_rows_kernel(float* __restrict__ p, const int32_t* __restrict__ rows, const float* __restrict__ g,
-                                       const int32_t* __restrict__ row_count, int32_t capacity, int32_t table_rows, int32_t width, float lr,
+__global__ void sparse_sgd_rows_kernel(float* __restrict__ p, const int32_t* rows, const float* g,
+                                       const int32_t* row_count, int32_t capacity, int32_t table_rows, int32_t width, float lr,
                                        int32_t* status) {
   const int lane = threadIdx.x & 31;
   int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = ((int64_t)gridDim.x * blockDim.x) >> 5;

@@ -200,7 +200,7 @@ cnhw_to_nchw_bias_kernel(const float* __restrict__ t, const float* __restrict__ 
 constexpr int kDbiasSlices = 16;
 template <int VEC>
 __global__ void __launch_bounds__(256)
-conv_dbias_partial_kernel(const float* __restrict__ g, int n, int cout, int plane, int per_slice, double* __restrict__ partial) {
+conv_dbias_partial_kernel(const float* g, int n, int cout, int plane, int per_slice, double* __restrict__ partial) {
   pdl_enter();
   __shared__ double sm[256];
   const int co = blockIdx.x, slice = blockIdx.y;
@@ -221,10 +221,10 @@ conv_dbias_partial_kernel(const float* __restrict__ g, int n, int cout, int plan
       if (i < i1) {
         const float* src = base + (int64_t)i * image + (int64_t)p * VEC;
         if (VEC == 4) {
-          const float4 t = __ldg(reinterpret_cast<const float4*>(src));
+          const float4 t = ld_global(reinterpret_cast<const float4*>(src));
           v[l][0] = t.x; v[l][VEC / 4] = t.y; v[l][VEC / 2] = t.z; v[l][VEC - 1] = t.w;
         } else {
-          v[l][0] = __ldg(src);
+          v[l][0] = ld_global(src);
         }
       }
       p += step_p;
@@ -247,7 +247,7 @@ conv_dbias_partial_kernel(const float* __restrict__ g, int n, int cout, int plan
   }
   if (threadIdx.x == 0) partial[(int64_t)slice * cout + co] = sm[0];
 }
-__global__ void conv_dbias_finish_kernel(const double* __restrict__ partial, int slices, int cout, float* __restrict__ dbias, int accumulate) {
+__global__ void conv_dbias_finish_kernel(const double* partial, int slices, int cout, float* dbias, int accumulate) {
   pdl_enter();
   int co = blockIdx.x * blockDim.x + threadIdx.x;
   if (co >= cout) return;
@@ -282,7 +282,7 @@ static bool pool_out(int size, int kernel, int stride, int pad, int* out) {
 // First maximum wins ties, NaN wins over numbers (ReferenceKernels.MaxPool2d, TensorKernels.cs:242-295).
 // IDX: int when the input has fewer than 2^31 elements (32-bit divisions).
 template <typename IDX>
-__global__ void maxpool_fwd_kernel(PoolGeom g, const float* __restrict__ x, int64_t total, float* __restrict__ y, int32_t* __restrict__ idx) {
+__global__ void maxpool_fwd_kernel(PoolGeom g, const float* x, int64_t total, float* __restrict__ y, int32_t* __restrict__ idx) {
   pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -315,7 +315,7 @@ __global__ void maxpool_fwd_kernel(PoolGeom g, const float* __restrict__ x, int6
 }
 
 // dx[j] = sum of g[i] over the outputs i (in increasing i) whose saved index is j.
-__global__ void maxpool_bwd_kernel(PoolGeom g, const float* __restrict__ gr, const int32_t* __restrict__ idx, int64_t total,
+__global__ void maxpool_bwd_kernel(PoolGeom g, const float* gr, const int32_t* idx, int64_t total,
                                    float* __restrict__ dx) {
   pdl_enter();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -339,8 +339,8 @@ __global__ void maxpool_bwd_kernel(PoolGeom g, const float* __restrict__ gr, con
 // dx[e] is g of that window when its saved index is e, else zero. 32-bit index arithmetic; a thread owns VEC adjacent
 // inputs of a row (one 16-byte store when VEC is 4: w a multiple of 4 and dx 16-byte aligned).
 template <int VEC>
-__global__ void maxpool_bwd_tiled_kernel(int h, int w, int oh, int ow, int kh, int kw, const float* __restrict__ gr,
-                                         const int32_t* __restrict__ idx, int groups, float* __restrict__ dx) {
+__global__ void maxpool_bwd_tiled_kernel(int h, int w, int oh, int ow, int kh, int kw, const float* gr,
+                                         const int32_t* idx, int groups, float* __restrict__ dx) {
   pdl_enter();
   const int stride = gridDim.x * blockDim.x;
   const int wg = w / VEC;
@@ -362,8 +362,8 @@ __global__ void maxpool_bwd_tiled_kernel(int h, int w, int oh, int ow, int kh, i
         if (ox < ow) {
           if (ox != last_ox) {
             last_ox = ox;
-            last_idx = __ldg(idx + obase + ox);
-            last_g = __ldg(gr + obase + ox);
+            last_idx = ld_global(idx + obase + ox);
+            last_g = ld_global(gr + obase + ox);
           }
           if (last_idx == e0 + j) v[j] = last_g;
         }
@@ -384,7 +384,7 @@ __global__ void maxpool_bwd_tiled_kernel(int h, int w, int oh, int ow, int kh, i
 // of 32 x 256 through 2 x 2 windows took 78 us forward and 75 backward (201 MB: 30 us).
 template <int KW>
 __global__ void __launch_bounds__(256)
-maxpool_fwd_windows_kernel(int h, int w, int kh, const float* __restrict__ x, int groups, float* __restrict__ y, int32_t* __restrict__ idx) {
+maxpool_fwd_windows_kernel(int h, int w, int kh, const float* x, int groups, float* __restrict__ y, int32_t* __restrict__ idx) {
   pdl_enter();
   constexpr int OUT = 4 / KW;
   const int wg = w / 4, oh = h / kh, ow = w / KW;
@@ -395,7 +395,7 @@ maxpool_fwd_windows_kernel(int h, int w, int kh, const float* __restrict__ x, in
     float best[OUT];
     int32_t where[OUT];
     for (int ky = 0; ky < kh; ky++) {
-      const float4 t = __ldg(reinterpret_cast<const float4*>(x + at + ky * w));
+      const float4 t = ld_global(reinterpret_cast<const float4*>(x + at + ky * w));
       const float v[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
       for (int j = 0; j < 4; j++) {
@@ -421,7 +421,7 @@ maxpool_fwd_windows_kernel(int h, int w, int kh, const float* __restrict__ x, in
 }
 template <int KW>
 __global__ void __launch_bounds__(256)
-maxpool_bwd_windows_kernel(int h, int w, int kh, const float* __restrict__ gr, const int32_t* __restrict__ idx, int groups, float* __restrict__ dx) {
+maxpool_bwd_windows_kernel(int h, int w, int kh, const float* gr, const int32_t* idx, int groups, float* __restrict__ dx) {
   pdl_enter();
   constexpr int OUT = 4 / KW;
   const int wg = w / 4, oh = h / kh, ow = w / KW;
@@ -432,18 +432,18 @@ maxpool_bwd_windows_kernel(int h, int w, int kh, const float* __restrict__ gr, c
     float g[OUT];
     int32_t where[OUT];
     if constexpr (OUT == 4) {
-      const float4 t = __ldg(reinterpret_cast<const float4*>(gr + out));
-      const int4 i = __ldg(reinterpret_cast<const int4*>(idx + out));
+      const float4 t = ld_global(reinterpret_cast<const float4*>(gr + out));
+      const int4 i = ld_global(reinterpret_cast<const int4*>(idx + out));
       g[0] = t.x; g[1] = t.y; g[2] = t.z; g[3] = t.w;
       where[0] = i.x; where[1] = i.y; where[2] = i.z; where[3] = i.w;
     } else if constexpr (OUT == 2) {
-      const float2 t = __ldg(reinterpret_cast<const float2*>(gr + out));
-      const int2 i = __ldg(reinterpret_cast<const int2*>(idx + out));
+      const float2 t = ld_global(reinterpret_cast<const float2*>(gr + out));
+      const int2 i = ld_global(reinterpret_cast<const int2*>(idx + out));
       g[0] = t.x; g[1] = t.y;
       where[0] = i.x; where[1] = i.y;
     } else {
-      g[0] = __ldg(gr + out);
-      where[0] = __ldg(idx + out);
+      g[0] = ld_global(gr + out);
+      where[0] = ld_global(idx + out);
     }
     for (int ky = 0; ky < kh; ky++) {
       float v[4];
