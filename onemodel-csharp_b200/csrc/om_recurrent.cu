@@ -9,6 +9,7 @@
 // own exp/log polynomials (Ctc.cs:515-616), one CTA per sequence; per-class sums run in increasing extended-label
 // order so the result has the reference's bits.
 #include <algorithm>
+#include <initializer_list>
 
 #include "om_common.cuh"
 #include "om_lstm_seq.cuh"
@@ -439,6 +440,13 @@ static int32_t lstm_fwd_seq(om_ctx* ctx, int dirs, const int32_t* reverse, int32
   return OM_OK;
 }
 
+// The whole-sequence kernels read these 16 bytes at a time (a view may start off that grid).
+static bool on_grid(std::initializer_list<const float*> pointers) {
+  for (const float* p : pointers)
+    if (reinterpret_cast<uintptr_t>(p) & 15) return false;
+  return true;
+}
+
 int32_t om_lstm_layer_fwd(om_ctx* ctx, int32_t reverse, int32_t t, int32_t b, int32_t i, int32_t h, const float* x,
                           const float* w_ih, const float* w_hh, const float* b_ih, const float* b_hh, const float* h0,
                           const float* c0, float* y, float* gates, float* c, float* tanh_c) {
@@ -446,7 +454,7 @@ int32_t om_lstm_layer_fwd(om_ctx* ctx, int32_t reverse, int32_t t, int32_t b, in
   if (t < 0 || b < 0 || i < 1 || h < 1) return fail(ctx, OM_ERR_SHAPE, "LstmLayer: T %d B %d I %d H %d", t, b, i, h);
   if (t == 0 || b == 0) return OM_OK;
   ProfileScope prof(ctx, "om_lstm_layer_fwd", 2.0 * t * b * 4.0 * h * (i + h), 4.0 * t * b * (double)(i + 7 * h));
-  if (lstm_seq_supported(ctx, 1, t, b, h, false))
+  if (on_grid({w_hh, h0, y}) && lstm_seq_supported(ctx, 1, t, b, h, false))
     return lstm_fwd_seq(ctx, 1, &reverse, t, b, i, h, x, &w_ih, &w_hh, &b_ih, &b_hh, &h0, &c0, &y, &gates, &c, &tanh_c);
   return lstm_fwd_body(ctx, reverse, t, b, i, h, x, w_ih, w_hh, b_ih, b_hh, h0, c0, y, gates, c, tanh_c);
 }
@@ -458,7 +466,7 @@ int32_t om_lstm_bilayer_fwd(om_ctx* ctx, int32_t t, int32_t b, int32_t i, int32_
   if (t < 0 || b < 0 || i < 1 || h < 1) return fail(ctx, OM_ERR_SHAPE, "LstmLayer: T %d B %d I %d H %d", t, b, i, h);
   if (t == 0 || b == 0) return OM_OK;
   ProfileScope prof(ctx, "om_lstm_layer_fwd", 2.0 * 2 * t * b * 4.0 * h * (i + h), 2.0 * 4.0 * t * b * (double)(i + 7 * h));
-  if (lstm_seq_supported(ctx, 2, t, b, h, false)) {
+  if (on_grid({w_hh[0], w_hh[1], y[0], y[1]}) && lstm_seq_supported(ctx, 2, t, b, h, false)) {
     const int32_t order[2] = {0, 1};
     return lstm_fwd_seq(ctx, 2, order, t, b, i, h, x, w_ih, w_hh, b_ih, b_hh, nullptr, nullptr, y, gates, c, tanh_c);
   }
@@ -583,7 +591,7 @@ int32_t om_lstm_layer_bwd(om_ctx* ctx, int32_t reverse, int32_t t, int32_t b, in
   if (t < 0 || b < 0 || i < 1 || h < 1) return fail(ctx, OM_ERR_SHAPE, "LstmBackward: T %d B %d I %d H %d", t, b, i, h);
   if (t == 0 || b == 0) return OM_OK;
   ProfileScope prof(ctx, "om_lstm_layer_bwd", 4.0 * t * b * 4.0 * h * (i + h), 4.0 * t * b * (double)(2 * i + 12 * h));
-  if (lstm_seq_supported(ctx, 1, t, b, h, true))
+  if (on_grid({w_hh}) && lstm_seq_supported(ctx, 1, t, b, h, true))
     return lstm_bwd_seq(ctx, 1, &reverse, t, b, i, h, &gy, &ghn, &gcn, x, &y, &w_ih, &w_hh, &h0, &c0, &gates, &c, &tanh_c, &dx, &dw_ih, &dw_hh,
                         &db_ih, &db_hh, &dh0, &dc0);
   return lstm_bwd_body(ctx, reverse, t, b, i, h, gy, ghn, gcn, x, y, w_ih, w_hh, h0, c0, gates, c, tanh_c, dx, dw_ih, dw_hh, db_ih, db_hh,
@@ -598,7 +606,7 @@ int32_t om_lstm_bilayer_bwd(om_ctx* ctx, int32_t t, int32_t b, int32_t i, int32_
   if (t < 0 || b < 0 || i < 1 || h < 1) return fail(ctx, OM_ERR_SHAPE, "LstmBackward: T %d B %d I %d H %d", t, b, i, h);
   if (t == 0 || b == 0) return OM_OK;
   ProfileScope prof(ctx, "om_lstm_layer_bwd", 2.0 * 4.0 * t * b * 4.0 * h * (i + h), 2.0 * 4.0 * t * b * (double)(2 * i + 12 * h));
-  if (lstm_seq_supported(ctx, 2, t, b, h, true)) {
+  if (on_grid({w_hh[0], w_hh[1]}) && lstm_seq_supported(ctx, 2, t, b, h, true)) {
     const int32_t order[2] = {0, 1};
     return lstm_bwd_seq(ctx, 2, order, t, b, i, h, gy, nullptr, nullptr, x, y, w_ih, w_hh, nullptr, nullptr, gates, c, tanh_c, dx, dw_ih, dw_hh,
                         db_ih, db_hh, nullptr, nullptr);

@@ -259,6 +259,33 @@ def test_whole_sequence_lstm_shapes(ctx, K, t, b, h):
         assert scaled_diff(q, p) <= 1e-4, k
 
 
+@pytest.mark.parametrize("off", [(1, 0, 0), (0, 1, 0), (0, 0, 1)])
+def test_lstm_of_arrays_off_the_16_byte_grid(ctx, off):
+    """Recurrent weights, initial state and outputs one float past a 16-byte boundary under OM_SEQ_KERNELS: the values of the step-by-step form, both directions
+    of the pass."""
+    t, b, n, h = 3, 5, 12, 32
+    x, w_ih, w_hh, h0, gy = normal(1, t, b, n), normal(2, 4 * h, n, scale=0.2), normal(3, 4 * h, h, scale=0.2), normal(4, b, h), normal(5, t, b, h)
+    runs = []
+    for flags, shift in ((0, (0, 0, 0)), (omb.OM_SEQ_KERNELS, off)):
+        ctx.set_flags(flags)
+        try:
+            X, WI, GY = (ctx.to_device(a) for a in (x, w_ih, gy))
+            WH, H0 = (ctx.to_device(np.concatenate([np.zeros(k, np.float32), a.ravel()])) for a, k in ((w_hh, shift[0]), (h0, shift[1])))
+            Y = ctx.empty((t * b * h + shift[2],))
+            G, CC, TC, DX, DWI, DWH = (ctx.empty(s) for s in ((t, b, 4 * h), (t, b, h), (t, b, h), (t, b, n), w_ih.shape, w_hh.shape))
+            pw, p0, py = (C.c_void_p(a.ptr.value + 4 * k) for a, k in zip((WH, H0, Y), shift))
+            sizes = [i32(t), i32(b), i32(n), i32(h)]
+            ctx.call("om_lstm_layer_fwd", ctx.handle, i32(0), *sizes, X.ptr, WI.ptr, pw, None, None, p0, None, py, G.ptr, CC.ptr, TC.ptr)
+            ctx.call("om_lstm_layer_bwd", ctx.handle, i32(0), *sizes, GY.ptr, None, None, X.ptr, py, WI.ptr, pw, p0, None, G.ptr, CC.ptr, TC.ptr, DX.ptr, DWI.ptr, DWH.ptr,
+                     None, None, None, None)
+            ctx.sync()
+            runs.append([Y.numpy()[shift[2]:], DX.numpy(), DWI.numpy(), DWH.numpy()])
+        finally:
+            ctx.set_flags(0)
+    for p, q in zip(*runs):
+        assert scaled_diff(q, p) <= 1e-4
+
+
 @pytest.mark.parametrize("case", [
     (80, 32, 16, 16, 96, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1), (20, 48, 32, 32, 64, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1),     # half a block of channels empty
     (33, 64, 16, 16, 129, 3, 3, 1, 1, (1, 1, 1, 1), 1, 1),     # a second block of one channel, images that no box divides
