@@ -27,7 +27,7 @@ __global__ void add_bias_rows_kernel(float* y, const float* bias, int64_t rows, 
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   if (ld != cols) {
     for (int64_t j = i; j < total; j += stride) y[(j / cols) * ld + (j % cols)] += bias[j % cols];
-  } else if ((cols & 3) == 0) {
+  } else if ((cols & 3) == 0 && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0) {
     int64_t n4 = total >> 2;
     int32_t c4 = cols >> 2;
     float4* y4 = reinterpret_cast<float4*>(y);

@@ -166,7 +166,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     constexpr int STG_LD = 36;                                   // floats per staged row: 144 bytes keeps float4 alignment and
     float* stg = reinterpret_cast<float*>(smem) + quad * 32 * STG_LD;   // spreads the eight rows of a phase over all banks
     const int row_base = m0 + quad * 32;
-    const bool aligned = ((reinterpret_cast<uintptr_t>(c) & 15) == 0) && ((p.ldc & 3) == 0);
+    const bool aligned = ((reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(p.bias)) & 15) == 0 && (p.ldc & 3) == 0;
     if (ok && row_base < p.m && p.tma_store) {
       // Bulk stores: each 32 x 32 block goes to its own 4 KB of the (dead) operand stages in the 128-byte-swizzled layout
       // of the C tensor map (16-byte chunk c of row r at chunk c ^ (r & 7): a quarter warp writes 128 distinct bytes),

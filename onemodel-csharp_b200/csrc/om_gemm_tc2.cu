@@ -176,7 +176,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     constexpr int STG_LD = 36;
     float* stg = reinterpret_cast<float*>(smem) + quad * 32 * STG_LD;
     const int row_base = m0 + quad * 32;
-    const bool aligned = ((reinterpret_cast<uintptr_t>(c) & 15) == 0) && ((p.ldc & 3) == 0);
+    const bool aligned = ((reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(p.bias)) & 15) == 0 && (p.ldc & 3) == 0;
     if (ok && row_base < p.m && p.tma_store) {
       // Bulk stores as in the one-CTA kernel: 32 x 32 blocks staged in the swizzled layout of the C map and handed to the
       // TMA unit. A warp cycles through four 4 KB staging blocks; before it overwrites one it waits until the bulk copy

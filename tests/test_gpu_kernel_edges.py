@@ -259,6 +259,25 @@ def test_whole_sequence_lstm_shapes(ctx, K, t, b, h):
         assert scaled_diff(q, p) <= 1e-4, k
 
 
+@pytest.mark.parametrize("tf32", [0, 1])
+@pytest.mark.parametrize("off", [(1, 0), (0, 1), (1, 1)])
+def test_linear_bias_off_the_16_byte_grid(ctx, tf32, off):
+    """Bias and outputs one float past a 16-byte boundary, where the fp32 product adds the bias in a pass of its own: the bits of the aligned call (TF32: 2e-5)."""
+    m, n, k = 640, 256, 36
+    x, w, b = to_tf32(normal(1, m, k)), to_tf32(normal(2, n, k)), normal(3, n)
+    ctx.set_flags(omb.OM_TF32 if tf32 else 0)
+    try:
+        X, W = ctx.to_device(x), ctx.to_device(w)
+        out = []
+        for shift in ((0, 0), off):
+            B, Y = ctx.to_device(np.concatenate([np.zeros(shift[0], np.float32), b])), ctx.empty((m * n + shift[1],))
+            ctx.call("om_linear_fwd", ctx.handle, X.ptr, W.ptr, C.c_void_p(B.ptr.value + 4 * shift[0]), i32(m), i32(k), i32(n), C.c_void_p(Y.ptr.value + 4 * shift[1]))
+            out.append(Y.numpy()[shift[1]:])
+    finally:
+        ctx.set_flags(0)
+    assert scaled_diff(out[1], out[0]) <= 2e-5 if tf32 else np.array_equal(out[0], out[1])
+
+
 @pytest.mark.parametrize("off", [(1, 0, 0), (0, 1, 0), (0, 0, 1)])
 def test_lstm_of_arrays_off_the_16_byte_grid(ctx, off):
     """Recurrent weights, initial state and outputs one float past a 16-byte boundary under OM_SEQ_KERNELS: the values of the step-by-step form, both directions
