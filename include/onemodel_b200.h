@@ -59,7 +59,7 @@ typedef enum om_status {
  * kernel that wrote past the end shows as OM_ERR_CANARY at the next om_sync. Index operands are range-checked on the
  * device with or without the flag. A debugging mode: two extra small launches per allocation. OM_PAIR_TILES (with OM_TF32): every plain product the
  * CTA-pair kernel can take runs on it (tcgen05 cta_group::2, 256-row tiles: fewer operand bytes per SM); without the
- * flag only products with several rounds of tiles over the device do.
+ * flag those with several rounds of tiles over the device, with one round of wide tiles and a short k, or with few tiles and a very deep k do.
  * OM_TWO_STREAMS: a backward entry point whose gradients are independent of one another (om_linear_bwd: the input
  * gradient on one side, the weight and bias gradients on the other) runs them on two streams of the context, forked
  * and joined inside the call, so that products too small to fill the device overlap; om_linear_bwd_bf16_b16 runs the
@@ -71,7 +71,8 @@ typedef enum om_status {
  * it only those of up to 1184 CTAs are, or of up to 296 while a step is being captured. OM_SERIAL_LAUNCHES: none is, whatever the other flags say:
  * what overlapped runs are compared with, and what a profiler's durations of single kernels need.
  * OM_PERSISTENT_TILES (with OM_TF32): plain products run on the persistent CTA-pair kernel that the bfloat16 products
- * always use (two accumulator buffers in tensor memory: a tile's read-back and stores run under the next tile's MMAs). */
+ * always use (two accumulator buffers in tensor memory: a tile's read-back and stores run under the next tile's MMAs); without the flag those do
+ * that give nearly every CTA pair a full tile, and half of the pairs one where k is deep. */
 #define OM_TF32 1u
 #define OM_BF16_OPERANDS 2u
 #define OM_CHECKED 4u

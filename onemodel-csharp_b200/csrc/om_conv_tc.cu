@@ -677,8 +677,9 @@ __device__ __forceinline__ bool cn_add_chains(float (&acc)[COLS], uint32_t tmem,
 // CHAINS: the sum over k in several accumulator chains that are added in fp32 in increasing order. The tensor core cuts what a step of its accumulator
 // cannot hold instead of rounding it, an error that grows with the number of steps (1.8e-8 of the result a step of eight k's: 4.9e-6 at k
 // = 2304). With a chain a tap, dx has the bits of the product on the unfolded matrix and its fold, and a tap outside the gradient's plane
-// is left out whatever its weight is; in one chain over all taps it was 7 times as far from the exact sums. Reading an accumulator back takes the
-// result warps about as long as a block of k takes the products, and goes on beside them.
+// is left out whatever its weight is; in one chain over all taps it was 7 times as far from the exact sums (128 channels
+// 2.6e-6 against 3.4e-7). Two accumulators, so that one is read back while the other is filled; us in one chain / a chain a tap: 256 x 64 x 32 x 32 from 128 with
+// stride 2 83 / 95, 64 x 64 x 16 x 128 from 128 99 / 119, 32 x 256 x 14 x 14 from 256 44 / 52.
 template <int NT, int STAGES, bool CHAINS>
 __global__ void __launch_bounds__(cn_threads(CHAINS), STAGES > 4 ? 1 : 2)
 conv_nhwc_kernel(const __grid_constant__ ConvNhwcMaps maps, const __grid_constant__ ConvNhwcParams p) {

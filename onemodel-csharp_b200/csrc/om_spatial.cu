@@ -820,12 +820,16 @@ int32_t om_conv2d_dbias(om_ctx* ctx, const om_conv_shape* s, const float* gr, fl
   return OM_OK;
 }
 
+// Weight and input gradient both take the channels-last copy of the output's gradient.
+static bool conv_bwd_shares(om_ctx* ctx, const ConvGeom& g) {
+  return g.n > 0 && g.n <= 65535 && conv_on_tensor_pipe(ctx, g, true) && conv_nhwc_wgrad_fits(g) && conv_nhwc_dgrad_fits(g);
+}
+
 int32_t om_conv2d_bwd_workspace(om_ctx* ctx, const om_conv_shape* s, int64_t* floats) {
   OM_CHECK_CTX(ctx);
   ConvGeom g;
   if (!s || !conv_geom(s, &g)) return fail(ctx, OM_ERR_SHAPE, "Invalid convolution geometry.");
-  const bool shared = g.n > 0 && g.n <= 65535 && conv_on_tensor_pipe(ctx, g, true) && conv_nhwc_wgrad_fits(g) && conv_nhwc_dgrad_fits(g);
-  *floats = shared ? conv_nhwc_turned_floats(g) : 0;
+  *floats = conv_bwd_shares(ctx, g) ? conv_nhwc_turned_floats(g) : 0;
   return OM_OK;
 }
 
@@ -834,7 +838,7 @@ int32_t om_conv2d_bwd_params(om_ctx* ctx, const om_conv_shape* s, const float* g
   OM_CHECK_CTX(ctx);
   ConvGeom g;
   if (!s || !conv_geom(s, &g)) return fail(ctx, OM_ERR_SHAPE, "Invalid convolution geometry.");
-  if (workspace) {
+  if (workspace && conv_bwd_shares(ctx, g)) {
     ProfileScope prof(ctx, "om_conv2d_bwd_params", dw ? 2.0 * g.n * g.cout * (double)g.cin * g.kh * g.kw * g.oh * g.ow : 0.0,
                       4.0 * g.n * ((double)g.cin * g.h * g.w + (double)g.cout * g.oh * g.ow));
     OM_TRY(conv_nhwc_turn_gradient(ctx, g, gr, workspace, dbias, accumulate_b));
@@ -847,9 +851,9 @@ int32_t om_conv2d_bwd_params(om_ctx* ctx, const om_conv_shape* s, const float* g
 
 int32_t om_conv2d_bwd_input(om_ctx* ctx, const om_conv_shape* s, const float* gr, const float* w, float* dx, const float* workspace) {
   OM_CHECK_CTX(ctx);
-  if (!workspace) return om_conv2d_dgrad(ctx, s, gr, w, dx);
   ConvGeom g;
   if (!s || !conv_geom(s, &g)) return fail(ctx, OM_ERR_SHAPE, "Invalid convolution geometry.");
+  if (!workspace || !conv_bwd_shares(ctx, g)) return om_conv2d_dgrad(ctx, s, gr, w, dx);
   ProfileScope prof(ctx, "om_conv2d_dgrad", 2.0 * g.n * g.cout * (double)g.cin * g.kh * g.kw * g.oh * g.ow,
                     4.0 * g.n * ((double)g.cin * g.h * g.w + (double)g.cout * g.oh * g.ow));
   return conv_nhwc_dgrad(ctx, g, gr, w, dx, workspace);
