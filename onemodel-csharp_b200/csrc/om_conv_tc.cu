@@ -1354,7 +1354,11 @@ int32_t conv_nhwc_wgrad(om_ctx* ctx, const ConvGeom& g, const float* gr, const f
   int splits = (int)std::max<long long>(1, std::min<long long>(kSplitSlots / ((long long)tn * tm), p.blocks / 8));
   p.blocks_per_split = (int)ceil_div(p.blocks, splits);
   splits = (int)ceil_div(p.blocks, p.blocks_per_split);
-  p.chain = std::min(p.blocks_per_split, product_chain_blocks(g.cout, g.cin * p.taps, g.n * g.oh * g.ow));
+  // No longer than the chains of the product on the unfolded matrix, and half of them where the boxes walk the pixels in another order than it does: of 90
+  // geometries three were 6 to 8 % further from float64 than that product with its length (60 x 128 x 8 x 54 by 256: 3.41e-6 / 3.66e-6).
+  const int plain = product_chain_blocks(g.cout, g.cin * p.taps, g.n * g.oh * g.ow);
+  const bool in_order = (p.box.w == g.ow && (p.box.h == g.oh || p.box.n == 1)) || (p.box.h == 1 && p.box.n == 1);
+  p.chain = std::min(p.blocks_per_split, in_order ? plain : (plain + 1) / 2);
   float *own = nullptr, *xt = nullptr;
   CUtensorMap map_g = {}, map_x = {};
   int32_t st = turned ? OM_OK : cn_turn(ctx, gr, g.n, g.cout, g.oh * g.ow, &own);
